@@ -1,4 +1,6 @@
 // extern "C" surface of libringrnn.so: argument checking, precision dispatch, error reporting.
+#include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <atomic>
@@ -66,6 +68,34 @@ static void drain_timed_locked() {
     cudaEventDestroy(t.stop);
   }
   g_timed.clear();
+}
+
+// ---- launch set-up, once per kernel and device --------------------------------------------------
+namespace {
+struct Residency { const void* kernel; int device, clusters; };
+std::mutex g_residency_mu;
+std::vector<Residency> g_residency;  // a handful of entries: one per kernel instantiation in use
+}  // namespace
+
+int resident_clusters(const void* kernel, cudaLaunchConfig_t* cfg, int cluster_size, int smem_bytes) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return -1; }
+  std::lock_guard<std::mutex> lk(g_residency_mu);
+  for (const Residency& r : g_residency)
+    if (r.kernel == kernel && r.device == device) return r.clusters;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  if (e != cudaSuccess) { set_last_cuda_error(e); return -1; }
+  int n = 0;
+  cfg->gridDim = dim3((unsigned)(148 / cluster_size * cluster_size), 1, 1);
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = 148 / cluster_size;
+  }
+  if (getenv("RINGRNN_DEBUG") != nullptr)
+    fprintf(stderr, "[ringrnn] cluster size %d: at most %d clusters resident\n", cluster_size, n);
+  g_residency.push_back({kernel, device, n});
+  return n;
 }
 
 // ---- deferred device status --------------------------------------------------------------------
@@ -172,6 +202,14 @@ extern "C" const char* ringrnn_last_cuda_error_string(void) { return cudaGetErro
 extern "C" size_t ringrnn_workspace_bytes(const RingRnnProblem* p, int which, int history_given) {
   if (p == nullptr || check_problem(*p) != RINGRNN_OK) return (size_t)-1;
   const bool bf16 = p->precision == RINGRNN_PREC_BF16;
+  if (bf16 && lane_supported(*p)) {
+    switch (which) {
+      case RINGRNN_WS_FWD: return lane_fwd_workspace_bytes(*p);
+      case RINGRNN_WS_SAVED: return lane_saved_bytes(*p);
+      case RINGRNN_WS_BWD: return lane_bwd_workspace_bytes(*p);
+      default: return (size_t)-1;
+    }
+  }
   if (bf16 && !bf16_supported(*p)) {
     // bf16 arithmetic, one GEMM per timestep: the shapes the persistent kernels do not take
     if (!stepwise_supported(*p)) return (size_t)-1;
@@ -207,7 +245,8 @@ extern "C" int ringrnn_fwd(const RingRnnFwdArgs* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
     if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    rc = bf16_supported(a->p) ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
+    rc = lane_supported(a->p) ? lane_forward(*a, dp, s)
+         : bf16_supported(a->p) ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }
@@ -231,7 +270,8 @@ extern "C" int ringrnn_bwd(const RingRnnBwdArgs* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
     if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    rc = bf16_supported(a->p) ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
+    rc = lane_supported(a->p) ? lane_backward(*a, dp, s)
+         : bf16_supported(a->p) ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }

@@ -95,6 +95,11 @@ int queue_status_report(const int* dev_status, cudaStream_t s);
 constexpr int GRAD_J_BLOCKS = 128;
 int launch_grad_j(const float* raw, const float* Wo, size_t NN, float* grad_J, double* scratch, cudaStream_t s);
 
+// Clusters of `kernel` that can be resident at once on the current device, its shared-memory limit raised on the way: asked
+// of the driver on the first call per kernel and device (it takes longer than a launch) and remembered.  cfg: everything but
+// the grid.  -1 on a CUDA error.
+int resident_clusters(const void* kernel, cudaLaunchConfig_t* cfg, int cluster_size, int smem_bytes);
+
 // fp32 (CUDA-core) path ----------------------------------------------------------------------
 size_t fp32_fwd_workspace_bytes(const RingRnnProblem& p);
 size_t fp32_saved_bytes(const RingRnnProblem& p, int history_given);
@@ -106,6 +111,9 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
 int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* out, int M, int N, long long K,
             int nsplit, int* status, cudaStream_t s);
 
+int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, int slabs, int cols, int nsplit, int* status,
+                  cudaStream_t s);
+
 int tc_gemm_pair(const void* A, const void* B, float* out, int M, int N, long long K, int* status, cudaStream_t s);
 
 // bf16 tensor-core path ----------------------------------------------------------------------
@@ -115,6 +123,14 @@ size_t bf16_saved_bytes(const RingRnnProblem& p);
 size_t bf16_bwd_workspace_bytes(const RingRnnProblem& p);
 int bf16_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s);
 int bf16_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s);
+
+// bf16, N <= 256 and up to two active columns: neurons on the tensor-memory lanes (ringrnn_lane.cu)
+bool lane_supported(const RingRnnProblem& p);
+size_t lane_fwd_workspace_bytes(const RingRnnProblem& p);
+size_t lane_saved_bytes(const RingRnnProblem& p);
+size_t lane_bwd_workspace_bytes(const RingRnnProblem& p);
+int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s);
+int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s);
 
 // bf16 stepwise path: one tensor-core GEMM per timestep (ringrnn_stepwise.cu), for the shapes the persistent
 // kernels do not take

@@ -73,12 +73,15 @@ struct GemmCfg {
 
 // out[split][M_total][N_total] fp32;  the CTA's output tile starts at (m0 = blockIdx.x*128, n0 = blockIdx.y*NT)
 // K-major:  tmA over A[M_total, K] box [128 x 64], tmB over B[N_total, K] box [min(NT,256) x 64]
+//           K may be cut into slabs of chunks_per_slab K chunks (KC columns each): slab i is columns [0, ..) of rows
+//           [i*M_total, (i+1)*M_total) of A and [i*N_total, ..) of B, e.g. one slab per timestep of [T][rows][samples]
+//           tensors; columns beyond the tensor read as zero.  K_total then counts KC per chunk.
 // MN-major: tmA over A[K, M_total] box [KC x 64],  tmB over B[K, N_total] box [KC x 64]
 template <bool MN_MAJOR, int NT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                float* __restrict__ out, int M_total, int N_total, long long K_total, long long k_per_split,
-               int* status) {
+               int chunks_per_slab, int* status) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -130,8 +133,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int blk = 0; blk < NT / 64; ++blk)
             tma_load_2d(b_dst + blk * Cfg::KC * 128, &tmB, full_bar(s), n0 + blk * 64, k);
         } else {
-          tma_load_2d(a_dst, &tmA, full_bar(s), k, m0);
-          for (int nh = 0; nh < Cfg::NI; ++nh) tma_load_2d(b_dst + nh * 256 * 128, &tmB, full_bar(s), k, n0 + nh * 256);
+          const int chunk = k / Cfg::KC, slab = chunk / chunks_per_slab, x = (chunk - slab * chunks_per_slab) * Cfg::KC;
+          tma_load_2d(a_dst, &tmA, full_bar(s), x, slab * M_total + m0);
+          for (int nh = 0; nh < Cfg::NI; ++nh)
+            tma_load_2d(b_dst + nh * 256 * 128, &tmB, full_bar(s), x, slab * N_total + n0 + nh * 256);
         }
       }
     }
@@ -352,7 +357,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int nspl
 
 template <bool MN_MAJOR, int NT>
 int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N_total, long long K_total, int nsplit,
-                int* status, cudaStream_t s) {
+                int* status, cudaStream_t s, int slabs = 1) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -360,10 +365,16 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
     ok = make_tmap_bf16_2d(&tmA, A, (uint64_t)K_total, (uint64_t)M_total, Cfg::KC, 64) &&
          make_tmap_bf16_2d(&tmB, B, (uint64_t)K_total, (uint64_t)N_total, Cfg::KC, 64);
   } else {
-    ok = make_tmap_bf16_2d(&tmA, A, (uint64_t)M_total, (uint64_t)K_total, 128, 64) &&
-         make_tmap_bf16_2d(&tmB, B, (uint64_t)N_total, (uint64_t)K_total, Cfg::NMMA, 64);
+    const uint64_t cols = (uint64_t)K_total / slabs;  // of one slab
+    ok = make_tmap_bf16_2d(&tmA, A, (uint64_t)slabs * M_total, cols, 128, 64) &&
+         make_tmap_bf16_2d(&tmB, B, (uint64_t)slabs * N_total, cols, Cfg::NMMA, 64);
   }
   if (!ok) return RINGRNN_ERR_CUDA;
+  int chunks_per_slab = 0x7fffffff;
+  if (slabs > 1) {
+    chunks_per_slab = (int)((K_total / slabs + Cfg::KC - 1) / Cfg::KC);
+    K_total = (long long)slabs * chunks_per_slab * Cfg::KC;
+  }
   long long kps = (K_total + nsplit - 1) / nsplit;
   kps = (kps + Cfg::KC - 1) / Cfg::KC * Cfg::KC;
   RINGRNN_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<MN_MAJOR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -372,7 +383,7 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
   {
     LaunchScope ls(K_DW, s);
     gemm_tc_kernel<MN_MAJOR, NT><<<grid, GEMM_THREADS, Cfg::SMEM, s>>>(tmA, tmB, partial, M_total, N_total, K_total,
-                                                                        kps, status);
+                                                                        kps, chunks_per_slab, status);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   return RINGRNN_OK;
@@ -406,6 +417,16 @@ int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* o
     RINGRNN_CUDA_TRY(cudaGetLastError());
   }
   return RINGRNN_OK;
+}
+
+// partial[split][M][N] = sum over slabs and columns of A[slab][M][cols] * B[slab][N][cols]^T (K-major operands)
+int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, int slabs, int cols, int nsplit, int* status,
+                  cudaStream_t s) {
+  if (M % 128 != 0 || nsplit < 1) return RINGRNN_ERR_SHAPE;
+  const long long K = (long long)slabs * cols;
+  if (N == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, slabs);
+  if (N == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, slabs);
+  return RINGRNN_ERR_SHAPE;
 }
 
 // CTA-pair K-major GEMM: out[M,N] = A[M,K] * B[N,K]^T, M % 256 == 0, N a multiple of 256, 224 or 128 (the pair MMA wants N % 32 == 0) (N % NT == 0)
