@@ -9,7 +9,10 @@
 // delta_t = alpha*F'(re_t)*g_t, and a batched-over-(t,b) product kernel forms
 // dW_m = sum_{t,b} s_m[t,b] * delta_t[b,:]^T r_{t-1}[b,:] with a fixed split of the (t,b) range and a
 // fixed-order reduction of the partial sums, so results are bit-reproducible (no atomics).
+#include <string.h>
+
 #include "ringrnn_common.cuh"
+#include "ringrnn_fp32_cluster.cuh"
 
 namespace ringrnn {
 
@@ -313,71 +316,115 @@ __global__ void __launch_bounds__(FT) bwd_fp32_kernel(DevProblem p, const float*
 }
 
 // ---- weight gradients: partial[s][m][i][j] = sum_{k in split s} scale_m[k] delta[k][i] rprev[k][j]
-constexpr int DW_TILE = 64;
-constexpr int DW_KC = 16;
+// A CTA of 128 threads forms a 128 x 128 tile of one matrix over its slice of k = (t, b), 8 x 16 per thread in packed pairs:
+// six 16-byte shared-memory loads (four wavefronts each) per 128 FMAs, which leaves the FMA pipe the bound (8 x 8 per thread
+// has it the other way round).  The next rows are loaded into registers, untouched until the current ones are multiplied.  N = 250, 20000 rows, 3 matrices: 369 -> 286 us.
+constexpr int DW_TILE = 128;
+constexpr int DW_KC = 8;
+constexpr int DW_PAD = DW_TILE + 4;
+constexpr int DW_THREADS = 128;
 
-__global__ void __launch_bounds__(256) dw_fp32_kernel(DevProblem p, const float* __restrict__ delta,
-                                                      const float* __restrict__ hist, float* __restrict__ partial,
-                                                      int ksplit, long long k_per_split) {
-  __shared__ __align__(16) float dsm[DW_KC][DW_TILE];
-  __shared__ __align__(16) float rsm[DW_KC][DW_TILE];
+__device__ __forceinline__ unsigned long long dw_pk(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+__global__ void __launch_bounds__(DW_THREADS, 2) dw_fp32_kernel(DevProblem p, const float* __restrict__ delta,
+                                                                const float* __restrict__ hist,
+                                                                float* __restrict__ partial, int ksplit,
+                                                                long long k_per_split) {
+  __shared__ __align__(16) float dsm[2][DW_KC][DW_PAD];
+  __shared__ __align__(16) float rsm[2][DW_KC][DW_PAD];
   const int N = p.N;
   const int m = blockIdx.z / ksplit, s = blockIdx.z % ksplit;
   const int i0 = blockIdx.y * DW_TILE, j0 = blockIdx.x * DW_TILE;
   const long long K = (long long)p.T * p.B;
   const long long k_begin = (long long)s * k_per_split;
   const long long k_end = (k_begin + k_per_split < K) ? k_begin + k_per_split : K;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int lr = threadIdx.x / 16;        // k row this thread loads
-  const int lc = (threadIdx.x % 16) * 4;  // first of 4 columns it loads
-  float acc[4][4];
+  const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
+  const int lc = threadIdx.x;  // the column this thread loads
+  const int col = m == 0 ? 0 : active_col(p, m - 1);
+  const bool di = i0 + lc < N, rj = j0 + lc < N;
+  unsigned long long acc[8][8];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int x = 0; x < 8; ++x)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-
-  for (long long kk = k_begin; kk < k_end; kk += DW_KC) {
-    const long long k = kk + lr;
-    float dv[4] = {0.f, 0.f, 0.f, 0.f}, rv[4] = {0.f, 0.f, 0.f, 0.f};
-    if (k < k_end) {
-      const int t = (int)(k / p.B), b = (int)(k % p.B);
-      const float sc = (m == 0) ? 1.f : __ldg(p.A + ((size_t)b * p.T + t) * p.a_dim + active_col(p, m - 1));
-      const float* drow = delta + (size_t)k * N;
-      const float* rrow = (t == 0) ? p.r_init + (size_t)b * N : hist + ((size_t)(t - 1) * p.B + b) * N;
+    for (int y = 0; y < 8; ++y) acc[x][y] = 0ull;
+  float dv[DW_KC], rv[DW_KC], sv[DW_KC];
+  // (t, b) of the next row, carried along from one set of rows to the next
+  int t = (int)(k_begin / p.B), b = (int)(k_begin - (long long)t * p.B);
+  const float* dp = delta + (size_t)k_begin * N + i0 + lc;
+  const float* ap = p.A + col;
+  auto load = [&](long long k0) {
+    const int left = k_end - k0 < DW_KC ? (int)(k_end - k0) : DW_KC;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (i0 + lc + c < N) dv[c] = sc * __ldg(drow + i0 + lc + c);
-        if (j0 + lc + c < N) rv[c] = __ldg(rrow + j0 + lc + c);
+    for (int x = 0; x < DW_KC; ++x) {
+      dv[x] = 0.f;
+      rv[x] = 0.f;
+      sv[x] = 1.f;
+      if (x < left) {
+        if (m > 0) sv[x] = __ldg(ap + ((size_t)b * p.T + t) * p.a_dim);
+        if (di) dv[x] = __ldg(dp);
+        if (rj) rv[x] = __ldg((t == 0 ? p.r_init + (size_t)b * N : hist + ((size_t)(t - 1) * p.B + b) * N) + j0 + lc);
+      }
+      dp += N;
+      if (++b == p.B) {
+        b = 0;
+        ++t;
       }
     }
-    __syncthreads();
+  };
+  auto put = [&](int buf) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      dsm[lr][lc + c] = dv[c];
-      rsm[lr][lc + c] = rv[c];
+    for (int x = 0; x < DW_KC; ++x) {
+      dsm[buf][x][lc] = dv[x] * sv[x];
+      rsm[buf][x][lc] = rv[x];
     }
-    __syncthreads();
-#pragma unroll
+  };
+  if (k_begin < k_end) {
+    load(k_begin);
+    put(0);
+  }
+  __syncthreads();
+  int buf = 0;
+  for (long long kk = k_begin; kk < k_end; kk += DW_KC, buf ^= 1) {
+    const bool more = kk + DW_KC < k_end;
+    if (more) load(kk + DW_KC);
+#pragma unroll 4
     for (int q = 0; q < DW_KC; ++q) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&dsm[q][ty * 4]);
-      const float4 b4 = *reinterpret_cast<const float4*>(&rsm[q][tx * 4]);
-      const float av[4] = {a4.x, a4.y, a4.z, a4.w};
-      const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+      const float4 a0 = *reinterpret_cast<const float4*>(&dsm[buf][q][ty * 4]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&dsm[buf][q][64 + ty * 4]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      unsigned long long bv[8];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int y = 0; y < 4; ++y) {
+        const float4 f = *reinterpret_cast<const float4*>(&rsm[buf][q][32 * y + tx * 4]);
+        bv[2 * y] = dw_pk(f.x, f.y);
+        bv[2 * y + 1] = dw_pk(f.z, f.w);
+      }
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+      for (int x = 0; x < 8; ++x) {
+        const unsigned long long a2 = dw_pk(av[x], av[x]);
+#pragma unroll
+        for (int y = 0; y < 8; ++y) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[x][y]) : "l"(a2), "l"(bv[y]));
+      }
     }
+    if (more) put(buf ^ 1);
+    __syncthreads();
   }
   float* out = partial + ((size_t)s * p.n_mat + m) * N * N;
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int i = i0 + ty * 4 + a;
+  for (int x = 0; x < 8; ++x) {
+    const int i = i0 + (x / 4) * 64 + ty * 4 + x % 4;
     if (i >= N) continue;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int j = j0 + tx * 4 + b;
-      if (j < N) out[(size_t)i * N + j] = acc[a][b];
+    for (int y = 0; y < 8; ++y) {
+      const int j = j0 + (y / 2) * 32 + tx * 4 + (y % 2) * 2;
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[x][y]));
+      if (j < N) out[(size_t)i * N + j] = lo;
+      if (j + 1 < N) out[(size_t)i * N + j + 1] = hi;
     }
   }
 }
@@ -431,12 +478,17 @@ __global__ void grad_j_partial_kernel(const float* __restrict__ raw, const float
   }
 }
 __global__ void grad_j_finish_kernel(const double* __restrict__ partial, int nblocks, float* grad_J) {
+  double a0 = 0.0, a1 = 0.0;  // one warp; fixed order
+  for (int b = threadIdx.x; b < nblocks; b += 32) {
+    a0 += partial[2 * b];
+    a1 += partial[2 * b + 1];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a0 += __shfl_down_sync(0xffffffffu, a0, o);
+    a1 += __shfl_down_sync(0xffffffffu, a1, o);
+  }
   if (threadIdx.x == 0) {
-    double a0 = 0.0, a1 = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
-      a0 += partial[2 * b];
-      a1 += partial[2 * b + 1];
-    }
     grad_J[0] = (float)a0;
     grad_J[1] = (float)a1;
   }
@@ -461,7 +513,7 @@ namespace {
 int pick_ksplit(const RingRnnProblem& p, int n_mat) {
   const int tiles = ((p.N + DW_TILE - 1) / DW_TILE) * ((p.N + DW_TILE - 1) / DW_TILE) * n_mat;
   long long K = (long long)p.T * p.B;
-  int ks = (4 * 148 + tiles - 1) / tiles;
+  int ks = 2 * 148 / tiles;  // two resident CTAs per SM
   if (ks < 1) ks = 1;
   if (ks > 64) ks = 64;
   while (ks > 1 && K / ks < 64) --ks;
@@ -532,17 +584,97 @@ int launch_transpose(const DevProblem& dp, float* WT, cudaStream_t s) {
   return RINGRNN_OK;
 }
 
+// ---- cluster kernels (ringrnn_fp32_cluster.cuh): which requests, and in what shape -------------------------------
+// The shape with the least estimated time per step among those whose weights and buffers fit shared memory:
+// rounds of resident clusters x (FMA issue of one CTA's neurons for the tile + exchange and barrier).  Resident clusters on
+// a B200 (148 SMs, GPCs of unequal size): 15 of 8, 33 of 4.  No shape fits: the kernels above, weights through L2.
+bool cluster_shape(const RingRnnProblem& p, int n_mat, fc::Shape* out) {
+  const int resident[4] = {148, 74, 33, 15};
+  double best = 1e300;
+  for (int lc = 0; lc < 4; ++lc) {
+    const int C = 1 << lc;
+    fc::Shape h;
+    h.C = C;
+    h.NP = (p.N + 31) / 32 * 32;
+    h.NC = ((p.N + C - 1) / C + 31) / 32 * 32;
+    if (C > 1 && h.NC * (C - 1) >= p.N) continue;  // a CTA without neurons
+    for (h.NO = 1; h.NO <= 4; ++h.NO) {
+      h.tiles = (p.B + 8 * h.NO - 1) / (8 * h.NO);
+      if (sizeof(float) * (size_t)fc::offsets(h, n_mat, 2).total > SMEM_MAX) continue;
+      const double rounds = (h.tiles + resident[lc] - 1) / resident[lc];
+      const double cost = rounds * (n_mat * (double)h.NC * h.NP * 8 * h.NO / 128 * 1.25 + 900 + (C > 1 ? 400 : 0));
+      if (cost < best) {
+        best = cost;
+        *out = h;
+      }
+    }
+  }
+  return best < 1e300;
+}
+
+template <int MODE, int ACT>
+int launch_cluster(const fc::Args& a, int splits, int slot, cudaStream_t s) {
+  auto kernel = fc::cluster_kernel<MODE, ACT>;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.blockDim = dim3(fc::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = sizeof(float) * (size_t)fc::offsets(a.sh, a.p.n_mat, MODE).total;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = a.sh.C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  RINGRNN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+  cfg.gridDim = dim3(a.sh.tiles * a.sh.C, splits, 1);
+  {
+    LaunchScope ls(slot, s);
+    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
+  }
+  return RINGRNN_OK;
+}
+
+template <int MODE>
+int launch_cluster_act(int act, const fc::Args& a, int splits, int slot, cudaStream_t s) {
+  switch (act) {
+    case RINGRNN_ACT_RELU: return launch_cluster<MODE, RINGRNN_ACT_RELU>(a, splits, slot, s);
+    case RINGRNN_ACT_GELU: return launch_cluster<MODE, RINGRNN_ACT_GELU>(a, splits, slot, s);
+    case RINGRNN_ACT_TANH: return launch_cluster<MODE, RINGRNN_ACT_TANH>(a, splits, slot, s);
+    default: return launch_cluster<MODE, RINGRNN_ACT_SILU>(a, splits, slot, s);
+  }
+}
+
+// grad_A[b,t,col_k] = sum over the CTAs of part[rank][k][b][t]
+__global__ void da_cluster_kernel(DevProblem p, const float* __restrict__ part, int C, float* grad_A) {
+  const size_t BT = (size_t)p.B * p.T, total = BT * (p.n_mat - 1);
+  for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
+    const int k = (int)(idx / BT);
+    const size_t bt = idx % BT;
+    float v = 0.f;
+    for (int r = 0; r < C; ++r) v += part[((size_t)r * (p.n_mat - 1) + k) * BT + bt];
+    grad_A[bt * p.a_dim + active_col(p, k)] = v;
+  }
+}
+
 }  // namespace
 
 // workspace layouts ----------------------------------------------------------------------------
 //   FWD : WT[n_mat][N][N]
-//   SAVED (only when the caller does not keep bump_history): hist[T][B][N]
-//   BWD : WT[n_mat][N][N] | delta[T][B][N] | partial[ksplit][n_mat][N][N] | raw[N][N]
+//   SAVED (only when the caller does not keep bump_history): hist[T][B][N], with cluster kernels also F'(re)[T][B][N]
+//   BWD : WT[n_mat][N][N] | delta[T][B][N] | partial[ksplit][n_mat][N][N] | raw[N][N] |
+//         with cluster kernels F'(re)[T][B][N] (when the forward could not keep it) | dL/dA sums [C][n_mat-1][B][T]
 size_t fp32_fwd_workspace_bytes(const RingRnnProblem& p) {
   return align_up(sizeof(float) * (size_t)n_mat_of(p) * p.N * p.N, 256);
 }
 size_t fp32_saved_bytes(const RingRnnProblem& p, int history_given) {
-  return history_given ? 0 : align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256);
+  if (history_given) return 0;
+  fc::Shape h;
+  return (cluster_shape(p, n_mat_of(p), &h) ? 2 : 1) * align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256);
+}
+static size_t cluster_da_bytes(const RingRnnProblem& p, const fc::Shape& h) {
+  return align_up(sizeof(float) * (size_t)h.C * (n_mat_of(p) - 1) * p.B * p.T, 256);
 }
 // bytes of the split-(t,b) partial sums; never less than the scratch the dJ reduction borrows from the same region
 static size_t partial_bytes(const RingRnnProblem& p, int n_mat) {
@@ -553,8 +685,11 @@ static size_t partial_bytes(const RingRnnProblem& p, int n_mat) {
 size_t fp32_bwd_workspace_bytes(const RingRnnProblem& p) {
   const int n_mat = n_mat_of(p);
   const size_t NN = (size_t)p.N * p.N;
-  return align_up(sizeof(float) * n_mat * NN, 256) + align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256) +
-         partial_bytes(p, n_mat) + align_up(sizeof(float) * NN, 256);
+  size_t n = align_up(sizeof(float) * n_mat * NN, 256) + align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256) +
+             partial_bytes(p, n_mat) + align_up(sizeof(float) * NN, 256);
+  fc::Shape h;
+  if (cluster_shape(p, n_mat, &h)) n += align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256) + cluster_da_bytes(p, h);
+  return n;
 }
 
 int fp32_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) {
@@ -564,6 +699,17 @@ int fp32_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   if (hist == nullptr && a.saved != nullptr) {
     if (a.saved_bytes < fp32_saved_bytes(p, 0)) return RINGRNN_ERR_WORKSPACE;
     hist = static_cast<float*>(a.saved);
+  }
+  fc::Args ca;
+  memset(&ca, 0, sizeof(ca));
+  if (cluster_shape(p, dp.n_mat, &ca.sh)) {
+    ca.p = dp;
+    ca.hist = hist;
+    if (a.bump_history == nullptr && a.saved != nullptr)
+      ca.dact = reinterpret_cast<float*>(static_cast<char*>(a.saved) + align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256));
+    ca.dec_x = a.dec_x; ca.dec_y = a.dec_y; ca.dec_ta = a.dec_ta; ca.dec_u = a.dec_u; ca.dec_v = a.dec_v;
+    ca.final_state = a.final_state;
+    return launch_cluster_act<0>(p.activation, ca, 1, K_FWD, s);
   }
   float* WT = static_cast<float*>(a.workspace);
   int rc = launch_transpose(dp, WT, s);
@@ -594,23 +740,55 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
   float* partial = reinterpret_cast<float*>(w);
   w += partial_bytes(p, n_mat);
   float* raw = reinterpret_cast<float*>(w);
+  w += align_up(sizeof(float) * NN, 256);
 
-  int rc = launch_transpose(dp, WT, s);
-  if (rc != RINGRNN_OK) return rc;
   if (a.grad_A != nullptr)
     RINGRNN_CUDA_TRY(cudaMemsetAsync(a.grad_A, 0, sizeof(float) * (size_t)p.B * p.T * p.a_dim, s));
-  Fp32BwdIn in{hist, a.grad_output, a.coef_x, a.coef_y, a.coef_s, a.dec_u, a.dec_v, delta, a.grad_r_init, a.grad_A};
-  if (bwd_smem(p.N, n_mat, 16) <= SMEM_MAX) rc = launch_bwd<16>(dp, p.activation, WT, in, s);
-  else if (bwd_smem(p.N, n_mat, 8) <= SMEM_MAX) rc = launch_bwd<8>(dp, p.activation, WT, in, s);
-  else if (bwd_smem(p.N, n_mat, 4) <= SMEM_MAX) rc = launch_bwd<4>(dp, p.activation, WT, in, s);
-  else rc = RINGRNN_ERR_SHAPE;
-  if (rc != RINGRNN_OK) return rc;
+  int rc;
+  fc::Args ca;
+  memset(&ca, 0, sizeof(ca));
+  if (cluster_shape(p, n_mat, &ca.sh)) {
+    ca.p = dp;
+    ca.hist = const_cast<float*>(hist);
+    const size_t tbn = align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256);
+    if (a.bump_history == nullptr) {  // the forward kept F'(re) beside the history
+      ca.dact = reinterpret_cast<float*>(static_cast<char*>(const_cast<void*>(a.saved)) + tbn);
+    } else {  // only the history: F'(re) of all steps at once first, off the sequential path
+      ca.dact = reinterpret_cast<float*>(w);
+      int splits = 148 / (ca.sh.tiles * ca.sh.C);
+      if (splits > p.T) splits = p.T;
+      rc = launch_cluster_act<1>(p.activation, ca, splits < 1 ? 1 : splits, K_BWD, s);
+      if (rc != RINGRNN_OK) return rc;
+    }
+    w += tbn;
+    ca.grad_output = a.grad_output;
+    ca.coef_x = a.coef_x; ca.coef_y = a.coef_y; ca.coef_s = a.coef_s; ca.dec_u = a.dec_u; ca.dec_v = a.dec_v;
+    ca.delta = delta;
+    ca.grad_r_init = a.grad_r_init;
+    ca.dA_part = a.grad_A != nullptr && n_mat > 1 ? reinterpret_cast<float*>(w) : nullptr;
+    rc = launch_cluster<2, RINGRNN_ACT_RELU>(ca, 1, K_BWD, s);  // (no activation is evaluated in reverse)
+    if (rc != RINGRNN_OK) return rc;
+    if (ca.dA_part != nullptr) {
+      LaunchScope ls(K_REDUCE, s);
+      da_cluster_kernel<<<296, 256, 0, s>>>(dp, ca.dA_part, ca.sh.C, a.grad_A);
+      RINGRNN_CUDA_TRY(cudaGetLastError());
+    }
+  } else {
+    rc = launch_transpose(dp, WT, s);
+    if (rc != RINGRNN_OK) return rc;
+    Fp32BwdIn in{hist, a.grad_output, a.coef_x, a.coef_y, a.coef_s, a.dec_u, a.dec_v, delta, a.grad_r_init, a.grad_A};
+    if (bwd_smem(p.N, n_mat, 16) <= SMEM_MAX) rc = launch_bwd<16>(dp, p.activation, WT, in, s);
+    else if (bwd_smem(p.N, n_mat, 8) <= SMEM_MAX) rc = launch_bwd<8>(dp, p.activation, WT, in, s);
+    else if (bwd_smem(p.N, n_mat, 4) <= SMEM_MAX) rc = launch_bwd<4>(dp, p.activation, WT, in, s);
+    else rc = RINGRNN_ERR_SHAPE;
+    if (rc != RINGRNN_OK) return rc;
+  }
 
   const long long K = (long long)p.T * p.B;
   long long kps = (K + ksplit - 1) / ksplit;
   kps = (kps + DW_KC - 1) / DW_KC * DW_KC;
   dim3 grid((p.N + DW_TILE - 1) / DW_TILE, (p.N + DW_TILE - 1) / DW_TILE, n_mat * ksplit);
-  { LaunchScope ls(K_DW, s); dw_fp32_kernel<<<grid, 256, 0, s>>>(dp, delta, hist, partial, ksplit, kps); }
+  { LaunchScope ls(K_DW, s); dw_fp32_kernel<<<grid, DW_THREADS, 0, s>>>(dp, delta, hist, partial, ksplit, kps); }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   RINGRNN_CUDA_TRY(cudaMemsetAsync(a.grad_Wa, 0, sizeof(float) * (size_t)p.a_dim * NN, s));
   { LaunchScope ls(K_REDUCE, s); dw_reduce_kernel<<<296, 256, 0, s>>>(dp, partial, ksplit, a.grad_Wa, a.grad_Wo, raw); }
