@@ -186,6 +186,40 @@ int ringrnn_last_device_code(void);
  * other, so the next ringrnn_fwd / ringrnn_bwd / ringrnn_device_status sees RINGRNN_ERR_DEVICE. */
 int ringrnn_selftest_wait(long long limit_cycles, int code, int* status, void* stream);
 
+/* One training step on the fused loss: ringrnn_fwd (every step saved, or checkpoints), ringrnn_angle_loss, ringrnn_bwd, out of
+ * one scratch buffer of ringrnn_train_bytes() bytes.  The loop body of train_general_ring_no_gain.py:312-334 without its
+ * optimizer.  dL/dW for a loss of loss_out[0] + bump_weight * loss_out[1].
+ *   target [B,T]; dec_u, dec_v [N]; loss_out float[2]; decoded [B,T], final_state [B,N], grad_J float[2]: NULL = skip
+ * A wait abandoned by the forward is reported to the next call, as everywhere. */
+typedef struct RingRnnTrainArgs {
+  RingRnnProblem p;
+  const float* target;
+  float bump_weight;
+  float inv_count;
+  const float* dec_u;
+  const float* dec_v;
+  float* grad_Wo;
+  float* grad_Wa;
+  float* grad_J;
+  float* loss_out;
+  float* decoded;
+  float* final_state;
+  void* workspace;
+  size_t workspace_bytes;
+} RingRnnTrainArgs;
+size_t ringrnn_train_bytes(const RingRnnProblem* p);
+int ringrnn_train_step(const RingRnnTrainArgs* args, void* stream);
+
+/* Which columns of an action signal [rows, a_dim] (a_dim <= 64) hold a non-zero value: bit k of *mask (host memory).  Waits
+ * for `stream`.  RINGRNN_ERR_UNSUPPORTED if more than 32 host threads ask at once.  The root training script pads [L, R]
+ * with zero columns (train_general_ring_no_gain.py:200-223), which both directions skip. */
+int ringrnn_active_columns(const float* A, long long rows, int a_dim, unsigned long long* mask, void* stream);
+
+/* angle[i] = atan2(y[i], x[i]) in [0, 2pi) (train/train_ring_attractor.py:196-206), and the circular distance
+ * min(d, 2pi - d), d = |pred - target| mod 2pi (compare/compare_models_fair.py:15-20); n elements. */
+int ringrnn_decode_angles(long long n, const float* x, const float* y, float* angle, void* stream);
+int ringrnn_angular_error(long long n, const float* pred, const float* target, float* error, void* stream);
+
 /* Decode + loss on the [B,T] scalars the forward emits.  Replaces the [B,T,N]-sized chain
  * `bump @ W_delta7`, max-normalise (train_general_ring_no_gain.py:113-116), cosine_similarity_loss
  * (train/train_ring_attractor.py:190-220) and bump_amplitude_loss (:275-298).
@@ -236,6 +270,16 @@ int ringrnn_generate_trials(int B, int T, int N, int a_dim, unsigned long long s
                             float max_av, float scale, float start_ratio, const float* zero_ratios, int n_ratios,
                             int bump_kind, float bump_param, float* A, float* target, float* r_init,
                             float* theta0_scratch, void* stream);
+
+/* The host generator's trials from the host's own uniform draws: what the reference does with them
+ * (utils/generate_av_integration_data.py:28-56: the j-th step after the first n0 keeps its velocity iff the index of the
+ * j-th smallest ordering draw is below the trial's keep count; the target lags by one step), the [L, R] signal divided by
+ * max_av, and the unit-norm Gaussian bump of width N/bump_width at the first target angle.
+ *   draws  device, for n_all >= n trials: theta [n_all] | keep [n_all] | value [n_all][T-n0] | order [n_all][T-n0], all float
+ *   A [n,T,2], target [n,T], r_init [n,N] out.  T - n0 <= 8192. */
+int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, const float* draws, float max_av, float bump_width,
+                            float* A, float* target, float* r_init, void* stream);
+
 
 /* Optimizer step on flat buffers, entirely on the device: clip the gradient to a global L2 norm of `max_norm`
  * (max_norm <= 0: no clipping), then one Adam update (no weight decay, no amsgrad).  Replaces the pair

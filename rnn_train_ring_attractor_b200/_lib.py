@@ -45,6 +45,13 @@ class BwdArgs(C.Structure):
                 ("workspace_bytes", C.c_size_t), ("status", C.c_void_p)]
 
 
+class TrainArgs(C.Structure):
+    _fields_ = [("p", Problem), ("target", C.c_void_p), ("bump_weight", C.c_float), ("inv_count", C.c_float),
+                ("dec_u", C.c_void_p), ("dec_v", C.c_void_p), ("grad_Wo", C.c_void_p), ("grad_Wa", C.c_void_p),
+                ("grad_J", C.c_void_p), ("loss_out", C.c_void_p), ("decoded", C.c_void_p), ("final_state", C.c_void_p),
+                ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t)]
+
+
 # every symbol include/ringrnn.h declares: name -> (restype, argtypes)
 SYMBOLS = {
     "ringrnn_version": (C.c_int, []),
@@ -66,9 +73,16 @@ SYMBOLS = {
     "ringrnn_angle_loss_static": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                             C.c_float, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                             C.c_void_p, C.c_void_p]),
+    "ringrnn_train_bytes": (C.c_size_t, [C.POINTER(Problem)]),
+    "ringrnn_train_step": (C.c_int, [C.POINTER(TrainArgs), C.c_void_p]),
+    "ringrnn_active_columns": (C.c_int, [C.c_void_p, C.c_longlong, C.c_int, C.POINTER(C.c_ulonglong), C.c_void_p]),
+    "ringrnn_decode_angles": (C.c_int, [C.c_longlong, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ringrnn_angular_error": (C.c_int, [C.c_longlong, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ringrnn_generate_trials": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_ulonglong, C.c_longlong, C.c_float,
                                           C.c_float, C.c_float, C.POINTER(C.c_float), C.c_int, C.c_int, C.c_float,
                                           C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ringrnn_assemble_trials": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_float, C.c_float,
+                                          C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ringrnn_clip_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_float, C.c_float,
                                     C.c_float, C.c_float, C.c_int, C.c_float, C.c_void_p, C.c_void_p]),
     "ringrnn_device_status": (C.c_int, [C.POINTER(C.c_int)]),

@@ -126,6 +126,28 @@ int queue_status_report(const int* dev_status, cudaStream_t s) {
   return RINGRNN_OK;
 }
 
+static __device__ int g_direct_status;          // one per device
+static volatile int* g_direct_host = nullptr;    // one pinned word for all devices
+static int* g_direct_dev[64];
+
+int direct_status(DirectStatus* out) {
+  int device = 0;
+  RINGRNN_CUDA_TRY(cudaGetDevice(&device));
+  if (device < 0 || device >= 64) return RINGRNN_ERR_UNSUPPORTED;
+  std::lock_guard<std::mutex> lk(g_status_mu);
+  if (g_direct_host == nullptr) {
+    void* h = nullptr;
+    RINGRNN_CUDA_TRY(cudaHostAlloc(&h, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    *static_cast<volatile int*>(h) = 0;
+    g_direct_host = static_cast<volatile int*>(h);
+  }
+  if (g_direct_dev[device] == nullptr)
+    RINGRNN_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&g_direct_dev[device]), g_direct_status));
+  out->dev = g_direct_dev[device];
+  out->host = g_direct_host;
+  return RINGRNN_OK;
+}
+
 // first unreported non-zero status word that has arrived on the host (0 if none); clears what it returns
 static int take_device_status() {
   std::lock_guard<std::mutex> lk(g_status_mu);
@@ -137,6 +159,13 @@ static int take_device_status() {
         if (code == 0) code = g_status_ring[i];
         g_status_ring[i] = 0;
       }
+  if (g_direct_host != nullptr && *g_direct_host != 0) {
+    if (code == 0) code = *g_direct_host;
+    *g_direct_host = 0;
+    // (a failure path: later waits must not find the old code)
+    for (int* d : g_direct_dev)
+      if (d != nullptr) (void)cudaMemset(d, 0, sizeof(int));
+  }
   return code;
 }
 static thread_local int g_last_device_code = 0;
@@ -245,8 +274,11 @@ extern "C" int ringrnn_fwd(const RingRnnFwdArgs* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
     if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    rc = lane_supported(a->p) ? lane_forward(*a, dp, s)
-         : bf16_supported(a->p) ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
+    if (lane_supported(a->p)) {
+      rc = lane_forward(*a, dp, s);
+      return rc != RINGRNN_OK || a->status == nullptr ? rc : queue_status_report(a->status, s);
+    }
+    rc = bf16_supported(a->p) ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }
@@ -270,8 +302,11 @@ extern "C" int ringrnn_bwd(const RingRnnBwdArgs* a, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
     if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    rc = lane_supported(a->p) ? lane_backward(*a, dp, s)
-         : bf16_supported(a->p) ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
+    if (lane_supported(a->p)) {
+      rc = lane_backward(*a, dp, s);
+      return rc != RINGRNN_OK || a->status == nullptr ? rc : queue_status_report(a->status, s);
+    }
+    rc = bf16_supported(a->p) ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }

@@ -91,6 +91,15 @@ __host__ __device__ __forceinline__ int active_col(const DevProblem& p, int k) {
 // on this process looks at the words that have arrived.
 int queue_status_report(const int* dev_status, cudaStream_t s);
 
+// The same without a copy behind every launch, for kernels whose waits report through all three words: `dev` is polled by
+// slow waits (library-owned, per device, zero unless a wait was abandoned), `host` is a pinned host word the failing thread
+// writes itself.  0 = ok.
+struct DirectStatus {
+  int* dev;
+  volatile int* host;
+};
+int direct_status(DirectStatus* out);
+
 // dJ0 / dJ1 from the unscaled Wo gradient (ringrnn_fp32.cu); scratch: GRAD_J_BLOCKS * 2 doubles
 constexpr int GRAD_J_BLOCKS = 128;
 int launch_grad_j(const float* raw, const float* Wo, size_t NN, float* grad_J, double* scratch, cudaStream_t s);
@@ -112,7 +121,7 @@ int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* o
             int nsplit, int* status, cudaStream_t s);
 
 int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, int slabs, int cols, int nsplit, int* status,
-                  cudaStream_t s);
+                  volatile int* host_status, cudaStream_t s);
 
 int tc_gemm_pair(const void* A, const void* B, float* out, int M, int N, long long K, int* status, cudaStream_t s);
 

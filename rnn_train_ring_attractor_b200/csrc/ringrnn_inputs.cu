@@ -111,6 +111,91 @@ __global__ void __launch_bounds__(128) initial_bump_kernel(int B, int N, const f
   }
 }
 
+// One block per trial.  The ordering draws are sorted in shared memory (bitonic, ties by index: a stable sort), then every
+// step's velocity, the running angle (fp64 like the host's cumulative sum, each thread a stretch of steps) and the action
+// signal.  Arithmetic in the order of the host generator.
+constexpr int ASSEMBLE_THREADS = 256;
+__global__ void __launch_bounds__(ASSEMBLE_THREADS) assemble_trials_kernel(int n_all, int T, int n0, int N,
+                                                                           const float* __restrict__ draws, float max_av,
+                                                                           float bump_width, int sort_len, float* __restrict__ A,
+                                                                           float* __restrict__ target,
+                                                                           float* __restrict__ r_init) {
+  extern __shared__ unsigned long long sorted[];  // [sort_len] (draw bits, index), then the velocities [T]
+  __shared__ double warp_sum[ASSEMBLE_THREADS / 32];
+  __shared__ float red[ASSEMBLE_THREADS / 32];
+  float* av = reinterpret_cast<float*>(sorted + sort_len);
+  const int b = blockIdx.x, rest = T - n0, tid = threadIdx.x;
+  const float two_pi = 6.283185307179586f;
+  const float theta0 = draws[b] * two_pi;
+  const int keep = (int)draws[n_all + b];
+  const float* value = draws + 2 * (size_t)n_all + (size_t)b * rest;
+  const float* order = draws + (size_t)n_all * (2 + rest) + (size_t)b * rest;
+  for (int i = tid; i < sort_len; i += ASSEMBLE_THREADS)
+    sorted[i] = i < rest ? ((unsigned long long)__float_as_uint(order[i]) << 32) | (unsigned)i : ~0ull;
+  __syncthreads();
+  for (int size = 2; size <= sort_len; size <<= 1)
+    for (int half = size >> 1; half > 0; half >>= 1) {
+      for (int i = tid; i < sort_len / 2; i += ASSEMBLE_THREADS) {
+        const int lo = 2 * i - (i & (half - 1)), hi = lo + half;
+        const unsigned long long x = sorted[lo], y = sorted[hi];
+        if ((x > y) == ((lo & size) == 0)) {
+          sorted[lo] = y;
+          sorted[hi] = x;
+        }
+      }
+      __syncthreads();
+    }
+  for (int t = tid; t < T; t += ASSEMBLE_THREADS) {
+    float v = 0.f;
+    if (t >= n0) {
+      const bool kept = (int)(unsigned)sorted[t - n0] < keep;
+      v = __fmul_rn(__fmul_rn(__fmul_rn(value[t - n0] - 0.5f, 2.f), max_av), kept ? 1.f : 0.f);
+    }
+    av[t] = v;
+    float2* a2 = reinterpret_cast<float2*>(A) + (size_t)b * T + t;
+    *a2 = make_float2(__fdiv_rn(fmaxf(-v, 0.f), max_av), __fdiv_rn(fmaxf(v, 0.f), max_av));
+  }
+  __syncthreads();
+  // target[t] = theta0 + sum_{u<t} av[u]
+  const int per = (T + ASSEMBLE_THREADS - 1) / ASSEMBLE_THREADS, lo = tid * per, hi = lo + per < T ? lo + per : T;
+  double sum = 0.0;
+  for (int t = lo; t < hi; ++t) sum += av[t];
+  double incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((tid & 31) >= o) incl += up;
+  }
+  if ((tid & 31) == 31) warp_sum[tid >> 5] = incl;
+  __syncthreads();
+  double before = incl - sum;
+  for (int w = 0; w < (tid >> 5); ++w) before += warp_sum[w];
+  for (int t = lo; t < hi; ++t) {
+    float ang = t == 0 ? theta0 : fmodf(theta0 + (float)before, two_pi);
+    if (ang < 0.f) ang += two_pi;
+    target[(size_t)b * T + t] = ang;
+    before += av[t];
+  }
+  // the bump
+  const float c = theta0 * (float)N / two_pi, w = (float)N / bump_width, denom = 2.f * w * w;
+  float ss = 0.f;
+  for (int i = tid; i < N; i += ASSEMBLE_THREADS) {
+    float d = fabsf((float)i - c);
+    d = fminf(d, (float)N - d);
+    const float v = expf(-(d * d) / denom);
+    r_init[(size_t)b * N + i] = v;
+    ss += v * v;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+  for (int i = 0; i < ASSEMBLE_THREADS / 32; ++i) ss += red[i];
+  const float norm = sqrtf(ss);
+  for (int i = tid; i < N; i += ASSEMBLE_THREADS) r_init[(size_t)b * N + i] /= norm;
+}
+
 }  // namespace
 }  // namespace ringrnn
 
@@ -142,5 +227,26 @@ extern "C" int ringrnn_generate_trials(int B, int T, int N, int a_dim, unsigned 
     initial_bump_kernel<<<B, 128, 0, s>>>(B, N, theta0_scratch, bump_kind, bump_param, r_init);
     RINGRNN_CUDA_TRY(cudaGetLastError());
   }
+  return RINGRNN_OK;
+}
+
+extern "C" int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, const float* draws, float max_av,
+                                       float bump_width, float* A, float* target, float* r_init, void* stream) {
+  using namespace ringrnn;
+  if (n <= 0 || n_all < n || T <= 0 || n0 < 0 || n0 >= T || N <= 0) return RINGRNN_ERR_SHAPE;
+  if (!draws || !A || !target || !r_init || !(max_av > 0.f) || !(bump_width > 0.f)) return RINGRNN_ERR_ARG;
+  if (T - n0 > 8192) return RINGRNN_ERR_TOO_LARGE;
+  int sort_len = 2;
+  while (sort_len < T - n0) sort_len <<= 1;
+  const int smem = sort_len * 8 + T * 4;
+  if (smem > 200 * 1024) return RINGRNN_ERR_TOO_LARGE;
+  RINGRNN_CUDA_TRY(cudaFuncSetAttribute(assemble_trials_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  {
+    LaunchScope ls(K_PREP, s);
+    assemble_trials_kernel<<<n, ASSEMBLE_THREADS, smem, s>>>(n_all, T, n0, N, draws, max_av, bump_width, sort_len, A, target,
+                                                            r_init);
+  }
+  RINGRNN_CUDA_TRY(cudaGetLastError());
   return RINGRNN_OK;
 }

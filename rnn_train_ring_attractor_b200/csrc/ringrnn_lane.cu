@@ -61,7 +61,7 @@ Saved saved_of(void* base, const LaneLayout& l, int T) {
   return s;
 }
 
-constexpr int FINISH_BLOCKS = 148;
+constexpr int FINISH_BLOCKS = 296;
 
 struct LaneBwdLayout {
   size_t dl, partial, jpart, da;
@@ -120,21 +120,32 @@ __global__ void __launch_bounds__(256) lane_finish_kernel(const float* __restric
   __shared__ bool last;
   const size_t NN = (size_t)N * N, slice = (size_t)3 * NP * NP;
   double a0 = 0.0, a1 = 0.0;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < NN; e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e / N), j = (int)(e % N);
-    const float* src = partial + (size_t)i * NP + j;
-    float gm[3] = {0.f, 0.f, 0.f};
-    for (int s = 0; s < nsplit; ++s)
-#pragma unroll
-      for (int m = 0; m < 3; ++m) gm[m] += src[s * slice + (size_t)m * NP * NP];
-    a0 += gm[0];
-    a1 += (double)gm[0] * Wo[e];
-    grad_Wo[e] = add ? grad_Wo[e] + J1 * gm[0] : J1 * gm[0];
-    for (int k = 0; k < a_dim; ++k) {
-      const float v = k == colL ? gm[1] : k == colR ? gm[2] : 0.f;
-      float* o = grad_Wa + (size_t)k * NN + e;
-      if (!add) *o = v;
-      else if (k == colL || k == colR) *o += v;
+  // element (m, i, j) of the three blocks per thread; then the columns of grad_Wa nobody uses
+  for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < 3 * NN; x += (size_t)gridDim.x * blockDim.x) {
+    const int m = (int)(x / NN);
+    const size_t e = x - m * NN;
+    if (m > 0 && (m == 1 ? colL : colR) < 0) continue;
+    const int i = (int)(e / N), j = (int)(e - (size_t)i * N);
+    const float* src = partial + ((size_t)m * NP + i) * NP + j;
+    float v = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < nsplit; ++s) v += src[s * slice];
+    float* o;
+    if (m == 0) {
+      a0 += v;
+      a1 += (double)v * Wo[e];
+      v *= J1;
+      o = grad_Wo + e;
+    } else {
+      o = grad_Wa + (size_t)(m == 1 ? colL : colR) * NN + e;
+    }
+    *o = add ? *o + v : v;
+  }
+  if (!add && a_dim > (colL >= 0) + (colR >= 0)) {
+    const size_t all = (size_t)a_dim * NN;
+    for (size_t x = blockIdx.x * (size_t)blockDim.x + threadIdx.x; x < all; x += (size_t)gridDim.x * blockDim.x) {
+      const int k = (int)(x / NN);
+      if (k != colL && k != colR) grad_Wa[x] = 0.f;
     }
   }
   if (grad_J == nullptr) return;
@@ -197,7 +208,7 @@ __global__ void lane_da_kernel(const float* __restrict__ part, int CL, int B, in
 }
 
 template <class P>
-void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneLayout& l, int T, int t0, int* status) {
+void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneLayout& l, int T, int t0, const DirectStatus& st, int* report, bool first) {
   memset(&q, 0, sizeof(q));
   q.B = p.B; q.T = T; q.N = p.N; q.BPs = l.BPs; q.n_ut = l.n_ut; q.a_dim = p.a_dim;
   q.colL = dp.n_mat > 1 ? dp.cols[0] : -1;
@@ -210,7 +221,10 @@ void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneL
   q.WR = q.colR >= 0 ? p.Wa + q.colR * NN : nullptr;
   q.A = p.A;
   q.t0 = t0; q.T_total = p.T;
-  q.status = status;
+  q.status = st.dev;
+  q.host = st.host;
+  q.report = report;
+  q.zero_report = first ? 1 : 0;
 }
 
 }  // namespace
@@ -250,14 +264,17 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   if (train && (a.saved_bytes < lane_saved_bytes(p) || (reinterpret_cast<uintptr_t>(a.saved) & 255) != 0))
     return RINGRNN_ERR_WORKSPACE;
   char* w = static_cast<char*>(a.workspace);
-  int* status = a.status != nullptr ? a.status : reinterpret_cast<int*>(w);
   float* dec1 = reinterpret_cast<float*>(w + 1024);
   const int K = train ? lane_ckpt_interval(p) : 0;
-  if (a.status == nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
+  DirectStatus st{a.status, nullptr};
+  if (a.status == nullptr) {
+    const int rc = direct_status(&st);
+    if (rc != RINGRNN_OK) return rc;
+  }
   if (K > 0)  // checkpoint 0 is the initial state
     RINGRNN_CUDA_TRY(cudaMemcpyAsync(a.saved, p.r_init, ckpt_slot(p), cudaMemcpyDeviceToDevice, s));
   LaneFwdParams q;
-  set_common(q, p, dp, l, p.T, 0, status);
+  set_common(q, p, dp, l, p.T, 0, st, a.status == nullptr ? reinterpret_cast<int*>(w) : nullptr, true);
   q.r_init = p.r_init;
   if (train && K == 0) {
     const Saved sv = saved_of(a.saved, l, p.T);
@@ -295,9 +312,14 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
   const int Tk = K > 0 ? K : p.T;  // steps of one stretch
   const LaneBwdLayout b = lane_bwd_layout(l, Tk);
   char* w = static_cast<char*>(a.workspace);
-  int* status = a.status != nullptr ? a.status : reinterpret_cast<int*>(w);
+  DirectStatus st{a.status, nullptr};
+  if (a.status == nullptr) {
+    const int rc = direct_status(&st);
+    if (rc != RINGRNN_OK) return rc;
+  }
+  int* report = a.status == nullptr ? reinterpret_cast<int*>(w) : nullptr;
   unsigned* done = reinterpret_cast<unsigned*>(w + 64);
-  RINGRNN_CUDA_TRY(cudaMemsetAsync(w, 0, 128, s));
+  if (a.grad_J != nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(unsigned), s));
   w += 1024;
   __nv_bfloat16* DL = reinterpret_cast<__nv_bfloat16*>(w);
   w += b.dl;
@@ -326,7 +348,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
     if (K > 0) {
       sv = saved_of(chunk_saved, l, Tc);
       LaneFwdParams f;
-      set_common(f, p, dp, l, Tc, t0, status);
+      set_common(f, p, dp, l, Tc, t0, st, report, c == n_ck - 1);
       f.r_init = static_cast<const float*>(a.saved) + (size_t)c * p.B * p.N;
       f.Rh = sv.Rh; f.Dh = sv.Dh; f.Sg = sv.Sg;
       const int rc = lane_forward_launch(p.activation, l.NP, l.S, l.units, f, s);
@@ -335,7 +357,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
       sv = saved_of(const_cast<void*>(a.saved), l, p.T);
     }
     LaneBwdParams q;
-    set_common(q, p, dp, l, Tc, t0, status);
+    set_common(q, p, dp, l, Tc, t0, st, report, K == 0);
     q.Rh = sv.Rh; q.Dh = sv.Dh; q.Sg = sv.Sg;
     q.grad_output = a.grad_output;
     q.coef_x = a.coef_x; q.coef_y = a.coef_y; q.coef_s = a.coef_s;
@@ -352,7 +374,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
       RINGRNN_CUDA_TRY(cudaGetLastError());
     }
     const int nsplit = lane_bwd_layout(l, Tc).nsplit;
-    rc = tc_gemm_slabs(DL, sv.Rh, partial, 3 * l.NP, l.NP, Tc, l.BPs, nsplit, status, s);
+    rc = tc_gemm_slabs(DL, sv.Rh, partial, 3 * l.NP, l.NP, Tc, l.BPs, nsplit, st.dev, st.host, s);
     if (rc != RINGRNN_OK) return rc;
     {
       LaunchScope ls(K_REDUCE, s);

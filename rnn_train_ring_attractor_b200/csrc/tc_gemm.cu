@@ -81,7 +81,7 @@ template <bool MN_MAJOR, int NT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                float* __restrict__ out, int M_total, int N_total, long long K_total, long long k_per_split,
-               int chunks_per_slab, int* status) {
+               int chunks_per_slab, int* status, volatile int* host_status) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -93,7 +93,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   volatile uint32_t* tmem_slot_p = reinterpret_cast<volatile uint32_t*>(gen + Cfg::NSTAGE * Cfg::STAGE + 8 * (2 * Cfg::NSTAGE + 1));
   volatile int* dead = reinterpret_cast<volatile int*>(gen + Cfg::NSTAGE * Cfg::STAGE + 8 * (2 * Cfg::NSTAGE + 1) + 4);
-  const WaitCtx wctx{dead, status};
+  const WaitCtx wctx{dead, status, WAIT_LIMIT_CYCLES, nullptr, host_status};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * 128, n0 = blockIdx.y * NT;
@@ -357,7 +357,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int nspl
 
 template <bool MN_MAJOR, int NT>
 int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N_total, long long K_total, int nsplit,
-                int* status, cudaStream_t s, int slabs = 1) {
+                int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -383,7 +383,7 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
   {
     LaunchScope ls(K_DW, s);
     gemm_tc_kernel<MN_MAJOR, NT><<<grid, GEMM_THREADS, Cfg::SMEM, s>>>(tmA, tmB, partial, M_total, N_total, K_total,
-                                                                        kps, chunks_per_slab, status);
+                                                                        kps, chunks_per_slab, status, host_status);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   return RINGRNN_OK;
@@ -421,11 +421,11 @@ int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* o
 
 // partial[split][M][N] = sum over slabs and columns of A[slab][M][cols] * B[slab][N][cols]^T (K-major operands)
 int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, int slabs, int cols, int nsplit, int* status,
-                  cudaStream_t s) {
+                  volatile int* host_status, cudaStream_t s) {
   if (M % 128 != 0 || nsplit < 1) return RINGRNN_ERR_SHAPE;
   const long long K = (long long)slabs * cols;
-  if (N == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, slabs);
-  if (N == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, slabs);
+  if (N == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, slabs, host_status);
+  if (N == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, slabs, host_status);
   return RINGRNN_ERR_SHAPE;
 }
 

@@ -50,7 +50,10 @@ struct LaneFwdParams {
   float* ckpt;           // as in TcFwdParams
   int ckpt_every;
   int t0, T_total;
-  int* status;
+  int* status;            // polled by slow waits
+  int* report;            // the caller's scratch word, or nullptr
+  int zero_report;        // the first kernel of a call clears it
+  volatile int* host;     // pinned host word, or nullptr
 };
 
 struct LaneBwdParams {
@@ -76,7 +79,10 @@ struct LaneBwdParams {
   float* dA_part;             // [CL][2][T][BPs] or nullptr
   const float* carry_in;      // [B,N] or nullptr
   int t0, T_total;
-  int* status;
+  int* status;            // polled by slow waits
+  int* report;            // the caller's scratch word, or nullptr
+  int zero_report;        // the first kernel of a call clears it
+  volatile int* host;     // pinned host word, or nullptr
 };
 
 // samples per unit: 16, 32 or 64 (see lane_unit_samples); units: 1 or 2 per CTA
@@ -147,14 +153,15 @@ struct Ctx {
 
 template <class C>
 __device__ __forceinline__ Ctx<C> setup(uint8_t* smem_raw, int units, const float* dec_u, const float* dec_v, int N,
-                                        int* status) {
+                                        int* status, int* report, int zero_report, volatile int* host) {
   Ctx<C> c;
   c.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   c.gen = smem_raw + (c.base - smem_u32(smem_raw));
   c.bars = c.base + C::OFF_BAR;
   c.rank = C::CL > 1 ? cluster_ctarank() : 0u;
   volatile int* dead = reinterpret_cast<volatile int*>(c.gen + C::OFF_BAR + B_DEAD);
-  c.w = WaitCtx{dead, status};
+  c.w = WaitCtx{dead, status, WAIT_LIMIT_CYCLES, report, host};
+  if (blockIdx.x == 0 && threadIdx.x == 0 && report != nullptr && zero_report) *report = 0;
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     *dead = 0;

@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
   using C = Cfg<NP, S, 1, 5, 2>;
   constexpr int E = C::E;
   extern __shared__ uint8_t smem_raw[];
-  const Ctx<C> c = setup<C>(smem_raw, 1, p.dec_u, p.dec_v, p.N, p.status);
+  const Ctx<C> c = setup<C>(smem_raw, 1, p.dec_u, p.dec_v, p.N, p.status, p.report, p.zero_report, p.host);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = (int)(blockIdx.x / C::CL), stride = (int)(gridDim.x / C::CL);
   const int T = p.T;

@@ -97,24 +97,22 @@ def train_step(step_fn, local_inputs, N, a_dim, global_batch, T, buf=None, group
     if buf is None:
         buf = torch.empty(grad_buffer_numel(N, a_dim), dtype=torch.float32, device=device)
     parts = step_fn(local_inputs, 1.0 / (global_batch * T), buf)
-    buf[-2:].copy_(parts)
+    tail = buf[-2:]
+    if parts.data_ptr() != tail.data_ptr():  # (the fused operator writes them there itself)
+        tail.copy_(parts)
     allreduce_grad_buffer(buf, group, timeout_s)
     out = split_grad_buffer(buf, N, a_dim)
-    loss = out["loss_parts"][0] + bump_weight * out["loss_parts"][1]
+    loss = torch.add(tail[0], tail[1], alpha=bump_weight)
     return loss, out
 
 
 def fused_step_fn(Wa, J0, J1, Wo, alpha, activation, bump_weight=0.2, precision=None, ckpt_every=0):
     """step_fn for :func:`train_step` backed by the fused CUDA operator (`ckpt_every`: see ring_rnn_fused)."""
-    from .fused import ring_rnn_fused
+    from .fused import TrainStep
+
+    step = TrainStep(Wa, J0, J1, Wo, alpha, activation, bump_weight, precision, ckpt_every)
 
     def fn(local_inputs, inv_count, buf):
-        A, r_init, target = local_inputs
-        Wa_ = Wa.detach().requires_grad_(True)
-        Wo_ = Wo.detach().requires_grad_(True)
-        loss, parts, _, _ = ring_rnn_fused(A, Wa_, J0, J1, Wo_, r_init, alpha, activation, target, bump_weight,
-                                           inv_count, precision, buf, ckpt_every)
-        loss.backward()
-        return parts
+        return step(*local_inputs, inv_count, buf)
 
     return fn

@@ -8,12 +8,22 @@ import math
 
 import torch
 
+from . import _lib
 from .fused import ring_rnn_rollout
-from .inputs import av_to_action_signal, generate_av, initial_bump_gaussian
+from .inputs import trials_from_host_draws
+from .ring_rnn_cuda import on_device, stream_of
 
 
 def angular_error(pred, target):
     """Circular |pred - target| in [0, pi] (compare/compare_models_fair.py:15-20)."""
+    if (pred.is_cuda and target.is_cuda and pred.device == target.device and pred.dtype == target.dtype == torch.float32
+            and pred.shape == target.shape and pred.is_contiguous() and target.is_contiguous() and pred.numel() > 0
+            and not (torch.is_grad_enabled() and (pred.requires_grad or target.requires_grad))):
+        out = torch.empty_like(pred)
+        with on_device(pred.device):
+            _lib.check(_lib.lib().ringrnn_angular_error(pred.numel(), pred.data_ptr(), target.data_ptr(), out.data_ptr(),
+                                                        stream_of(pred.device)))
+        return out
     d = torch.abs(pred - target) % (2 * math.pi)
     return torch.minimum(d, 2 * math.pi - d)
 
@@ -21,16 +31,9 @@ def angular_error(pred, target):
 def evaluate_angular_error(Wa, J0, J1, Wo, alpha, activation, n_trials=200, seq_len=500, batch=50, seed=123,
                            max_av=0.1 * math.pi, precision=None):
     """dict(mean, std, max, final_mean, errors[n_trials, seq_len]) in radians for the given weights (device tensors)."""
-    dev = Wo.device
-    N = Wo.shape[0]
     g = torch.Generator().manual_seed(seed)
-    errs = []
-    for _ in range((n_trials + batch - 1) // batch):
-        av, angle = generate_av(batch, seq_len, max_av=max_av, generator=g)
-        A = av_to_action_signal(av, max_av).to(dev)
-        r0 = initial_bump_gaussian(angle[:, 0], N).to(dev)
-        decoded, _ = ring_rnn_rollout(A, Wa, J0, J1, Wo, r0, alpha, activation, precision=precision)
-        errs.append(angular_error(decoded, angle.to(dev)))
-    e = torch.cat(errs, dim=0)[:n_trials]
-    return {"mean": float(e.mean()), "std": float(e.std()), "max": float(e.max()), "final_mean": float(e[:, -1].mean()),
-            "errors": e}
+    x = trials_from_host_draws(n_trials, seq_len, Wo.shape[0], batch, max_av, g, Wo.device)
+    decoded, _ = ring_rnn_rollout(x["A"], Wa, J0, J1, Wo, x["r_init"], alpha, activation, precision=precision)
+    e = angular_error(decoded, x["target"])
+    mean, std, top, final = torch.stack((e.mean(), e.std(), e.max(), e[:, -1].mean())).tolist()
+    return {"mean": mean, "std": std, "max": top, "final_mean": final, "errors": e}

@@ -15,14 +15,14 @@ import torch
 from torch.autograd import Function
 
 from . import _lib
-from .ring_rnn_cuda import _check_tensor, _scalar, _scratch, active_columns, choose_precision, nvtx_range
+from .ring_rnn_cuda import _check_tensor, _scalar, _scratch, active_columns, nvtx_range, on_device, plan, stream_of
 
 _decode_cache = {}
 
 
 def decode_vectors(N, device):
     """u, v [N] fp32 on `device` (computed in float64 once per (N, device))."""
-    key = (N, str(device))
+    key = (N, device)
     if key not in _decode_cache:
         idx = torch.arange(N, dtype=torch.float64)
         W = torch.cos(2 * math.pi * (idx[:, None] - idx[None, :]) / N)
@@ -52,13 +52,13 @@ class RingRnnFusedFunc(Function):
             raise RuntimeError("target_angle must be (batch, seq_len)")
         dev = action_signal.device
         active = list(range(a_dim)) if ctx.needs_input_grad[0] else active_columns(action_signal)
-        prec = choose_precision(B, T, N, a_dim, act, len(active), precision)
+        prec, n_fwd, n_saved, n_bwd = plan(B, T, N, a_dim, act, len(active), precision, 0, int(ckpt_every))
         if inv_count is None:
             inv_count = 1.0 / (B * T)
         u, v = decode_vectors(N, dev)
         L = _lib.lib()
-        with torch.cuda.device(dev), nvtx_range("ringrnn_fused_fwd"):
-            stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with on_device(dev), nvtx_range("ringrnn_fused_fwd"):
+            stream = stream_of(dev)
             p = _lib.make_problem(B, T, N, a_dim, act, prec, _scalar(J0), _scalar(J1), alpha,
                                   action_signal.data_ptr(), Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active,
                                   ckpt_every=ckpt_every)
@@ -66,8 +66,8 @@ class RingRnnFusedFunc(Function):
             decoded = torch.empty(B, T, device=dev, dtype=torch.float32)
             final_state = torch.empty(B, N, device=dev, dtype=torch.float32)
             parts = torch.empty(2, device=dev, dtype=torch.float32)
-            ws = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_FWD, 0), dev)
-            saved = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_SAVED, 0), dev)
+            ws = _scratch(n_fwd, dev)
+            saved = _scratch(n_saved, dev)
             a = _lib.FwdArgs()
             a.p = p
             a.saved, a.saved_bytes = saved.data_ptr(), saved.numel()
@@ -88,6 +88,8 @@ class RingRnnFusedFunc(Function):
         ctx.J0, ctx.J1, ctx.alpha, ctx.act, ctx.active, ctx.prec = J0, J1, alpha, act, active, prec
         ctx.grad_buffer = grad_buffer
         ctx.ckpt_every = ckpt_every
+        ctx.n_bwd = n_bwd
+        ctx.set_materialize_grads(False)  # parts, decoded and final_state have no gradient: no zeros for them
         ctx.mark_non_differentiable(parts, decoded, final_state)
         return loss, parts, decoded, final_state
 
@@ -101,7 +103,9 @@ class RingRnnFusedFunc(Function):
         want_r = ctx.needs_input_grad[5]
         want_a = ctx.needs_input_grad[0]
         L = _lib.lib()
-        with torch.cuda.device(dev), nvtx_range("ringrnn_fused_bwd"):
+        if g_loss is None:
+            return (None,) * 14
+        with on_device(dev), nvtx_range("ringrnn_fused_bwd"):
             p = _lib.make_problem(B, T, N, a_dim, ctx.act, ctx.prec, _scalar(ctx.J0), _scalar(ctx.J1), ctx.alpha,
                                   action_signal.data_ptr(), Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(),
                                   ctx.active, ckpt_every=ctx.ckpt_every)
@@ -117,7 +121,7 @@ class RingRnnFusedFunc(Function):
                 grad_J = torch.empty(2, device=dev, dtype=torch.float32) if want_j else None
             grad_r = torch.empty_like(r_init) if want_r else None
             grad_a = torch.empty_like(action_signal) if want_a else None
-            ws = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_BWD, 0), dev)
+            ws = _scratch(ctx.n_bwd, dev)
             a = _lib.BwdArgs()
             a.p = p
             a.grad_A = None if grad_a is None else grad_a.data_ptr()
@@ -128,7 +132,7 @@ class RingRnnFusedFunc(Function):
             a.grad_J = None if grad_J is None else grad_J.data_ptr()
             a.grad_r_init = None if grad_r is None else grad_r.data_ptr()
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            _lib.check(L.ringrnn_bwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            _lib.check(L.ringrnn_bwd(C.byref(a), stream_of(dev)))
             if ctx.prec == _lib.PREC["bf16"]:
                 _lib.check_device_status(ws, "backward")
             if ctx.grad_buffer is not None:
@@ -173,21 +177,82 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
         _check_tensor(name, t)
     dev = action_signal.device
     active = active_columns(action_signal)
-    prec = choose_precision(B, T, N, a_dim, act, len(active), precision)
+    prec, n_fwd, _, _ = plan(B, T, N, a_dim, act, len(active), precision, 0)
     u, v = decode_vectors(N, dev)
     L = _lib.lib()
-    with torch.cuda.device(dev), torch.no_grad(), nvtx_range("ringrnn_rollout"):
+    with on_device(dev), torch.no_grad(), nvtx_range("ringrnn_rollout"):
         p = _lib.make_problem(B, T, N, a_dim, act, prec, _scalar(J0), _scalar(J1), alpha, action_signal.data_ptr(),
                               Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active)
         xy = torch.empty(2, B, T, device=dev, dtype=torch.float32)
         final_state = torch.empty(B, N, device=dev, dtype=torch.float32)
-        ws = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_FWD, 0), dev)
+        ws = _scratch(n_fwd, dev)
         a = _lib.FwdArgs()
         a.p = p
         a.dec_x, a.dec_y = xy[0].data_ptr(), xy[1].data_ptr()
         a.dec_u, a.dec_v = u.data_ptr(), v.data_ptr()
         a.final_state = final_state.data_ptr()
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        _lib.check(L.ringrnn_fwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
-        decoded = torch.remainder(torch.atan2(xy[1], xy[0]) + 2 * math.pi, 2 * math.pi)
+        stream = stream_of(dev)
+        _lib.check(L.ringrnn_fwd(C.byref(a), stream))
+        decoded = xy[0]  # in place of x
+        _lib.check(L.ringrnn_decode_angles(B * T, xy[0].data_ptr(), xy[1].data_ptr(), decoded.data_ptr(), stream))
     return decoded, final_state
+
+
+class TrainStep:
+    """Loss and weight gradients of one batch in ONE library call (ringrnn_train_step), for callers that need no autograd
+    graph: ``step(A, r_init, target, inv_count, grad_buffer)`` fills ``grad_buffer`` = [dWo | dWa | dJ0 dJ1] and returns the
+    two loss parts -- as the next two elements of the buffer where it is that long (dp.grad_buffer_numel)."""
+
+    def __init__(self, Wa, J0, J1, Wo, alpha, activation, bump_weight=0.2, precision=None, ckpt_every=0):
+        if activation not in _lib.ACT:
+            raise ValueError(f"Invalid activation '{activation}'. Must be one of {list(_lib.ACT.keys())}.")
+        self.Wa, self.Wo = Wa.detach(), Wo.detach()
+        self.J0, self.J1, self.alpha, self.act = J0, J1, alpha, _lib.ACT[activation]
+        self.bump_weight, self.precision, self.ckpt_every = bump_weight, precision, int(ckpt_every)
+        self._bytes = {}
+
+    def __call__(self, A, r_init, target, inv_count, grad_buffer):
+        Wa, Wo = self.Wa, self.Wo
+        B, T, a_dim = A.shape
+        N = Wa.shape[1]
+        for name, t in (("A", A), ("Wa", Wa), ("Wo", Wo), ("r_init", r_init), ("target_angle", target),
+                        ("grad_buffer", grad_buffer)):
+            _check_tensor(name, t)
+        if target.shape != (B, T):
+            raise RuntimeError("target_angle must be (batch, seq_len)")
+        if Wa.shape != (a_dim, N, N) or Wo.shape != (N, N) or r_init.shape != (B, N):
+            raise RuntimeError("shape mismatch between action_signal, Wa, Wo and r_init")
+        n_grad = (1 + a_dim) * N * N
+        if grad_buffer.numel() < n_grad + 2:
+            raise RuntimeError("grad_buffer must hold [dWo | dWa | dJ0 dJ1]")
+        dev = A.device
+        active = active_columns(A)
+        prec = plan(B, T, N, a_dim, self.act, len(active), self.precision, 0, self.ckpt_every)[0]
+        u, v = decode_vectors(N, dev)
+        L = _lib.lib()
+        with on_device(dev), nvtx_range("ringrnn_train_step"):
+            a = _lib.TrainArgs()
+            a.p = _lib.make_problem(B, T, N, a_dim, self.act, prec, _scalar(self.J0), _scalar(self.J1), self.alpha,
+                                    A.data_ptr(), Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active, self.ckpt_every)
+            key = (B, T, N, a_dim, len(active), prec)
+            n_bytes = self._bytes.get(key)
+            if n_bytes is None:
+                n_bytes = L.ringrnn_train_bytes(C.byref(a.p))
+                if len(self._bytes) >= 64:
+                    self._bytes.clear()
+                self._bytes[key] = n_bytes
+            ws = _scratch(n_bytes, dev)
+            parts = grad_buffer[n_grad + 2:n_grad + 4]
+            if parts.numel() < 2:
+                parts = torch.empty(2, device=dev, dtype=torch.float32)
+            g = grad_buffer.data_ptr()
+            a.target, a.bump_weight, a.inv_count = target.data_ptr(), self.bump_weight, inv_count
+            a.dec_u, a.dec_v = u.data_ptr(), v.data_ptr()
+            a.grad_Wo, a.grad_Wa, a.grad_J, a.loss_out = g, g + 4 * N * N, g + 4 * n_grad, parts.data_ptr()
+            a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+            _lib.check(L.ringrnn_train_step(C.byref(a), stream_of(dev)))
+            if _lib.CHECK_DEVICE_STATUS:
+                torch.cuda.synchronize()
+                _lib.raise_if_device_error()
+        return parts

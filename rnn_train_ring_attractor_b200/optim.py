@@ -12,6 +12,7 @@ import ctypes as C
 import torch
 
 from . import _lib
+from .ring_rnn_cuda import on_device, stream_of
 
 
 class FlatRingParams:
@@ -69,8 +70,8 @@ class FusedClipAdam:
         if flat_grads.shape != self.params.shape or flat_grads.dtype != torch.float32 or not flat_grads.is_contiguous():
             raise ValueError("flat_grads must match the parameter buffer (contiguous fp32)")
         self.step_count += 1
-        with torch.cuda.device(self.params.device):
-            stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        with on_device(self.params.device):
+            stream = stream_of(self.params.device)
             _lib.check(_lib.lib().ringrnn_clip_adam(
                 self.params.data_ptr(), flat_grads.data_ptr(), self.exp_avg.data_ptr(), self.exp_avg_sq.data_ptr(),
                 self.n_updated, self.lr, self.betas[0], self.betas[1], self.eps, self.step_count, self.max_norm,

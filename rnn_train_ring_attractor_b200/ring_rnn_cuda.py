@@ -27,21 +27,38 @@ from torch.autograd import Function
 from . import _lib
 
 
-@contextlib.contextmanager
-def nvtx_range(name):
+class nvtx_range:
     """NVTX range around a library call (the reference brackets its fwd/bwd the same way for its profiles,
     legacy/bwd_fp32.py:705-740); a no-op when torch has no CUDA runtime to push to."""
-    pushed = False
-    try:
-        torch.cuda.nvtx.range_push(name)
-        pushed = True
-    except Exception:
-        pass
-    try:
-        yield
-    finally:
-        if pushed:
+    __slots__ = ("name", "pushed")
+
+    def __init__(self, name):
+        self.name, self.pushed = name, False
+
+    def __enter__(self):
+        try:
+            torch.cuda.nvtx.range_push(self.name)
+            self.pushed = True
+        except Exception:
+            pass
+
+    def __exit__(self, *exc):
+        if self.pushed:
             torch.cuda.nvtx.range_pop()
+        return False
+
+
+_same_device = contextlib.nullcontext()
+
+
+def on_device(dev):
+    """torch.cuda.device(dev), or nothing at all when it is the current device already."""
+    return _same_device if dev.index == torch.cuda.current_device() else torch.cuda.device(dev)
+
+
+def stream_of(dev):
+    return C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+
 
 _precision = os.environ.get("RINGRNN_PRECISION", "auto")
 
@@ -94,8 +111,20 @@ def active_columns(action_signal):
     hit = _active_cache.get(key)
     if hit is not None and hit[0]() is action_signal and hit[1] == action_signal._version:
         return hit[2]
-    flags = (action_signal != 0).flatten(0, 1).any(dim=0)
-    cols = torch.nonzero(flags).flatten().tolist()
+    cols = None
+    if action_signal.is_cuda and a_dim <= _lib.MAX_ACTIVE and action_signal.dtype == torch.float32 and action_signal.is_contiguous():
+        mask = C.c_ulonglong(0)
+        dev = action_signal.device
+        with on_device(dev):
+            rc = _lib.lib().ringrnn_active_columns(action_signal.data_ptr(), action_signal.shape[0] * action_signal.shape[1],
+                                                   a_dim, C.byref(mask), stream_of(dev))
+        if rc == 0:
+            cols = [k for k in range(a_dim) if mask.value >> k & 1]
+        elif rc != _lib.ERR_UNSUPPORTED:
+            _lib.check(rc)
+    if cols is None:
+        flags = (action_signal != 0).flatten(0, 1).any(dim=0)
+        cols = torch.nonzero(flags).flatten().tolist()
     if len(cols) > _lib.MAX_ACTIVE:
         cols = list(range(a_dim))
     try:
@@ -104,6 +133,31 @@ def active_columns(action_signal):
     except TypeError:
         pass
     return cols
+
+
+_plans = {}  # (shape, precision asked for, history) -> (precision, forward / saved / backward bytes); sizes only, bounded
+
+
+def plan(B, T, N, a_dim, act_code, n_active, requested, history, ckpt_every=0):
+    """(precision code, forward scratch, saved state, backward scratch in bytes) of a request: the precision resolved as
+    choose_precision does, the sizes as ringrnn_workspace_bytes reports them.  They depend on the shape alone, so a
+    training loop asks the library once."""
+    key = (B, T, N, a_dim, act_code, n_active, requested or _precision, history, ckpt_every)
+    hit = _plans.get(key)
+    if hit is None:
+        prec = choose_precision(B, T, N, a_dim, act_code, n_active, requested)
+        p = _lib.Problem()
+        p.B, p.T, p.N, p.a_dim, p.activation, p.precision = B, T, N, a_dim, act_code, prec
+        p.n_active = n_active if n_active <= _lib.MAX_ACTIVE else -1
+        p.ckpt_every = ckpt_every
+        for k in range(max(p.n_active, 0)):
+            p.active_cols[k] = k
+        L = _lib.lib()
+        sizes = [L.ringrnn_workspace_bytes(C.byref(p), w, history) for w in (_lib.WS_FWD, _lib.WS_SAVED, _lib.WS_BWD)]
+        if len(_plans) >= 256:
+            _plans.clear()
+        hit = _plans[key] = (prec, *sizes)
+    return hit
 
 
 def choose_precision(B, T, N, a_dim, act_code, n_active, requested=None):
@@ -166,20 +220,22 @@ class RingRnnCudaFunc(Function):
         dev = action_signal.device
         # zero columns may be skipped only if nobody asks for the gradient with respect to the action signal
         active = list(range(a_dim)) if ctx.needs_input_grad[0] else active_columns(action_signal)
-        prec = choose_precision(batch_size, seq_len, N, a_dim, act, len(active))
+        prec, n_fwd, n_saved, n_bwd = plan(batch_size, seq_len, N, a_dim, act, len(active), None, 1)
         L = _lib.lib()
-        with torch.cuda.device(dev), nvtx_range("ringrnn_fwd"):
+        with on_device(dev), nvtx_range("ringrnn_fwd"):
             p = _lib.make_problem(batch_size, seq_len, N, a_dim, act, prec, _scalar(J0), _scalar(J1), alpha,
                                   action_signal.data_ptr(), Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active)
             bump_history = torch.empty(seq_len, batch_size, N, device=dev, dtype=action_signal.dtype)
-            ws = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_FWD, 1), dev)
-            saved = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_SAVED, 1), dev)
+            ws = _scratch(n_fwd, dev)
             a = _lib.FwdArgs()
             a.p = p
             a.bump_history = bump_history.data_ptr()
-            a.saved, a.saved_bytes = saved.data_ptr(), saved.numel()
+            saved = None
+            if any(ctx.needs_input_grad):  # nothing is kept for a backward that cannot come
+                saved = _scratch(n_saved, dev)
+                a.saved, a.saved_bytes = saved.data_ptr(), saved.numel()
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            _lib.check(L.ringrnn_fwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            _lib.check(L.ringrnn_fwd(C.byref(a), stream_of(dev)))
             if prec == _lib.PREC["bf16"]:
                 _lib.check_device_status(ws, "forward")
         ctx.save_for_backward(action_signal, Wa, Wo, bump_history, r_init, saved)
@@ -189,6 +245,7 @@ class RingRnnCudaFunc(Function):
         ctx.activation_name = activation_name
         ctx.active = active
         ctx.prec = prec
+        ctx.n_bwd = n_bwd
         return bump_history
 
     @staticmethod
@@ -203,7 +260,7 @@ class RingRnnCudaFunc(Function):
         want_r = ctx.needs_input_grad[5]
         want_a = ctx.needs_input_grad[0]
         L = _lib.lib()
-        with torch.cuda.device(dev), nvtx_range("ringrnn_bwd"):
+        with on_device(dev), nvtx_range("ringrnn_bwd"):
             p = _lib.make_problem(batch_size, seq_len, N, a_dim, act, ctx.prec, _scalar(ctx.J0), _scalar(ctx.J1),
                                   ctx.alpha, action_signal.data_ptr(), Wa.data_ptr(), Wo.data_ptr(),
                                   r_init.data_ptr(), ctx.active)
@@ -212,7 +269,7 @@ class RingRnnCudaFunc(Function):
             grad_J = torch.empty(2, device=dev, dtype=torch.float32) if want_j else None
             grad_r = torch.empty_like(r_init) if want_r else None
             grad_a = torch.empty_like(action_signal) if want_a else None
-            ws = _scratch(L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_BWD, 1), dev)
+            ws = _scratch(ctx.n_bwd, dev)
             a = _lib.BwdArgs()
             a.p = p
             a.grad_A = None if grad_a is None else grad_a.data_ptr()
@@ -223,7 +280,7 @@ class RingRnnCudaFunc(Function):
             a.grad_J = None if grad_J is None else grad_J.data_ptr()
             a.grad_r_init = None if grad_r is None else grad_r.data_ptr()
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-            _lib.check(L.ringrnn_bwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            _lib.check(L.ringrnn_bwd(C.byref(a), stream_of(dev)))
             if ctx.prec == _lib.PREC["bf16"]:
                 _lib.check_device_status(ws, "backward")
         gJ0 = grad_J[0].reshape(ctx.J0.shape) if (torch.is_tensor(ctx.J0) and ctx.J0.requires_grad) else None

@@ -1,0 +1,113 @@
+"""Edges of the kernels whose CTAs own few samples, and of the host-side compositions, on the GPU.
+
+Tolerances: bf16 mode 1e-2 and fp32 mode 1e-4 relative, the bounds of the parity tests (two bf16 roundings of 2^-9 per
+product, fp32 sums over at most a few thousand terms); what two entry points compute with the same kernels must be equal."""
+import math
+import os
+import sys
+
+import pytest
+import torch
+
+sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+from oracle import ring_oracle as orc  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp32": 1e-4, "bf16": 1e-2}
+
+
+def _case(N, B, T, a_dim, seed):
+    g = torch.Generator().manual_seed(seed)
+    s = 1.0 / math.sqrt(N)
+    return (torch.rand(B, T, a_dim, generator=g), torch.randn(a_dim, N, N, generator=g) * s,
+            torch.randn(N, N, generator=g) * s, torch.rand(B, N, generator=g) - 0.5, torch.randn(T, B, N, generator=g))
+
+
+# neurons around the 128-lane and two-CTA limits; batches around 16, 32, 64 samples per unit (148 or 74 units resident) and
+# beyond one round of units; steps around the eight whose scalars are staged at a time; J1 = 0 (no ratio to J1)
+LANE = [(1, 1, 1, 2, "tanh", -0.1, 0.1), (2, 17, 8, 1, "silu", -0.1, 0.1), (127, 16, 9, 2, "gelu", -0.1, 0.1),
+        (128, 2369, 7, 2, "tanh", -0.07, 0.3), (129, 15, 16, 2, "silu", -0.1, 0.1), (255, 1185, 3, 2, "gelu", -0.031, 0.1),
+        (256, 2400, 9, 2, "tanh", -0.05, 0.0), (120, 9500, 2, 2, "silu", 0.0, 0.1), (100, 20001, 3, 2, "tanh", -0.1, 0.1)]
+# fp32 clusters: one CTA, two, four, eight; a last CTA with few neurons; several column counts; no shape that fits
+CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), (97, 9, 4, 2, "gelu", -0.1, 0.1),
+           (200, 300, 3, 2, "tanh", -0.1, 0.1), (257, 70, 3, 1, "silu", -0.05, 0.2), (320, 33, 2, 2, "tanh", -0.04, 0.1)]
+
+
+@pytest.mark.parametrize("prec,shape", [("bf16", s) for s in LANE] + [("fp32", s) for s in CLUSTER],
+                         ids=lambda v: v if isinstance(v, str) else "N%d-B%d-T%d-a%d-%s" % v[:5])
+def test_small_tile_kernels_match_the_oracle(prec, shape):
+    from gpu_helpers import canaries_intact, run_backward, run_forward
+    N, B, T, a_dim, act, J0, J1 = shape
+    A, Wa, Wo, r0, cot = _case(N, B, T, a_dim, N + B)
+    f64 = [x.double() for x in (A, Wa, Wo, r0, cot)]
+    hist = orc.ring_forward_lean(f64[0], f64[1], J0, J1, f64[2], f64[3], 0.1, act)
+    ref = orc.ring_backward_manual(f64[4], f64[0], f64[1], J0, J1, f64[2], hist, f64[3], 0.1, act)
+    dev = [x.cuda() for x in (A, Wa, Wo, r0)]
+    f = run_forward(*dev, J0, J1, 0.1, act, prec, None, history=True, decode=True)
+    b = run_backward(*dev, J0, J1, 0.1, act, f, grad_output=cot.cuda(), prec=prec)
+    assert all(canaries_intact(x) for x in f["backs"] + b["backs"])
+    tol = TOL[prec]
+    assert orc.rel_err(f["hist"], hist) < tol
+    for k, name in (("dWo", "dWo"), ("dWa", "dWa"), ("dr_init", "dr_init"), ("dA", "dA")):
+        assert orc.rel_err(b[k], ref[name]) < tol, k
+    u, v = f["u"].cpu().double(), f["v"].cpu().double()
+    h = f["hist"].cpu().double()  # the decode sums belong to this history: fp32 sums over N terms
+    for k, want in (("x", h @ u), ("y", h @ v), ("ta", h.abs().sum(2))):
+        scale = (h.abs() @ (u.abs() if k == "x" else v.abs() if k == "y" else torch.ones(N, dtype=torch.float64))).T
+        assert float(((f[k].cpu().double() - want.T).abs() / scale.clamp(min=1e-30)).max()) < (N + 8) * 2.0 ** -24, k
+
+
+@pytest.mark.parametrize("a_dim,cols", [(3, [0, 2]), (16, [0, 1]), (16, []), (64, [5, 63]), (7, list(range(7)))])
+def test_active_columns(a_dim, cols):
+    from rnn_train_ring_attractor_b200.ring_rnn_cuda import active_columns
+    A = torch.zeros(37, 61, a_dim, device="cuda")
+    for k in cols:
+        A[(k * 5) % 37, (k * 7) % 61, k] = -1e-30
+    assert active_columns(A) == cols
+
+
+@pytest.mark.parametrize("n,batch,T", [(200, 50, 500), (7, 3, 11), (5, 4, 2)])
+def test_trials_from_host_draws_are_the_host_generators(n, batch, T):
+    from rnn_train_ring_attractor_b200 import inputs
+    x = inputs.trials_from_host_draws(n, T, 120, batch, 0.1 * math.pi, torch.Generator().manual_seed(4), "cuda")
+    g = torch.Generator().manual_seed(4)
+    parts = [inputs.generate_av(batch, T, generator=g) for _ in range((n + batch - 1) // batch)]
+    av, angle = (torch.cat(p)[:n] for p in zip(*parts))
+    assert torch.equal(x["A"].cpu(), inputs.av_to_action_signal(av, 0.1 * math.pi))
+    d = (x["target"].cpu() - angle).abs()
+    assert float(torch.minimum(d, 2 * math.pi - d).max()) < 4e-6  # a few ulp of 2 pi
+    assert orc.rel_err(x["r_init"], inputs.initial_bump_gaussian(angle[:, 0], 120)) < 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 5, 4096, 100003])
+def test_angles_and_errors(n):
+    from rnn_train_ring_attractor_b200 import _lib
+    from rnn_train_ring_attractor_b200.evaluate import angular_error
+    g = torch.Generator().manual_seed(n)
+    x, y = torch.randn(n, generator=g).cuda(), torch.randn(n, generator=g).cuda()
+    out = torch.empty(n, device="cuda")
+    _lib.check(_lib.lib().ringrnn_decode_angles(n, x.data_ptr(), y.data_ptr(), out.data_ptr(), None))
+    want = torch.remainder(torch.atan2(y.double(), x.double()), 2 * math.pi)
+    d = (out.double() - want).abs()
+    assert float(torch.minimum(d, 2 * math.pi - d).max()) < 2e-6 and float(out.min()) >= 0 and float(out.max()) < 2 * math.pi
+    t = (torch.rand(n, generator=g) * 20 - 10).cuda()
+    e = (out.double() - t.double()).abs() % (2 * math.pi)
+    assert float((angular_error(out, t).double() - torch.minimum(e, 2 * math.pi - e)).abs().max()) < 4e-6
+
+
+@pytest.mark.parametrize("N,B,T,prec,ckpt", [(40, 20, 12, None, 0), (200, 33, 9, None, 4), (300, 130, 5, None, 0), (60, 9, 7, "fp32", 0)])
+def test_one_call_training_step_equals_the_autograd_surface(N, B, T, prec, ckpt):
+    from rnn_train_ring_attractor_b200 import dp
+    from rnn_train_ring_attractor_b200.fused import ring_rnn_fused
+    case = orc.make_case(N, B, T, "tanh", seed=2)
+    A, Wa, Wo, r0, tgt = (t.cuda() for t in (case.A, case.Wa, case.Wo, case.r_init, case.target))
+    buf = torch.full((dp.grad_buffer_numel(N, 2),), float("nan"), device="cuda")
+    loss, out = dp.train_step(dp.fused_step_fn(Wa, -0.1, 0.1, Wo, 0.1, "tanh", precision=prec, ckpt_every=ckpt), (A, r0, tgt), N,
+                              2, B, T, buf=buf)
+    want = torch.empty_like(buf)
+    Wa.requires_grad_(True), Wo.requires_grad_(True)
+    l2, parts, _, _ = ring_rnn_fused(A, Wa, -0.1, 0.1, Wo, r0, 0.1, "tanh", tgt, precision=prec, grad_buffer=want,
+                                     ckpt_every=ckpt)
+    l2.backward()
+    assert torch.equal(buf[:-2], want[:-2]) and torch.equal(buf[-2:], parts)
+    assert abs(float(loss) - float(l2)) <= 2.0 ** -22 * abs(float(l2))
