@@ -235,6 +235,7 @@ extern "C" int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, c
   using namespace ringrnn;
   if (n <= 0 || n_all < n || T <= 0 || n0 < 0 || n0 >= T || N <= 0) return RINGRNN_ERR_SHAPE;
   if (!draws || !A || !target || !r_init || !(max_av > 0.f) || !(bump_width > 0.f)) return RINGRNN_ERR_ARG;
+  if ((reinterpret_cast<uintptr_t>(A) & 7) != 0) return RINGRNN_ERR_ARG;  // written two floats at a time
   if (T - n0 > 8192) return RINGRNN_ERR_TOO_LARGE;
   int sort_len = 2;
   while (sort_len < T - n0) sort_len <<= 1;

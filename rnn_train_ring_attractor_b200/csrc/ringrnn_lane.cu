@@ -207,6 +207,11 @@ __global__ void lane_da_kernel(const float* __restrict__ part, int CL, int B, in
   }
 }
 
+bool aligned16(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; }  // (nullptr is)
+
+// A caller's matrix may be a slice of something larger and start at any float.
+void set_weight_loads(LaneFwdParams& q) { q.w_vec = q.N % 4 == 0 && aligned16(q.Wo) && aligned16(q.WL) && aligned16(q.WR); }
+
 template <class P>
 void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneLayout& l, int T, int t0, const DirectStatus& st, int* report, bool first) {
   memset(&q, 0, sizeof(q));
@@ -275,6 +280,7 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
     RINGRNN_CUDA_TRY(cudaMemcpyAsync(a.saved, p.r_init, ckpt_slot(p), cudaMemcpyDeviceToDevice, s));
   LaneFwdParams q;
   set_common(q, p, dp, l, p.T, 0, st, a.status == nullptr ? reinterpret_cast<int*>(w) : nullptr, true);
+  set_weight_loads(q);
   q.r_init = p.r_init;
   if (train && K == 0) {
     const Saved sv = saved_of(a.saved, l, p.T);
@@ -287,6 +293,7 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
     q.dec[0][k] = dec[k];
     if (l.CL > 1 && dec[k] != nullptr) q.dec[1][k] = dec1 + (size_t)k * p.B * p.T;
   }
+  q.dec_vec = p.T % 4 == 0 && aligned16(a.dec_x) && aligned16(a.dec_y) && aligned16(a.dec_ta) && aligned16(dec1);
   q.dec_u = a.dec_u; q.dec_v = a.dec_v;
   q.final_state = a.final_state;
   q.ckpt = K > 0 ? static_cast<float*>(a.saved) : nullptr;
@@ -349,6 +356,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
       sv = saved_of(chunk_saved, l, Tc);
       LaneFwdParams f;
       set_common(f, p, dp, l, Tc, t0, st, report, c == n_ck - 1);
+      set_weight_loads(f);
       f.r_init = static_cast<const float*>(a.saved) + (size_t)c * p.B * p.N;
       f.Rh = sv.Rh; f.Dh = sv.Dh; f.Sg = sv.Sg;
       const int rc = lane_forward_launch(p.activation, l.NP, l.S, l.units, f, s);

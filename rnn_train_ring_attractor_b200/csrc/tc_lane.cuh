@@ -37,6 +37,8 @@ struct LaneFwdParams {
   const float* Wo;       // [N,N]
   const float* WL;       // [N,N] or nullptr
   const float* WR;
+  int w_vec;             // 16-byte loads of matrix rows are aligned (N a multiple of four and every matrix so aligned)
+  int dec_vec;           // likewise 16-byte stores of four steps' decode sums
   const float* A;        // [B,T_total,a_dim]
   const float* r_init;   // [B,N]
   __nv_bfloat16* Rh;     // [T+1][NP][BPs] (slot 0 = r_init) or nullptr
@@ -209,8 +211,8 @@ __device__ __forceinline__ void teardown(const Ctx<C>& c) {
 // from the caller's fp32 tensors.  Forward: row n of the operand is row n of W (a thread reads along its row, four columns
 // at a time); reverse: column n of W (consecutive lanes read consecutive columns).
 template <class C, int NP, bool TRANSPOSED>
-__device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const* W, int N, const float* cterm, int n, int row,
-                                             int h, uint32_t lane_base) {
+__device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const* W, int N, bool vec, const float* cterm, int n,
+                                             int row, int h, uint32_t lane_base) {
   for (int m = 0; m < 3; ++m) {
     const float* w = W[m];
     const bool live = w != nullptr && n < N;
@@ -220,7 +222,7 @@ __device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const
       if (TRANSPOSED) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = (live && k0 + i < N) ? __ldg(w + (size_t)(k0 + i) * N + n) : 0.f;
-      } else if ((N & 3) == 0) {
+      } else if (vec) {
 #pragma unroll
         for (int i = 0; i < 16; i += 4) {
           float4 f = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
 
   if (epi) {
     const float* const W[3] = {p.use_wo ? p.Wo : nullptr, p.WL, p.WR};
-    load_weights<C, NP, true>(c, W, p.N, p.cterm, n, row, h, lane_base);
+    load_weights<C, NP, true>(c, W, p.N, false, p.cterm, n, row, h, lane_base);
   }
   tcgen05_fence_before();
   __syncthreads();

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
 
   if (epi && u == 0) {
     const float* const W[3] = {p.use_wo ? p.Wo : nullptr, p.WL, p.WR};
-    load_weights<C, NP, false>(c, W, p.N, p.cterm, n, row, h, lane_base);
+    load_weights<C, NP, false>(c, W, p.N, p.w_vec != 0, p.cterm, n, row, h, lane_base);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
               if (b < p.B && o != nullptr) {
                 o += (size_t)b * T + (t - 8);
                 const float4 x = lds4(src + i * 8), y = lds4(src + i * 8 + 4);
-                if ((T & 3) == 0) {
+                if (p.dec_vec) {
                   reinterpret_cast<float4*>(o)[0] = x;
                   reinterpret_cast<float4*>(o)[1] = y;
                 } else {

@@ -96,10 +96,12 @@ def train_step(step_fn, local_inputs, N, a_dim, global_batch, T, buf=None, group
     device = local_inputs[0].device
     if buf is None:
         buf = torch.empty(grad_buffer_numel(N, a_dim), dtype=torch.float32, device=device)
-    parts = step_fn(local_inputs, 1.0 / (global_batch * T), buf)
     tail = buf[-2:]
-    if parts.data_ptr() != tail.data_ptr():  # (the fused operator writes them there itself)
-        tail.copy_(parts)
+    write = getattr(step_fn, "write", None)
+    if write is not None:  # the fused operator puts the loss parts behind the gradients itself
+        write(local_inputs, 1.0 / (global_batch * T), buf)
+    else:
+        tail.copy_(step_fn(local_inputs, 1.0 / (global_batch * T), buf))
     allreduce_grad_buffer(buf, group, timeout_s)
     out = split_grad_buffer(buf, N, a_dim)
     loss = torch.add(tail[0], tail[1], alpha=bump_weight)
@@ -110,9 +112,4 @@ def fused_step_fn(Wa, J0, J1, Wo, alpha, activation, bump_weight=0.2, precision=
     """step_fn for :func:`train_step` backed by the fused CUDA operator (`ckpt_every`: see ring_rnn_fused)."""
     from .fused import TrainStep
 
-    step = TrainStep(Wa, J0, J1, Wo, alpha, activation, bump_weight, precision, ckpt_every)
-
-    def fn(local_inputs, inv_count, buf):
-        return step(*local_inputs, inv_count, buf)
-
-    return fn
+    return TrainStep(Wa, J0, J1, Wo, alpha, activation, bump_weight, precision, ckpt_every)

@@ -7,6 +7,7 @@ four statistics the script prints (mean, std, max, mean error at the final step)
 import math
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from .fused import ring_rnn_rollout
@@ -14,11 +15,18 @@ from .inputs import trials_from_host_draws
 from .ring_rnn_cuda import on_device, stream_of
 
 
+def _plain(t):
+    """An ordinary contiguous fp32 CUDA tensor that nothing differentiates, batches or traces."""
+    return (type(t) is torch.Tensor and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()
+            and not (t.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(t))
+
+
 def angular_error(pred, target):
     """Circular |pred - target| in [0, pi] (compare/compare_models_fair.py:15-20)."""
-    if (pred.is_cuda and target.is_cuda and pred.device == target.device and pred.dtype == target.dtype == torch.float32
-            and pred.shape == target.shape and pred.is_contiguous() and target.is_contiguous() and pred.numel() > 0
-            and not (torch.is_grad_enabled() and (pred.requires_grad or target.requires_grad))):
+    # one kernel instead of five passes over the tensors: 65536 x 4000 angles in 0.5 instead of 2 ms
+    if (_plain(pred) and _plain(target) and pred.device == target.device and pred.shape == target.shape and pred.numel() > 0
+            and forward_ad._current_level < 0 and torch._C._len_torch_dispatch_stack() == 0 and not torch.compiler.is_compiling()
+            and not torch.jit.is_tracing()):
         out = torch.empty_like(pred)
         with on_device(pred.device):
             _lib.check(_lib.lib().ringrnn_angular_error(pred.numel(), pred.data_ptr(), target.data_ptr(), out.data_ptr(),

@@ -201,21 +201,32 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
 
 class TrainStep:
     """Loss and weight gradients of one batch in ONE library call (ringrnn_train_step), for callers that need no autograd
-    graph: ``step(A, r_init, target, inv_count, grad_buffer)`` fills ``grad_buffer`` = [dWo | dWa | dJ0 dJ1] and returns the
-    two loss parts -- as the next two elements of the buffer where it is that long (dp.grad_buffer_numel)."""
+    graph: ``step((A, r_init, target), inv_count, grad_buffer)`` fills ``grad_buffer`` = [dWo | dWa | dJ0 dJ1] (None: a
+    buffer of its own) and returns the two loss parts, a tensor of their own.  ``write`` is the same with the parts as the
+    next two elements of the buffer (dp.grad_buffer_numel), for a caller that wants them there."""
 
     def __init__(self, Wa, J0, J1, Wo, alpha, activation, bump_weight=0.2, precision=None, ckpt_every=0):
         if activation not in _lib.ACT:
             raise ValueError(f"Invalid activation '{activation}'. Must be one of {list(_lib.ACT.keys())}.")
-        self.Wa, self.Wo = Wa.detach(), Wo.detach()
+        self.Wa, self.Wo = Wa, Wo
         self.J0, self.J1, self.alpha, self.act = J0, J1, alpha, _lib.ACT[activation]
         self.bump_weight, self.precision, self.ckpt_every = bump_weight, precision, int(ckpt_every)
         self._bytes = {}
 
-    def __call__(self, A, r_init, target, inv_count, grad_buffer):
+    def __call__(self, local_inputs, inv_count, grad_buffer):
+        return self._step(local_inputs, inv_count, grad_buffer, False)
+
+    def write(self, local_inputs, inv_count, grad_buffer):
+        return self._step(local_inputs, inv_count, grad_buffer, True)
+
+    def _step(self, local_inputs, inv_count, grad_buffer, parts_in_buffer):
+        A, r_init, target = local_inputs
         Wa, Wo = self.Wa, self.Wo
         B, T, a_dim = A.shape
         N = Wa.shape[1]
+        n_grad = (1 + a_dim) * N * N
+        if grad_buffer is None:
+            grad_buffer = torch.empty(n_grad + 2, device=A.device, dtype=torch.float32)
         for name, t in (("A", A), ("Wa", Wa), ("Wo", Wo), ("r_init", r_init), ("target_angle", target),
                         ("grad_buffer", grad_buffer)):
             _check_tensor(name, t)
@@ -223,8 +234,7 @@ class TrainStep:
             raise RuntimeError("target_angle must be (batch, seq_len)")
         if Wa.shape != (a_dim, N, N) or Wo.shape != (N, N) or r_init.shape != (B, N):
             raise RuntimeError("shape mismatch between action_signal, Wa, Wo and r_init")
-        n_grad = (1 + a_dim) * N * N
-        if grad_buffer.numel() < n_grad + 2:
+        if grad_buffer.numel() < n_grad + (4 if parts_in_buffer else 2):
             raise RuntimeError("grad_buffer must hold [dWo | dWa | dJ0 dJ1]")
         dev = A.device
         active = active_columns(A)
@@ -243,8 +253,9 @@ class TrainStep:
                     self._bytes.clear()
                 self._bytes[key] = n_bytes
             ws = _scratch(n_bytes, dev)
-            parts = grad_buffer[n_grad + 2:n_grad + 4]
-            if parts.numel() < 2:
+            if parts_in_buffer:
+                parts = grad_buffer[n_grad + 2:n_grad + 4]
+            else:
                 parts = torch.empty(2, device=dev, dtype=torch.float32)
             g = grad_buffer.data_ptr()
             a.target, a.bump_weight, a.inv_count = target.data_ptr(), self.bump_weight, inv_count

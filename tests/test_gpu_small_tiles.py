@@ -111,3 +111,54 @@ def test_one_call_training_step_equals_the_autograd_surface(N, B, T, prec, ckpt)
     l2.backward()
     assert torch.equal(buf[:-2], want[:-2]) and torch.equal(buf[-2:], parts)
     assert abs(float(loss) - float(l2)) <= 2.0 ** -22 * abs(float(l2))
+
+
+@pytest.mark.parametrize("N,T", [(64, 8), (200, 12)])
+@pytest.mark.parametrize("prec", ["fp32", "bf16"])
+def test_weights_may_start_at_any_float(N, T, prec):
+    from rnn_train_ring_attractor_b200.fused import ring_rnn_fused
+    case = orc.make_case(N, 20, T, "tanh", seed=4)
+    A, Wa, Wo, r0, tgt = (t.cuda() for t in (case.A, case.Wa, case.Wo, case.r_init, case.target))
+
+    def shifted(t):
+        room = torch.empty(t.numel() + 1, device="cuda")
+        return room[1:].view(t.shape).copy_(t)
+
+    def grads(Wa, Wo):
+        Wa, Wo = Wa.detach().requires_grad_(True), Wo.detach().requires_grad_(True)
+        loss, _, decoded, _ = ring_rnn_fused(A, Wa, -0.1, 0.1, Wo, r0, 0.1, "tanh", tgt, precision=prec)
+        loss.backward()
+        return loss.detach(), decoded, Wa.grad, Wo.grad
+
+    for a, b in zip(grads(Wa, Wo), grads(shifted(Wa), shifted(Wo))):
+        assert torch.equal(a, b)
+
+
+def test_step_function_called_directly():
+    """Loss parts are the caller's to keep, the buffer may be left out, and weights are looked up at each call."""
+    from rnn_train_ring_attractor_b200 import dp
+    case = orc.make_case(40, 20, 6, "tanh", seed=5)
+    A, Wa, Wo, r0, tgt = (t.cuda() for t in (case.A, case.Wa, case.Wo, case.r_init, case.target))
+    Wo = torch.nn.Parameter(Wo)
+    step = dp.fused_step_fn(Wa, -0.1, 0.1, Wo, 0.1, "tanh")
+    buf = torch.zeros(dp.grad_buffer_numel(40, 2), device="cuda")
+    first = step((A, r0, tgt), 1.0 / 120, buf)
+    kept = first.clone()
+    buf.zero_()
+    assert torch.equal(first, kept) and torch.equal(step((A, r0, tgt), 1.0 / 120, None), kept)
+    Wo.data = Wo.data * 3.0
+    changed = step((A, r0, tgt), 1.0 / 120, buf)
+    assert torch.equal(dp.fused_step_fn(Wa, -0.1, 0.1, Wo.detach(), 0.1, "tanh")((A, r0, tgt), 1.0 / 120, buf), changed)
+    assert not torch.equal(changed, kept)
+
+
+def test_angular_error_transforms():
+    from torch.autograd import forward_ad
+    from rnn_train_ring_attractor_b200.evaluate import angular_error
+    p, t = torch.tensor([0.5, 3.0], device="cuda"), torch.tensor([[0.25, 6.0], [1.0, 1.0]], device="cuda")
+    want = torch.stack([angular_error(p, row) for row in t])
+    assert torch.allclose(torch.vmap(angular_error, in_dims=(None, 0))(p, t), want, atol=4e-6)
+    with forward_ad.dual_level():
+        out = forward_ad.unpack_dual(angular_error(forward_ad.make_dual(p, torch.ones_like(p)), t[0]))
+        assert out.tangent is not None and torch.equal(out.tangent.cpu(), torch.tensor([1.0, -1.0]))
+    assert torch.equal(torch.func.grad(lambda x: angular_error(x, t[0]).sum())(p).cpu(), torch.tensor([1.0, -1.0]))
