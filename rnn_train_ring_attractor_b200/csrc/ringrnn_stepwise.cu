@@ -7,15 +7,19 @@
 // cpp/kernels/bwd_mixed_precision_aggressive.cuh:564-671), without materialising W_eff[B,N,N].
 //
 // With m = 0 for Wo and m = 1..n for the active action matrices (coefficient c_0 = 1 -- J1 is folded into the
-// stacked weights -- and c_m = A[b,t,cols[m-1]]):
-//   forward   X_t[b, m*NP + j] = c_m r_{t-1}[b,j]  (bf16)      re_t = X_t . Wst^T + J0 sum_j r_{t-1}[b,j]
-//             Wst[i, m*NP + j] = W_m[i,j]                       (one GEMM [BP,(1+n)NP] x [(1+n)NP,NP] per step)
-//   backward  Z_t = delta_t . WstT^T,  WstT[m*NP + j, i] = W_m[i,j]   ([BP,NP] x [NP,(1+n)NP] per step)
+// stacked weights -- and c_m = A[b,t,cols[m-1]]), both directions form all products of a step with one GEMM and mix them
+// in fp32 in the row kernel:
+//   forward   Z_t = r_{t-1} . Wf^T,  Wf[m*NP + i, j] = W_m[i,j]     ([BP,NP] x [NP,(1+n)NP] per step)
+//             re_t[b,i] = J0 sum_j r_{t-1}[b,j] + sum_m c_m Z_t[b, m*NP + i]
+//   backward  Z_t = delta_t . Wt^T,  Wt[m*NP + j, i] = W_m[i,j]
 //             carry[b,j] = (1-alpha) g_t[b,j] + J0 sum_i delta_t[b,i] + sum_m c_m Z_t[b, m*NP + j]
 //             dL/dA[b,t,cols[k]] = sum_j r_{t-1}[b,j] Z_t[b,(1+k)*NP + j]
-//   weights   dWst = sum_t delta_t^T X_t: one split-K GEMM over all (t, b) at the end.
+//   weights   dWst = sum_t delta_t^T X_t, X_t[b, m*NP + j] = c_m r_{t-1}[b,j]: one split-K GEMM over all (t, b) at the end.
 // Between the GEMMs a row kernel (one block per sample) applies the epilogue of one step and prepares the operand
 // of the next, so a step costs two launches.  Split-K partial sums are reduced in fixed order: bit-reproducible.
+//
+// Forward, large batches (the [BP,NP] output alone fills the machine): re_t = X_t . Wst^T with the scaled copies of the state
+// as one long operand, because Z would be (1+n) times the output.
 #include <string.h>
 
 #include "ringrnn_common.cuh"
@@ -24,7 +28,7 @@ namespace ringrnn {
 
 namespace {
 
-constexpr int ROW_THREADS = 256;
+constexpr int ROW_MAX = 512;  // threads of a row kernel: four neurons each, several rounds beyond 2048
 
 struct SwCols {
   int n;
@@ -34,7 +38,9 @@ struct SwCols {
 struct SwLayout {
   int NP, BP, n_act, blocks;  // blocks = 1 + n_act column blocks of NP
   long long KX;               // (1 + n_act) * NP
-  int ns_fwd, ns_bwd, ns_dw;  // split-K factors of the three GEMMs
+  bool concat;                // forward: one long operand X instead of all products Z
+  int nt_z, ns_z;             // tile width and split-K factor of the Z GEMM
+  int ns_dw;                  // split-K factor of the weight-gradient GEMM
 };
 
 int sw_active(const RingRnnProblem& p) { return p.n_active < 0 ? p.a_dim : p.n_active; }
@@ -45,6 +51,26 @@ int splits_for(long long tiles, long long K) {
   return (int)(ns < 1 ? 1 : ns);
 }
 
+// Tile width and K splits of the Z GEMM by estimated cycles: waves of 148 CTAs x (start-up + operand bytes at the 50 B/clk
+// that enter an SM + the tile's way out at about 24 B/clk), plus the partial sums written and read back at 2.5 KB/clk.
+void z_shape(int BP, long long KX, int K, int* nt_out, int* ns_out) {
+  double best = 1e300;
+  for (int nt = 512; nt >= 128; nt /= 2) {
+    if (KX % nt != 0) continue;
+    for (int ns = 1; ns <= 8 && K / ns >= 128; ++ns) {
+      const double ctas = (double)(BP / 128) * (KX / nt) * ns;
+      const long long chunks = (K / 64 + ns - 1) / ns;
+      const double waves = (double)(((long long)ctas + 147) / 148);
+      const double cost = waves * (1500 + chunks * (128.0 + nt) * 128 / 50 + nt * 512.0 / 24) + 8.0 * ns * BP * KX / 2500;
+      if (cost < best) {
+        best = cost;
+        *nt_out = nt;
+        *ns_out = ns;
+      }
+    }
+  }
+}
+
 SwLayout sw_layout(const RingRnnProblem& p) {
   SwLayout l;
   l.NP = (p.N + 127) / 128 * 128;
@@ -53,16 +79,49 @@ SwLayout sw_layout(const RingRnnProblem& p) {
   l.blocks = 1 + l.n_act;
   l.KX = (long long)l.blocks * l.NP;
   const int nt_fwd = (l.NP % 512 == 0) ? 512 : (l.NP % 256 == 0) ? 256 : 128;
-  l.ns_fwd = splits_for((long long)(l.BP / 128) * (l.NP / nt_fwd), l.KX);
-  const int nt_bwd = (l.KX % 512 == 0) ? 512 : (l.KX % 256 == 0) ? 256 : 128;
-  l.ns_bwd = splits_for((long long)(l.BP / 128) * (l.KX / nt_bwd), l.NP);
-  l.ns_dw = splits_for((long long)(l.NP / 128) * (l.KX / nt_bwd), (long long)p.T * l.BP);
+  l.concat = splits_for((long long)(l.BP / 128) * (l.NP / nt_fwd), l.KX) == 1;
+  z_shape(l.BP, l.KX, l.NP, &l.nt_z, &l.ns_z);
+  const int nt_dw = (l.KX % 512 == 0) ? 512 : (l.KX % 256 == 0) ? 256 : 128;
+  l.ns_dw = splits_for((long long)(l.NP / 128) * (l.KX / nt_dw), (long long)p.T * l.BP);
   return l;
 }
 
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+int row_threads(int NP) { return NP / 4 < ROW_MAX ? NP / 4 : ROW_MAX; }  // NP is a multiple of 128
 
-// block-wide sum (blockDim.x == ROW_THREADS); every thread gets the result
+// four consecutive elements
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ uint2 to_bf16x4(float4 v) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+__device__ __forceinline__ float4 of_bf16x4(uint2 v) {
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                     __uint_as_float(v.y & 0xffff0000u));
+}
+// elements i .. i+3 of a caller's row of N: single floats where the row ends or starts off a 16-byte boundary
+__device__ __forceinline__ float4 row_ld(const float* row, int i, int N, bool vec) {
+  if (vec && i + 3 < N) return __ldg(reinterpret_cast<const float4*>(row + i));
+  return make_float4(i < N ? __ldg(row + i) : 0.f, i + 1 < N ? __ldg(row + i + 1) : 0.f, i + 2 < N ? __ldg(row + i + 2) : 0.f,
+                     i + 3 < N ? __ldg(row + i + 3) : 0.f);
+}
+__device__ __forceinline__ void row_st(float* row, int i, int N, bool vec, float4 v) {
+  if (vec && i + 3 < N) {
+    st4(row + i, v);
+  } else {
+    if (i < N) row[i] = v.x;
+    if (i + 1 < N) row[i + 1] = v.y;
+    if (i + 2 < N) row[i + 2] = v.z;
+    if (i + 3 < N) row[i + 3] = v.w;
+  }
+}
+__device__ __forceinline__ float4 fma4(float c, float4 x, float4 y) {
+  return make_float4(fmaf(c, x.x, y.x), fmaf(c, x.y, y.y), fmaf(c, x.z, y.z), fmaf(c, x.w, y.w));
+}
+__device__ __forceinline__ float sum4(float4 v) { return (v.x + v.y) + (v.z + v.w); }
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return fmaf(a.x, b.x, a.y * b.y) + fmaf(a.z, b.z, a.w * b.w); }
+
+// block-wide sum; every thread gets the result
 __device__ __forceinline__ float block_sum(float v, float* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -70,39 +129,59 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   float tot = 0.f;
-#pragma unroll
-  for (int w = 0; w < ROW_THREADS / 32; ++w) tot += red[w];
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += red[w];
   return tot;
 }
 
-// Wst [NP][KX] and WstT [KX][NP] (bf16, zero padded); block 0 carries J1.  grid (NP, blocks), block 256
-__global__ void sw_prep_weights_kernel(const float* __restrict__ Wo, const float* __restrict__ Wa, SwCols cols, float J1,
-                                       int N, int NP, long long KX, __nv_bfloat16* __restrict__ Wst,
-                                       __nv_bfloat16* __restrict__ WstT) {
-  const int i = blockIdx.x, m = blockIdx.y;
+// bf16 copy of the matrices, zero padded, block 0 scaled by J1: element (i, j) of block m at i*ld_i + m*ld_m + j.
+// grid (x, blocks), block 256.  Streams 4 bytes in and 2 out per element; 17 matrices of 2048^2: 427 MB.
+__global__ void __launch_bounds__(256) sw_prep_weights_kernel(const float* __restrict__ Wo, const float* __restrict__ Wa,
+                                                              SwCols cols, float J1, int N, int NP, long long ld_i,
+                                                              long long ld_m, bool vec, __nv_bfloat16* __restrict__ out) {
+  const int m = blockIdx.y;
   const float* W = (m == 0) ? Wo : Wa + (size_t)cols.c[m - 1] * N * N;
   const float scale = (m == 0) ? J1 : 1.f;
-  for (int j = threadIdx.x; j < NP; j += blockDim.x) {
-    const float v = (i < N && j < N) ? scale * W[(size_t)i * N + j] : 0.f;
-    if (Wst != nullptr) Wst[(size_t)i * KX + (size_t)m * NP + j] = __float2bfloat16(v);
-    // WstT row (m, j) holds W_m[:, j]: written from the same thread's transposed element for coalescing
-    if (WstT != nullptr) {
-      const float vt = (i < N && j < N) ? scale * W[(size_t)j * N + i] : 0.f;  // W_m[j, i] -> WstT[(m, i), j]
-      WstT[((size_t)m * NP + i) * NP + j] = __float2bfloat16(vt);
-    }
+  const int quads = NP / 4, total = NP * quads, stride = gridDim.x * 256;
+#pragma unroll 4
+  for (int e = blockIdx.x * 256 + threadIdx.x; e < total; e += stride) {
+    const int i = e / quads, j = (e - i * quads) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < N) v = row_ld(W + (size_t)i * N, j, N, vec);
+    v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+    *reinterpret_cast<uint2*>(out + i * ld_i + m * ld_m + j) = to_bf16x4(v);
   }
+}
+
+// The transposed copy for reverse time, out[m*NP + j][i] = W_m[i][j], by tiles of 32 x 32.  grid (NP/32, NP/32, blocks), block 256
+__global__ void __launch_bounds__(256) sw_prep_transposed_kernel(const float* __restrict__ Wo, const float* __restrict__ Wa,
+                                                                 SwCols cols, float J1, int N, int NP,
+                                                                 __nv_bfloat16* __restrict__ out) {
+  __shared__ float tile[32][33];
+  const int m = blockIdx.z, j0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
+  const float* W = (m == 0) ? Wo : Wa + (size_t)cols.c[m - 1] * N * N;
+  const float scale = (m == 0) ? J1 : 1.f;
+  const int c = threadIdx.x & 31;
+#pragma unroll
+  for (int r = threadIdx.x >> 5; r < 32; r += 8)
+    tile[r][c] = (i0 + r < N && j0 + c < N) ? scale * __ldg(W + (size_t)(i0 + r) * N + j0 + c) : 0.f;
+  __syncthreads();
+  const int j = threadIdx.x >> 3, i = (threadIdx.x & 7) * 4;
+  *reinterpret_cast<uint2*>(out + ((size_t)m * NP + j0 + j) * NP + i0 + i) =
+      to_bf16x4(make_float4(tile[i][j], tile[i + 1][j], tile[i + 2][j], tile[i + 3][j]));
 }
 
 struct SwFwd {
   int B, T, N, NP, BP, a_dim, nsplit;
   long long KX;
+  bool concat;             // partial [nsplit = 1][BP][NP] and X; otherwise Z [nsplit][BP][KX]
+  bool vec;                // the caller's rows of N floats start on 16-byte boundaries
   float J0, alpha;
   const float* A;
   const float* r_init;
-  const float* partial;    // [nsplit][BP][NP]
+  const float* partial;
   float* state;            // [BP][NP] fp32 master state
   float* rowsum;           // [BP]
-  __nv_bfloat16* X;        // [BP][KX]
+  __nv_bfloat16* X;        // [BP][KX] (concat) or [BP][NP] or nullptr: the operand of the next step, unless Rh is it
   __nv_bfloat16* Rh;       // [T+1][BP][NP] or nullptr
   __nv_bfloat16* Dh;       // [T][BP][NP] or nullptr
   float* hist;             // [T,B,N] or nullptr
@@ -115,58 +194,84 @@ struct SwFwd {
   SwCols cols;
 };
 
-// One block per padded sample row.  t >= 0: finishes step t (r_t from the GEMM of step t), then builds the operand
-// of step t+1.  t = -1: loads r_init and builds the operand of step 0.
+// One block per padded sample row, four neurons per thread.  t >= 0: finishes step t (r_t from the GEMM of step t), then
+// builds the operand of step t+1.  t = -1: loads r_init and builds the operand of step 0.  Bound by the latency of its
+// loads: all of a thread's products of a step are in flight together.
 template <int ACT>
-__global__ void sw_forward_row_kernel(SwFwd q, int t) {
-  __shared__ float red[ROW_THREADS / 32];
-  const int b = blockIdx.x;
+__global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t) {
+  __shared__ float red[ROW_MAX / 32];
+  __shared__ float coef[1 + RINGRNN_MAX_ACTIVE];  // of step t (products) or, concat, of step t+1 (operand)
+  const int b = blockIdx.x, n = q.cols.n;
   const bool valid = b < q.B;
   float* st = q.state + (size_t)b * q.NP;
   float px = 0.f, py = 0.f, pa = 0.f, rs = 0.f;
   const float s_prev = (t >= 0) ? q.rowsum[b] : 0.f;
   const bool build = t + 1 < q.T;
-  const float* a_next = q.A + ((size_t)b * q.T + (t + 1)) * q.a_dim;  // read only when valid && build
-  __nv_bfloat16* xrow = q.X + (size_t)b * q.KX;
-  for (int i = threadIdx.x; i < q.NP; i += ROW_THREADS) {
-    float r = 0.f;
-    if (valid && i < q.N) {
-      if (t < 0) {
-        r = q.r_init[(size_t)b * q.N + i];
-      } else {
-        float re = q.J0 * s_prev;
-        for (int s = 0; s < q.nsplit; ++s) re += q.partial[((size_t)s * q.BP + b) * q.NP + i];
-        r = fmaf(q.alpha, act_fn<ACT>(re), (1.f - q.alpha) * st[i]);
-        if (q.Dh != nullptr) q.Dh[((size_t)t * q.BP + b) * q.NP + i] = __float2bfloat16(act_grad<ACT>(re));
-        if (q.hist != nullptr) q.hist[((size_t)t * q.B + b) * q.N + i] = r;
-        if (q.final_state != nullptr && t + 1 == q.T) q.final_state[(size_t)b * q.N + i] = r;
-        if (q.dec_x != nullptr || q.dec_y != nullptr) {
-          px = fmaf(r, q.dec_u[i], px);
-          py = fmaf(r, q.dec_v[i], py);
+  const int t_c = q.concat ? t + 1 : t;
+  for (int k = threadIdx.x; k <= n; k += blockDim.x)
+    coef[k] = k == 0 ? 1.f : (valid && t_c >= 0 && t_c < q.T) ? __ldg(q.A + ((size_t)b * q.T + t_c) * q.a_dim + q.cols.c[k - 1]) : 0.f;
+  __syncthreads();
+  const int blocks = q.concat ? 1 : 1 + n;
+  const size_t ld = q.concat ? q.NP : q.KX;
+  const bool dec = q.dec_x != nullptr || q.dec_y != nullptr;
+  for (int i = threadIdx.x * 4; i < q.NP; i += blockDim.x * 4) {
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+    if (t < 0) {
+      if (valid) {
+        const float4 r0 = row_ld(q.r_init + (size_t)b * q.N, i, q.N, q.vec);
+        r[0] = r0.x; r[1] = r0.y; r[2] = r0.z; r[3] = r0.w;
+      }
+    } else {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      if (valid) {
+        float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s = 0; s < q.nsplit; ++s) {
+          const float* src = q.partial + ((size_t)s * q.BP + b) * ld + i;
+#pragma unroll 8
+          for (int m = 0; m < blocks; ++m) z = fma4(coef[m], ld4(src + (size_t)m * q.NP), z);
         }
-        pa += fabsf(r);
+        const float zz[4] = {z.x, z.y, z.z, z.w};
+        const float4 old4 = ld4(st + i);
+        const float old[4] = {old4.x, old4.y, old4.z, old4.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (i + x < q.N) {
+            const float re = fmaf(q.J0, s_prev, zz[x]);
+            r[x] = fmaf(q.alpha, act_fn<ACT>(re), (1.f - q.alpha) * old[x]);
+            if (q.Dh != nullptr) d[x] = act_grad<ACT>(re);
+            if (dec) {
+              px = fmaf(r[x], q.dec_u[i + x], px);
+              py = fmaf(r[x], q.dec_v[i + x], py);
+            }
+            pa += fabsf(r[x]);
+          }
+        const float4 r4 = make_float4(r[0], r[1], r[2], r[3]);
+        if (q.hist != nullptr) row_st(q.hist + ((size_t)t * q.B + b) * q.N, i, q.N, q.vec, r4);
+        if (q.final_state != nullptr && t + 1 == q.T) row_st(q.final_state + (size_t)b * q.N, i, q.N, q.vec, r4);
       }
-    } else if (t >= 0 && q.Dh != nullptr) {
-      q.Dh[((size_t)t * q.BP + b) * q.NP + i] = __float2bfloat16(0.f);
+      if (q.Dh != nullptr)
+        *reinterpret_cast<uint2*>(q.Dh + ((size_t)t * q.BP + b) * q.NP + i) = to_bf16x4(make_float4(d[0], d[1], d[2], d[3]));
     }
-    st[i] = r;
-    const __nv_bfloat16 rb = __float2bfloat16(r);
-    if (q.Rh != nullptr) q.Rh[((size_t)(t + 1) * q.BP + b) * q.NP + i] = rb;
-    if (build) {
-      const float rf = __bfloat162float(rb);
-      rs += rf;
-      xrow[i] = rb;
-      for (int k = 0; k < q.cols.n; ++k) {
-        const float ck = valid ? __ldg(a_next + q.cols.c[k]) : 0.f;
-        xrow[(size_t)(1 + k) * q.NP + i] = __float2bfloat16(ck * rf);
-      }
+    st4(st + i, make_float4(r[0], r[1], r[2], r[3]));
+    const uint2 rb = to_bf16x4(make_float4(r[0], r[1], r[2], r[3]));
+    const float4 rf = of_bf16x4(rb);
+    rs += sum4(rf);
+    if (q.Rh != nullptr) *reinterpret_cast<uint2*>(q.Rh + ((size_t)(t + 1) * q.BP + b) * q.NP + i) = rb;
+    if (build && q.X != nullptr) {
+      __nv_bfloat16* x = q.X + (size_t)b * (q.concat ? q.KX : (long long)q.NP) + i;
+      *reinterpret_cast<uint2*>(x) = rb;
+      if (q.concat)
+        for (int k = 1; k <= n; ++k) {
+          const float c = coef[k];
+          *reinterpret_cast<uint2*>(x + (size_t)k * q.NP) = to_bf16x4(make_float4(c * rf.x, c * rf.y, c * rf.z, c * rf.w));
+        }
     }
   }
   if (build) {
     const float tot = block_sum(rs, red);
     if (threadIdx.x == 0) q.rowsum[b] = tot;
   }
-  if (t >= 0 && valid && (q.dec_x != nullptr || q.dec_y != nullptr || q.dec_ta != nullptr)) {
+  if (t >= 0 && valid && (dec || q.dec_ta != nullptr)) {
     const float sx = block_sum(px, red), sy = block_sum(py, red), sa = block_sum(pa, red);
     if (threadIdx.x == 0) {
       const size_t o = (size_t)b * q.T + t;
@@ -180,6 +285,7 @@ __global__ void sw_forward_row_kernel(SwFwd q, int t) {
 struct SwBwd {
   int B, T, N, NP, BP, a_dim, nsplit;
   long long KX;
+  bool vec;                  // as in SwFwd
   float J0, alpha;
   const float* A;
   const float* grad_output;  // [T,B,N] or nullptr
@@ -199,94 +305,116 @@ struct SwBwd {
   SwCols cols;
 };
 
-// One block per padded sample row.  t_carry >= 0: forms the carry out of step t_carry from Z (and dL/dA of that
-// step); t_delta >= 0: g and delta of step t_delta from the carry (zero when t_carry < 0).
-__global__ void sw_backward_row_kernel(SwBwd q, int t_carry, int t_delta) {
-  __shared__ float red[ROW_THREADS / 32];
-  const int b = blockIdx.x;
+// One block per padded sample row, four neurons per thread.  t_carry >= 0: forms the carry out of step t_carry from Z (and
+// dL/dA of that step, WANT_DA); t_delta >= 0: g and delta of step t_delta from the carry (zero when t_carry < 0).
+template <bool WANT_DA>
+__global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t_carry, int t_delta) {
+  __shared__ float red[ROW_MAX / 32];
+  __shared__ float coef[1 + RINGRNN_MAX_ACTIVE];
+  __shared__ float da[WANT_DA ? (1 + RINGRNN_MAX_ACTIVE) * (ROW_MAX / 32) : 1];  // [matrix][warp]
+  const int b = blockIdx.x, n = q.cols.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool valid = b < q.B;
   float* g = q.g + (size_t)b * q.NP;
   const float beta = 1.f - q.alpha;
   const float sd = (t_carry >= 0) ? q.sum_delta[b] : 0.f;
-  const float* a_c = q.A + ((size_t)b * q.T + (t_carry >= 0 ? t_carry : 0)) * q.a_dim;
   float cx = 0.f, cy = 0.f, cs = 0.f;
   if (valid && t_delta >= 0 && q.coef_x != nullptr) {
     cx = q.coef_x[(size_t)b * q.T + t_delta];
     cy = q.coef_y[(size_t)b * q.T + t_delta];
     cs = q.coef_s[(size_t)b * q.T + t_delta];
   }
+  for (int k = threadIdx.x; k <= n; k += blockDim.x)
+    coef[k] = k == 0 ? 1.f : (valid && t_carry >= 0) ? __ldg(q.A + ((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k - 1]) : 0.f;
+  if (WANT_DA)
+    for (int x = threadIdx.x; x < (1 + n) * (ROW_MAX / 32); x += blockDim.x) da[x] = 0.f;
+  __syncthreads();
   float ds = 0.f;
-  for (int j = threadIdx.x; j < q.NP; j += ROW_THREADS) {
-    float carry = 0.f;
-    const bool live = valid && j < q.N;
-    if (t_carry >= 0 && live) {
-      carry = fmaf(beta, g[j], q.J0 * sd);
-      for (int m = 0; m <= q.cols.n; ++m) {
-        float z = 0.f;
-        for (int s = 0; s < q.nsplit; ++s) z += q.partial[((size_t)s * q.BP + b) * q.KX + (size_t)m * q.NP + j];
-        const float cm = (m == 0) ? 1.f : __ldg(a_c + q.cols.c[m - 1]);
-        carry = fmaf(cm, z, carry);
+  for (int j = threadIdx.x * 4; j < q.NP; j += blockDim.x * 4) {  // whole warps: NP is a multiple of 128
+    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t_carry >= 0 && valid) {
+      float4 rp = make_float4(0.f, 0.f, 0.f, 0.f);  // (zero beyond N)
+      if (WANT_DA) rp = of_bf16x4(*reinterpret_cast<const uint2*>(q.Rh + ((size_t)t_carry * q.BP + b) * q.NP + j));
+      for (int s = 0; s < q.nsplit; ++s) {
+        const float* src = q.partial + ((size_t)s * q.BP + b) * q.KX + j;
+#pragma unroll 8
+        for (int m = 0; m <= n; ++m) {
+          const float4 z = ld4(src + (size_t)m * q.NP);
+          carry = fma4(coef[m], z, carry);
+          if (WANT_DA && m > 0) {
+            float v = dot4(rp, z);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) da[m * (ROW_MAX / 32) + warp] += v;
+          }
+        }
       }
+      const float4 go = ld4(g + j);
+      const float js = q.J0 * sd;
+      carry = make_float4(carry.x + fmaf(beta, go.x, js), carry.y + fmaf(beta, go.y, js), carry.z + fmaf(beta, go.z, js),
+                          carry.w + fmaf(beta, go.w, js));
     }
     if (t_delta >= 0) {
-      float gg = carry;
-      if (live) {
-        if (q.grad_output != nullptr) gg += q.grad_output[((size_t)t_delta * q.B + b) * q.N + j];
-        if (q.coef_x != nullptr) {
-          const float r = __bfloat162float(q.Rh[((size_t)(t_delta + 1) * q.BP + b) * q.NP + j]);
-          gg = fmaf(cx, q.dec_u[j], gg);
-          gg = fmaf(cy, q.dec_v[j], gg);
-          gg = fmaf(cs, (r > 0.f) ? 1.f : ((r < 0.f) ? -1.f : 0.f), gg);
+      float gg[4] = {carry.x, carry.y, carry.z, carry.w};
+      float4 go = make_float4(0.f, 0.f, 0.f, 0.f), rt = go;
+      if (valid && q.grad_output != nullptr) go = row_ld(q.grad_output + ((size_t)t_delta * q.B + b) * q.N, j, q.N, q.vec);
+      if (valid && q.coef_x != nullptr)
+        rt = of_bf16x4(*reinterpret_cast<const uint2*>(q.Rh + ((size_t)(t_delta + 1) * q.BP + b) * q.NP + j));
+      const float gs[4] = {go.x, go.y, go.z, go.w}, rr[4] = {rt.x, rt.y, rt.z, rt.w};
+      const float4 dact = of_bf16x4(*reinterpret_cast<const uint2*>(q.Dh + ((size_t)t_delta * q.BP + b) * q.NP + j));
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        if (!valid || j + x >= q.N) {
+          gg[x] = 0.f;
+          continue;
         }
-      } else {
-        gg = 0.f;
+        gg[x] += gs[x];
+        if (q.coef_x != nullptr) {
+          gg[x] = fmaf(cx, q.dec_u[j + x], gg[x]);
+          gg[x] = fmaf(cy, q.dec_v[j + x], gg[x]);
+          gg[x] = fmaf(cs, (rr[x] > 0.f) ? 1.f : ((rr[x] < 0.f) ? -1.f : 0.f), gg[x]);
+        }
       }
-      g[j] = gg;
-      const float dact = __bfloat162float(q.Dh[((size_t)t_delta * q.BP + b) * q.NP + j]);
-      const __nv_bfloat16 db = __float2bfloat16(q.alpha * dact * gg);
-      q.Delta[((size_t)t_delta * q.BP + b) * q.NP + j] = db;
-      ds += __bfloat162float(db);
-    } else if (live && q.grad_r_init != nullptr) {
-      q.grad_r_init[(size_t)b * q.N + j] = carry;
+      st4(g + j, make_float4(gg[0], gg[1], gg[2], gg[3]));
+      const uint2 db = to_bf16x4(make_float4(q.alpha * dact.x * gg[0], q.alpha * dact.y * gg[1], q.alpha * dact.z * gg[2],
+                                             q.alpha * dact.w * gg[3]));
+      *reinterpret_cast<uint2*>(q.Delta + ((size_t)t_delta * q.BP + b) * q.NP + j) = db;
+      ds += sum4(of_bf16x4(db));
+    } else if (valid && q.grad_r_init != nullptr) {
+      row_st(q.grad_r_init + (size_t)b * q.N, j, q.N, q.vec, carry);
     }
   }
   if (t_delta >= 0) {
     const float tot = block_sum(ds, red);
     if (threadIdx.x == 0) q.sum_delta[b] = tot;
   }
-  if (t_carry >= 0 && valid && q.grad_A != nullptr) {
-    // dL/dA[b,t,cols[k]] = sum_j r_{t-1}[b,j] Z[b,(1+k)NP + j]
-    const __nv_bfloat16* rprev = q.Rh + ((size_t)t_carry * q.BP + b) * q.NP;
-    for (int k = 0; k < q.cols.n; ++k) {
-      float acc = 0.f;
-      for (int j = threadIdx.x; j < q.N; j += ROW_THREADS) {
-        float z = 0.f;
-        for (int s = 0; s < q.nsplit; ++s) z += q.partial[((size_t)s * q.BP + b) * q.KX + (size_t)(1 + k) * q.NP + j];
-        acc = fmaf(__bfloat162float(rprev[j]), z, acc);
-      }
-      const float tot = block_sum(acc, red);
-      if (threadIdx.x == 0) q.grad_A[((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k]] = tot;
+  if (WANT_DA && t_carry >= 0 && valid) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+      float v = 0.f;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += da[(1 + k) * (ROW_MAX / 32) + w];
+      q.grad_A[((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k]] = v;
     }
   }
 }
 
 // Xall[t][b][m*NP + j] = c_m(b,t) * r_{t-1}[b,j] for all t: the B operand of the weight-gradient GEMM.
-// grid (BP, T), block 256
-__global__ void sw_build_xall_kernel(const __nv_bfloat16* __restrict__ Rh, const float* __restrict__ A, SwCols cols,
-                                     int B, int T, int a_dim, int NP, int BP, long long KX,
-                                     __nv_bfloat16* __restrict__ Xall) {
+// grid (BP, T), four neurons per thread
+__global__ void __launch_bounds__(ROW_MAX) sw_build_xall_kernel(const __nv_bfloat16* __restrict__ Rh, const float* __restrict__ A,
+                                                                SwCols cols, int B, int T, int a_dim, int NP, int BP,
+                                                                long long KX, __nv_bfloat16* __restrict__ Xall) {
   const int b = blockIdx.x, t = blockIdx.y;
   const bool valid = b < B;
   const __nv_bfloat16* r = Rh + ((size_t)t * BP + b) * NP;
   __nv_bfloat16* x = Xall + ((size_t)t * BP + b) * KX;
   const float* at = A + ((size_t)b * T + t) * a_dim;
-  for (int j = threadIdx.x; j < NP; j += blockDim.x) {
-    const __nv_bfloat16 rb = r[j];
-    const float rf = __bfloat162float(rb);
-    x[j] = rb;
+  for (int j = threadIdx.x * 4; j < NP; j += blockDim.x * 4) {
+    const uint2 rb = *reinterpret_cast<const uint2*>(r + j);
+    const float4 rf = of_bf16x4(rb);
+    *reinterpret_cast<uint2*>(x + j) = rb;
+#pragma unroll 4
     for (int k = 0; k < cols.n; ++k) {
-      const float ck = valid ? __ldg(at + cols.c[k]) : 0.f;
-      x[(size_t)(1 + k) * NP + j] = __float2bfloat16(ck * rf);
+      const float c = valid ? __ldg(at + cols.c[k]) : 0.f;
+      *reinterpret_cast<uint2*>(x + (size_t)(1 + k) * NP + j) = to_bf16x4(make_float4(c * rf.x, c * rf.y, c * rf.z, c * rf.w));
     }
   }
 }
@@ -315,7 +443,7 @@ SwCols cols_of(const DevProblem& dp) {
 template <int ACT>
 void launch_forward_row(const SwFwd& q, int t, cudaStream_t s) {
   LaunchScope ls(K_FWD, s);
-  sw_forward_row_kernel<ACT><<<q.BP, ROW_THREADS, 0, s>>>(q, t);
+  sw_forward_row_kernel<ACT><<<q.BP, row_threads(q.NP), 0, s>>>(q, t);
 }
 
 void forward_row(int act, const SwFwd& q, int t, cudaStream_t s) {
@@ -338,12 +466,23 @@ bool stepwise_supported(const RingRnnProblem& p) {
   return NP <= 16384 && (1 + n_act) * NP <= (1ll << 30);
 }
 
-// FWD workspace: status(1024) | Wst | X | state | rowsum | split-K partials
+namespace {
+size_t x_bytes(const SwLayout& l) { return align_up((size_t)l.BP * (l.concat ? l.KX : l.NP) * 2, 1024); }
+size_t z_bytes(const SwLayout& l, bool concat) {
+  return align_up((concat ? (size_t)l.BP * l.NP : (size_t)l.ns_z * l.BP * l.KX) * 4, 1024);
+}
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }  // (nullptr is)
+int prep_blocks(const SwLayout& l) {
+  const long long n = (long long)l.NP * l.NP / 4 / (256 * 4);
+  return n < 1 ? 1 : n > 592 ? 592 : (int)n;
+}
+}  // namespace
+
+// FWD workspace: status(1024) | weights | X | state | rowsum | products
 size_t stepwise_fwd_workspace_bytes(const RingRnnProblem& p) {
   const SwLayout l = sw_layout(p);
-  return 1024 + align_up((size_t)l.NP * l.KX * 2, 1024) + align_up((size_t)l.BP * l.KX * 2, 1024) +
-         align_up((size_t)l.BP * l.NP * 4, 1024) + align_up((size_t)l.BP * 4, 1024) +
-         align_up((size_t)l.ns_fwd * l.BP * l.NP * 4, 1024);
+  return 1024 + align_up((size_t)l.NP * l.KX * 2, 1024) + x_bytes(l) + align_up((size_t)l.BP * l.NP * 4, 1024) +
+         align_up((size_t)l.BP * 4, 1024) + z_bytes(l, l.concat);
 }
 // SAVED: Rh [T+1][BP][NP] | Dh [T][BP][NP] (bf16)
 size_t stepwise_saved_bytes(const RingRnnProblem& p) {
@@ -356,7 +495,7 @@ size_t stepwise_bwd_workspace_bytes(const RingRnnProblem& p) {
   const SwLayout l = sw_layout(p);
   return 1024 + align_up((size_t)l.KX * l.NP * 2, 1024) + align_up((size_t)p.T * l.BP * l.NP * 2, 1024) +
          align_up((size_t)l.BP * l.NP * 4, 1024) + align_up((size_t)l.BP * 4, 1024) +
-         align_up((size_t)l.ns_bwd * l.BP * l.KX * 4, 1024) + align_up((size_t)p.T * l.BP * l.KX * 2, 1024) +
+         z_bytes(l, false) + align_up((size_t)p.T * l.BP * l.KX * 2, 1024) +
          align_up((size_t)l.ns_dw * l.NP * l.KX * 4, 1024) + align_up((size_t)l.NP * l.KX * 4, 1024) +
          align_up((size_t)p.N * p.N * 4, 1024);
 }
@@ -375,7 +514,7 @@ int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t
   __nv_bfloat16* Wst = reinterpret_cast<__nv_bfloat16*>(w);
   w += align_up((size_t)l.NP * l.KX * 2, 1024);
   __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
-  w += align_up((size_t)l.BP * l.KX * 2, 1024);
+  w += x_bytes(l);
   float* state = reinterpret_cast<float*>(w);
   w += align_up((size_t)l.BP * l.NP * 4, 1024);
   float* rowsum = reinterpret_cast<float*>(w);
@@ -386,19 +525,25 @@ int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t
   const SwCols cols = cols_of(dp);
   {
     LaunchScope ls(K_PREP, s);
-    sw_prep_weights_kernel<<<dim3(l.NP, l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP, l.KX, Wst, nullptr);
+    const bool vec = p.N % 4 == 0 && aligned16(p.Wo) && aligned16(dp.Wa);
+    sw_prep_weights_kernel<<<dim3(prep_blocks(l), l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP,
+                                                                          l.concat ? l.KX : l.NP,
+                                                                          l.concat ? l.NP : (long long)l.NP * l.NP, vec, Wst);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
 
   SwFwd q;
   memset(&q, 0, sizeof(q));
-  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.ns_fwd;
+  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.concat ? 1 : l.ns_z;
+  q.concat = l.concat;
+  q.vec = p.N % 4 == 0 && aligned16(p.r_init) && aligned16(a.bump_history) && aligned16(a.final_state);
   q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
-  q.A = p.A; q.r_init = p.r_init; q.partial = partial; q.state = state; q.rowsum = rowsum; q.X = X;
+  q.A = p.A; q.r_init = p.r_init; q.partial = partial; q.state = state; q.rowsum = rowsum;
   q.Rh = train ? static_cast<__nv_bfloat16*>(a.saved) : nullptr;
   q.Dh = train ? reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(a.saved) +
                                                    align_up((size_t)(p.T + 1) * l.BP * l.NP * 2, 1024))
                : nullptr;
+  q.X = l.concat || !train ? X : nullptr;
   q.hist = a.bump_history; q.final_state = a.final_state;
   q.dec_x = a.dec_x; q.dec_y = a.dec_y; q.dec_ta = a.dec_ta; q.dec_u = a.dec_u; q.dec_v = a.dec_v;
   q.cols = cols;
@@ -406,8 +551,12 @@ int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t
   forward_row(p.activation, q, -1, s);
   RINGRNN_CUDA_TRY(cudaGetLastError());
   for (int t = 0; t < p.T; ++t) {
-    // partial[s] = X_t[BP, KX] x Wst[NP, KX]^T over the s-th slice of KX (summed by the row kernel)
-    int rc = tc_gemm(0, X, Wst, partial, nullptr, l.BP, l.NP, l.KX, l.ns_fwd, status, s);
+    int rc;
+    if (l.concat)
+      rc = tc_gemm(0, X, Wst, partial, nullptr, l.BP, l.NP, l.KX, 1, status, s);
+    else
+      rc = tc_gemm(0, train ? q.Rh + (size_t)t * l.BP * l.NP : X, Wst, partial, nullptr, l.BP, (int)l.KX, l.NP, l.ns_z, status,
+                   s, l.nt_z);
     if (rc != RINGRNN_OK) return rc;
     forward_row(p.activation, q, t, s);
     RINGRNN_CUDA_TRY(cudaGetLastError());
@@ -434,7 +583,7 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
   float* sum_delta = reinterpret_cast<float*>(w);
   w += align_up((size_t)l.BP * 4, 1024);
   float* zpart = reinterpret_cast<float*>(w);
-  w += align_up((size_t)l.ns_bwd * l.BP * l.KX * 4, 1024);
+  w += z_bytes(l, false);
   __nv_bfloat16* Xall = reinterpret_cast<__nv_bfloat16*>(w);
   w += align_up((size_t)p.T * l.BP * l.KX * 2, 1024);
   float* dwpart = reinterpret_cast<float*>(w);
@@ -450,7 +599,7 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
   const SwCols cols = cols_of(dp);
   {
     LaunchScope ls(K_PREP, s);
-    sw_prep_weights_kernel<<<dim3(l.NP, l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP, l.KX, nullptr, WstT);
+    sw_prep_transposed_kernel<<<dim3(l.NP / 32, l.NP / 32, l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP, WstT);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   if (a.grad_A != nullptr)
@@ -458,7 +607,8 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
 
   SwBwd q;
   memset(&q, 0, sizeof(q));
-  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.ns_bwd;
+  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.ns_z;
+  q.vec = p.N % 4 == 0 && aligned16(a.grad_output) && aligned16(a.grad_r_init);
   q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
   q.A = p.A; q.grad_output = a.grad_output;
   q.coef_x = a.coef_x; q.coef_y = a.coef_y; q.coef_s = a.coef_s; q.dec_u = a.dec_u; q.dec_v = a.dec_v;
@@ -467,22 +617,24 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
 
   {
     LaunchScope ls(K_BWD, s);
-    sw_backward_row_kernel<<<l.BP, ROW_THREADS, 0, s>>>(q, -1, p.T - 1);
+    sw_backward_row_kernel<false><<<l.BP, row_threads(l.NP), 0, s>>>(q, -1, p.T - 1);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   for (int t = p.T - 1; t >= 0; --t) {
     // Z_t[BP, KX] = delta_t[BP, NP] x WstT[KX, NP]^T
-    int rc = tc_gemm(0, Delta + (size_t)t * l.BP * l.NP, WstT, zpart, nullptr, l.BP, (int)l.KX, l.NP, l.ns_bwd, status, s);
+    int rc = tc_gemm(0, Delta + (size_t)t * l.BP * l.NP, WstT, zpart, nullptr, l.BP, (int)l.KX, l.NP, l.ns_z, status, s,
+                     l.nt_z);
     if (rc != RINGRNN_OK) return rc;
     {
       LaunchScope ls(K_BWD, s);
-      sw_backward_row_kernel<<<l.BP, ROW_THREADS, 0, s>>>(q, t, t - 1);
+      if (q.grad_A != nullptr) sw_backward_row_kernel<true><<<l.BP, row_threads(l.NP), 0, s>>>(q, t, t - 1);
+      else sw_backward_row_kernel<false><<<l.BP, row_threads(l.NP), 0, s>>>(q, t, t - 1);
     }
     RINGRNN_CUDA_TRY(cudaGetLastError());
   }
   {
     LaunchScope ls(K_PREP, s);
-    sw_build_xall_kernel<<<dim3(l.BP, p.T), 256, 0, s>>>(Rh, p.A, cols, p.B, p.T, p.a_dim, l.NP, l.BP, l.KX, Xall);
+    sw_build_xall_kernel<<<dim3(l.BP, p.T), row_threads(l.NP), 0, s>>>(Rh, p.A, cols, p.B, p.T, p.a_dim, l.NP, l.BP, l.KX, Xall);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   // dWst[NP, KX] = Delta^T [NP, T*BP] x Xall [T*BP, KX]

@@ -393,12 +393,13 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
 
 // C[M,N] (fp32, partial sums over nsplit slices then reduced into `out`) = A * B with bf16 operands.
 //   mn_major = 1: A is [K, M], B is [K, N] (row-major);  mn_major = 0: A is [M, K], B is [N, K].
+// nt: tile width to use (128, 256 or 512), 0 = the largest that divides N.
 // M multiple of 128; N in {128, 256, 512} or a multiple of 512 (N % NT == 0).  partial: nsplit*M*N floats.
 int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* out, int M, int N, long long K,
-            int nsplit, int* status, cudaStream_t s) {
+            int nsplit, int* status, cudaStream_t s, int nt) {
   if (M % 128 != 0 || nsplit < 1) return RINGRNN_ERR_SHAPE;
   int rc;
-  const int NT = (N % 512 == 0) ? 512 : (N % 256 == 0) ? 256 : (N % 128 == 0) ? 128 : 0;
+  const int NT = nt > 0 ? nt : (N % 512 == 0) ? 512 : (N % 256 == 0) ? 256 : (N % 128 == 0) ? 128 : 0;
   if (NT == 0) return RINGRNN_ERR_SHAPE;
 #define RINGRNN_GEMM_CASE(MN, NTV)                                                            \
   if (mn_major == MN && NT == NTV) rc = launch_gemm<MN != 0, NTV>(A, B, partial, M, N, K, nsplit, status, s); else
