@@ -1,7 +1,7 @@
-// bf16 mode, N <= 256 with up to two active action columns: host side of the kernels of tc_lane.cuh (buffer layouts,
+// bf16 mode, N <= 512 with up to two active action columns: host side of the kernels of tc_lane.cuh (buffer layouts,
 // choice of the samples per unit, weight gradients, checkpoints).
 //
-// Layouts (NP = 128 or 256, S samples per unit tile, n_ut = ceil(B/S) unit tiles, BPs = n_ut * S):
+// Layouts (NP = 128, 256 or 512, S samples per unit tile, n_ut = ceil(B/S) unit tiles, BPs = n_ut * S):
 //   saved            Rh [T+1][NP][BPs] bf16 (slot 0 = r_init, slot t+1 = r_t; the last slot stays unwritten: nothing reads
 //                    r_T) | Dh = F'(re), T*NP*BPs bf16 in the threads' own order | sign words, likewise
 //   backward scratch DL [T][3][NP][BPs] bf16 = delta, L*delta, R*delta | split-K partials [ns][3*NP][NP] | dJ partials |
@@ -25,12 +25,12 @@ struct LaneLayout {
 
 LaneLayout lane_layout(const RingRnnProblem& p) {
   LaneLayout l;
-  l.NP = p.N <= 128 ? 128 : 256;
+  l.NP = p.N <= 128 ? 128 : p.N <= 256 ? 256 : 512;
   l.CL = l.NP / 128;
   // A step costs its latency chain, which grows with the samples per unit; so the fewest samples at which the batch still
   // fits the 148 SMs in one go.  Beyond 64 per CTA (NP = 128) two units of 64 run side by side in a CTA.
   const int fit = 148 / l.CL;
-  l.S = p.B <= 16 * fit ? 16 : p.B <= 32 * fit ? 32 : 64;
+  l.S = l.NP == 512 || p.B <= 16 * fit ? 16 : p.B <= 32 * fit ? 32 : 64;
   l.n_ut = (p.B + l.S - 1) / l.S;
   l.BPs = l.n_ut * l.S;
   l.units = (l.NP == 128 && l.S == 64 && l.n_ut > fit) ? 2 : 1;
@@ -69,7 +69,7 @@ struct LaneBwdLayout {
 };
 LaneBwdLayout lane_bwd_layout(const LaneLayout& l, int T) {
   LaneBwdLayout b;
-  const int tiles = 3 * l.NP / 128;
+  const int tiles = 3 * l.NP / 128 * (l.NP > 256 ? l.NP / 256 : 1);
   const long long chunks = (long long)T * ((l.BPs + 63) / 64);
   long long ns = 148 / tiles;
   if (ns > chunks / 8) ns = chunks / 8;  // at least eight K chunks per CTA: a partial tile costs as much as a few of them
@@ -101,12 +101,15 @@ void set_inhibition(P& q, float J0, float J1) {
   }
 }
 
-// out[i] += add[i]
-__global__ void add_into_kernel(float* o0, float* o1, float* o2, const float* __restrict__ add, size_t n) {
+// out[k][i] += sum over the parts of add[part][k][i]
+__global__ void add_into_kernel(float* o0, float* o1, float* o2, const float* __restrict__ add, int parts, size_t n) {
   float* o = blockIdx.y == 0 ? o0 : blockIdx.y == 1 ? o1 : o2;
   if (o == nullptr) return;
-  const float* a = add + blockIdx.y * n;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) o[i] += a[i];
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    float v = o[i];
+    for (int p = 0; p < parts; ++p) v += add[((size_t)p * 3 + blockIdx.y) * n + i];
+    o[i] = v;
+  }
 }
 
 // From the split-K partials of dWcat [3*NP][NP]: grad_Wo = J1 * block 0, grad_Wa[colL], [colR] = blocks 1, 2, every other
@@ -234,17 +237,22 @@ void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneL
 
 }  // namespace
 
+// N in (256, 512]: two rounds of 33 resident clusters of 16 samples.  Training step N=512, T=128, against the tiles of 128
+// samples (tc_fwd.cu, tc_bwd.cu), which take one round up to 4096 samples: B = 64 1.37 against 2.67 ms, 512 1.50 / 2.84, 1024
+// 2.82 / 2.89 (with dL/dA, N=400 B=1000 T=100: 2.38 / 2.75), a third round 4.16 / 2.97.
+constexpr int LANE_512_MAX_B = 33 * 16 * 2;
+
 bool lane_supported(const RingRnnProblem& p) {
   static const bool force_stepwise = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
   if (force_stepwise) return false;
   const int n_act = p.n_active < 0 ? p.a_dim : p.n_active;
-  return p.N >= 1 && p.N <= 256 && n_act <= 2 && p.B >= 1 && p.T >= 1;
+  return p.N >= 1 && (p.N <= 256 || (p.N <= 512 && p.B <= LANE_512_MAX_B)) && n_act <= 2 && p.B >= 1 && p.T >= 1;
 }
 
-// FWD workspace: status(1024) | second CTA's decode sums [3][B][T] (NP = 256)
+// FWD workspace: status(1024) | the other CTAs' decode sums [CL-1][3][B][T]
 size_t lane_fwd_workspace_bytes(const RingRnnProblem& p) {
   const LaneLayout l = lane_layout(p);
-  return 1024 + (l.CL > 1 ? align_up((size_t)3 * p.B * p.T * 4, 1024) : 0);
+  return 1024 + (l.CL > 1 ? align_up((size_t)3 * (l.CL - 1) * p.B * p.T * 4, 1024) : 0);
 }
 size_t lane_saved_bytes(const RingRnnProblem& p) {
   const int K = lane_ckpt_interval(p);
@@ -291,7 +299,7 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   const bool want_dec = a.dec_x || a.dec_y || a.dec_ta;
   for (int k = 0; k < 3; ++k) {
     q.dec[0][k] = dec[k];
-    if (l.CL > 1 && dec[k] != nullptr) q.dec[1][k] = dec1 + (size_t)k * p.B * p.T;
+    for (int r = 1; r < l.CL && dec[k] != nullptr; ++r) q.dec[r][k] = dec1 + ((size_t)(r - 1) * 3 + k) * p.B * p.T;
   }
   q.dec_vec = p.T % 4 == 0 && aligned16(a.dec_x) && aligned16(a.dec_y) && aligned16(a.dec_ta) && aligned16(dec1);
   q.dec_u = a.dec_u; q.dec_v = a.dec_v;
@@ -302,7 +310,7 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   if (rc != RINGRNN_OK) return rc;
   if (want_dec && l.CL > 1) {
     LaunchScope ls(K_LOSS, s);
-    add_into_kernel<<<dim3(148, 3), 256, 0, s>>>(a.dec_x, a.dec_y, a.dec_ta, dec1, (size_t)p.B * p.T);
+    add_into_kernel<<<dim3(148, 3), 256, 0, s>>>(a.dec_x, a.dec_y, a.dec_ta, dec1, l.CL - 1, (size_t)p.B * p.T);
     RINGRNN_CUDA_TRY(cudaGetLastError());
   }
   return RINGRNN_OK;

@@ -426,7 +426,7 @@ int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, in
   if (M % 128 != 0 || nsplit < 1) return RINGRNN_ERR_SHAPE;
   const long long K = (long long)slabs * cols;
   if (N == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, slabs, host_status);
-  if (N == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, slabs, host_status);
+  if (N % 256 == 0) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, slabs, host_status);
   return RINGRNN_ERR_SHAPE;
 }
 

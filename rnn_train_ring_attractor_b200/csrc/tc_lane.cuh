@@ -1,4 +1,4 @@
-// Recurrent kernels with neurons on the tensor-memory lanes (bf16 mode, N <= 256, up to two active action columns).
+// Recurrent kernels with neurons on the tensor-memory lanes (bf16 mode, N <= 512, up to two active action columns).
 //
 // The products of a step are taken as  D_m[neuron, sample] = W_m[128 neurons, NP] x r^T[NP, S samples]: the weights are the
 // A operand and stay on the chip for the whole sequence, the state of S samples is the B operand.  Compared with samples on
@@ -10,14 +10,17 @@
 //   state into both CTAs' operand buffers (16-byte distributed-shared-memory stores; the buffers alternate, so nobody waits
 //   for a peer's MMAs: a peer that has sent r_t has finished the MMAs that read r_{t-2}).
 //
+//   NP = 512: a cluster of four, likewise, 16 samples per cluster.
+//
 // A operand.  Matrices that fit are kept in TENSOR MEMORY (128 lanes x NP/2 columns each): an MMA with a 16-column B operand
 // is bound by fetching its A tile, 4 KB at 128 B/clk from shared memory against 8-16 cycles from tensor memory.  The rest
-// of the three (only where 64 samples per unit leave no columns) are in shared memory, K-major, 128-byte swizzle.
+// of the three (where 64 samples per unit leave no columns; at NP = 512, 44 of the 96 K steps) are in shared memory,
+// K-major, 128-byte swizzle.
 // Global inhibition.  J0 * sum_j r_j joins the Wo product: J1 * (Yo + (J0/J1) * S) with S from an MMA whose A tile is
 // constant along both dimensions, the same 16-column tile for every K step.  J0/J1 enters as up to three bf16 terms (24
 // bits); one is enough for the usual J0 = -J1.
 // B operand.  [NP rows = neurons] x [64 samples] bf16, 128 bytes per row, 128-byte swizzle ("MN-major"); an MMA reads the
-// first S samples.  A thread owns a neuron, so it writes its new values as 16-byte pieces of a row.
+// first S samples.  NP = 512, where shared memory is short: 16 samples, 32 bytes per row, 32-byte swizzle.  A thread owns a neuron, so it writes its new values as 16-byte pieces of a row.
 //
 // Roles (128 + 256 U threads): warp 0 issues the MMAs, warp 1 allocates tensor memory, warp 2 stages the per-sample
 // scalars (action signal, loss coefficients) eight steps at a time, the last 8 U warps are the epilogue: unit u has eight,
@@ -45,7 +48,7 @@ struct LaneFwdParams {
   __nv_bfloat16* Dh;     // F'(re), private layout, T*NP*BPs elements
   uint32_t* Sg;          // sign / zero bits of r_t, private layout, T*NP*BPs/4 bytes
   float* hist;           // [T,B,N] or nullptr
-  float* dec[2][3];      // [B][T] decode sums r.u, r.v, sum|r| over the neurons of CTA 0 and 1; nullptr = not wanted
+  float* dec[4][3];      // [B][T] decode sums r.u, r.v, sum|r| over the neurons of each CTA; nullptr = not wanted
   const float* dec_u;    // [N]
   const float* dec_v;
   float* final_state;    // [B,N] or nullptr
@@ -113,24 +116,27 @@ struct Cfg {
   // tensor memory columns: accumulators [unit][3][S] | three constant tiles of 8 | weights, NP/2 per matrix
   static constexpr int C_CONST = 3 * S * U;
   static constexpr int C_W = (C_CONST + 24 + 31) / 32 * 32;
-  static constexpr int NTM = (512 - C_W) / (NP / 2) > 3 ? 3 : (512 - C_W) / (NP / 2);  // matrices kept there
-  static constexpr int NSM = 3 - NTM;                                                  // matrices in shared memory
+  // K steps (of the 3*KS of the three matrices, in order) kept there; the rest in shared memory, tiles of four K steps
+  static constexpr int NTK = NP == 512 ? (512 - C_W) / 32 * 4 : ((512 - C_W) / (NP / 2) > 3 ? 3 : (512 - C_W) / (NP / 2)) * KS;
+  static constexpr int SM_TILES = (3 * KS - NTK) / 4;
   // shared memory
   static constexpr int ST_BUFS = CL > 1 ? 2 : 1;
-  static constexpr int ST_BYTES = NP * 128;
-  static constexpr int RED_BUFS = S < 64 ? 2 : 1;  // alternating, so that one barrier per step is enough
+  static constexpr int ST_ROW = NP == 512 ? 32 : 128;  // bytes of an operand row
+  static constexpr int ST_BYTES = NP * ST_ROW;
+  static constexpr int RED_BUFS = S < 64 && NP < 512 ? 2 : 1;  // alternating, so that one barrier per step is enough
   static constexpr int RED_BYTES = 128 * S * 4;
   static constexpr int OFF_W = U * ST_BUFS * ST_BYTES;
-  static constexpr int OFF_RED = OFF_W + NSM * (NP / 64) * 16384;
+  static constexpr int OFF_RED = OFF_W + SM_TILES * 16384;
   static constexpr int OFF_SC = OFF_RED + U * NRED * RED_BUFS * RED_BYTES;
   static constexpr int SC_BYTES = 2 * CH * Q * S * 4;             // per unit
   static constexpr int OFF_DEC = OFF_SC + U * SC_BYTES;
-  static constexpr int DEC_BYTES = NRED == 1 ? 2 * 3 * S * 8 * 4 : 0;  // forward: eight steps of decode sums, twice
+  static constexpr int DEC_BYTES = Q == 2 ? 2 * 3 * S * 8 * 4 : 0;  // forward: eight steps of decode sums, twice
   static constexpr int OFF_UV = OFF_DEC + U * DEC_BYTES;
   static constexpr int OFF_BAR = OFF_UV + 128 * 8;
   static constexpr int SMEM = OFF_BAR + 256 + 1024;
   static_assert(SMEM <= tcr::SMEM_LIMIT, "shared memory");
-  static_assert(NTM >= 1 && C_W + NTM * (NP / 2) <= 512, "tensor memory");
+  static_assert(NTK % 4 == 0 && NTK >= KS && C_W + NTK * 8 <= 512, "tensor memory");
+  static_assert(NP < 512 || S == 16, "operand rows of 16 samples");
   // registers: launched with LAUNCH_REGS per thread; the four service warps hand theirs to the epilogue
   static constexpr int LAUNCH_REGS = 65536 / THREADS / 8 * 8;
   static constexpr int LOW = U == 1 ? 72 : 40, HIGH = U == 1 ? 208 : 104;
@@ -138,12 +144,13 @@ struct Cfg {
 };
 
 // barrier block
-constexpr uint32_t B_STATE = 0;      // [2 units] the operand of the next step is complete
-constexpr uint32_t B_DFULL = 16;     // [2] the accumulators of the step are complete
-constexpr uint32_t B_SC_FULL = 32;   // [2 units][2]
-constexpr uint32_t B_SC_FREE = 64;   // [2 units][2]
-constexpr uint32_t B_TMEM = 96;
-constexpr uint32_t B_DEAD = 100;
+constexpr uint32_t B_STATE = 0;      // [2 units][2] the operand of the next step is complete: used alternately, because a CTA
+                                     // may send the state after the next before a third one's arrival for this one lands
+constexpr uint32_t B_DFULL = 32;     // [2] the accumulators of the step are complete
+constexpr uint32_t B_SC_FULL = 48;   // [2 units][2]
+constexpr uint32_t B_SC_FREE = 80;   // [2 units][2]
+constexpr uint32_t B_TMEM = 112;
+constexpr uint32_t B_DEAD = 116;
 
 template <class C>
 struct Ctx {
@@ -168,9 +175,9 @@ __device__ __forceinline__ Ctx<C> setup(uint8_t* smem_raw, int units, const floa
   if (threadIdx.x == 0) {
     *dead = 0;
     for (int u = 0; u < units; ++u) {
-      mbar_init(c.bars + B_STATE + 8 * u, 8 * C::CL);  // the epilogue warps of every CTA of the cluster
       mbar_init(c.bars + B_DFULL + 8 * u, 1);
       for (int i = 0; i < 2; ++i) {
+        mbar_init(c.bars + B_STATE + 16 * u + 8 * i, 8 * C::CL);  // the epilogue warps of every CTA of the cluster
         mbar_init(c.bars + B_SC_FULL + 16 * u + 8 * i, 1);
         mbar_init(c.bars + B_SC_FREE + 16 * u + 8 * i, 8);
       }
@@ -216,7 +223,7 @@ __device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const
   for (int m = 0; m < 3; ++m) {
     const float* w = W[m];
     const bool live = w != nullptr && n < N;
-#pragma unroll 1
+#pragma unroll(NP < 512 ? 1 : 2)
     for (int k0 = h * (NP / 2); k0 < (h + 1) * (NP / 2); k0 += 16) {
       float v[16];
       if (TRANSPOSED) {
@@ -236,11 +243,12 @@ __device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const
       uint32_t pk[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) pk[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-      if (m < C::NTM) {
-        tmem_st8(c.tmem + lane_base + C::C_W + m * (NP / 2) + k0 / 2, pk);
+      const int ks = m * C::KS + k0 / 16;
+      if (ks < C::NTK) {
+        tmem_st8(c.tmem + lane_base + C::C_W + ks * 8, pk);
       } else {
-        const uint32_t tile = c.base + C::OFF_W + ((m - C::NTM) * (NP / 64) + k0 / 64) * 16384 + row * 128;
-        const uint32_t u0 = (uint32_t)(k0 % 64) / 8;
+        const uint32_t tile = c.base + C::OFF_W + (ks - C::NTK) / 4 * 16384 + row * 128;
+        const uint32_t u0 = (uint32_t)((ks - C::NTK) & 3) * 2;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(tile + (((u0 + i) ^ ((uint32_t)row & 7u)) << 4)),
@@ -257,7 +265,7 @@ __device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const
     }
   }
   tmem_st_wait();
-  if (C::NSM > 0) fence_proxy_async_smem();
+  if (C::SM_TILES > 0) fence_proxy_async_smem();
 }
 
 // MMA issuer (one whole warp, see umma_ts_warp; everything the instructions are built from is uniform).  Unit u's tile of
@@ -275,22 +283,24 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (tile + u >= n_ut) continue;
-        const bool ok = mbar_wait<(C::CL > 1)>(c.bars + B_STATE + 8 * u, g[u] & 1u, c.w, code);
+        const bool ok = mbar_wait<(C::CL > 1)>(c.bars + B_STATE + 16 * u + 8 * (g[u] & 1u), (g[u] >> 1) & 1u, c.w, code);
         if (!__all_sync(0xffffffffu, ok)) return;
         if (C::CL > 1) fence_proxy_async_all();
         tcgen05_fence_after();
         const uint32_t st = base + (u * C::ST_BUFS + (C::ST_BUFS > 1 ? (g[u] & 1u) : 0u)) * C::ST_BYTES;
-        const uint64_t b0 = desc_sw128(desc_lo(st, 16));
+        const uint64_t b0 = C::ST_ROW == 32 ? desc_sw32(desc_lo(st, 16)) : desc_sw128(desc_lo(st, 16));
+        constexpr uint32_t B_STEP = C::ST_ROW;  // 16 rows, in units of 16 bytes
         const uint32_t d = tmem + u * 3 * S;
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
 #pragma unroll
           for (int ks = 0; ks < C::KS; ++ks) {
-            if (m < C::NTM) {
-              umma_ts_warp(d + m * S, tmem + C::C_W + m * (NP / 2) + ks * 8, b0 + ks * 128, idesc, ks > 0, lead);
+            const int w = m * C::KS + ks;
+            if (w < C::NTK) {
+              umma_ts_warp(d + m * S, tmem + C::C_W + w * 8, b0 + ks * B_STEP, idesc, ks > 0, lead);
             } else {
-              const uint64_t a0 = desc_sw128(desc_lo(base + C::OFF_W + (m - C::NTM) * (NP / 64) * 16384, 16));
-              umma_ss_warp(d + m * S, a0 + (ks / 4) * 1024 + 2 * (ks & 3), b0 + ks * 128, idesc, ks > 0, lead);
+              const uint64_t a0 = desc_sw128(desc_lo(base + C::OFF_W, 16));
+              umma_ss_warp(d + m * S, a0 + (w - C::NTK) / 4 * 1024 + 2 * ((w - C::NTK) & 3), b0 + ks * B_STEP, idesc, ks > 0, lead);
             }
           }
         }
@@ -298,7 +308,7 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
         for (int i = 0; i < n_const; ++i) {
 #pragma unroll
           for (int ks = 0; ks < C::KS; ++ks)
-            umma_ts_warp(d, tmem + C::C_CONST + 8 * i, b0 + ks * 128, idesc, true, lead);
+            umma_ts_warp(d, tmem + C::C_CONST + 8 * i, b0 + ks * B_STEP, idesc, true, lead);
         }
         if (lead) umma_commit(c.bars + B_DFULL + 8 * u);
         __syncwarp();
@@ -308,29 +318,33 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
   }
 }
 
-// Publishes this thread's E new state values (packed bf16 pairs): into row `row` of the operand buffer, here and in the
-// peer, then one arrival per warp on the state barriers.  Local arrival first: a peer may only start the next step once
-// every warp of this CTA has arrived here too, so no barrier ever sees two phases at once.
+// Publishes this thread's E new state values (packed bf16 pairs): into row `row` of operand buffer g & 1, here and in the
+// peers, then one arrival per warp on the state barriers of that buffer.
 template <class C, int S>
-__device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed, uint32_t parity, int u, int row_k, int h,
+__device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed, uint32_t g, int u, int row_k, int h,
                                         int lane) {
-  const uint32_t buf = c.base + (u * C::ST_BUFS + (C::ST_BUFS > 1 ? parity : 0u)) * C::ST_BYTES + row_k * 128;
+  const uint32_t parity = g & 1u;
+  const uint32_t buf = c.base + (u * C::ST_BUFS + (C::ST_BUFS > 1 ? parity : 0u)) * C::ST_BYTES + row_k * C::ST_ROW;
+  const uint32_t swizzle = C::ST_ROW == 32 ? ((uint32_t)row_k >> 2) & 1u : (uint32_t)row_k & 7u;
 #pragma unroll
   for (int v = 0; v < C::E / 8; ++v) {
-    const uint32_t addr = buf + (((uint32_t)(h * (C::E / 8) + v) ^ ((uint32_t)row_k & 7u)) << 4);
+    const uint32_t addr = buf + (((uint32_t)(h * (C::E / 8) + v) ^ swizzle) << 4);
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(packed[4 * v]), "r"(packed[4 * v + 1]),
                  "r"(packed[4 * v + 2]), "r"(packed[4 * v + 3])
                  : "memory");
-    if (C::CL > 1)
-      st_cluster_v4(mapa(addr, c.rank ^ 1u), packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+#pragma unroll
+    for (uint32_t peer = 1; peer < C::CL; ++peer)
+      st_cluster_v4(mapa(addr, c.rank ^ peer), packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
   }
   if (C::CL > 1) fence_proxy_async_all();
   else fence_proxy_async_smem();
   tcgen05_fence_before();  // this thread's accumulator reads precede the MMAs the arrival releases
   __syncwarp();
   if (lane == 0) {
-    mbar_arrive(c.bars + B_STATE + 8 * u);
-    if (C::CL > 1) mbar_arrive_cluster(c.bars + B_STATE + 8 * u, c.rank ^ 1u);
+    const uint32_t bar = c.bars + B_STATE + 16 * u + 8 * parity;
+    mbar_arrive(bar);
+#pragma unroll
+    for (uint32_t peer = 1; peer < C::CL; ++peer) mbar_arrive_cluster(bar, c.rank ^ peer);
   }
 }
 

@@ -1,4 +1,4 @@
-// bf16 mode, reverse time, N <= 256: neurons on the tensor-memory lanes (see tc_lane.cuh for the decomposition).  Per step
+// bf16 mode, reverse time, N <= 512: neurons on the tensor-memory lanes (see tc_lane.cuh for the decomposition).  Per step
 //   D_m[j, sample] = W_m^T x delta_t      carry = (1-alpha) g + J0 sum_i delta + J1 Zo + L Zl + R Zr
 //   g_{t-1} = carry + dL/dr_{t-1}         delta_{t-1} = alpha F'(re_{t-1}) g_{t-1}
 // delta, L*delta and R*delta go to DL, [T][3][NP][samples], the K-major A operand of the weight-gradient GEMM.
@@ -12,8 +12,9 @@ using namespace lane;
 
 template <int NP, int S>
 __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant__ LaneBwdParams p) {
-  using C = Cfg<NP, S, 1, 5, 2>;
+  using C = Cfg<NP, S, 1, 5, NP < 512 ? 2 : 1>;
   constexpr int E = C::E;
+  constexpr int NRED = NP < 512 ? 2 : 1;  // dL/dA: both products side by side, or one after the other
   extern __shared__ uint8_t smem_raw[];
   const Ctx<C> c = setup<C>(smem_raw, 1, p.dec_u, p.dec_v, p.N, p.status, p.report, p.zero_report, p.host);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
           packed[j / 2] = pack_bf16x2(x0, x1);
           packed[j / 2 + 1] = pack_bf16x2(x2, x3);
         }
-        publish<C, S>(c, packed, g & 1u, 0, n, h, lane);
+        publish<C, S>(c, packed, g, 0, n, h, lane);
       };
       // off the critical path: delta_t and its scaled copies (packed bf16 products, the scalars rounded to bf16)
       auto write_dl = [&](int t, int e) {
@@ -174,8 +175,9 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
         if (t > 0) wait_entry(e + 1);
         mbar_wait(c.bars + B_DFULL, g & 1u, c.w, 305);
         tcgen05_fence_after();
-        float* red = reinterpret_cast<float*>(c.gen + C::OFF_RED) + (C::RED_BUFS > 1 ? (t & 1) : 0) * (2 * C::RED_BYTES / 4);
+        float* red = reinterpret_cast<float*>(c.gen + C::OFF_RED) + (C::RED_BUFS > 1 ? (t & 1) : 0) * (NRED * C::RED_BYTES / 4);
         if (want_dA && C::RED_BUFS == 1) named_bar_sync(4, 256);  // the previous step's readers are done
+        float later[NRED == 1 ? E : 4];
         constexpr int GR = E < 16 ? E : 16;
 #pragma unroll
         for (int j0 = 0; j0 < E; j0 += GR) {
@@ -211,11 +213,17 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
               const uint4 r8 = rp[(j0 + x) / 8];
               const uint32_t w0 = (x & 4) ? r8.z : r8.x, w1 = (x & 4) ? r8.w : r8.y;
               const float r0 = tcr::bf16_lo(w0), r1 = tcr::bf16_hi(w0), r2 = tcr::bf16_lo(w1), r3 = tcr::bf16_hi(w1);
+              if constexpr (NRED == 1) {  // the second product waits in registers
+                later[j0 + x] = r0 * __uint_as_float(zr[x]);
+                later[j0 + x + 1] = r1 * __uint_as_float(zr[x + 1]);
+                later[j0 + x + 2] = r2 * __uint_as_float(zr[x + 2]);
+                later[j0 + x + 3] = r3 * __uint_as_float(zr[x + 3]);
+              }
               uint8_t* dst = reinterpret_cast<uint8_t*>(red) + red_offset<S>(row, (h * E + j0 + x) / 4);
               *reinterpret_cast<float4*>(dst) = make_float4(r0 * __uint_as_float(zl[x]), r1 * __uint_as_float(zl[x + 1]),
                                                             r2 * __uint_as_float(zl[x + 2]), r3 * __uint_as_float(zl[x + 3]));
-              *reinterpret_cast<float4*>(dst + C::RED_BYTES) =
-                  make_float4(r0 * __uint_as_float(zr[x]), r1 * __uint_as_float(zr[x + 1]), r2 * __uint_as_float(zr[x + 2]),
+              if constexpr (NRED == 2)
+                *reinterpret_cast<float4*>(dst + C::RED_BYTES) = make_float4(r0 * __uint_as_float(zr[x]), r1 * __uint_as_float(zr[x + 1]), r2 * __uint_as_float(zr[x + 2]),
                               r3 * __uint_as_float(zr[x + 3]));
             }
           }
@@ -237,25 +245,40 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
         }
         if (t > 1) prefetch(t - 2);
         if (want_dA) {
-          named_bar_sync(2, 256);
-          if (tid < 4 * S) {
-            const int part = tid & 15, quad = tid >> 4;
-            float a[8];
+          const int part = tid & 15, quad = tid >> 4;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = 0.f;
+          for (int pass = 0; pass < 3 - NRED; ++pass) {
+            if constexpr (NRED == 1) {
+              if (pass == 1) {
+                named_bar_sync(4, 256);  // the first product's readers are done
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint8_t* src = reinterpret_cast<const uint8_t*>(red) + red_offset<S>(part + 16 * i, quad);
-              const float4 l = lds4(reinterpret_cast<const float*>(src)), r = lds4(reinterpret_cast<const float*>(src + C::RED_BYTES));
-              a[0] += l.x; a[1] += l.y; a[2] += l.z; a[3] += l.w;
-              a[4] += r.x; a[5] += r.y; a[6] += r.z; a[7] += r.w;
+                for (int x = 0; x < E; x += 4)
+                  *reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(red) + red_offset<S>(row, (h * E + x) / 4)) =
+                      make_float4(later[x], later[x + 1], later[x + 2], later[x + 3]);
+              }
             }
-            half_warp_sums<8>(a, lane);
-            if ((lane & 3) == 0) {
-              const int v0 = 4 * ((lane >> 3) & 1) + 2 * ((lane >> 2) & 1);
+            named_bar_sync(2, 256);
+            if (tid < 4 * S) {
+              float a[4 * NRED];
 #pragma unroll
-              for (int i = 0; i < 2; ++i)
-                p.dA_part[(((size_t)c.rank * 2 + (v0 + i) / 4) * T + t) * p.BPs + ut * S + quad * 4 + (v0 + i) % 4] = a[i];
+              for (int i = 0; i < 4 * NRED; ++i) a[i] = 0.f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int k = 0; k < NRED; ++k) {
+                  const float4 v = lds4(reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(red) + k * C::RED_BYTES +
+                                                                       red_offset<S>(part + 16 * i, quad)));
+                  a[4 * k] += v.x; a[4 * k + 1] += v.y; a[4 * k + 2] += v.z; a[4 * k + 3] += v.w;
+                }
+              half_warp_sums<4 * NRED>(a, lane);
+              if ((lane & 3) == 0) {
+                const int v0 = NRED * (2 * ((lane >> 3) & 1) + ((lane >> 2) & 1));
+#pragma unroll
+                for (int i = 0; i < NRED; ++i) {
+                  const int k = NRED == 2 ? (v0 + i) / 4 : pass;
+                  p.dA_part[(((size_t)c.rank * 2 + k) * T + t) * p.BPs + ut * S + quad * 4 + (v0 + i) % 4] = a[i];
+                }
+              }
             }
           }
         }
@@ -270,7 +293,7 @@ namespace {
 
 template <int NP, int S>
 int launch(const LaneBwdParams& p, cudaStream_t s) {
-  using C = Cfg<NP, S, 1, 5, 2>;
+  using C = Cfg<NP, S, 1, 5, NP < 512 ? 2 : 1>;
   auto kernel = bwd_lane_kernel<NP, S>;
   return launch_lane<C>(K_BWD, reinterpret_cast<const void*>(kernel), p.n_ut, s,
                         [&](const cudaLaunchConfig_t* cfg) { return cudaLaunchKernelEx(cfg, kernel, p); });
@@ -280,6 +303,7 @@ int launch(const LaneBwdParams& p, cudaStream_t s) {
 
 int lane_backward_launch(int NP, int S, const LaneBwdParams& p, cudaStream_t s) {
   if (NP == 128) return S == 16 ? launch<128, 16>(p, s) : S == 32 ? launch<128, 32>(p, s) : launch<128, 64>(p, s);
+  if (NP == 512) return launch<512, 16>(p, s);
   return S == 16 ? launch<256, 16>(p, s) : S == 32 ? launch<256, 32>(p, s) : launch<256, 64>(p, s);
 }
 

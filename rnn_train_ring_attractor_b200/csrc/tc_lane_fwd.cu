@@ -1,4 +1,4 @@
-// bf16 mode, forward, N <= 256: neurons on the tensor-memory lanes (see tc_lane.cuh for the decomposition).  One launch
+// bf16 mode, forward, N <= 512: neurons on the tensor-memory lanes (see tc_lane.cuh for the decomposition).  One launch
 // runs all T steps; the fp32 master state of S samples x 128 neurons lives in the registers of a unit's eight epilogue
 // warps, S/2 values per thread.
 #include <string.h>
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
       for (int j = 0; j < E; ++j) master[j] = (live && b0 + j < p.B) ? __ldg(p.r_init + (size_t)(b0 + j) * p.N + n) : 0.f;
 #pragma unroll
       for (int j = 0; j < E / 2; ++j) packed[j] = pack_bf16x2(master[2 * j], master[2 * j + 1]);
-      publish<C, S>(c, packed, g & 1u, u, n, h, lane);
+      publish<C, S>(c, packed, g, u, n, h, lane);
       if (p.Rh != nullptr) {
         uint4* dst = reinterpret_cast<uint4*>(p.Rh + (size_t)n * p.BPs + b0);
 #pragma unroll
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
             }
           }
         }
-        if (t + 1 < T) publish<C, S>(c, packed, (g + 1) & 1u, u, n, h, lane);
+        if (t + 1 < T) publish<C, S>(c, packed, g + 1, u, n, h, lane);
         // ---- off the critical path: the next step's MMAs are running
         if (k == CH - 1 || t + 1 == T) {  // the scalars of this chunk are no longer needed
           __syncwarp();
@@ -267,6 +267,7 @@ int by_shape(int NP, int S, int U, const LaneFwdParams& p, cudaStream_t s) {
     if (S == 32) return launch<ACT, 128, 32, 1>(p, s);
     return launch<ACT, 128, 64, 1>(p, s);
   }
+  if (NP == 512) return launch<ACT, 512, 16, 1>(p, s);
   if (S == 16) return launch<ACT, 256, 16, 1>(p, s);
   if (S == 32) return launch<ACT, 256, 32, 1>(p, s);
   return launch<ACT, 256, 64, 1>(p, s);

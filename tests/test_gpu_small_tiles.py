@@ -27,7 +27,10 @@ def _case(N, B, T, a_dim, seed):
 # beyond one round of units; steps around the eight whose scalars are staged at a time; J1 = 0 (no ratio to J1)
 LANE = [(1, 1, 1, 2, "tanh", -0.1, 0.1), (2, 17, 8, 1, "silu", -0.1, 0.1), (127, 16, 9, 2, "gelu", -0.1, 0.1),
         (128, 2369, 7, 2, "tanh", -0.07, 0.3), (129, 15, 16, 2, "silu", -0.1, 0.1), (255, 1185, 3, 2, "gelu", -0.031, 0.1),
-        (256, 2400, 9, 2, "tanh", -0.05, 0.0), (120, 9500, 2, 2, "silu", 0.0, 0.1), (100, 20001, 3, 2, "tanh", -0.1, 0.1)]
+        (256, 2400, 9, 2, "tanh", -0.05, 0.0), (120, 9500, 2, 2, "silu", 0.0, 0.1), (100, 20001, 3, 2, "tanh", -0.1, 0.1),
+        # four CTAs: neurons around 256 and 512, one and several rounds of 33 clusters of 16 samples, the last batch taken
+        (257, 1, 1, 2, "tanh", -0.1, 0.1), (384, 17, 9, 1, "silu", -0.05, 0.1), (510, 33, 8, 2, "gelu", -0.013, 0.1),
+        (512, 1056, 3, 2, "tanh", -0.02, 0.1), (300, 1057, 2, 2, "tanh", -0.02, 0.1)]
 # fp32 clusters: one CTA, two, four, eight; a last CTA with few neurons; several column counts; no shape that fits
 CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), (97, 9, 4, 2, "gelu", -0.1, 0.1),
            (200, 300, 3, 2, "tanh", -0.1, 0.1), (257, 70, 3, 1, "silu", -0.05, 0.2), (320, 33, 2, 2, "tanh", -0.04, 0.1)]
