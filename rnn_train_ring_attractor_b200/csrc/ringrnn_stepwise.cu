@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include "ringrnn_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace ringrnn {
 
@@ -53,7 +54,9 @@ int splits_for(long long tiles, long long K) {
 
 // Tile width and K splits of the Z GEMM by estimated cycles: waves of 148 CTAs x (start-up + operand bytes at the 50 B/clk
 // that enter an SM + the tile's way out at about 24 B/clk), plus the partial sums written and read back at 2.5 KB/clk.
+// CTA pairs (an even number of row tiles) fetch half of the B rows each.
 void z_shape(int BP, long long KX, int K, int* nt_out, int* ns_out) {
+  const bool pair = BP % 256 == 0;
   double best = 1e300;
   for (int nt = 512; nt >= 128; nt /= 2) {
     if (KX % nt != 0) continue;
@@ -61,7 +64,7 @@ void z_shape(int BP, long long KX, int K, int* nt_out, int* ns_out) {
       const double ctas = (double)(BP / 128) * (KX / nt) * ns;
       const long long chunks = (K / 64 + ns - 1) / ns;
       const double waves = (double)(((long long)ctas + 147) / 148);
-      const double cost = waves * (1500 + chunks * (128.0 + nt) * 128 / 50 + nt * 512.0 / 24) + 8.0 * ns * BP * KX / 2500;
+      const double cost = waves * (1500 + chunks * (128.0 + (pair ? nt / 2 : nt)) * 128 / 50 + nt * 512.0 / 24) + 8.0 * ns * BP * KX / 2500;
       if (cost < best) {
         best = cost;
         *nt_out = nt;
@@ -205,11 +208,13 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
   const bool valid = b < q.B;
   float* st = q.state + (size_t)b * q.NP;
   float px = 0.f, py = 0.f, pa = 0.f, rs = 0.f;
-  const float s_prev = (t >= 0) ? q.rowsum[b] : 0.f;
   const bool build = t + 1 < q.T;
   const int t_c = q.concat ? t + 1 : t;
   for (int k = threadIdx.x; k <= n; k += blockDim.x)
     coef[k] = k == 0 ? 1.f : (valid && t_c >= 0 && t_c < q.T) ? __ldg(q.A + ((size_t)b * q.T + t_c) * q.a_dim + q.cols.c[k - 1]) : 0.f;
+  tc::grid_launch_dependents();
+  tc::grid_wait();  // everything below may depend on the kernels before
+  const float s_prev = (t >= 0) ? q.rowsum[b] : 0.f;
   __syncthreads();
   const int blocks = q.concat ? 1 : 1 + n;
   const size_t ld = q.concat ? q.NP : q.KX;
@@ -316,7 +321,6 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
   const bool valid = b < q.B;
   float* g = q.g + (size_t)b * q.NP;
   const float beta = 1.f - q.alpha;
-  const float sd = (t_carry >= 0) ? q.sum_delta[b] : 0.f;
   float cx = 0.f, cy = 0.f, cs = 0.f;
   if (valid && t_delta >= 0 && q.coef_x != nullptr) {
     cx = q.coef_x[(size_t)b * q.T + t_delta];
@@ -327,6 +331,9 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
     coef[k] = k == 0 ? 1.f : (valid && t_carry >= 0) ? __ldg(q.A + ((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k - 1]) : 0.f;
   if (WANT_DA)
     for (int x = threadIdx.x; x < (1 + n) * (ROW_MAX / 32); x += blockDim.x) da[x] = 0.f;
+  tc::grid_launch_dependents();
+  tc::grid_wait();
+  const float sd = (t_carry >= 0) ? q.sum_delta[b] : 0.f;
   __syncthreads();
   float ds = 0.f;
   for (int j = threadIdx.x * 4; j < q.NP; j += blockDim.x * 4) {  // whole warps: NP is a multiple of 128
@@ -440,10 +447,26 @@ SwCols cols_of(const DevProblem& dp) {
   return c;
 }
 
+// `chained`: starts while the GEMM before it still runs (programmatic dependent launch)
+template <class K, class... Args>
+cudaError_t launch_row(K kernel, int rows, int NP, cudaStream_t s, bool chained, Args... args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(rows, 1, 1);
+  cfg.blockDim = dim3(row_threads(NP), 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <int ACT>
 void launch_forward_row(const SwFwd& q, int t, cudaStream_t s) {
   LaunchScope ls(K_FWD, s);
-  sw_forward_row_kernel<ACT><<<q.BP, row_threads(q.NP), 0, s>>>(q, t);
+  launch_row(sw_forward_row_kernel<ACT>, q.BP, q.NP, s, t >= 0 && !q.concat, q, t);
 }
 
 void forward_row(int act, const SwFwd& q, int t, cudaStream_t s) {
@@ -555,8 +578,8 @@ int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t
     if (l.concat)
       rc = tc_gemm(0, X, Wst, partial, nullptr, l.BP, l.NP, l.KX, 1, status, s);
     else
-      rc = tc_gemm(0, train ? q.Rh + (size_t)t * l.BP * l.NP : X, Wst, partial, nullptr, l.BP, (int)l.KX, l.NP, l.ns_z, status,
-                   s, l.nt_z);
+      rc = tc_gemm_chained(train ? q.Rh + (size_t)t * l.BP * l.NP : X, Wst, partial, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z,
+                           status, s);
     if (rc != RINGRNN_OK) return rc;
     forward_row(p.activation, q, t, s);
     RINGRNN_CUDA_TRY(cudaGetLastError());
@@ -617,18 +640,17 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
 
   {
     LaunchScope ls(K_BWD, s);
-    sw_backward_row_kernel<false><<<l.BP, row_threads(l.NP), 0, s>>>(q, -1, p.T - 1);
+    RINGRNN_CUDA_TRY(launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, false, q, -1, p.T - 1));
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   for (int t = p.T - 1; t >= 0; --t) {
     // Z_t[BP, KX] = delta_t[BP, NP] x WstT[KX, NP]^T
-    int rc = tc_gemm(0, Delta + (size_t)t * l.BP * l.NP, WstT, zpart, nullptr, l.BP, (int)l.KX, l.NP, l.ns_z, status, s,
-                     l.nt_z);
+    int rc = tc_gemm_chained(Delta + (size_t)t * l.BP * l.NP, WstT, zpart, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z, status, s);
     if (rc != RINGRNN_OK) return rc;
     {
       LaunchScope ls(K_BWD, s);
-      if (q.grad_A != nullptr) sw_backward_row_kernel<true><<<l.BP, row_threads(l.NP), 0, s>>>(q, t, t - 1);
-      else sw_backward_row_kernel<false><<<l.BP, row_threads(l.NP), 0, s>>>(q, t, t - 1);
+      RINGRNN_CUDA_TRY(q.grad_A != nullptr ? launch_row(sw_backward_row_kernel<true>, l.BP, l.NP, s, true, q, t, t - 1)
+                                           : launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, true, q, t, t - 1));
     }
     RINGRNN_CUDA_TRY(cudaGetLastError());
   }

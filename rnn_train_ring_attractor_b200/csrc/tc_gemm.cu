@@ -116,11 +116,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_p;
+  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
+      grid_wait();
       for (int it = 0; it < iters; ++it) {
         const int s = it % Cfg::NSTAGE;
         const uint32_t round = it / Cfg::NSTAGE;
@@ -170,6 +172,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     // epilogue: warp w owns TMEM lanes 32*(w%4)..+31 = output rows m0 + that
     const int q = warp & 3;
+    grid_wait();  // earlier kernels may still read what this one writes
     const bool ok = mbar_wait(done_bar, 0, wctx, 103);
     tcgen05_fence_after();
     const int row = m0 + q * 32 + lane;
@@ -200,8 +203,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 
 // ---- CTA-pair variant (K-major operands): a cluster of two CTAs owns a 256 x NT output tile; each CTA loads its
-// own 128 rows of A and half of the B rows, the even CTA issues cta_group::2 MMAs for both.  Used by the
-// library self-test to validate the pair building blocks the recurrent kernels rely on.
+// own 128 rows of A and half of the B rows, the even CTA issues cta_group::2 MMAs for both, so that a B tile enters the two
+// SMs once and not twice.  out[split][M_total][N_total], split = blockIdx.z.
+// B must not be written by the kernel before this one: its first stages are fetched while that one still runs.
 template <int NT>
 struct PairCfg {
   static constexpr int KC = 64;
@@ -210,15 +214,16 @@ struct PairCfg {
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int NSTAGE = (200 * 1024) / STAGE < 8 ? (200 * 1024) / STAGE : 8;
   static constexpr int SMEM = NSTAGE * STAGE + 1024 + 256;
+  static constexpr int NI = NT > 256 ? NT / 256 : 1;  // MMA instructions along N per k-step
+  static constexpr int NMMA = NT / NI;
   static constexpr int TMEM_COLS = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : NT <= 256 ? 256 : 512;  // power of two
 };
 
 template <int NT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 float* __restrict__ out, int M_total, int N_total, long long K_total, int* status) {
+                 float* __restrict__ out, int M_total, int N_total, long long K_total, long long k_per_split, int* status) {
   using Cfg = PairCfg<NT>;
-  static_assert(NT <= 256, "one MMA instruction along N");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bars = base + Cfg::NSTAGE * Cfg::STAGE;
@@ -235,7 +240,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t h = cluster_ctarank();  // 0 = even CTA (issues the MMAs), 1 = odd CTA
   const int pair = blockIdx.x >> 1;
   const int m0 = pair * 256 + (int)h * 128, n0 = blockIdx.y * NT;
-  const int iters = (int)((K_total + Cfg::KC - 1) / Cfg::KC);
+  const int k_begin = (int)(blockIdx.z * k_per_split);
+  const int k_end = K_total - k_begin < k_per_split ? (int)K_total : (int)(k_begin + k_per_split);
+  const int iters = k_end > k_begin ? (k_end - k_begin + Cfg::KC - 1) / Cfg::KC : 0;
 
   if (threadIdx.x == 0) {
     *dead = 0;
@@ -253,25 +260,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_wait();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_p;
+  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
+      auto load_b = [&](int it) {
+        const int s = it % Cfg::NSTAGE;
+        const uint32_t b_dst = base + s * Cfg::STAGE + Cfg::A_BYTES;
+        if (h == 0) mbar_arrive_expect_tx(full_bar(s), 2 * Cfg::STAGE);  // both CTAs' bytes land on this barrier
+        for (int nh = 0; nh < Cfg::NI; ++nh)
+          tma_load_2d_pair(b_dst + nh * (Cfg::NMMA / 2) * 128, &tmB, full_bar(s), k_begin + it * Cfg::KC,
+                           n0 + nh * Cfg::NMMA + (int)h * (Cfg::NMMA / 2));
+      };
+      const int early = iters < Cfg::NSTAGE ? iters : Cfg::NSTAGE;
+      for (int it = 0; it < early; ++it) load_b(it);
+      grid_wait();
       for (int it = 0; it < iters; ++it) {
         const int s = it % Cfg::NSTAGE;
-        const uint32_t round = it / Cfg::NSTAGE;
-        if (it >= Cfg::NSTAGE && !mbar_wait(empty_bar(s), (round - 1) & 1u, wctx, 111)) break;
-        const uint32_t a_dst = base + s * Cfg::STAGE, b_dst = a_dst + Cfg::A_BYTES;
-        if (h == 0) mbar_arrive_expect_tx(full_bar(s), 2 * Cfg::STAGE);  // both CTAs' bytes land on this barrier
-        const int k = it * Cfg::KC;
-        tma_load_2d_pair(a_dst, &tmA, full_bar(s), k, m0);
-        tma_load_2d_pair(b_dst, &tmB, full_bar(s), k, n0 + (int)h * (NT / 2));
+        if (it >= Cfg::NSTAGE) {
+          if (!mbar_wait(empty_bar(s), (it / Cfg::NSTAGE - 1) & 1u, wctx, 111)) break;
+          load_b(it);
+        }
+        tma_load_2d_pair(base + s * Cfg::STAGE, &tmA, full_bar(s), k_begin + it * Cfg::KC, m0);
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && h == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(256, NT, 0, 0);
+      constexpr uint32_t idesc = make_idesc_bf16(256, Cfg::NMMA, 0, 0);
       bool ok = true;
       for (int it = 0; it < iters && ok; ++it) {
         const int s = it % Cfg::NSTAGE;
@@ -282,17 +299,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t a_src = base + s * Cfg::STAGE, b_src = a_src + Cfg::A_BYTES;
         const uint32_t a_lo = desc_lo(a_src, 16), b_lo = desc_lo(b_src, 16);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) umma_ss_pair_lo(tmem_base, a_lo + 2 * ks, b_lo + 2 * ks, idesc, (it > 0 || ks > 0) ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+          for (int nh = 0; nh < Cfg::NI; ++nh)
+            umma_ss_pair_lo(tmem_base + nh * Cfg::NMMA, a_lo + 2 * ks, b_lo + nh * ((Cfg::NMMA / 2) * 128 >> 4) + 2 * ks, idesc,
+                            (it > 0 || ks > 0) ? 1u : 0u);
         umma_commit_pair(empty_bar(s), 3);
       }
       umma_commit_pair(done_bar, 3);
     }
   } else {
     const int q = warp & 3;
+    grid_wait();
     const bool ok = mbar_wait(done_bar, 0, wctx, 113);
     tcgen05_fence_after();
     const int row = m0 + q * 32 + lane;
-    float* orow = out + (size_t)row * N_total + n0;
+    float* orow = out + ((size_t)blockIdx.z * M_total + row) * N_total + n0;
     for (int c0 = 0; c0 < NT; c0 += 32) {
       uint32_t v[32];
       if (iters > 0 && ok) {
@@ -318,30 +340,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 }
 
 template <int NT>
-int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int N_total, long long K_total, int* status,
-                     cudaStream_t s) {
+int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int N_total, long long K_total, int nsplit,
+                     bool overlap, int* status, cudaStream_t s) {
   using Cfg = PairCfg<NT>;
   CUtensorMap tmA, tmB;
   if (!make_tmap_bf16_2d(&tmA, A, (uint64_t)M_total, (uint64_t)K_total, 128, 64) ||
-      !make_tmap_bf16_2d(&tmB, B, (uint64_t)N_total, (uint64_t)K_total, NT / 2, 64))
+      !make_tmap_bf16_2d(&tmB, B, (uint64_t)N_total, (uint64_t)K_total, Cfg::NMMA / 2, 64))
     return RINGRNN_ERR_CUDA;
   RINGRNN_CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * (M_total / 256), N_total / NT, 1);
+  cfg.gridDim = dim3(2 * (M_total / 256), N_total / NT, nsplit);
   cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 2 : 1;
+  long long kps = (K_total + nsplit - 1) / nsplit;
+  kps = (kps + Cfg::KC - 1) / Cfg::KC * Cfg::KC;
   {
     LaunchScope ls(K_DW, s);
-    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NT>, tmA, tmB, out, M_total, N_total, K_total, status));
+    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NT>, tmA, tmB, out, M_total, N_total, K_total, kps, status));
   }
   return RINGRNN_OK;
 }
@@ -357,7 +383,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int nspl
 
 template <bool MN_MAJOR, int NT>
 int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N_total, long long K_total, int nsplit,
-                int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr) {
+                int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr, bool overlap = false) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   CUtensorMap tmA, tmB;
   bool ok;
@@ -382,8 +408,19 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
   dim3 grid((M_total + 127) / 128, (N_total + NT - 1) / NT, nsplit);
   {
     LaunchScope ls(K_DW, s);
-    gemm_tc_kernel<MN_MAJOR, NT><<<grid, GEMM_THREADS, Cfg::SMEM, s>>>(tmA, tmB, partial, M_total, N_total, K_total,
-                                                                        kps, chunks_per_slab, status, host_status);
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MN_MAJOR, NT>, tmA, tmB, partial, M_total, N_total, K_total, kps,
+                                        chunks_per_slab, status, host_status));
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   return RINGRNN_OK;
@@ -393,13 +430,12 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
 
 // C[M,N] (fp32, partial sums over nsplit slices then reduced into `out`) = A * B with bf16 operands.
 //   mn_major = 1: A is [K, M], B is [K, N] (row-major);  mn_major = 0: A is [M, K], B is [N, K].
-// nt: tile width to use (128, 256 or 512), 0 = the largest that divides N.
 // M multiple of 128; N in {128, 256, 512} or a multiple of 512 (N % NT == 0).  partial: nsplit*M*N floats.
 int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* out, int M, int N, long long K,
-            int nsplit, int* status, cudaStream_t s, int nt) {
+            int nsplit, int* status, cudaStream_t s) {
   if (M % 128 != 0 || nsplit < 1) return RINGRNN_ERR_SHAPE;
   int rc;
-  const int NT = nt > 0 ? nt : (N % 512 == 0) ? 512 : (N % 256 == 0) ? 256 : (N % 128 == 0) ? 128 : 0;
+  const int NT = (N % 512 == 0) ? 512 : (N % 256 == 0) ? 256 : (N % 128 == 0) ? 128 : 0;
   if (NT == 0) return RINGRNN_ERR_SHAPE;
 #define RINGRNN_GEMM_CASE(MN, NTV)                                                            \
   if (mn_major == MN && NT == NTV) rc = launch_gemm<MN != 0, NTV>(A, B, partial, M, N, K, nsplit, status, s); else
@@ -433,9 +469,25 @@ int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, in
 // CTA-pair K-major GEMM: out[M,N] = A[M,K] * B[N,K]^T, M % 256 == 0, N a multiple of 256, 224 or 128 (the pair MMA wants N % 32 == 0) (N % NT == 0)
 int tc_gemm_pair(const void* A, const void* B, float* out, int M, int N, long long K, int* status, cudaStream_t s) {
   if (M % 256 != 0) return RINGRNN_ERR_SHAPE;
-  if (N % 256 == 0) return launch_gemm_pair<256>(A, B, out, M, N, K, status, s);
-  if (N % 224 == 0) return launch_gemm_pair<224>(A, B, out, M, N, K, status, s);
-  if (N % 128 == 0) return launch_gemm_pair<128>(A, B, out, M, N, K, status, s);
+  if (N % 256 == 0) return launch_gemm_pair<256>(A, B, out, M, N, K, 1, false, status, s);
+  if (N % 224 == 0) return launch_gemm_pair<224>(A, B, out, M, N, K, 1, false, status, s);
+  if (N % 128 == 0) return launch_gemm_pair<128>(A, B, out, M, N, K, 1, false, status, s);
+  return RINGRNN_ERR_SHAPE;
+}
+
+// One GEMM of a chain of kernels with programmatic dependent launch: partial[split][M][N] = A[M,K] * B[N,K]^T with tiles of nt
+// columns, by CTA pairs where M allows.  B must be older than the kernel before this one.
+int tc_gemm_chained(const void* A, const void* B, float* partial, int M, int N, long long K, int nsplit, int nt, int* status,
+                    cudaStream_t s) {
+  if (M % 256 == 0) {
+    if (nt == 512) return launch_gemm_pair<512>(A, B, partial, M, N, K, nsplit, true, status, s);
+    if (nt == 256) return launch_gemm_pair<256>(A, B, partial, M, N, K, nsplit, true, status, s);
+    if (nt == 128) return launch_gemm_pair<128>(A, B, partial, M, N, K, nsplit, true, status, s);
+  } else {
+    if (nt == 512) return launch_gemm<false, 512>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
+    if (nt == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
+    if (nt == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
+  }
   return RINGRNN_ERR_SHAPE;
 }
 
