@@ -56,6 +56,56 @@ namespace {
 
 using namespace tc;
 
+// 2-D fp32 row-major tensor, box of 32 x 32 (128 bytes per row), 128-byte swizzle: what an epilogue warp stores at a time
+bool make_tmap_f32_out(CUtensorMap* out, void* base, uint64_t rows, uint64_t cols) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {cols * 4};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Epilogue warp q (tensor-memory lanes 32q..) writes its 32 rows x NT columns to rows y.. of `out`, 32 columns at a time through
+// eight buffers of 4 KB in the (no longer needed) operand stages.  A thread owns a row: stored from registers, each instruction
+// touches 32 lines, about 9 us for a tile of 128 x 512; TMA stores take what a row's buffer holds in whole lines.
+constexpr int OUT_BUFS = 8, OUT_BYTES = 4 * OUT_BUFS * 4096;
+template <int NT>
+__device__ __forceinline__ void store_tile(const CUtensorMap* out, uint32_t smem, uint32_t tmem, int q, int lane, int x0, int y,
+                                           bool zero) {
+  const uint32_t mine = smem + q * OUT_BUFS * 4096;
+#pragma unroll 1
+  for (int c = 0; c < NT / 32; ++c) {
+    uint32_t v[32];
+    if (!zero) {
+      tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c * 32, v);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = 0u;
+    }
+    if (c >= OUT_BUFS) {
+      if (lane == 0) bulk_wait_read<OUT_BUFS - 1>();
+      __syncwarp();
+    }
+    const uint32_t buf = mine + (c % OUT_BUFS) * 4096;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + lane * 128 + ((j ^ (lane & 7)) << 4)), "r"(v[4 * j]),
+                   "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                   : "memory");
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_2d(out, buf, x0 + c * 32, y);
+      bulk_commit();
+    }
+  }
+  if (lane == 0) bulk_wait_all<0>();
+}
+
 constexpr int GEMM_THREADS = 192;
 
 template <bool MN_MAJOR, int NT>
@@ -80,7 +130,7 @@ struct GemmCfg {
 template <bool MN_MAJOR, int NT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               float* __restrict__ out, int M_total, int N_total, long long K_total, long long k_per_split,
+               const __grid_constant__ CUtensorMap tmOut, int M_total, int N_total, long long K_total, long long k_per_split,
                int chunks_per_slab, int* status, volatile int* host_status) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   extern __shared__ uint8_t smem_raw[];
@@ -175,26 +225,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     grid_wait();  // earlier kernels may still read what this one writes
     const bool ok = mbar_wait(done_bar, 0, wctx, 103);
     tcgen05_fence_after();
-    const int row = m0 + q * 32 + lane;
-    float* orow = out + ((size_t)blockIdx.z * M_total + row) * N_total + n0;
-    for (int c0 = 0; c0 < NT; c0 += 32) {
-      uint32_t v[32];
-      if (iters > 0 && ok) {
-        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c0, v);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0u;
-      }
-      if (row < M_total) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          if (n0 + c0 + j < N_total)
-            *reinterpret_cast<float4*>(orow + c0 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                     __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-        }
-      }
-    }
+    store_tile<NT>(&tmOut, base, tmem_base, q, lane, n0, (int)blockIdx.z * M_total + m0 + q * 32, iters == 0 || !ok);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -205,6 +236,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // ---- CTA-pair variant (K-major operands): a cluster of two CTAs owns a 256 x NT output tile; each CTA loads its
 // own 128 rows of A and half of the B rows, the even CTA issues cta_group::2 MMAs for both, so that a B tile enters the two
 // SMs once and not twice.  out[split][M_total][N_total], split = blockIdx.z.
+// B tiles of the first `keep` columns of the grid are asked to stay in L2, the rest to leave it first.
 // B must not be written by the kernel before this one: its first stages are fetched while that one still runs.
 template <int NT>
 struct PairCfg {
@@ -222,7 +254,7 @@ struct PairCfg {
 template <int NT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 float* __restrict__ out, int M_total, int N_total, long long K_total, long long k_per_split, int* status) {
+                 const __grid_constant__ CUtensorMap tmOut, int M_total, long long K_total, long long k_per_split, int keep, int* status) {
   using Cfg = PairCfg<NT>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -266,13 +298,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
+      const uint64_t policy = (int)blockIdx.y < keep ? l2_policy_evict_last() : l2_policy_evict_first();
       auto load_b = [&](int it) {
         const int s = it % Cfg::NSTAGE;
         const uint32_t b_dst = base + s * Cfg::STAGE + Cfg::A_BYTES;
         if (h == 0) mbar_arrive_expect_tx(full_bar(s), 2 * Cfg::STAGE);  // both CTAs' bytes land on this barrier
         for (int nh = 0; nh < Cfg::NI; ++nh)
-          tma_load_2d_pair(b_dst + nh * (Cfg::NMMA / 2) * 128, &tmB, full_bar(s), k_begin + it * Cfg::KC,
-                           n0 + nh * Cfg::NMMA + (int)h * (Cfg::NMMA / 2));
+          tma_load_2d_pair_hint(b_dst + nh * (Cfg::NMMA / 2) * 128, &tmB, full_bar(s), k_begin + it * Cfg::KC,
+                                n0 + nh * Cfg::NMMA + (int)h * (Cfg::NMMA / 2), policy);
       };
       const int early = iters < Cfg::NSTAGE ? iters : Cfg::NSTAGE;
       for (int it = 0; it < early; ++it) load_b(it);
@@ -313,24 +346,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     grid_wait();
     const bool ok = mbar_wait(done_bar, 0, wctx, 113);
     tcgen05_fence_after();
-    const int row = m0 + q * 32 + lane;
-    float* orow = out + ((size_t)blockIdx.z * M_total + row) * N_total + n0;
-    for (int c0 = 0; c0 < NT; c0 += 32) {
-      uint32_t v[32];
-      if (iters > 0 && ok) {
-        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c0, v);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0u;
-      }
-      if (row < M_total) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(orow + c0 + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
-                                                                   __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-      }
-    }
+    store_tile<NT>(&tmOut, base, tmem_base, q, lane, n0, (int)blockIdx.z * M_total + m0 + q * 32, iters == 0 || !ok);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -343,8 +359,9 @@ template <int NT>
 int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int N_total, long long K_total, int nsplit,
                      bool overlap, int* status, cudaStream_t s) {
   using Cfg = PairCfg<NT>;
-  CUtensorMap tmA, tmB;
-  if (!make_tmap_bf16_2d(&tmA, A, (uint64_t)M_total, (uint64_t)K_total, 128, 64) ||
+  CUtensorMap tmA, tmB, tmOut;
+  if (!make_tmap_f32_out(&tmOut, out, (uint64_t)nsplit * M_total, (uint64_t)N_total) ||
+      !make_tmap_bf16_2d(&tmA, A, (uint64_t)M_total, (uint64_t)K_total, 128, 64) ||
       !make_tmap_bf16_2d(&tmB, B, (uint64_t)N_total, (uint64_t)K_total, Cfg::NMMA / 2, 64))
     return RINGRNN_ERR_CUDA;
   RINGRNN_CUDA_TRY(cudaFuncSetAttribute(gemm_pair_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
@@ -365,9 +382,13 @@ int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int 
   cfg.numAttrs = overlap ? 2 : 1;
   long long kps = (K_total + nsplit - 1) / nsplit;
   kps = (kps + Cfg::KC - 1) / Cfg::KC * Cfg::KC;
+  // A chain reads B again each step.  More of it than L2 holds (126 MB, of which the products take some) would push out all of
+  // itself before it comes round again: 72 MB stay, the rest streams past.
+  const double b_bytes = 2.0 * N_total * K_total, l2 = 72e6;
+  const int tiles = N_total / NT, keep = b_bytes <= l2 ? tiles : (int)(tiles * (l2 / b_bytes));
   {
     LaunchScope ls(K_DW, s);
-    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NT>, tmA, tmB, out, M_total, N_total, K_total, kps, status));
+    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NT>, tmA, tmB, tmOut, M_total, K_total, kps, keep, status));
   }
   return RINGRNN_OK;
 }
@@ -385,7 +406,7 @@ template <bool MN_MAJOR, int NT>
 int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N_total, long long K_total, int nsplit,
                 int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr, bool overlap = false) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmOut;
   bool ok;
   if (MN_MAJOR) {
     ok = make_tmap_bf16_2d(&tmA, A, (uint64_t)K_total, (uint64_t)M_total, Cfg::KC, 64) &&
@@ -395,7 +416,7 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
     ok = make_tmap_bf16_2d(&tmA, A, (uint64_t)slabs * M_total, cols, 128, 64) &&
          make_tmap_bf16_2d(&tmB, B, (uint64_t)slabs * N_total, cols, Cfg::NMMA, 64);
   }
-  if (!ok) return RINGRNN_ERR_CUDA;
+  if (!ok || !make_tmap_f32_out(&tmOut, partial, (uint64_t)nsplit * M_total, (uint64_t)N_total)) return RINGRNN_ERR_CUDA;
   int chunks_per_slab = 0x7fffffff;
   if (slabs > 1) {
     chunks_per_slab = (int)((K_total / slabs + Cfg::KC - 1) / Cfg::KC);
@@ -419,7 +440,7 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MN_MAJOR, NT>, tmA, tmB, partial, M_total, N_total, K_total, kps,
+    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MN_MAJOR, NT>, tmA, tmB, tmOut, M_total, N_total, K_total, kps,
                                         chunks_per_slab, status, host_status));
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
