@@ -25,7 +25,8 @@
 // Roles (128 + 256 U threads): warp 0 issues the MMAs, warp 1 allocates tensor memory, warp 2 stages the per-sample
 // scalars (action signal, loss coefficients) eight steps at a time, the last 8 U warps are the epilogue: unit u has eight,
 // warp w of them owns lanes 32 (w & 3).. and the half h = w >> 2 of the unit's samples (E = S/2 per thread).
-// U = 2 units of S samples run side by side in a CTA, one unit's MMAs under the other's epilogue.
+// U = 2 units of S samples run side by side in a CTA, one unit's MMAs under the other's epilogue.  Unit u of the c-th of G
+// clusters takes tiles c + G (u + U round), so that a last round of up to G tiles has one, and is faster, in every CTA.
 #pragma once
 
 #include "tc_recurrent.cuh"
@@ -144,13 +145,14 @@ struct Cfg {
 };
 
 // barrier block
-constexpr uint32_t B_STATE = 0;      // [2 units][2] the operand of the next step is complete: used alternately, because a CTA
-                                     // may send the state after the next before a third one's arrival for this one lands
-constexpr uint32_t B_DFULL = 32;     // [2] the accumulators of the step are complete
-constexpr uint32_t B_SC_FULL = 48;   // [2 units][2]
-constexpr uint32_t B_SC_FREE = 80;   // [2 units][2]
-constexpr uint32_t B_TMEM = 112;
-constexpr uint32_t B_DEAD = 116;
+constexpr uint32_t B_STATE = 0;      // [units x CTAs of the cluster <= 4][2] that CTA's neurons of the next operand are complete:
+                                     // the two are used alternately, because a CTA may send the state after the next before
+                                     // a third one's arrival for this one lands
+constexpr uint32_t B_DFULL = 64;     // [2] the accumulators of the step are complete
+constexpr uint32_t B_SC_FULL = 80;   // [2 units][2]
+constexpr uint32_t B_SC_FREE = 112;  // [2 units][2]
+constexpr uint32_t B_TMEM = 144;
+constexpr uint32_t B_DEAD = 148;
 
 template <class C>
 struct Ctx {
@@ -177,7 +179,7 @@ __device__ __forceinline__ Ctx<C> setup(uint8_t* smem_raw, int units, const floa
     for (int u = 0; u < units; ++u) {
       mbar_init(c.bars + B_DFULL + 8 * u, 1);
       for (int i = 0; i < 2; ++i) {
-        mbar_init(c.bars + B_STATE + 16 * u + 8 * i, 8 * C::CL);  // the epilogue warps of every CTA of the cluster
+        for (int q = 0; q < C::CL; ++q) mbar_init(c.bars + B_STATE + 16 * (u * C::CL + q) + 8 * i, 8);  // its epilogue warps
         mbar_init(c.bars + B_SC_FULL + 16 * u + 8 * i, 1);
         mbar_init(c.bars + B_SC_FREE + 16 * u + 8 * i, 8);
       }
@@ -269,12 +271,13 @@ __device__ __forceinline__ void load_weights(const Ctx<C>& c, const float* const
 }
 
 // MMA issuer (one whole warp, see umma_ts_warp; everything the instructions are built from is uniform).  Unit u's tile of
-// a round exists iff tile + u < n_ut.
+// a round exists iff tile + u * stride / U < n_ut.
 template <class C, int NP, int S, int U>
 __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride, int n_ut, int T, int n_const, int code) {
   constexpr uint32_t idesc = make_idesc_bf16(128, S, 0, 1);
   const uint32_t lead = elect_one();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, c.tmem, 0), base = __shfl_sync(0xffffffffu, c.base, 0);
+  const uint32_t tmem = __shfl_sync(0xffffffffu, c.tmem, 0), base = __shfl_sync(0xffffffffu, c.base, 0),
+                 rank = __shfl_sync(0xffffffffu, c.rank, 0);
   uint32_t g[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) g[u] = 0;
@@ -282,33 +285,42 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
     for (int t = 0; t < T; ++t) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (tile + u >= n_ut) continue;
-        const bool ok = mbar_wait<(C::CL > 1)>(c.bars + B_STATE + 16 * u + 8 * (g[u] & 1u), (g[u] >> 1) & 1u, c.w, code);
-        if (!__all_sync(0xffffffffu, ok)) return;
-        if (C::CL > 1) fence_proxy_async_all();
-        tcgen05_fence_after();
+        if (tile + u * (stride / U) >= n_ut) continue;
         const uint32_t st = base + (u * C::ST_BUFS + (C::ST_BUFS > 1 ? (g[u] & 1u) : 0u)) * C::ST_BYTES;
-        const uint64_t b0 = C::ST_ROW == 32 ? desc_sw32(desc_lo(st, 16)) : desc_sw128(desc_lo(st, 16));
-        constexpr uint32_t B_STEP = C::ST_ROW;  // 16 rows, in units of 16 bytes
         const uint32_t d = tmem + u * 3 * S;
+        constexpr uint32_t B_STEP = C::ST_ROW;  // 16 rows, in units of 16 bytes
+        // the neurons of one CTA at a time, this CTA's own first: the peers' are still on their way
+#pragma unroll 1
+        for (uint32_t i = 0; i < C::CL; ++i) {
+          const uint32_t q = rank ^ i;
+          const bool ok = mbar_wait<(C::CL > 1)>(c.bars + B_STATE + 16 * (u * C::CL + q) + 8 * (g[u] & 1u), (g[u] >> 1) & 1u, c.w, code);
+          if (!__all_sync(0xffffffffu, ok)) return;
+          if (C::CL > 1) fence_proxy_async_all();
+          tcgen05_fence_after();
+          const uint64_t b0 = (C::ST_ROW == 32 ? desc_sw32(desc_lo(st, 16)) : desc_sw128(desc_lo(st, 16))) + q * 8 * B_STEP;
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
+          for (int m = 0; m < 3; ++m) {
 #pragma unroll
-          for (int ks = 0; ks < C::KS; ++ks) {
-            const int w = m * C::KS + ks;
-            if (w < C::NTK) {
-              umma_ts_warp(d + m * S, tmem + C::C_W + w * 8, b0 + ks * B_STEP, idesc, ks > 0, lead);
-            } else {
-              const uint64_t a0 = desc_sw128(desc_lo(base + C::OFF_W, 16));
-              umma_ss_warp(d + m * S, a0 + (w - C::NTK) / 4 * 1024 + 2 * ((w - C::NTK) & 3), b0 + ks * B_STEP, idesc, ks > 0, lead);
+            for (int ks = 0; ks < 8; ++ks) {
+              const int w = m * C::KS + (int)q * 8 + ks;
+              const bool acc = ks > 0 || i > 0;
+              // where the K step is kept: known at compile time except for the one matrix that is cut (NP = 512)
+              const bool in_tmem = (C::NTK % C::KS != 0 && m == C::NTK / C::KS) ? w < C::NTK : m < C::NTK / C::KS;
+              if (in_tmem) {
+                umma_ts_warp(d + m * S, tmem + C::C_W + w * 8, b0 + ks * B_STEP, idesc, acc, lead);
+              } else {
+                const uint64_t a0 = desc_sw128(desc_lo(base + C::OFF_W, 16));
+                umma_ss_warp(d + m * S, a0 + (uint32_t)((w - C::NTK) / 4 * 1024 + 2 * ((w - C::NTK) & 3)), b0 + ks * B_STEP, idesc,
+                             acc, lead);
+              }
             }
           }
-        }
 #pragma unroll 1
-        for (int i = 0; i < n_const; ++i) {
+          for (int x = 0; x < n_const; ++x) {
 #pragma unroll
-          for (int ks = 0; ks < C::KS; ++ks)
-            umma_ts_warp(d, tmem + C::C_CONST + 8 * i, b0 + ks * B_STEP, idesc, true, lead);
+            for (int ks = 0; ks < 8; ++ks)
+              umma_ts_warp(d, tmem + C::C_CONST + 8 * x, b0 + ks * B_STEP, idesc, true, lead);
+          }
         }
         if (lead) umma_commit(c.bars + B_DFULL + 8 * u);
         __syncwarp();
@@ -318,33 +330,37 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
   }
 }
 
-// Publishes this thread's E new state values (packed bf16 pairs): into row `row` of operand buffer g & 1, here and in the
-// peers, then one arrival per warp on the state barriers of that buffer.
+// Publishes this thread's E new state values (packed bf16 pairs): into row `row` of operand buffer g & 1, first here, so that
+// the MMAs on this CTA's own neurons start, then in the peers; one arrival per warp each.
 template <class C, int S>
 __device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed, uint32_t g, int u, int row_k, int h,
                                         int lane) {
   const uint32_t parity = g & 1u;
   const uint32_t buf = c.base + (u * C::ST_BUFS + (C::ST_BUFS > 1 ? parity : 0u)) * C::ST_BYTES + row_k * C::ST_ROW;
   const uint32_t swizzle = C::ST_ROW == 32 ? ((uint32_t)row_k >> 2) & 1u : (uint32_t)row_k & 7u;
+  const uint32_t bar = c.bars + B_STATE + 16 * (u * C::CL + c.rank) + 8 * parity;
+  auto addr = [&](int v) { return buf + (((uint32_t)(h * (C::E / 8) + v) ^ swizzle) << 4); };
 #pragma unroll
-  for (int v = 0; v < C::E / 8; ++v) {
-    const uint32_t addr = buf + (((uint32_t)(h * (C::E / 8) + v) ^ swizzle) << 4);
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(packed[4 * v]), "r"(packed[4 * v + 1]),
+  for (int v = 0; v < C::E / 8; ++v)
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr(v)), "r"(packed[4 * v]), "r"(packed[4 * v + 1]),
                  "r"(packed[4 * v + 2]), "r"(packed[4 * v + 3])
                  : "memory");
-#pragma unroll
-    for (uint32_t peer = 1; peer < C::CL; ++peer)
-      st_cluster_v4(mapa(addr, c.rank ^ peer), packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-  }
-  if (C::CL > 1) fence_proxy_async_all();
-  else fence_proxy_async_smem();
+  fence_proxy_async_smem();
   tcgen05_fence_before();  // this thread's accumulator reads precede the MMAs the arrival releases
   __syncwarp();
-  if (lane == 0) {
-    const uint32_t bar = c.bars + B_STATE + 16 * u + 8 * parity;
-    mbar_arrive(bar);
+  if (lane == 0) mbar_arrive(bar);
+  if (C::CL > 1) {
 #pragma unroll
-    for (uint32_t peer = 1; peer < C::CL; ++peer) mbar_arrive_cluster(bar, c.rank ^ peer);
+    for (uint32_t peer = 1; peer < C::CL; ++peer)
+#pragma unroll
+      for (int v = 0; v < C::E / 8; ++v)
+        st_cluster_v4(mapa(addr(v), c.rank ^ peer), packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+    fence_proxy_async_all();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+      for (uint32_t peer = 1; peer < C::CL; ++peer) mbar_arrive_cluster(bar, c.rank ^ peer);
+    }
   }
 }
 
@@ -355,7 +371,7 @@ __device__ __forceinline__ void scalar_role(const Ctx<C>& c, int u, int first, i
                                             Src src) {
   const int lane = threadIdx.x & 31;
   uint32_t chunk = 0;
-  for (int tile = first + u; tile < n_ut; tile += stride) {
+  for (int tile = first; tile < n_ut; tile += stride) {
     const int b0 = tile * S;
     for (int e0 = 0; e0 < T; e0 += CH, ++chunk) {
       const uint32_t buf = chunk & 1u;

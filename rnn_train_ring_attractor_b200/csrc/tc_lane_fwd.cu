@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
   extern __shared__ uint8_t smem_raw[];
   const Ctx<C> c = setup<C>(smem_raw, U, p.dec_u, p.dec_v, p.N, p.status, p.report, p.zero_report, p.host);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int first = (int)(blockIdx.x / C::CL) * U, stride = (int)(gridDim.x / C::CL) * U;
+  const int first = (int)(blockIdx.x / C::CL), groups = (int)(gridDim.x / C::CL), stride = groups * U;
   const int T = p.T;
   const bool epi = warp >= 4;
   const int u = epi ? (warp - 4) >> 3 : 0;            // unit
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
     if (warp == 0) {
       mma_role<C, NP, S, U>(c, first, stride, p.n_ut, T, p.n_const, 202);
     } else if (warp >= 2 && warp - 2 < U) {
-      scalar_role<C, S, 2>(c, warp - 2, first, stride, p.n_ut, T, p.B, 203, [&](int i, int b, int e) {
+      scalar_role<C, S, 2>(c, warp - 2, first + (warp - 2) * groups, stride, p.n_ut, T, p.B, 203, [&](int i, int b, int e) {
         const int col = i == 0 ? p.colL : p.colR;
         return col >= 0 ? __ldg(p.A + ((size_t)b * p.T_total + p.t0 + e) * p.a_dim + col) : 0.f;
       });
@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
     const bool live = n < p.N;
     const float J1 = live ? p.J1 : 0.f;  // padding neurons: the constant tile reaches them too, their state stays zero
     const f32x2 J1p = pk2(J1, J1), alphap = pk2(p.alpha, p.alpha), betap = pk2(1.f - p.alpha, 1.f - p.alpha);
+    const bool want_ta = p.dec[0][2] != nullptr, want_dh = p.Dh != nullptr;
     const bool want_dec = p.dec[0][0] != nullptr || p.dec[0][1] != nullptr || p.dec[0][2] != nullptr;
     const int tid = threadIdx.x - 128 - 256 * u;  // within the unit
     const uint32_t d_base = c.tmem + lane_base + u * 3 * S + h * E;
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
     float* const decb = reinterpret_cast<float*>(c.gen + C::OFF_DEC + u * C::DEC_BYTES);
     const float2* const uv = reinterpret_cast<const float2*>(c.gen + C::OFF_UV);
     uint32_t g = 0, chunk = 0;
-    for (int ut = first + u; ut < p.n_ut; ut += stride) {
+    for (int ut = first + u * groups; ut < p.n_ut; ut += stride) {
       const int b0 = ut * S + h * E;
       float master[E];
       uint32_t packed[E / 2];
@@ -114,9 +115,11 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
               const f32x2 r2 = fma2(alphap, f2[i], mul2(betap, pk2(master[e], master[e + 1])));
               upk2(r2, master[e], master[e + 1]);
               packed[e / 2] = pack_bf16x2(master[e], master[e + 1]);
-              float da, db;
-              upk2(d2[i], da, db);
-              dpk[e / 2] = pack_bf16x2(da, db);
+              if (want_dh) {
+                float da, db;
+                upk2(d2[i], da, db);
+                dpk[e / 2] = pack_bf16x2(da, db);
+              }
             }
           }
         }
@@ -127,7 +130,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
           if (lane == 0) mbar_arrive(c.bars + B_SC_FREE + 16 * u + 8 * (chunk & 1u));
           ++chunk;
         }
-        if (p.Dh != nullptr) {
+        if (want_dh) {
 #pragma unroll
           for (int v = 0; v < E / 8; ++v)
             st_cs_v4(p.Dh + dh_offset<C, S>(t, p.n_ut, ut, c.rank, h, v, row), dpk[4 * v], dpk[4 * v + 1], dpk[4 * v + 2],
@@ -192,16 +195,21 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
               const float2 w = uv[nn];
               a[0] = fmaf(r.x, w.x, a[0]); a[1] = fmaf(r.y, w.x, a[1]); a[2] = fmaf(r.z, w.x, a[2]); a[3] = fmaf(r.w, w.x, a[3]);
               a[4] = fmaf(r.x, w.y, a[4]); a[5] = fmaf(r.y, w.y, a[5]); a[6] = fmaf(r.z, w.y, a[6]); a[7] = fmaf(r.w, w.y, a[7]);
-              a[8] += fabsf(r.x); a[9] += fabsf(r.y); a[10] += fabsf(r.z); a[11] += fabsf(r.w);
-            }
-            half_warp_sums<12>(a, lane);
-            if ((lane & 3) == 0) {
-              const int v0 = 6 * ((lane >> 3) & 1) + 3 * ((lane >> 2) & 1);
-#pragma unroll
-              for (int i = 0; i < 3; ++i) {
-                const int kind = (v0 + i) / 4, s = quad * 4 + (v0 + i) % 4;
-                dec_t[(kind * S + s) * 8 + (t & 7)] = a[i];
+              if (want_ta) {
+                a[8] += fabsf(r.x); a[9] += fabsf(r.y); a[10] += fabsf(r.z); a[11] += fabsf(r.w);
               }
+            }
+            auto put = [&](int v0, int n) {  // the first n of a[] are values v0.. of [kind][sample of the quad]
+#pragma unroll
+              for (int i = 0; i < 3; ++i)
+                if (i < n) dec_t[((v0 + i) / 4 * S + quad * 4 + (v0 + i) % 4) * 8 + (t & 7)] = a[i];
+            };
+            if (want_ta) {
+              half_warp_sums<12>(a, lane);
+              if ((lane & 3) == 0) put(6 * ((lane >> 3) & 1) + 3 * ((lane >> 2) & 1), 3);
+            } else {  // a roll-out asks for the two angles' sums only
+              half_warp_sums<8>(a, lane);
+              if ((lane & 3) == 0) put(4 * ((lane >> 3) & 1) + 2 * ((lane >> 2) & 1), 2);
             }
           }
           // eight steps at a time to global memory, one chunk behind: the barrier above orders the sums of the
