@@ -41,7 +41,6 @@ struct SwLayout {
   long long KX;               // (1 + n_act) * NP
   bool concat;                // forward: one long operand X instead of all products Z
   int nt_z, ns_z;             // tile width and split-K factor of the Z GEMM
-  int ns_dw;                  // split-K factor of the weight-gradient GEMM
 };
 
 int sw_active(const RingRnnProblem& p) { return p.n_active < 0 ? p.a_dim : p.n_active; }
@@ -84,10 +83,15 @@ SwLayout sw_layout(const RingRnnProblem& p) {
   const int nt_fwd = (l.NP % 512 == 0) ? 512 : (l.NP % 256 == 0) ? 256 : 128;
   l.concat = splits_for((long long)(l.BP / 128) * (l.NP / nt_fwd), l.KX) == 1;
   z_shape(l.BP, l.KX, l.NP, &l.nt_z, &l.ns_z);
-  const int nt_dw = (l.KX % 512 == 0) ? 512 : (l.KX % 256 == 0) ? 256 : 128;
-  l.ns_dw = splits_for((long long)(l.NP / 128) * (l.KX / nt_dw), (long long)p.T * l.BP);
   return l;
 }
+// split-K factor of the weight-gradient GEMM over T steps
+int dw_splits(const SwLayout& l, int T) {
+  const int nt_dw = (l.KX % 512 == 0) ? 512 : (l.KX % 256 == 0) ? 256 : 128;
+  return splits_for((long long)(l.NP / 128) * (l.KX / nt_dw), (long long)T * l.BP);
+}
+int sw_ckpt_interval(const RingRnnProblem& p) { return (p.ckpt_every > 0 && p.ckpt_every < p.T) ? p.ckpt_every : 0; }
+size_t ckpt_slot(const RingRnnProblem& p) { return sizeof(float) * (size_t)p.B * p.N; }
 
 int row_threads(int NP) { return NP / 4 < ROW_MAX ? NP / 4 : ROW_MAX; }  // NP is a multiple of 128
 
@@ -173,8 +177,10 @@ __global__ void __launch_bounds__(256) sw_prep_transposed_kernel(const float* __
       to_bf16x4(make_float4(tile[i][j], tile[i + 1][j], tile[i + 2][j], tile[i + 3][j]));
 }
 
+// A pass may cover steps [t0, t0 + T) of a sequence of T_total (a stretch between checkpoints): the action signal, the decode
+// sums, grad_output and the loss coefficients are indexed with the global step, everything else with the local one.
 struct SwFwd {
-  int B, T, N, NP, BP, a_dim, nsplit;
+  int B, T, N, NP, BP, a_dim, nsplit, t0, T_total;
   long long KX;
   bool concat;             // partial [nsplit = 1][BP][NP] and X; otherwise Z [nsplit][BP][KX]
   bool vec;                // the caller's rows of N floats start on 16-byte boundaries
@@ -194,6 +200,8 @@ struct SwFwd {
   float* dec_ta;
   const float* dec_u;
   const float* dec_v;
+  float* ckpt;             // [ceil(T/ckpt_every)][B][N]: slot c receives the state after step c*ckpt_every - 1, or nullptr
+  int ckpt_every;
   SwCols cols;
 };
 
@@ -211,7 +219,7 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
   const bool build = t + 1 < q.T;
   const int t_c = q.concat ? t + 1 : t;
   for (int k = threadIdx.x; k <= n; k += blockDim.x)
-    coef[k] = k == 0 ? 1.f : (valid && t_c >= 0 && t_c < q.T) ? __ldg(q.A + ((size_t)b * q.T + t_c) * q.a_dim + q.cols.c[k - 1]) : 0.f;
+    coef[k] = k == 0 ? 1.f : (valid && t_c >= 0 && t_c < q.T) ? __ldg(q.A + ((size_t)b * q.T_total + q.t0 + t_c) * q.a_dim + q.cols.c[k - 1]) : 0.f;
   tc::grid_launch_dependents();
   tc::grid_wait();  // everything below may depend on the kernels before
   const float s_prev = (t >= 0) ? q.rowsum[b] : 0.f;
@@ -252,6 +260,8 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
           }
         const float4 r4 = make_float4(r[0], r[1], r[2], r[3]);
         if (q.hist != nullptr) row_st(q.hist + ((size_t)t * q.B + b) * q.N, i, q.N, q.vec, r4);
+        if (q.ckpt != nullptr && t + 1 < q.T && (t + 1) % q.ckpt_every == 0)
+          row_st(q.ckpt + ((size_t)((t + 1) / q.ckpt_every) * q.B + b) * q.N, i, q.N, q.vec, r4);
         if (q.final_state != nullptr && t + 1 == q.T) row_st(q.final_state + (size_t)b * q.N, i, q.N, q.vec, r4);
       }
       if (q.Dh != nullptr)
@@ -279,7 +289,7 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
   if (t >= 0 && valid && (dec || q.dec_ta != nullptr)) {
     const float sx = block_sum(px, red), sy = block_sum(py, red), sa = block_sum(pa, red);
     if (threadIdx.x == 0) {
-      const size_t o = (size_t)b * q.T + t;
+      const size_t o = (size_t)b * q.T_total + q.t0 + t;
       if (q.dec_x != nullptr) q.dec_x[o] = sx;
       if (q.dec_y != nullptr) q.dec_y[o] = sy;
       if (q.dec_ta != nullptr) q.dec_ta[o] = sa;
@@ -288,7 +298,8 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
 }
 
 struct SwBwd {
-  int B, T, N, NP, BP, a_dim, nsplit;
+  int B, T, N, NP, BP, a_dim, nsplit, t0, T_total;
+  bool resume;               // the first carry is what the stretch after this one left in g; otherwise zero
   long long KX;
   bool vec;                  // as in SwFwd
   float J0, alpha;
@@ -323,12 +334,13 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
   const float beta = 1.f - q.alpha;
   float cx = 0.f, cy = 0.f, cs = 0.f;
   if (valid && t_delta >= 0 && q.coef_x != nullptr) {
-    cx = q.coef_x[(size_t)b * q.T + t_delta];
-    cy = q.coef_y[(size_t)b * q.T + t_delta];
-    cs = q.coef_s[(size_t)b * q.T + t_delta];
+    const size_t bt = (size_t)b * q.T_total + q.t0 + t_delta;
+    cx = q.coef_x[bt];
+    cy = q.coef_y[bt];
+    cs = q.coef_s[bt];
   }
   for (int k = threadIdx.x; k <= n; k += blockDim.x)
-    coef[k] = k == 0 ? 1.f : (valid && t_carry >= 0) ? __ldg(q.A + ((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k - 1]) : 0.f;
+    coef[k] = k == 0 ? 1.f : (valid && t_carry >= 0) ? __ldg(q.A + ((size_t)b * q.T_total + q.t0 + t_carry) * q.a_dim + q.cols.c[k - 1]) : 0.f;
   if (WANT_DA)
     for (int x = threadIdx.x; x < (1 + n) * (ROW_MAX / 32); x += blockDim.x) da[x] = 0.f;
   tc::grid_launch_dependents();
@@ -359,11 +371,13 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
       const float js = q.J0 * sd;
       carry = make_float4(carry.x + fmaf(beta, go.x, js), carry.y + fmaf(beta, go.y, js), carry.z + fmaf(beta, go.z, js),
                           carry.w + fmaf(beta, go.w, js));
+    } else if (t_carry < 0 && q.resume) {
+      carry = ld4(g + j);
     }
     if (t_delta >= 0) {
       float gg[4] = {carry.x, carry.y, carry.z, carry.w};
       float4 go = make_float4(0.f, 0.f, 0.f, 0.f), rt = go;
-      if (valid && q.grad_output != nullptr) go = row_ld(q.grad_output + ((size_t)t_delta * q.B + b) * q.N, j, q.N, q.vec);
+      if (valid && q.grad_output != nullptr) go = row_ld(q.grad_output + ((size_t)(q.t0 + t_delta) * q.B + b) * q.N, j, q.N, q.vec);
       if (valid && q.coef_x != nullptr)
         rt = of_bf16x4(*reinterpret_cast<const uint2*>(q.Rh + ((size_t)(t_delta + 1) * q.BP + b) * q.NP + j));
       const float gs[4] = {go.x, go.y, go.z, go.w}, rr[4] = {rt.x, rt.y, rt.z, rt.w};
@@ -386,8 +400,9 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
                                              q.alpha * dact.w * gg[3]));
       *reinterpret_cast<uint2*>(q.Delta + ((size_t)t_delta * q.BP + b) * q.NP + j) = db;
       ds += sum4(of_bf16x4(db));
-    } else if (valid && q.grad_r_init != nullptr) {
-      row_st(q.grad_r_init + (size_t)b * q.N, j, q.N, q.vec, carry);
+    } else {
+      if (valid && q.grad_r_init != nullptr) row_st(q.grad_r_init + (size_t)b * q.N, j, q.N, q.vec, carry);
+      if (q.t0 > 0) st4(g + j, carry);
     }
   }
   if (t_delta >= 0) {
@@ -399,7 +414,7 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       float v = 0.f;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += da[(1 + k) * (ROW_MAX / 32) + w];
-      q.grad_A[((size_t)b * q.T + t_carry) * q.a_dim + q.cols.c[k]] = v;
+      q.grad_A[((size_t)b * q.T_total + q.t0 + t_carry) * q.a_dim + q.cols.c[k]] = v;
     }
   }
 }
@@ -407,13 +422,13 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
 // Xall[t][b][m*NP + j] = c_m(b,t) * r_{t-1}[b,j] for all t: the B operand of the weight-gradient GEMM.
 // grid (BP, T), four neurons per thread
 __global__ void __launch_bounds__(ROW_MAX) sw_build_xall_kernel(const __nv_bfloat16* __restrict__ Rh, const float* __restrict__ A,
-                                                                SwCols cols, int B, int T, int a_dim, int NP, int BP,
+                                                                SwCols cols, int B, int t0, int T_total, int a_dim, int NP, int BP,
                                                                 long long KX, __nv_bfloat16* __restrict__ Xall) {
   const int b = blockIdx.x, t = blockIdx.y;
   const bool valid = b < B;
   const __nv_bfloat16* r = Rh + ((size_t)t * BP + b) * NP;
   __nv_bfloat16* x = Xall + ((size_t)t * BP + b) * KX;
-  const float* at = A + ((size_t)b * T + t) * a_dim;
+  const float* at = A + ((size_t)b * T_total + t0 + t) * a_dim;
   for (int j = threadIdx.x * 4; j < NP; j += blockDim.x * 4) {
     const uint2 rb = *reinterpret_cast<const uint2*>(r + j);
     const float4 rf = of_bf16x4(rb);
@@ -424,6 +439,10 @@ __global__ void __launch_bounds__(ROW_MAX) sw_build_xall_kernel(const __nv_bfloa
       *reinterpret_cast<uint2*>(x + (size_t)(1 + k) * NP + j) = to_bf16x4(make_float4(c * rf.x, c * rf.y, c * rf.z, c * rf.w));
     }
   }
+}
+
+__global__ void sw_accumulate_kernel(float* __restrict__ out, const float* __restrict__ in, size_t n) {
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) out[e] += in[e];
 }
 
 // dWst [NP][KX] -> grad_Wo = J1 * block 0 (the operand block 0 is the unscaled state), raw = block 0,
@@ -507,21 +526,77 @@ size_t stepwise_fwd_workspace_bytes(const RingRnnProblem& p) {
   return 1024 + align_up((size_t)l.NP * l.KX * 2, 1024) + x_bytes(l) + align_up((size_t)l.BP * l.NP * 4, 1024) +
          align_up((size_t)l.BP * 4, 1024) + z_bytes(l, l.concat);
 }
-// SAVED: Rh [T+1][BP][NP] | Dh [T][BP][NP] (bf16)
-size_t stepwise_saved_bytes(const RingRnnProblem& p) {
-  const SwLayout l = sw_layout(p);
-  return align_up((size_t)(p.T + 1) * l.BP * l.NP * 2, 1024) + align_up((size_t)p.T * l.BP * l.NP * 2, 1024);
+// SAVED: Rh [T+1][BP][NP] | Dh [T][BP][NP] (bf16); with checkpoints fp32 states [ceil(T/K)][B][N]
+static size_t every_step_bytes(const SwLayout& l, int T) {
+  return align_up((size_t)(T + 1) * l.BP * l.NP * 2, 1024) + align_up((size_t)T * l.BP * l.NP * 2, 1024);
 }
-// BWD workspace: status(1024) | WstT | Delta [T][BP][NP] | g | sum_delta | Z partials | Xall [T][BP][KX] |
-//                dW partials | dWst | raw
+size_t stepwise_saved_bytes(const RingRnnProblem& p) {
+  const int K = sw_ckpt_interval(p);
+  if (K > 0) return align_up((size_t)((p.T + K - 1) / K) * ckpt_slot(p), 1024);
+  return every_step_bytes(sw_layout(p), p.T);
+}
+// BWD workspace (K = p.T without checkpoints): status(1024) | WstT | Delta [K][BP][NP] | g | sum_delta | Z | Xall [K][BP][KX] |
+//                dW partials | dWst | raw; with checkpoints also weights | X | state | rowsum | saved stretch | dWst of a stretch
 size_t stepwise_bwd_workspace_bytes(const RingRnnProblem& p) {
   const SwLayout l = sw_layout(p);
-  return 1024 + align_up((size_t)l.KX * l.NP * 2, 1024) + align_up((size_t)p.T * l.BP * l.NP * 2, 1024) +
-         align_up((size_t)l.BP * l.NP * 4, 1024) + align_up((size_t)l.BP * 4, 1024) +
-         z_bytes(l, false) + align_up((size_t)p.T * l.BP * l.KX * 2, 1024) +
-         align_up((size_t)l.ns_dw * l.NP * l.KX * 4, 1024) + align_up((size_t)l.NP * l.KX * 4, 1024) +
-         align_up((size_t)p.N * p.N * 4, 1024);
+  const int K = sw_ckpt_interval(p), T = K > 0 ? K : p.T;
+  const size_t w_bytes = align_up((size_t)l.KX * l.NP * 2, 1024), dw_bytes = align_up((size_t)l.NP * l.KX * 4, 1024);
+  const size_t state_bytes = align_up((size_t)l.BP * l.NP * 4, 1024), row_bytes = align_up((size_t)l.BP * 4, 1024);
+  size_t n = 1024 + w_bytes + align_up((size_t)T * l.BP * l.NP * 2, 1024) + state_bytes + row_bytes + z_bytes(l, false) +
+             align_up((size_t)T * l.BP * l.KX * 2, 1024) + align_up((size_t)dw_splits(l, T) * l.NP * l.KX * 4, 1024) + dw_bytes +
+             align_up((size_t)p.N * p.N * 4, 1024);
+  if (K > 0) n += w_bytes + x_bytes(l) + state_bytes + row_bytes + every_step_bytes(l, K) + dw_bytes;
+  return n;
 }
+
+namespace {
+
+struct SwFwdBuffers {
+  __nv_bfloat16* W;
+  __nv_bfloat16* X;
+  float* state;
+  float* rowsum;
+  float* partial;
+  int* status;
+};
+
+int prepare_forward(const RingRnnProblem& p, const DevProblem& dp, const SwLayout& l, const SwFwdBuffers& m, cudaStream_t s) {
+  LaunchScope ls(K_PREP, s);
+  const bool vec = p.N % 4 == 0 && aligned16(p.Wo) && aligned16(dp.Wa);
+  sw_prep_weights_kernel<<<dim3(prep_blocks(l), l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols_of(dp), p.J1, p.N, l.NP,
+                                                                        l.concat ? l.KX : l.NP,
+                                                                        l.concat ? l.NP : (long long)l.NP * l.NP, vec, m.W);
+  RINGRNN_CUDA_TRY(cudaGetLastError());
+  return RINGRNN_OK;
+}
+
+// Steps [q.t0, q.t0 + q.T) from q.r_init; the caller has set the outputs it wants.
+int run_forward(const RingRnnProblem& p, const DevProblem& dp, const SwLayout& l, const SwFwdBuffers& m, SwFwd q, cudaStream_t s) {
+  q.B = p.B; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.concat ? 1 : l.ns_z;
+  q.T_total = p.T;
+  q.concat = l.concat;
+  q.vec = p.N % 4 == 0 && aligned16(q.r_init) && aligned16(q.hist) && aligned16(q.final_state) && aligned16(q.ckpt);
+  q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
+  q.A = p.A; q.partial = m.partial; q.state = m.state; q.rowsum = m.rowsum;
+  q.X = l.concat || q.Rh == nullptr ? m.X : nullptr;
+  q.cols = cols_of(dp);
+  forward_row(p.activation, q, -1, s);
+  RINGRNN_CUDA_TRY(cudaGetLastError());
+  for (int t = 0; t < q.T; ++t) {
+    int rc;
+    if (l.concat)
+      rc = tc_gemm(0, m.X, m.W, m.partial, nullptr, l.BP, l.NP, l.KX, 1, m.status, s);
+    else
+      rc = tc_gemm_chained(q.Rh != nullptr ? q.Rh + (size_t)t * l.BP * l.NP : m.X, m.W, m.partial, l.BP, (int)l.KX, l.NP, l.ns_z,
+                           l.nt_z, m.status, s);
+    if (rc != RINGRNN_OK) return rc;
+    forward_row(p.activation, q, t, s);
+    RINGRNN_CUDA_TRY(cudaGetLastError());
+  }
+  return RINGRNN_OK;
+}
+
+}  // namespace
 
 int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) {
   const RingRnnProblem& p = a.p;
@@ -532,59 +607,37 @@ int stepwise_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t
   if (train && (a.saved_bytes < stepwise_saved_bytes(p) || (reinterpret_cast<uintptr_t>(a.saved) & 255) != 0))
     return RINGRNN_ERR_WORKSPACE;
   char* w = static_cast<char*>(a.workspace);
-  int* status = a.status != nullptr ? a.status : reinterpret_cast<int*>(w);
+  SwFwdBuffers m;
+  m.status = a.status != nullptr ? a.status : reinterpret_cast<int*>(w);
   w += 1024;
-  __nv_bfloat16* Wst = reinterpret_cast<__nv_bfloat16*>(w);
+  m.W = reinterpret_cast<__nv_bfloat16*>(w);
   w += align_up((size_t)l.NP * l.KX * 2, 1024);
-  __nv_bfloat16* X = reinterpret_cast<__nv_bfloat16*>(w);
+  m.X = reinterpret_cast<__nv_bfloat16*>(w);
   w += x_bytes(l);
-  float* state = reinterpret_cast<float*>(w);
+  m.state = reinterpret_cast<float*>(w);
   w += align_up((size_t)l.BP * l.NP * 4, 1024);
-  float* rowsum = reinterpret_cast<float*>(w);
+  m.rowsum = reinterpret_cast<float*>(w);
   w += align_up((size_t)l.BP * 4, 1024);
-  float* partial = reinterpret_cast<float*>(w);
-  if (a.status == nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
-
-  const SwCols cols = cols_of(dp);
-  {
-    LaunchScope ls(K_PREP, s);
-    const bool vec = p.N % 4 == 0 && aligned16(p.Wo) && aligned16(dp.Wa);
-    sw_prep_weights_kernel<<<dim3(prep_blocks(l), l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP,
-                                                                          l.concat ? l.KX : l.NP,
-                                                                          l.concat ? l.NP : (long long)l.NP * l.NP, vec, Wst);
-  }
-  RINGRNN_CUDA_TRY(cudaGetLastError());
-
+  m.partial = reinterpret_cast<float*>(w);
+  if (a.status == nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(m.status, 0, sizeof(int), s));
+  const int K = train ? sw_ckpt_interval(p) : 0;
+  if (K > 0)  // checkpoint 0 is the initial state
+    RINGRNN_CUDA_TRY(cudaMemcpyAsync(a.saved, p.r_init, ckpt_slot(p), cudaMemcpyDeviceToDevice, s));
+  const int rc = prepare_forward(p, dp, l, m, s);
+  if (rc != RINGRNN_OK) return rc;
   SwFwd q;
   memset(&q, 0, sizeof(q));
-  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.concat ? 1 : l.ns_z;
-  q.concat = l.concat;
-  q.vec = p.N % 4 == 0 && aligned16(p.r_init) && aligned16(a.bump_history) && aligned16(a.final_state);
-  q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
-  q.A = p.A; q.r_init = p.r_init; q.partial = partial; q.state = state; q.rowsum = rowsum;
-  q.Rh = train ? static_cast<__nv_bfloat16*>(a.saved) : nullptr;
-  q.Dh = train ? reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(a.saved) +
-                                                   align_up((size_t)(p.T + 1) * l.BP * l.NP * 2, 1024))
-               : nullptr;
-  q.X = l.concat || !train ? X : nullptr;
+  q.T = p.T;
+  q.r_init = p.r_init;
+  if (train && K == 0) {
+    q.Rh = static_cast<__nv_bfloat16*>(a.saved);
+    q.Dh = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(a.saved) + align_up((size_t)(p.T + 1) * l.BP * l.NP * 2, 1024));
+  }
+  q.ckpt = K > 0 ? static_cast<float*>(a.saved) : nullptr;
+  q.ckpt_every = K;
   q.hist = a.bump_history; q.final_state = a.final_state;
   q.dec_x = a.dec_x; q.dec_y = a.dec_y; q.dec_ta = a.dec_ta; q.dec_u = a.dec_u; q.dec_v = a.dec_v;
-  q.cols = cols;
-
-  forward_row(p.activation, q, -1, s);
-  RINGRNN_CUDA_TRY(cudaGetLastError());
-  for (int t = 0; t < p.T; ++t) {
-    int rc;
-    if (l.concat)
-      rc = tc_gemm(0, X, Wst, partial, nullptr, l.BP, l.NP, l.KX, 1, status, s);
-    else
-      rc = tc_gemm_chained(train ? q.Rh + (size_t)t * l.BP * l.NP : X, Wst, partial, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z,
-                           status, s);
-    if (rc != RINGRNN_OK) return rc;
-    forward_row(p.activation, q, t, s);
-    RINGRNN_CUDA_TRY(cudaGetLastError());
-  }
-  return RINGRNN_OK;
+  return run_forward(p, dp, l, m, q, s);
 }
 
 int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s) {
@@ -594,29 +647,35 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
   if ((reinterpret_cast<uintptr_t>(a.workspace) & 255) != 0) return RINGRNN_ERR_WORKSPACE;
   if (a.saved == nullptr || a.saved_bytes < stepwise_saved_bytes(p) || (reinterpret_cast<uintptr_t>(a.saved) & 255) != 0)
     return RINGRNN_ERR_WORKSPACE;
+  const int K = sw_ckpt_interval(p), Tk = K > 0 ? K : p.T;  // steps of one stretch
+  const size_t w_bytes = align_up((size_t)l.KX * l.NP * 2, 1024), dw_bytes = align_up((size_t)l.NP * l.KX * 4, 1024);
   char* w = static_cast<char*>(a.workspace);
-  int* status = a.status != nullptr ? a.status : reinterpret_cast<int*>(w);
-  w += 1024;
-  __nv_bfloat16* WstT = reinterpret_cast<__nv_bfloat16*>(w);
-  w += align_up((size_t)l.KX * l.NP * 2, 1024);
-  __nv_bfloat16* Delta = reinterpret_cast<__nv_bfloat16*>(w);
-  w += align_up((size_t)p.T * l.BP * l.NP * 2, 1024);
-  float* g = reinterpret_cast<float*>(w);
-  w += align_up((size_t)l.BP * l.NP * 4, 1024);
-  float* sum_delta = reinterpret_cast<float*>(w);
-  w += align_up((size_t)l.BP * 4, 1024);
-  float* zpart = reinterpret_cast<float*>(w);
-  w += z_bytes(l, false);
-  __nv_bfloat16* Xall = reinterpret_cast<__nv_bfloat16*>(w);
-  w += align_up((size_t)p.T * l.BP * l.KX * 2, 1024);
-  float* dwpart = reinterpret_cast<float*>(w);
-  w += align_up((size_t)l.ns_dw * l.NP * l.KX * 4, 1024);
-  float* dWst = reinterpret_cast<float*>(w);
-  w += align_up((size_t)l.NP * l.KX * 4, 1024);
-  float* raw = reinterpret_cast<float*>(w);
-  const __nv_bfloat16* Rh = static_cast<const __nv_bfloat16*>(a.saved);
-  const __nv_bfloat16* Dh = reinterpret_cast<const __nv_bfloat16*>(static_cast<const char*>(a.saved) +
-                                                                    align_up((size_t)(p.T + 1) * l.BP * l.NP * 2, 1024));
+  auto take = [&w](size_t bytes) { char* at = w; w += bytes; return at; };
+  int* scratch_status = reinterpret_cast<int*>(take(1024));
+  int* status = a.status != nullptr ? a.status : scratch_status;
+  __nv_bfloat16* WstT = reinterpret_cast<__nv_bfloat16*>(take(w_bytes));
+  __nv_bfloat16* Delta = reinterpret_cast<__nv_bfloat16*>(take(align_up((size_t)Tk * l.BP * l.NP * 2, 1024)));
+  float* g = reinterpret_cast<float*>(take(align_up((size_t)l.BP * l.NP * 4, 1024)));
+  float* sum_delta = reinterpret_cast<float*>(take(align_up((size_t)l.BP * 4, 1024)));
+  float* zpart = reinterpret_cast<float*>(take(z_bytes(l, false)));
+  __nv_bfloat16* Xall = reinterpret_cast<__nv_bfloat16*>(take(align_up((size_t)Tk * l.BP * l.KX * 2, 1024)));
+  float* dwpart = reinterpret_cast<float*>(take(align_up((size_t)dw_splits(l, Tk) * l.NP * l.KX * 4, 1024)));
+  float* dWst = reinterpret_cast<float*>(take(dw_bytes));
+  float* raw = reinterpret_cast<float*>(take(align_up((size_t)p.N * p.N * 4, 1024)));
+  SwFwdBuffers m;
+  memset(&m, 0, sizeof(m));
+  char* stretch = nullptr;
+  float* dWst_stretch = nullptr;
+  if (K > 0) {
+    m.W = reinterpret_cast<__nv_bfloat16*>(take(w_bytes));
+    m.X = reinterpret_cast<__nv_bfloat16*>(take(x_bytes(l)));
+    m.state = reinterpret_cast<float*>(take(align_up((size_t)l.BP * l.NP * 4, 1024)));
+    m.rowsum = reinterpret_cast<float*>(take(align_up((size_t)l.BP * 4, 1024)));
+    m.partial = zpart;
+    m.status = status;
+    stretch = take(every_step_bytes(l, K));
+    dWst_stretch = reinterpret_cast<float*>(take(dw_bytes));
+  }
   if (a.status == nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
 
   const SwCols cols = cols_of(dp);
@@ -625,43 +684,70 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
     sw_prep_transposed_kernel<<<dim3(l.NP / 32, l.NP / 32, l.blocks), 256, 0, s>>>(p.Wo, dp.Wa, cols, p.J1, p.N, l.NP, WstT);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
+  if (K > 0) {
+    const int rc = prepare_forward(p, dp, l, m, s);
+    if (rc != RINGRNN_OK) return rc;
+  }
   if (a.grad_A != nullptr)
     RINGRNN_CUDA_TRY(cudaMemsetAsync(a.grad_A, 0, sizeof(float) * (size_t)p.B * p.T * p.a_dim, s));
 
-  SwBwd q;
-  memset(&q, 0, sizeof(q));
-  q.B = p.B; q.T = p.T; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.ns_z;
-  q.vec = p.N % 4 == 0 && aligned16(a.grad_output) && aligned16(a.grad_r_init);
-  q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
-  q.A = p.A; q.grad_output = a.grad_output;
-  q.coef_x = a.coef_x; q.coef_y = a.coef_y; q.coef_s = a.coef_s; q.dec_u = a.dec_u; q.dec_v = a.dec_v;
-  q.Rh = Rh; q.Dh = Dh; q.partial = zpart; q.g = g; q.sum_delta = sum_delta; q.Delta = Delta;
-  q.grad_r_init = a.grad_r_init; q.grad_A = a.grad_A; q.cols = cols;
-
-  {
-    LaunchScope ls(K_BWD, s);
-    RINGRNN_CUDA_TRY(launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, false, q, -1, p.T - 1));
-  }
-  RINGRNN_CUDA_TRY(cudaGetLastError());
-  for (int t = p.T - 1; t >= 0; --t) {
-    // Z_t[BP, KX] = delta_t[BP, NP] x WstT[KX, NP]^T
-    int rc = tc_gemm_chained(Delta + (size_t)t * l.BP * l.NP, WstT, zpart, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z, status, s);
-    if (rc != RINGRNN_OK) return rc;
+  // With checkpoints the stretches of K steps are taken last to first: each is recomputed from its fp32 state, then run in
+  // reverse from the carry the later stretch left in g, and its weight gradients are added to the total.
+  const int n_ck = (p.T + Tk - 1) / Tk;
+  for (int c = n_ck - 1; c >= 0; --c) {
+    const int t0 = c * Tk, Tc = p.T - t0 < Tk ? p.T - t0 : Tk;
+    char* kept = K > 0 ? stretch : static_cast<char*>(const_cast<void*>(a.saved));
+    __nv_bfloat16* Rh = reinterpret_cast<__nv_bfloat16*>(kept);
+    __nv_bfloat16* Dh = reinterpret_cast<__nv_bfloat16*>(kept + align_up((size_t)(Tc + 1) * l.BP * l.NP * 2, 1024));
+    if (K > 0) {
+      SwFwd f;
+      memset(&f, 0, sizeof(f));
+      f.T = Tc; f.t0 = t0;
+      f.r_init = static_cast<const float*>(a.saved) + (size_t)c * p.B * p.N;
+      f.Rh = Rh; f.Dh = Dh;
+      const int rc = run_forward(p, dp, l, m, f, s);
+      if (rc != RINGRNN_OK) return rc;
+    }
+    SwBwd q;
+    memset(&q, 0, sizeof(q));
+    q.B = p.B; q.T = Tc; q.N = p.N; q.NP = l.NP; q.BP = l.BP; q.a_dim = p.a_dim; q.nsplit = l.ns_z;
+    q.t0 = t0; q.T_total = p.T;
+    q.resume = c != n_ck - 1;
+    q.grad_r_init = c == 0 ? a.grad_r_init : nullptr;
+    q.vec = p.N % 4 == 0 && aligned16(a.grad_output) && aligned16(q.grad_r_init);
+    q.KX = l.KX; q.J0 = p.J0; q.alpha = p.alpha;
+    q.A = p.A; q.grad_output = a.grad_output;
+    q.coef_x = a.coef_x; q.coef_y = a.coef_y; q.coef_s = a.coef_s; q.dec_u = a.dec_u; q.dec_v = a.dec_v;
+    q.Rh = Rh; q.Dh = Dh; q.partial = zpart; q.g = g; q.sum_delta = sum_delta; q.Delta = Delta;
+    q.grad_A = a.grad_A; q.cols = cols;
     {
+      LaunchScope ls(K_BWD, s);
+      RINGRNN_CUDA_TRY(launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, false, q, -1, Tc - 1));
+    }
+    for (int t = Tc - 1; t >= 0; --t) {
+      // Z_t[BP, KX] = delta_t[BP, NP] x WstT[KX, NP]^T
+      const int rc = tc_gemm_chained(Delta + (size_t)t * l.BP * l.NP, WstT, zpart, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z, status, s);
+      if (rc != RINGRNN_OK) return rc;
       LaunchScope ls(K_BWD, s);
       RINGRNN_CUDA_TRY(q.grad_A != nullptr ? launch_row(sw_backward_row_kernel<true>, l.BP, l.NP, s, true, q, t, t - 1)
                                            : launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, true, q, t, t - 1));
     }
+    {
+      LaunchScope ls(K_PREP, s);
+      sw_build_xall_kernel<<<dim3(l.BP, Tc), row_threads(l.NP), 0, s>>>(Rh, p.A, cols, p.B, t0, p.T, p.a_dim, l.NP, l.BP, l.KX, Xall);
+    }
     RINGRNN_CUDA_TRY(cudaGetLastError());
+    // dWst[NP, KX] = Delta^T [NP, Tc*BP] x Xall [Tc*BP, KX]
+    const bool first = c == n_ck - 1;
+    const int rc = tc_gemm(1, Delta, Xall, dwpart, first ? dWst : dWst_stretch, l.NP, (int)l.KX, (long long)Tc * l.BP,
+                           dw_splits(l, Tc), status, s);
+    if (rc != RINGRNN_OK) return rc;
+    if (!first) {
+      LaunchScope ls(K_REDUCE, s);
+      sw_accumulate_kernel<<<592, 256, 0, s>>>(dWst, dWst_stretch, (size_t)l.NP * l.KX);
+      RINGRNN_CUDA_TRY(cudaGetLastError());
+    }
   }
-  {
-    LaunchScope ls(K_PREP, s);
-    sw_build_xall_kernel<<<dim3(l.BP, p.T), row_threads(l.NP), 0, s>>>(Rh, p.A, cols, p.B, p.T, p.a_dim, l.NP, l.BP, l.KX, Xall);
-  }
-  RINGRNN_CUDA_TRY(cudaGetLastError());
-  // dWst[NP, KX] = Delta^T [NP, T*BP] x Xall [T*BP, KX]
-  int rc = tc_gemm(1, Delta, Xall, dwpart, dWst, l.NP, (int)l.KX, (long long)p.T * l.BP, l.ns_dw, status, s);
-  if (rc != RINGRNN_OK) return rc;
   const size_t NN = (size_t)p.N * p.N;
   RINGRNN_CUDA_TRY(cudaMemsetAsync(a.grad_Wa, 0, sizeof(float) * (size_t)p.a_dim * NN, s));
   {
@@ -671,7 +757,7 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
   RINGRNN_CUDA_TRY(cudaGetLastError());
   if (a.grad_J != nullptr) {
     // the dW split-K partials are dead after the reduction inside tc_gemm: their storage serves as scratch
-    rc = launch_grad_j(raw, p.Wo, NN, a.grad_J, reinterpret_cast<double*>(dwpart), s);
+    const int rc = launch_grad_j(raw, p.Wo, NN, a.grad_J, reinterpret_cast<double*>(dwpart), s);
     if (rc != RINGRNN_OK) return rc;
   }
   return RINGRNN_OK;
