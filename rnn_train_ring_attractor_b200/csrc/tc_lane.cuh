@@ -7,7 +7,7 @@
 // 32 or 64 small MMAs, one accumulator read of S/2 columns per thread, the activation, a store of the new state.
 //
 //   NP = 128: one CTA.  NP = 256: a cluster of two CTAs, CTA q owns neurons [128q, 128q+128) and stores its half of the new
-//   state into both CTAs' operand buffers (16-byte distributed-shared-memory stores; the buffers alternate, so nobody waits
+//   state into both CTAs' operand buffers (16-byte asynchronous stores through distributed shared memory; the buffers alternate, so nobody waits
 //   for a peer's MMAs: a peer that has sent r_t has finished the MMAs that read r_{t-2}).
 //
 //   NP = 512: a cluster of four, likewise, 16 samples per cluster.
@@ -179,7 +179,9 @@ __device__ __forceinline__ Ctx<C> setup(uint8_t* smem_raw, int units, const floa
     for (int u = 0; u < units; ++u) {
       mbar_init(c.bars + B_DFULL + 8 * u, 1);
       for (int i = 0; i < 2; ++i) {
-        for (int q = 0; q < C::CL; ++q) mbar_init(c.bars + B_STATE + 16 * (u * C::CL + q) + 8 * i, 8);  // its epilogue warps
+        // own neurons: one arrival per epilogue warp; a peer's: counted in bytes, armed by the MMA warp
+        for (int q = 0; q < C::CL; ++q)
+          mbar_init(c.bars + B_STATE + 16 * (u * C::CL + q) + 8 * i, q == (int)c.rank ? 8 : 1);
         mbar_init(c.bars + B_SC_FULL + 16 * u + 8 * i, 1);
         mbar_init(c.bars + B_SC_FREE + 16 * u + 8 * i, 8);
       }
@@ -290,6 +292,11 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
         const uint32_t d = tmem + u * 3 * S;
         constexpr uint32_t B_STEP = C::ST_ROW;  // 16 rows, in units of 16 bytes
         // the neurons of one CTA at a time, this CTA's own first: the peers' are still on their way
+        if (C::CL > 1 && lead) {
+          for (uint32_t i = 1; i < C::CL; ++i)
+            mbar_arrive_expect_tx(c.bars + B_STATE + 16 * (u * C::CL + (rank ^ i)) + 8 * (g[u] & 1u), 128 * S * 2);
+        }
+        __syncwarp();
 #pragma unroll 1
         for (uint32_t i = 0; i < C::CL; ++i) {
           const uint32_t q = rank ^ i;
@@ -330,8 +337,9 @@ __device__ __forceinline__ void mma_role(const Ctx<C>& c, int first, int stride,
   }
 }
 
-// Publishes this thread's E new state values (packed bf16 pairs): into row `row` of operand buffer g & 1, first here, so that
-// the MMAs on this CTA's own neurons start, then in the peers; one arrival per warp each.
+// Publishes this thread's E new state values (packed bf16 pairs) into row `row` of operand buffer g & 1: sent to the peers
+// (asynchronous stores, counted on their barriers), then stored here, where the MMAs on this CTA's own neurons start first.
+// The reader of a peer's part orders it against the tensor core's reads by a proxy fence behind its wait.
 template <class C, int S>
 __device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed, uint32_t g, int u, int row_k, int h,
                                         int lane) {
@@ -341,6 +349,13 @@ __device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed,
   const uint32_t bar = c.bars + B_STATE + 16 * (u * C::CL + c.rank) + 8 * parity;
   auto addr = [&](int v) { return buf + (((uint32_t)(h * (C::E / 8) + v) ^ swizzle) << 4); };
 #pragma unroll
+  for (uint32_t peer = 1; peer < C::CL; ++peer) {
+    const uint32_t peer_bar = mapa(bar, c.rank ^ peer);
+#pragma unroll
+    for (int v = 0; v < C::E / 8; ++v)
+      st_async_v4(mapa(addr(v), c.rank ^ peer), peer_bar, packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
+  }
+#pragma unroll
   for (int v = 0; v < C::E / 8; ++v)
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr(v)), "r"(packed[4 * v]), "r"(packed[4 * v + 1]),
                  "r"(packed[4 * v + 2]), "r"(packed[4 * v + 3])
@@ -349,19 +364,6 @@ __device__ __forceinline__ void publish(const Ctx<C>& c, const uint32_t* packed,
   tcgen05_fence_before();  // this thread's accumulator reads precede the MMAs the arrival releases
   __syncwarp();
   if (lane == 0) mbar_arrive(bar);
-  if (C::CL > 1) {
-#pragma unroll
-    for (uint32_t peer = 1; peer < C::CL; ++peer)
-#pragma unroll
-      for (int v = 0; v < C::E / 8; ++v)
-        st_cluster_v4(mapa(addr(v), c.rank ^ peer), packed[4 * v], packed[4 * v + 1], packed[4 * v + 2], packed[4 * v + 3]);
-    fence_proxy_async_all();
-    __syncwarp();
-    if (lane == 0) {
-#pragma unroll
-      for (uint32_t peer = 1; peer < C::CL; ++peer) mbar_arrive_cluster(bar, c.rank ^ peer);
-    }
-  }
 }
 
 // Scalar stage (one warp per unit): scalars of entry e = eight at a time, entry e of quantity i for sample s at

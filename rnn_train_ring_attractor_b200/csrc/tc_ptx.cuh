@@ -206,6 +206,14 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// 16 bytes into another CTA of the cluster, counted on a barrier there (both addresses from mapa): the waiter sees the data
+// without a fence and a separate arrival of the sender
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];" ::"r"(addr), "r"(bar),
+               "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+
 // ---- programmatic dependent launch: let the next kernel of the stream start its set-up / wait for the previous kernels
 // and their writes.  Both do nothing in a launch without the attribute.
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
