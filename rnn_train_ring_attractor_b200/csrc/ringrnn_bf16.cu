@@ -128,13 +128,16 @@ Layout layout_of(const RingRnnProblem& p) {
 // ringrnn_stepwise.cu) is faster up to 2048 samples.  Operator forward and backward, T = 32, stepwise against persistent, ms:
 // B = 2048: N = 256 with 6 columns 1.11 / 1.43, N = 384 with 3 1.23 / 1.54, N = 512 with 8 1.99 / 2.10, N = 128 with 6 1.02 /
 // 1.02; B = 4096, N = 256 with 6: 1.85 / 1.49.
+// N > 512 with up to two columns: clusters of eight take 18 us per step of either direction at any batch, one GEMM per step
+// less than that up to 512 samples.  Training step, T = 64, stepwise against persistent, ms: N = 1024 B = 32 1.79 / 2.44, 256
+// 2.00 / 2.55, 512 2.29 / 2.62, 1024 3.22 / 2.75; N = 600 B = 100 1.53 / 2.42, 1000 2.71 / 2.69.
 // RINGRNN_STEPWISE=1 sends every bf16 request to the stepwise path (for comparisons).
 bool bf16_supported(const RingRnnProblem& p) {
   static const bool force_stepwise = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
   if (force_stepwise) return false;
   const int NP = padded_n(p.N), n_act = n_active_of(p);
   if (NP == 0 || p.B < 1 || p.T < 1) return false;
-  if (n_act <= 2) return true;
+  if (n_act <= 2) return NP <= 512 || p.B > 512;
   return NP <= 512 && n_act <= RINGRNN_MAX_ACTIVE && p.B > 2048;
 }
 

@@ -39,10 +39,10 @@ CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), 
 # one GEMM per step (more than two action columns): neurons off and on multiples of four (single and 16-byte accesses) and
 # beyond one round of 512 threads x 4 neurons, one and several K splits, and a batch that takes the concatenated operand
 STEPWISE = [(65, 3, 2, 3, "tanh", -0.1, 0.1), (130, 129, 3, 4, "silu", -0.1, 0.1), (384, 200, 3, 8, "gelu", -0.05, 0.1),
-            (600, 1900, 2, 3, "tanh", -0.02, 0.1), (2180, 5, 2, 3, "tanh", -0.01, 0.1)]
+            (600, 1900, 2, 3, "tanh", -0.02, 0.1), (2180, 5, 2, 3, "tanh", -0.01, 0.1), (513, 512, 2, 2, "tanh", -0.02, 0.1)]
 
-# persistent tiles of 128 samples with several weight groups: batches above the stepwise path's
-GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1)]
+# persistent tiles of 128 samples with several weight groups, and with two K rounds: batches above the stepwise path's
+GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1), (1000, 513, 3, 2, "tanh", -0.02, 0.1)]
 
 
 @pytest.mark.parametrize("prec,shape", [("bf16", s) for s in LANE + STEPWISE + GENERIC] + [("fp32", s) for s in CLUSTER],
