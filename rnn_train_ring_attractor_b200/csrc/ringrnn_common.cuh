@@ -135,7 +135,7 @@ size_t bf16_bwd_workspace_bytes(const RingRnnProblem& p);
 int bf16_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s);
 int bf16_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s);
 
-// bf16, N <= 256 and up to two active columns: neurons on the tensor-memory lanes (ringrnn_lane.cu)
+// bf16, N <= 256 (small batches: 512) and up to two active columns: neurons on the tensor-memory lanes (ringrnn_lane.cu)
 bool lane_supported(const RingRnnProblem& p);
 size_t lane_fwd_workspace_bytes(const RingRnnProblem& p);
 size_t lane_saved_bytes(const RingRnnProblem& p);

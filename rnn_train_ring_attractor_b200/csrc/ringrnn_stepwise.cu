@@ -1,8 +1,8 @@
 // bf16 mode, stepwise variant: one tensor-core GEMM per timestep instead of a persistent kernel.
 //
-// Used for shapes the persistent tcgen05 kernels do not take (N > 1024, or N > 512 with more than two active action
-// columns), i.e. the large-N, wide-action-signal rows of the reference's published latency table, where the batch
-// is small (256) and one step is already a full-machine GEMM.  Replaces, for those shapes, the same reference
+// Used for shapes the persistent tcgen05 kernels do not take, or would leave most of the machine idle on (bf16_supported in
+// ringrnn_bf16.cu has the lines): N > 1024, more than two active action columns at N > 512 or up to 2048 samples, N > 512 up to
+// 512 samples.  Replaces, for those shapes, the same reference
 // kernels as the persistent path (cpp/kernels/fwd_1loop_tc_idx.cuh:265-277 and the five per-step launches of
 // cpp/kernels/bwd_mixed_precision_aggressive.cuh:564-671), without materialising W_eff[B,N,N].
 //
@@ -141,7 +141,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // bf16 copy of the matrices, zero padded, block 0 scaled by J1: element (i, j) of block m at i*ld_i + m*ld_m + j.
-// grid (x, blocks), block 256.  Streams 4 bytes in and 2 out per element; 17 matrices of 2048^2: 427 MB.
+// grid (x, blocks), block 256.  Bound by memory: 4 bytes in and 2 out per element, 17 matrices of 2048^2 (428 MB) in 67 us =
+// 6.4 TB/s.
 __global__ void __launch_bounds__(256) sw_prep_weights_kernel(const float* __restrict__ Wo, const float* __restrict__ Wa,
                                                               SwCols cols, float J1, int N, int NP, long long ld_i,
                                                               long long ld_m, bool vec, __nv_bfloat16* __restrict__ out) {
@@ -207,7 +208,8 @@ struct SwFwd {
 
 // One block per padded sample row, four neurons per thread.  t >= 0: finishes step t (r_t from the GEMM of step t), then
 // builds the operand of step t+1.  t = -1: loads r_init and builds the operand of step 0.  Bound by the latency of its
-// loads: all of a thread's products of a step are in flight together.
+// loads: all of a thread's products of a step are in flight together (one float at a time, eight neurons per thread in turn:
+// 256 samples of N = 2048 with 18 partial sums took about 40 us, now 12 with the products coming from HBM).
 template <int ACT>
 __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t) {
   __shared__ float red[ROW_MAX / 32];

@@ -634,7 +634,7 @@ int tc_backward_launch(int NP, bool pair, const CUtensorMap& tmW, const CUtensor
     if (NP == 512) return launch_bwd_tc<512, false, true>(tmW, tmDL, tmDL32, p, s);
     return RINGRNN_ERR_UNSUPPORTED;
   }
-  // (two active columns and N <= 256: tc_lane_bwd.cu)
+  // (two active columns, N <= 256 and small batches of N <= 512: tc_lane_bwd.cu)
   if (NP == 512) return pair ? launch_bwd_tc<512, true>(tmW, tmDL, tmDL32, p, s) : launch_bwd_tc<512, false>(tmW, tmDL, tmDL32, p, s);
   if (NP == 1024 && !pair) return launch_bwd_tc<1024, false>(tmW, tmDL, tmDL32, p, s);  // two K rounds per step, clusters of 8
   return RINGRNN_ERR_UNSUPPORTED;

@@ -411,7 +411,7 @@ int tc_forward_launch(int act, int NP, bool pair, const CUtensorMap& tmW, const 
 #undef RINGRNN_TCG
     return RINGRNN_ERR_UNSUPPORTED;
   }
-// (two active columns and N <= 256: tc_lane_fwd.cu)
+// (two active columns, N <= 256 and small batches of N <= 512: tc_lane_fwd.cu)
 #define RINGRNN_TCF(ACT, NPV)                                                              \
   if (act == ACT && NP == NPV)                                                             \
     return pair ? launch_fwd_tc<ACT, NPV, true>(tmW, tmR0, p, s) : launch_fwd_tc<ACT, NPV, false>(tmW, tmR0, p, s);

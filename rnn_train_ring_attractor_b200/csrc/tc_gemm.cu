@@ -235,7 +235,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ---- CTA-pair variant (K-major operands): a cluster of two CTAs owns a 256 x NT output tile; each CTA loads its
 // own 128 rows of A and half of the B rows, the even CTA issues cta_group::2 MMAs for both, so that a B tile enters the two
-// SMs once and not twice.  out[split][M_total][N_total], split = blockIdx.z.
+// SMs once and not twice.  [256 x 2048] x [2048 x 34816]: 57 us by single CTAs with tiles of 128 x 512, 50 by pairs, 37 with the
+// TMA stores and the L2 policy.  out[split][M_total][N_total], split = blockIdx.z.
 // B tiles of the first `keep` columns of the grid are asked to stay in L2, the rest to leave it first.
 // B must not be written by the kernel before this one: its first stages are fetched while that one still runs.
 template <int NT>

@@ -22,6 +22,9 @@
 // B operand.  [NP rows = neurons] x [64 samples] bf16, 128 bytes per row, 128-byte swizzle ("MN-major"); an MMA reads the
 // first S samples.  NP = 512, where shared memory is short: 16 samples, 32 bytes per row, 32-byte swizzle.  A thread owns a neuron, so it writes its new values as 16-byte pieces of a row.
 //
+// What it gives over tiles of 128 samples, training steps: N = 120 B = 128 T = 120 1274 -> 315 us (428 with the old host path),
+// N = 256 B = 1024 T = 256 3390 -> 1200, N = 512 B = 64 T = 64 1464 -> 772; roll-out N = 120 B = 65536 T = 4000 65.0 -> 46.1 ms.
+//
 // Roles (128 + 256 U threads): warp 0 issues the MMAs, warp 1 allocates tensor memory, warp 2 stages the per-sample
 // scalars (action signal, loss coefficients) eight steps at a time, the last 8 U warps are the epilogue: unit u has eight,
 // warp w of them owns lanes 32 (w & 3).. and the half h = w >> 2 of the unit's samples (E = S/2 per thread).
