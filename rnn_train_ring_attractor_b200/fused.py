@@ -200,16 +200,18 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
 
 
 class TrainStep:
-    """Loss and weight gradients of one batch in ONE library call (ringrnn_train_step), for callers that need no autograd
-    graph: ``step((A, r_init, target), inv_count, grad_buffer)`` fills ``grad_buffer`` = [dWo | dWa | dJ0 dJ1] (None: a
-    buffer of its own) and returns the two loss parts, a tensor of their own.  ``write`` is the same with the parts as the
-    next two elements of the buffer (dp.grad_buffer_numel), for a caller that wants them there."""
+    """Loss and weight gradients of one batch in ONE library call (ringrnn_train_step): ``step((A, r_init, target),
+    inv_count, grad_buffer)`` fills ``grad_buffer`` = [dWo | dWa | dJ0 dJ1] (None: a buffer of its own) and returns the two
+    loss parts, a tensor of their own.  ``write`` is the same with the parts as the next two elements of the buffer
+    (dp.grad_buffer_numel), for a caller that wants them there.  Inputs that require a gradient (A, r_init, J0, J1) receive
+    theirs too, by way of ring_rnn_fused and its autograd graph."""
 
     def __init__(self, Wa, J0, J1, Wo, alpha, activation, bump_weight=0.2, precision=None, ckpt_every=0):
         if activation not in _lib.ACT:
             raise ValueError(f"Invalid activation '{activation}'. Must be one of {list(_lib.ACT.keys())}.")
         self.Wa, self.Wo = Wa, Wo
-        self.J0, self.J1, self.alpha, self.act = J0, J1, alpha, _lib.ACT[activation]
+        self.J0, self.J1, self.alpha = J0, J1, alpha
+        self.activation, self.act = activation, _lib.ACT[activation]
         self.bump_weight, self.precision, self.ckpt_every = bump_weight, precision, int(ckpt_every)
         self._bytes = {}
 
@@ -236,6 +238,13 @@ class TrainStep:
             raise RuntimeError("shape mismatch between action_signal, Wa, Wo and r_init")
         if grad_buffer.numel() < n_grad + (4 if parts_in_buffer else 2):
             raise RuntimeError("grad_buffer must hold [dWo | dWa | dJ0 dJ1]")
+        if torch.is_grad_enabled() and any(torch.is_tensor(t) and t.requires_grad for t in (A, r_init, self.J0, self.J1)):
+            # somebody upstream (a gain network, an encoder of the initial state, trained J0 / J1) waits for a gradient
+            loss, parts, _, _ = ring_rnn_fused(A, Wa.detach(), self.J0, self.J1, Wo.detach(), r_init, self.alpha,
+                                               self.activation, target, self.bump_weight, inv_count, self.precision,
+                                               grad_buffer, self.ckpt_every)
+            loss.backward()
+            return grad_buffer[n_grad + 2:n_grad + 4].copy_(parts) if parts_in_buffer else parts
         dev = A.device
         active = active_columns(A)
         prec = plan(B, T, N, a_dim, self.act, len(active), self.precision, 0, self.ckpt_every)[0]

@@ -164,6 +164,37 @@ def test_step_function_called_directly():
     assert not torch.equal(changed, kept)
 
 
+@pytest.mark.parametrize("through_train_step", [False, True])
+def test_step_function_reaches_what_requires_grad(through_train_step):
+    """A signal out of a gain network, a learnt initial state and trained J0 / J1 receive their gradients."""
+    from rnn_train_ring_attractor_b200 import dp
+    from rnn_train_ring_attractor_b200.fused import ring_rnn_fused
+    N, B, T = 40, 20, 6
+    case = orc.make_case(N, B, T, "tanh", seed=6)
+    A0, Wa, Wo, r0, tgt = (t.cuda() for t in (case.A, case.Wa, case.Wo, case.r_init, case.target))
+
+    def leaves():
+        return [torch.ones(2, device="cuda", requires_grad=True), r0.clone().requires_grad_(True)] + [
+            torch.tensor(x, device="cuda", requires_grad=True) for x in (-0.1, 0.1)]
+
+    gain, r, J0, J1 = got = leaves()
+    buf = torch.full((dp.grad_buffer_numel(N, 2),), float("nan"), device="cuda")
+    step = dp.fused_step_fn(Wa, J0, J1, Wo, 0.1, "tanh")
+    if through_train_step:
+        dp.train_step(step, (A0 * gain, r, tgt), N, 2, B, T, buf=buf)
+        parts = buf[-2:]
+    else:
+        parts = step((A0 * gain, r, tgt), 1.0 / (B * T), buf)
+    gain, r, J0, J1 = want = leaves()
+    ref = torch.empty_like(buf)
+    loss, ref_parts, _, _ = ring_rnn_fused(A0 * gain, Wa.requires_grad_(True), J0, J1, Wo.requires_grad_(True), r, 0.1, "tanh", tgt,
+                                           grad_buffer=ref)
+    loss.backward()
+    assert torch.equal(buf[:-2], ref[:-2]) and torch.equal(parts, ref_parts)
+    for a, b in zip(got, want):
+        assert a.grad is not None and torch.equal(a.grad, b.grad)
+
+
 def test_angular_error_transforms():
     from torch.autograd import forward_ad
     from rnn_train_ring_attractor_b200.evaluate import angular_error
