@@ -422,23 +422,26 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
 }
 
 // Xall[t][b][m*NP + j] = c_m(b,t) * r_{t-1}[b,j] for all t: the B operand of the weight-gradient GEMM.
-// grid (BP, T), four neurons per thread
+// grid (BP, T or as many rows as a grid may have), four neurons per thread
+constexpr int MAX_GRID_Y = 65535;
 __global__ void __launch_bounds__(ROW_MAX) sw_build_xall_kernel(const __nv_bfloat16* __restrict__ Rh, const float* __restrict__ A,
-                                                                SwCols cols, int B, int t0, int T_total, int a_dim, int NP, int BP,
-                                                                long long KX, __nv_bfloat16* __restrict__ Xall) {
-  const int b = blockIdx.x, t = blockIdx.y;
+                                                                SwCols cols, int B, int T, int t0, int T_total, int a_dim, int NP,
+                                                                int BP, long long KX, __nv_bfloat16* __restrict__ Xall) {
+  const int b = blockIdx.x;
   const bool valid = b < B;
-  const __nv_bfloat16* r = Rh + ((size_t)t * BP + b) * NP;
-  __nv_bfloat16* x = Xall + ((size_t)t * BP + b) * KX;
-  const float* at = A + ((size_t)b * T_total + t0 + t) * a_dim;
-  for (int j = threadIdx.x * 4; j < NP; j += blockDim.x * 4) {
-    const uint2 rb = *reinterpret_cast<const uint2*>(r + j);
-    const float4 rf = of_bf16x4(rb);
-    *reinterpret_cast<uint2*>(x + j) = rb;
+  for (int t = blockIdx.y; t < T; t += gridDim.y) {
+    const __nv_bfloat16* r = Rh + ((size_t)t * BP + b) * NP;
+    __nv_bfloat16* x = Xall + ((size_t)t * BP + b) * KX;
+    const float* at = A + ((size_t)b * T_total + t0 + t) * a_dim;
+    for (int j = threadIdx.x * 4; j < NP; j += blockDim.x * 4) {
+      const uint2 rb = *reinterpret_cast<const uint2*>(r + j);
+      const float4 rf = of_bf16x4(rb);
+      *reinterpret_cast<uint2*>(x + j) = rb;
 #pragma unroll 4
-    for (int k = 0; k < cols.n; ++k) {
-      const float c = valid ? __ldg(at + cols.c[k]) : 0.f;
-      *reinterpret_cast<uint2*>(x + (size_t)(1 + k) * NP + j) = to_bf16x4(make_float4(c * rf.x, c * rf.y, c * rf.z, c * rf.w));
+      for (int k = 0; k < cols.n; ++k) {
+        const float c = valid ? __ldg(at + cols.c[k]) : 0.f;
+        *reinterpret_cast<uint2*>(x + (size_t)(1 + k) * NP + j) = to_bf16x4(make_float4(c * rf.x, c * rf.y, c * rf.z, c * rf.w));
+      }
     }
   }
 }
@@ -736,7 +739,8 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
     }
     {
       LaunchScope ls(K_PREP, s);
-      sw_build_xall_kernel<<<dim3(l.BP, Tc), row_threads(l.NP), 0, s>>>(Rh, p.A, cols, p.B, t0, p.T, p.a_dim, l.NP, l.BP, l.KX, Xall);
+      sw_build_xall_kernel<<<dim3(l.BP, Tc < MAX_GRID_Y ? Tc : MAX_GRID_Y), row_threads(l.NP), 0, s>>>(Rh, p.A, cols, p.B, Tc, t0, p.T, p.a_dim,
+                                                                                                       l.NP, l.BP, l.KX, Xall);
     }
     RINGRNN_CUDA_TRY(cudaGetLastError());
     // dWst[NP, KX] = Delta^T [NP, Tc*BP] x Xall [Tc*BP, KX]

@@ -69,6 +69,29 @@ def test_small_tile_kernels_match_the_oracle(prec, shape):
         assert float(((f[k].cpu().double() - want.T).abs() / scale.clamp(min=1e-30)).max()) < (N + 8) * 2.0 ** -24, k
 
 
+def test_more_steps_than_a_grid_has_rows():
+    """65535 is the largest extent of a grid's second dimension: sequences beyond it on the one-GEMM-per-step path, against
+    the fp32 mode.  Bound: weights, state and delta are rounded to bf16 (2^-9 each), and what a step gets wrong the next ones
+    amplify by 1 / (1 - g), g the gain of the step's matrix: about 0.3 with the action matrices at a quarter of their size
+    (three of spectral radius 1/4, signal 1/2 on average).  3 * 2^-9 / 0.7 = 8e-3 < 1e-2."""
+    from rnn_train_ring_attractor_b200 import ring_rnn_cuda as op
+    N, B, T = 16, 2, 65538
+    A, Wa, Wo, r0, cot = (t.cuda() for t in _case(N, B, T, 3, 3))
+    Wa *= 0.25
+    Wo.requires_grad_(True), Wa.requires_grad_(True)
+    got = {}
+    for prec in ("bf16", "fp32"):
+        op.set_precision(prec)
+        try:
+            hist = op.ring_rnn_cuda_func(A, Wa, -0.1, 0.1, Wo, r0, 0.1, "tanh")
+            got[prec] = [hist.detach()] + list(torch.autograd.grad(hist, [Wo, Wa], cot))
+        finally:
+            op.set_precision("auto")
+    for a, b in zip(got["bf16"], got["fp32"]):
+        assert orc.rel_err(a, b) < TOL["bf16"]
+    assert orc.rel_err(got["bf16"][0][-3:], got["fp32"][0][-3:]) < TOL["bf16"]
+
+
 @pytest.mark.parametrize("a_dim,cols", [(3, [0, 2]), (16, [0, 1]), (16, []), (64, [5, 63]), (7, list(range(7)))])
 def test_active_columns(a_dim, cols):
     from rnn_train_ring_attractor_b200.ring_rnn_cuda import active_columns
