@@ -4,8 +4,9 @@
  * Plain pointers and sizes only; every pointer named "device" is CUDA device memory owned by
  * the caller, including all scratch ("workspace") and saved-for-backward storage, whose sizes
  * ringrnn_workspace_bytes() reports.  No entry point allocates device memory, exits the process
- * or throws: each returns a RINGRNN_* status.  (Host side, the library keeps one 256-byte block of pinned
- * host memory for the deferred status reports described at RingRnnFwdArgs, allocated once on first use.)  Calls are asynchronous on `stream` (a cudaStream_t
+ * or throws: each returns a RINGRNN_* status.  (Host side, the library keeps a few hundred bytes of pinned host
+ * memory, allocated once on first use: a ring of 64 words and one word for the deferred status reports described at
+ * RingRnnFwdArgs, and the 32 results of ringrnn_active_columns.)  Calls are asynchronous on `stream` (a cudaStream_t
  * passed as void*; NULL = the legacy default stream) and may come from any host thread.
  *
  * Each declaration cites the interface of the reference project (chongxi/rnn_train_ring_attractor,
@@ -84,7 +85,8 @@ typedef struct RingRnnProblem {
  *                 bounded device-side wait ran out, and once it is non-zero every later wait of kernels that share the
  *                 word gives up at once (NULL = the library uses, and zeroes, the first word of `workspace`).
  * Error reporting is deferred, because the call returns before its kernels have run (the reference synchronises and
- * exits instead, cpp/cuda_common.cuh:30-39): the status word is copied to the host behind the kernels, and the NEXT
+ * exits instead, cpp/cuda_common.cuh:30-39): the status word is copied to the host behind the kernels (or, where the
+ * library supplies the word and the kernels can, the failing thread writes a pinned host word itself), and the NEXT
  * ringrnn_fwd / ringrnn_bwd call of the process returns RINGRNN_ERR_DEVICE if a word that has arrived is non-zero --
  * the results of the launches since the last successful report are then invalid.  ringrnn_device_status() does the same
  * check on demand, e.g. right after the caller's own synchronisation. */
@@ -185,6 +187,9 @@ int ringrnn_last_device_code(void);
  * normally, `*status` (device int, zeroed by the caller) receives `code` (non-zero), and the report is queued like any
  * other, so the next ringrnn_fwd / ringrnn_bwd / ringrnn_device_status sees RINGRNN_ERR_DEVICE. */
 int ringrnn_selftest_wait(long long limit_cycles, int code, int* status, void* stream);
+/* The same with the other way of reporting: nothing is copied behind the kernel, the thread that gives up writes the code to
+ * `*status` and to the library's pinned host word. */
+int ringrnn_selftest_wait_direct(long long limit_cycles, int code, int* status, void* stream);
 
 /* One training step on the fused loss: ringrnn_fwd (every step saved, or checkpoints), ringrnn_angle_loss, ringrnn_bwd, out of
  * one scratch buffer of ringrnn_train_bytes() bytes.  The loop body of train_general_ring_no_gain.py:312-334 without its

@@ -88,6 +88,7 @@ SYMBOLS = {
     "ringrnn_device_status": (C.c_int, [C.POINTER(C.c_int)]),
     "ringrnn_last_device_code": (C.c_int, []),
     "ringrnn_selftest_wait": (C.c_int, [C.c_longlong, C.c_int, C.c_void_p, C.c_void_p]),
+    "ringrnn_selftest_wait_direct": (C.c_int, [C.c_longlong, C.c_int, C.c_void_p, C.c_void_p]),
     "ringrnn_launch_count": (C.c_longlong, []),
     "ringrnn_timing_slots": (C.c_int, []),
     "ringrnn_timing_name": (C.c_char_p, [C.c_int]),

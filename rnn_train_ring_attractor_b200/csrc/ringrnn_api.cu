@@ -15,14 +15,14 @@ namespace ringrnn {
 // Self-test of the bounded wait every tensor-core kernel is built on: one thread waits, through the same mbar_wait(),
 // for a barrier phase that nothing will ever complete.  After `limit` cycles the wait gives up, records `code` in the
 // status word and the kernel ends normally.
-__global__ void wait_selftest_kernel(int* status, long long limit, int code) {
+__global__ void wait_selftest_kernel(int* status, volatile int* host, long long limit, int code) {
   __shared__ alignas(8) unsigned long long bar;
   __shared__ int dead;
   if (threadIdx.x == 0) {
     dead = 0;
     tc::mbar_init(tc::smem_u32(&bar), 1);
     tc::fence_mbar_init();
-    tc::WaitCtx w{&dead, status, limit};
+    tc::WaitCtx w{&dead, status, limit, host};
     (void)tc::mbar_wait(tc::smem_u32(&bar), 0, w, code);
   }
 }
@@ -126,25 +126,17 @@ int queue_status_report(const int* dev_status, cudaStream_t s) {
   return RINGRNN_OK;
 }
 
-static __device__ int g_direct_status;          // one per device
-static volatile int* g_direct_host = nullptr;    // one pinned word for all devices
-static int* g_direct_dev[64];
+static volatile int* g_status_direct = nullptr;  // pinned and mapped: one word for all devices
 
-int direct_status(DirectStatus* out) {
-  int device = 0;
-  RINGRNN_CUDA_TRY(cudaGetDevice(&device));
-  if (device < 0 || device >= 64) return RINGRNN_ERR_UNSUPPORTED;
+int host_status_word(volatile int** out) {
   std::lock_guard<std::mutex> lk(g_status_mu);
-  if (g_direct_host == nullptr) {
+  if (g_status_direct == nullptr) {
     void* h = nullptr;
     RINGRNN_CUDA_TRY(cudaHostAlloc(&h, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
     *static_cast<volatile int*>(h) = 0;
-    g_direct_host = static_cast<volatile int*>(h);
+    g_status_direct = static_cast<volatile int*>(h);
   }
-  if (g_direct_dev[device] == nullptr)
-    RINGRNN_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&g_direct_dev[device]), g_direct_status));
-  out->dev = g_direct_dev[device];
-  out->host = g_direct_host;
+  *out = g_status_direct;
   return RINGRNN_OK;
 }
 
@@ -159,12 +151,9 @@ static int take_device_status() {
         if (code == 0) code = g_status_ring[i];
         g_status_ring[i] = 0;
       }
-  if (g_direct_host != nullptr && *g_direct_host != 0) {
-    if (code == 0) code = *g_direct_host;
-    *g_direct_host = 0;
-    // (a failure path: later waits must not find the old code)
-    for (int* d : g_direct_dev)
-      if (d != nullptr) (void)cudaMemset(d, 0, sizeof(int));
+  if (g_status_direct != nullptr && *g_status_direct != 0) {
+    if (code == 0) code = *g_status_direct;
+    *g_status_direct = 0;
   }
   return code;
 }
@@ -357,10 +346,24 @@ extern "C" int ringrnn_selftest_wait(long long limit_cycles, int code, int* stat
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   {
     LaunchScope ls(K_PREP, s);
-    wait_selftest_kernel<<<1, 32, 0, s>>>(status, limit_cycles, code);
+    wait_selftest_kernel<<<1, 32, 0, s>>>(status, nullptr, limit_cycles, code);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   return queue_status_report(status, s);
+}
+
+extern "C" int ringrnn_selftest_wait_direct(long long limit_cycles, int code, int* status, void* stream) {
+  if (status == nullptr || limit_cycles < 0 || limit_cycles > 4000000000LL || code == 0) return RINGRNN_ERR_ARG;
+  volatile int* host = nullptr;
+  const int rc = host_status_word(&host);
+  if (rc != RINGRNN_OK) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  {
+    LaunchScope ls(K_PREP, s);
+    wait_selftest_kernel<<<1, 32, 0, s>>>(status, host, limit_cycles, code);
+  }
+  RINGRNN_CUDA_TRY(cudaGetLastError());
+  return RINGRNN_OK;
 }
 
 extern "C" int ringrnn_device_status(int* code) {

@@ -91,14 +91,9 @@ __host__ __device__ __forceinline__ int active_col(const DevProblem& p, int k) {
 // on this process looks at the words that have arrived.
 int queue_status_report(const int* dev_status, cudaStream_t s);
 
-// The same without a copy behind every launch, for kernels whose waits report through all three words: `dev` is polled by
-// slow waits (library-owned, per device, zero unless a wait was abandoned), `host` is a pinned host word the failing thread
-// writes itself.  0 = ok.
-struct DirectStatus {
-  int* dev;
-  volatile int* host;
-};
-int direct_status(DirectStatus* out);
+// The same without a copy behind every launch: a pinned host word, one for the process, that the thread which abandons a wait
+// writes itself.  Which launches give up together is still decided by the status word of their call.
+int host_status_word(volatile int** out);
 
 // dJ0 / dJ1 from the unscaled Wo gradient (ringrnn_fp32.cu); scratch: GRAD_J_BLOCKS * 2 doubles
 constexpr int GRAD_J_BLOCKS = 128;

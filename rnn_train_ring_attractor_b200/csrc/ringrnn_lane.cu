@@ -216,7 +216,7 @@ bool aligned16(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 
 void set_weight_loads(LaneFwdParams& q) { q.w_vec = q.N % 4 == 0 && aligned16(q.Wo) && aligned16(q.WL) && aligned16(q.WR); }
 
 template <class P>
-void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneLayout& l, int T, int t0, const DirectStatus& st, int* report, bool first) {
+void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneLayout& l, int T, int t0, int* status, volatile int* host) {
   memset(&q, 0, sizeof(q));
   q.B = p.B; q.T = T; q.N = p.N; q.BPs = l.BPs; q.n_ut = l.n_ut; q.a_dim = p.a_dim;
   q.colL = dp.n_mat > 1 ? dp.cols[0] : -1;
@@ -229,10 +229,8 @@ void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneL
   q.WR = q.colR >= 0 ? p.Wa + q.colR * NN : nullptr;
   q.A = p.A;
   q.t0 = t0; q.T_total = p.T;
-  q.status = st.dev;
-  q.host = st.host;
-  q.report = report;
-  q.zero_report = first ? 1 : 0;
+  q.status = status;
+  q.host = host;
 }
 
 }  // namespace
@@ -279,15 +277,18 @@ int lane_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   char* w = static_cast<char*>(a.workspace);
   float* dec1 = reinterpret_cast<float*>(w + 1024);
   const int K = train ? lane_ckpt_interval(p) : 0;
-  DirectStatus st{a.status, nullptr};
-  if (a.status == nullptr) {
-    const int rc = direct_status(&st);
+  int* status = a.status;
+  volatile int* host = nullptr;
+  if (status == nullptr) {  // the call's own word, and no copy of it behind the kernels
+    status = reinterpret_cast<int*>(w);
+    const int rc = host_status_word(&host);
     if (rc != RINGRNN_OK) return rc;
+    RINGRNN_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
   }
   if (K > 0)  // checkpoint 0 is the initial state
     RINGRNN_CUDA_TRY(cudaMemcpyAsync(a.saved, p.r_init, ckpt_slot(p), cudaMemcpyDeviceToDevice, s));
   LaneFwdParams q;
-  set_common(q, p, dp, l, p.T, 0, st, a.status == nullptr ? reinterpret_cast<int*>(w) : nullptr, true);
+  set_common(q, p, dp, l, p.T, 0, status, host);
   set_weight_loads(q);
   q.r_init = p.r_init;
   if (train && K == 0) {
@@ -327,14 +328,15 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
   const int Tk = K > 0 ? K : p.T;  // steps of one stretch
   const LaneBwdLayout b = lane_bwd_layout(l, Tk);
   char* w = static_cast<char*>(a.workspace);
-  DirectStatus st{a.status, nullptr};
-  if (a.status == nullptr) {
-    const int rc = direct_status(&st);
+  int* status = a.status;
+  volatile int* host = nullptr;
+  if (status == nullptr) {
+    status = reinterpret_cast<int*>(w);
+    const int rc = host_status_word(&host);
     if (rc != RINGRNN_OK) return rc;
   }
-  int* report = a.status == nullptr ? reinterpret_cast<int*>(w) : nullptr;
   unsigned* done = reinterpret_cast<unsigned*>(w + 64);
-  if (a.grad_J != nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(unsigned), s));
+  if (a.status == nullptr || a.grad_J != nullptr) RINGRNN_CUDA_TRY(cudaMemsetAsync(w, 0, 128, s));  // both words
   w += 1024;
   __nv_bfloat16* DL = reinterpret_cast<__nv_bfloat16*>(w);
   w += b.dl;
@@ -363,7 +365,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
     if (K > 0) {
       sv = saved_of(chunk_saved, l, Tc);
       LaneFwdParams f;
-      set_common(f, p, dp, l, Tc, t0, st, report, c == n_ck - 1);
+      set_common(f, p, dp, l, Tc, t0, status, host);
       set_weight_loads(f);
       f.r_init = static_cast<const float*>(a.saved) + (size_t)c * p.B * p.N;
       f.Rh = sv.Rh; f.Dh = sv.Dh; f.Sg = sv.Sg;
@@ -373,7 +375,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
       sv = saved_of(const_cast<void*>(a.saved), l, p.T);
     }
     LaneBwdParams q;
-    set_common(q, p, dp, l, Tc, t0, st, report, K == 0);
+    set_common(q, p, dp, l, Tc, t0, status, host);
     q.Rh = sv.Rh; q.Dh = sv.Dh; q.Sg = sv.Sg;
     q.grad_output = a.grad_output;
     q.coef_x = a.coef_x; q.coef_y = a.coef_y; q.coef_s = a.coef_s;
@@ -390,7 +392,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
       RINGRNN_CUDA_TRY(cudaGetLastError());
     }
     const int nsplit = lane_bwd_layout(l, Tc).nsplit;
-    rc = tc_gemm_slabs(DL, sv.Rh, partial, 3 * l.NP, l.NP, Tc, l.BPs, nsplit, st.dev, st.host, s);
+    rc = tc_gemm_slabs(DL, sv.Rh, partial, 3 * l.NP, l.NP, Tc, l.BPs, nsplit, status, host, s);
     if (rc != RINGRNN_OK) return rc;
     {
       LaunchScope ls(K_REDUCE, s);

@@ -59,10 +59,8 @@ struct LaneFwdParams {
   float* ckpt;           // as in TcFwdParams
   int ckpt_every;
   int t0, T_total;
-  int* status;            // polled by slow waits
-  int* report;            // the caller's scratch word, or nullptr
-  int zero_report;        // the first kernel of a call clears it
-  volatile int* host;     // pinned host word, or nullptr
+  int* status;            // receives the code of an abandoned wait; polled by slow waits
+  volatile int* host;     // pinned host word that receives it too, or nullptr
 };
 
 struct LaneBwdParams {
@@ -88,10 +86,8 @@ struct LaneBwdParams {
   float* dA_part;             // [CL][2][T][BPs] or nullptr
   const float* carry_in;      // [B,N] or nullptr
   int t0, T_total;
-  int* status;            // polled by slow waits
-  int* report;            // the caller's scratch word, or nullptr
-  int zero_report;        // the first kernel of a call clears it
-  volatile int* host;     // pinned host word, or nullptr
+  int* status;            // receives the code of an abandoned wait; polled by slow waits
+  volatile int* host;     // pinned host word that receives it too, or nullptr
 };
 
 // samples per unit: 16, 32 or 64 (see lane_unit_samples); units: 1 or 2 per CTA
@@ -167,15 +163,14 @@ struct Ctx {
 
 template <class C>
 __device__ __forceinline__ Ctx<C> setup(uint8_t* smem_raw, int units, const float* dec_u, const float* dec_v, int N,
-                                        int* status, int* report, int zero_report, volatile int* host) {
+                                        int* status, volatile int* host) {
   Ctx<C> c;
   c.base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   c.gen = smem_raw + (c.base - smem_u32(smem_raw));
   c.bars = c.base + C::OFF_BAR;
   c.rank = C::CL > 1 ? cluster_ctarank() : 0u;
   volatile int* dead = reinterpret_cast<volatile int*>(c.gen + C::OFF_BAR + B_DEAD);
-  c.w = WaitCtx{dead, status, WAIT_LIMIT_CYCLES, report, host};
-  if (blockIdx.x == 0 && threadIdx.x == 0 && report != nullptr && zero_report) *report = 0;
+  c.w = WaitCtx{dead, status, WAIT_LIMIT_CYCLES, host};
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     *dead = 0;

@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(384, 1) bwd_lane_kernel(const __grid_constant_
   constexpr int E = C::E;
   constexpr int NRED = NP < 512 ? 2 : 1;  // dL/dA: both products side by side, or one after the other
   extern __shared__ uint8_t smem_raw[];
-  const Ctx<C> c = setup<C>(smem_raw, 1, p.dec_u, p.dec_v, p.N, p.status, p.report, p.zero_report, p.host);
+  const Ctx<C> c = setup<C>(smem_raw, 1, p.dec_u, p.dec_v, p.N, p.status, p.host);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = (int)(blockIdx.x / C::CL), stride = (int)(gridDim.x / C::CL);
   const int T = p.T;

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(128 + 256 * U, 1) fwd_lane_kernel(const __grid
   using C = Cfg<NP, S, U, 2, 1>;
   constexpr int E = C::E;
   extern __shared__ uint8_t smem_raw[];
-  const Ctx<C> c = setup<C>(smem_raw, U, p.dec_u, p.dec_v, p.N, p.status, p.report, p.zero_report, p.host);
+  const Ctx<C> c = setup<C>(smem_raw, U, p.dec_u, p.dec_v, p.N, p.status, p.host);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = (int)(blockIdx.x / C::CL), groups = (int)(gridDim.x / C::CL), stride = groups * U;
   const int T = p.T;

@@ -98,12 +98,10 @@ struct WaitCtx {
   volatile int* dead;  // shared memory flag of this CTA
   int* status;         // global status word (may be nullptr)
   long long limit = WAIT_LIMIT_CYCLES;  // cycles after which a wait is abandoned
-  int* report = nullptr;       // further words that receive the code: the caller's scratch,
-  volatile int* host = nullptr;  // and pinned host memory (see direct_status in ringrnn_common.cuh)
+  volatile int* host = nullptr;  // pinned host word that receives the code too (see host_status_word in ringrnn_common.cuh)
 };
 __device__ __forceinline__ void report_abandoned(const WaitCtx& w, int code) {
   if (w.status != nullptr) atomicCAS(w.status, 0, code);
-  if (w.report != nullptr) *w.report = code;
   if (w.host != nullptr) {
     *w.host = code;
     __threadfence_system();
@@ -126,7 +124,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const W
       if (*w.dead) return false;
       if (w.status != nullptr && *reinterpret_cast<volatile int*>(w.status) != 0) {
         *w.dead = 1;
-        if (w.report != nullptr) *w.report = *reinterpret_cast<volatile int*>(w.status);
         return false;
       }
       if (clock64() - t0 > w.limit) {

@@ -195,6 +195,8 @@ def test_device_status_surface_without_a_gpu(L):
     assert L.ringrnn_selftest_wait(1000, 7, None, None) == 1      # no status word
     assert L.ringrnn_selftest_wait(-1, 7, 1, None) == 1           # negative limit
     assert L.ringrnn_selftest_wait(1000, 0, 1, None) == 1         # code 0 would be indistinguishable from success
+    for bad in ((1000, 7, None), (-1, 7, 1), (1000, 0, 1)):
+        assert L.ringrnn_selftest_wait_direct(*bad, None) == 1
     _lib.raise_if_device_error()
 
 

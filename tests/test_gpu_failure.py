@@ -73,3 +73,30 @@ def test_a_nonzero_status_word_makes_later_waits_give_up_at_once():
     assert int(status[0]) == 5
     assert L.ringrnn_device_status(None) == _lib.ERR_DEVICE
     _drain()
+
+
+def test_a_wait_that_reports_without_a_copy():
+    """Kernels of small tiles have no copy of their status word queued behind them: the failing thread writes the call's word
+    and a pinned host word.  A call of its own, on another stream, neither sees nor hides that failure."""
+    from gpu_helpers import run_forward
+    L = _lib.lib()
+    _drain()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert L.ringrnn_selftest_wait_direct(200000, 31, status.data_ptr(), side.cuda_stream) == 0
+    side.synchronize()
+    code = C.c_int(0)
+    assert int(status[0]) == 31
+    assert L.ringrnn_device_status(C.byref(code)) == _lib.ERR_DEVICE and code.value == 31
+    assert L.ringrnn_device_status(C.byref(code)) == 0 and code.value == 0
+    g = torch.Generator().manual_seed(0)
+    args = [torch.rand(40, 9, 2, generator=g).cuda(), (torch.randn(2, 130, 130, generator=g) * 0.1).cuda(),
+            (torch.randn(130, 130, generator=g) * 0.1).cuda(), torch.rand(40, 130, generator=g).cuda()]
+    want = run_forward(*args, -0.1, 0.1, 0.1, "tanh", "bf16")["hist"].clone()
+    assert L.ringrnn_selftest_wait_direct(200000, 32, status.zero_().data_ptr(), side.cuda_stream) == 0
+    with pytest.raises(_lib.RingRnnError):
+        torch.cuda.synchronize()
+        run_forward(*args, -0.1, 0.1, 0.1, "tanh", "bf16")
+    assert torch.equal(run_forward(*args, -0.1, 0.1, 0.1, "tanh", "bf16")["hist"], want)  # its own word is zero throughout
+    _lib.raise_if_device_error()
