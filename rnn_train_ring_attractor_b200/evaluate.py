@@ -36,12 +36,21 @@ def angular_error(pred, target):
     return torch.minimum(d, 2 * math.pi - d)
 
 
+TRIAL_STEPS = 1 << 22  # trials x steps in hand at a time: what the roll-out of one stretch holds is about 28 bytes per step
+
+
 def evaluate_angular_error(Wa, J0, J1, Wo, alpha, activation, n_trials=200, seq_len=500, batch=50, seed=123,
                            max_av=0.1 * math.pi, precision=None):
-    """dict(mean, std, max, final_mean, errors[n_trials, seq_len]) in radians for the given weights (device tensors)."""
+    """dict(mean, std, max, final_mean, errors[n_trials, seq_len]) in radians for the given weights (device tensors).
+    ``batch`` trials are drawn at a time (it decides which trials a seed stands for); whole batches are rolled out together,
+    as many as ``TRIAL_STEPS`` allows and at least one."""
     g = torch.Generator().manual_seed(seed)
-    x = trials_from_host_draws(n_trials, seq_len, Wo.shape[0], batch, max_av, g, Wo.device)
-    decoded, _ = ring_rnn_rollout(x["A"], Wa, J0, J1, Wo, x["r_init"], alpha, activation, precision=precision)
-    e = angular_error(decoded, x["target"])
+    per = max(1, TRIAL_STEPS // max(1, batch * seq_len)) * batch
+    errs = []
+    for lo in range(0, n_trials, per):
+        x = trials_from_host_draws(min(per, n_trials - lo), seq_len, Wo.shape[0], batch, max_av, g, Wo.device)
+        decoded, _ = ring_rnn_rollout(x["A"], Wa, J0, J1, Wo, x["r_init"], alpha, activation, precision=precision)
+        errs.append(angular_error(decoded, x["target"]))
+    e = errs[0] if len(errs) == 1 else torch.cat(errs, dim=0)
     mean, std, top, final = torch.stack((e.mean(), e.std(), e.max(), e[:, -1].mean())).tolist()
     return {"mean": mean, "std": std, "max": top, "final_mean": final, "errors": e}

@@ -114,6 +114,30 @@ def test_trials_from_host_draws_are_the_host_generators(n, batch, T):
     assert orc.rel_err(x["r_init"], inputs.initial_bump_gaussian(angle[:, 0], 120)) < 1e-5
 
 
+def test_evaluation_rolls_out_whole_batches_up_to_a_bound(monkeypatch):
+    """The trials in hand at a time are bounded, and how many they are changes nothing."""
+    from rnn_train_ring_attractor_b200 import evaluate, inputs
+    Wo, Wl, Wr = (w.cuda() for w in inputs.ideal_weights(24))
+    sizes = []
+    inner = evaluate.ring_rnn_rollout
+
+    def rollout(A, *args, **kw):
+        sizes.append(A.shape[0] * A.shape[1])
+        return inner(A, *args, **kw)
+
+    monkeypatch.setattr(evaluate, "ring_rnn_rollout", rollout)
+    args = (torch.stack([Wl, Wr]), -0.1, 0.1, Wo, 0.1, "tanh")
+    evaluate.evaluate_angular_error(*args, n_trials=9000, seq_len=1000, batch=50)
+    assert max(sizes) <= 1 << 22 and sum(sizes) == 9000 * 1000
+    del sizes[:]
+    once = evaluate.evaluate_angular_error(*args, n_trials=23, seq_len=30, batch=4)
+    assert sizes == [23 * 30]
+    monkeypatch.setattr(evaluate, "TRIAL_STEPS", 300)
+    parts = evaluate.evaluate_angular_error(*args, n_trials=23, seq_len=30, batch=4)
+    assert sizes[1:] == [8 * 30, 8 * 30, 7 * 30]
+    assert torch.equal(once["errors"], parts["errors"])
+
+
 @pytest.mark.parametrize("n", [1, 5, 4096, 100003])
 def test_angles_and_errors(n):
     from rnn_train_ring_attractor_b200 import _lib
