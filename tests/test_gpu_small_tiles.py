@@ -114,6 +114,16 @@ def test_trials_from_host_draws_are_the_host_generators(n, batch, T):
     assert orc.rel_err(x["r_init"], inputs.initial_bump_gaussian(angle[:, 0], 120)) < 1e-5
 
 
+@pytest.mark.parametrize("T,ratio,max_av", [(40, 0.1, -0.3), (60000, 0.9, 0.1), (12000, 0.1, 0.1)])
+def test_trials_the_device_does_not_rank_come_from_the_host(T, ratio, max_av):
+    """A negative max_av, a trial whose velocities and ordering draws together exceed shared memory, more than 8192 draws."""
+    from rnn_train_ring_attractor_b200 import inputs
+    x = inputs.trials_from_host_draws(3, T, 24, 2, max_av, torch.Generator().manual_seed(4), "cuda", ratio)
+    g = torch.Generator().manual_seed(4)
+    av, angle = (torch.cat(p)[:3] for p in zip(*[inputs.generate_av(2, T, ratio, max_av=max_av, generator=g) for _ in range(2)]))
+    assert torch.equal(x["A"].cpu(), inputs.av_to_action_signal(av, max_av)) and torch.equal(x["target"].cpu(), angle)
+
+
 def test_evaluation_rolls_out_whole_batches_up_to_a_bound(monkeypatch):
     """The trials in hand at a time are bounded, and how many they are changes nothing."""
     from rnn_train_ring_attractor_b200 import evaluate, inputs
