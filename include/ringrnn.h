@@ -221,7 +221,8 @@ int ringrnn_train_step(const RingRnnTrainArgs* args, void* stream);
 int ringrnn_active_columns(const float* A, long long rows, int a_dim, unsigned long long* mask, void* stream);
 
 /* angle[i] = atan2(y[i], x[i]) in [0, 2pi) (train/train_ring_attractor.py:196-206), and the circular distance
- * min(d, 2pi - d), d = |pred - target| mod 2pi (compare/compare_models_fair.py:15-20); n elements. */
+ * min(d, 2pi - d), d = |pred - target| mod 2pi (compare/compare_models_fair.py:15-20); n elements.  The output may be one of
+ * the inputs. */
 int ringrnn_decode_angles(long long n, const float* x, const float* y, float* angle, void* stream);
 int ringrnn_angular_error(long long n, const float* pred, const float* target, float* error, void* stream);
 

@@ -66,9 +66,9 @@ __device__ __forceinline__ float circular_one(float p, float t) {
   const float d = fmodf(fabsf(p - t), two_pi);
   return fminf(d, two_pi - d);
 }
-// four elements per thread; `vec`: both inputs and the output are 16-byte aligned
+// four elements per thread; `vec`: both inputs and the output are 16-byte aligned.  The output may be one of the inputs.
 template <class F>
-__device__ __forceinline__ void map2(size_t n, bool vec, const float* __restrict__ a, const float* __restrict__ b, float* o, F f) {
+__device__ __forceinline__ void map2(size_t n, bool vec, const float* a, const float* b, float* o, F f) {
   const size_t stride = (size_t)gridDim.x * blockDim.x, first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   const size_t n4 = vec ? n / 4 : 0;
   for (size_t i = first; i < n4; i += stride) {

@@ -194,7 +194,7 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
         a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
         stream = stream_of(dev)
         _lib.check(L.ringrnn_fwd(C.byref(a), stream))
-        decoded = xy[0]  # in place of x
+        decoded = torch.empty(B, T, device=dev, dtype=torch.float32)  # (not a row of xy: a result keeps nothing else alive)
         _lib.check(L.ringrnn_decode_angles(B * T, xy[0].data_ptr(), xy[1].data_ptr(), decoded.data_ptr(), stream))
     return decoded, final_state
 

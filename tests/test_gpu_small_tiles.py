@@ -148,6 +148,14 @@ def test_evaluation_rolls_out_whole_batches_up_to_a_bound(monkeypatch):
     assert torch.equal(once["errors"], parts["errors"])
 
 
+def test_rollout_result_keeps_nothing_else_alive():
+    from rnn_train_ring_attractor_b200.fused import ring_rnn_rollout
+    case = orc.make_case(24, 6, 5, "tanh", seed=2)
+    A, Wa, Wo, r0 = (t.cuda() for t in (case.A, case.Wa, case.Wo, case.r_init))
+    decoded, _ = ring_rnn_rollout(A, Wa, -0.1, 0.1, Wo, r0, 0.1, "tanh")
+    assert decoded.shape == (6, 5) and decoded.untyped_storage().nbytes() == 4 * decoded.numel()
+
+
 @pytest.mark.parametrize("n", [1, 5, 4096, 100003])
 def test_angles_and_errors(n):
     from rnn_train_ring_attractor_b200 import _lib
@@ -159,6 +167,9 @@ def test_angles_and_errors(n):
     want = torch.remainder(torch.atan2(y.double(), x.double()), 2 * math.pi)
     d = (out.double() - want).abs()
     assert float(torch.minimum(d, 2 * math.pi - d).max()) < 2e-6 and float(out.min()) >= 0 and float(out.max()) < 2 * math.pi
+    same = x.clone()
+    _lib.check(_lib.lib().ringrnn_decode_angles(n, same.data_ptr(), y.data_ptr(), same.data_ptr(), None))
+    assert torch.equal(same, out)
     t = (torch.rand(n, generator=g) * 20 - 10).cuda()
     e = (out.double() - t.double()).abs() % (2 * math.pi)
     assert float((angular_error(out, t).double() - torch.minimum(e, 2 * math.pi - e)).abs().max()) < 4e-6
