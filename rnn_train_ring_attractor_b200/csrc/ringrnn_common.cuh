@@ -114,7 +114,7 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
 // split-K bf16 tensor-core GEMM (tc_gemm.cu); see there for the argument contract
 int tc_gemm(int mn_major, const void* A, const void* B, float* partial, float* out, int M, int N, long long K,
             int nsplit, int* status, cudaStream_t s);
-int tc_gemm_chained(const void* A, const void* B, float* partial, int M, int N, long long K, int nsplit, int nt, int* status,
+int tc_gemm_products(const void* A, const void* B, float* partial, int M, int N, long long K, int nsplit, int nt, int* status,
                     cudaStream_t s);
 
 int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, int slabs, int cols, int nsplit, int* status,

@@ -222,8 +222,6 @@ __global__ void __launch_bounds__(ROW_MAX) sw_forward_row_kernel(SwFwd q, int t)
   const int t_c = q.concat ? t + 1 : t;
   for (int k = threadIdx.x; k <= n; k += blockDim.x)
     coef[k] = k == 0 ? 1.f : (valid && t_c >= 0 && t_c < q.T) ? __ldg(q.A + ((size_t)b * q.T_total + q.t0 + t_c) * q.a_dim + q.cols.c[k - 1]) : 0.f;
-  tc::grid_launch_dependents();
-  tc::grid_wait();  // everything below may depend on the kernels before
   const float s_prev = (t >= 0) ? q.rowsum[b] : 0.f;
   __syncthreads();
   const int blocks = q.concat ? 1 : 1 + n;
@@ -345,8 +343,6 @@ __global__ void __launch_bounds__(ROW_MAX) sw_backward_row_kernel(SwBwd q, int t
     coef[k] = k == 0 ? 1.f : (valid && t_carry >= 0) ? __ldg(q.A + ((size_t)b * q.T_total + q.t0 + t_carry) * q.a_dim + q.cols.c[k - 1]) : 0.f;
   if (WANT_DA)
     for (int x = threadIdx.x; x < (1 + n) * (ROW_MAX / 32); x += blockDim.x) da[x] = 0.f;
-  tc::grid_launch_dependents();
-  tc::grid_wait();
   const float sd = (t_carry >= 0) ? q.sum_delta[b] : 0.f;
   __syncthreads();
   float ds = 0.f;
@@ -471,26 +467,16 @@ SwCols cols_of(const DevProblem& dp) {
   return c;
 }
 
-// `chained`: starts while the GEMM before it still runs (programmatic dependent launch)
 template <class K, class... Args>
-cudaError_t launch_row(K kernel, int rows, int NP, cudaStream_t s, bool chained, Args... args) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(rows, 1, 1);
-  cfg.blockDim = dim3(row_threads(NP), 1, 1);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+cudaError_t launch_row(K kernel, int rows, int NP, cudaStream_t s, Args... args) {
+  kernel<<<rows, row_threads(NP), 0, s>>>(args...);
+  return cudaGetLastError();
 }
 
 template <int ACT>
 void launch_forward_row(const SwFwd& q, int t, cudaStream_t s) {
   LaunchScope ls(K_FWD, s);
-  launch_row(sw_forward_row_kernel<ACT>, q.BP, q.NP, s, t >= 0 && !q.concat, q, t);
+  launch_row(sw_forward_row_kernel<ACT>, q.BP, q.NP, s, q, t);
 }
 
 void forward_row(int act, const SwFwd& q, int t, cudaStream_t s) {
@@ -592,7 +578,7 @@ int run_forward(const RingRnnProblem& p, const DevProblem& dp, const SwLayout& l
     if (l.concat)
       rc = tc_gemm(0, m.X, m.W, m.partial, nullptr, l.BP, l.NP, l.KX, 1, m.status, s);
     else
-      rc = tc_gemm_chained(q.Rh != nullptr ? q.Rh + (size_t)t * l.BP * l.NP : m.X, m.W, m.partial, l.BP, (int)l.KX, l.NP, l.ns_z,
+      rc = tc_gemm_products(q.Rh != nullptr ? q.Rh + (size_t)t * l.BP * l.NP : m.X, m.W, m.partial, l.BP, (int)l.KX, l.NP, l.ns_z,
                            l.nt_z, m.status, s);
     if (rc != RINGRNN_OK) return rc;
     forward_row(p.activation, q, t, s);
@@ -727,15 +713,15 @@ int stepwise_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_
     q.grad_A = a.grad_A; q.cols = cols;
     {
       LaunchScope ls(K_BWD, s);
-      RINGRNN_CUDA_TRY(launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, false, q, -1, Tc - 1));
+      RINGRNN_CUDA_TRY(launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, q, -1, Tc - 1));
     }
     for (int t = Tc - 1; t >= 0; --t) {
       // Z_t[BP, KX] = delta_t[BP, NP] x WstT[KX, NP]^T
-      const int rc = tc_gemm_chained(Delta + (size_t)t * l.BP * l.NP, WstT, zpart, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z, status, s);
+      const int rc = tc_gemm_products(Delta + (size_t)t * l.BP * l.NP, WstT, zpart, l.BP, (int)l.KX, l.NP, l.ns_z, l.nt_z, status, s);
       if (rc != RINGRNN_OK) return rc;
       LaunchScope ls(K_BWD, s);
-      RINGRNN_CUDA_TRY(q.grad_A != nullptr ? launch_row(sw_backward_row_kernel<true>, l.BP, l.NP, s, true, q, t, t - 1)
-                                           : launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, true, q, t, t - 1));
+      RINGRNN_CUDA_TRY(q.grad_A != nullptr ? launch_row(sw_backward_row_kernel<true>, l.BP, l.NP, s, q, t, t - 1)
+                                           : launch_row(sw_backward_row_kernel<false>, l.BP, l.NP, s, q, t, t - 1));
     }
     {
       LaunchScope ls(K_PREP, s);

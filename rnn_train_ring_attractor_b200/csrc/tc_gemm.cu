@@ -118,6 +118,7 @@ struct GemmCfg {
   static constexpr int SMEM = NSTAGE * STAGE + 1024 /*align*/ + 256 /*barriers*/;
   static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
   static constexpr int NI = NT > 256 ? NT / 256 : 1;  // MMA instructions along N per k-step
+  static_assert(OUT_BYTES <= NSTAGE * STAGE, "the epilogue's buffers");
   static constexpr int NMMA = NT > 256 ? 256 : NT;
 };
 
@@ -166,13 +167,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_p;
-  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
-      grid_wait();
       for (int it = 0; it < iters; ++it) {
         const int s = it % Cfg::NSTAGE;
         const uint32_t round = it / Cfg::NSTAGE;
@@ -222,7 +221,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     // epilogue: warp w owns TMEM lanes 32*(w%4)..+31 = output rows m0 + that
     const int q = warp & 3;
-    grid_wait();  // earlier kernels may still read what this one writes
     const bool ok = mbar_wait(done_bar, 0, wctx, 103);
     tcgen05_fence_after();
     store_tile<NT>(&tmOut, base, tmem_base, q, lane, n0, (int)blockIdx.z * M_total + m0 + q * 32, iters == 0 || !ok);
@@ -238,7 +236,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // SMs once and not twice.  [256 x 2048] x [2048 x 34816]: 57 us by single CTAs with tiles of 128 x 512, 50 by pairs, 37 with the
 // TMA stores and the L2 policy.  out[split][M_total][N_total], split = blockIdx.z.
 // B tiles of the first `keep` columns of the grid are asked to stay in L2, the rest to leave it first.
-// B must not be written by the kernel before this one: its first stages are fetched while that one still runs.
 template <int NT>
 struct PairCfg {
   static constexpr int KC = 64;
@@ -248,6 +245,7 @@ struct PairCfg {
   static constexpr int NSTAGE = (200 * 1024) / STAGE < 8 ? (200 * 1024) / STAGE : 8;
   static constexpr int SMEM = NSTAGE * STAGE + 1024 + 256;
   static constexpr int NI = NT > 256 ? NT / 256 : 1;  // MMA instructions along N per k-step
+  static_assert(OUT_BYTES <= NSTAGE * STAGE, "the epilogue's buffers");
   static constexpr int NMMA = NT / NI;
   static constexpr int TMEM_COLS = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : NT <= 256 ? 256 : 512;  // power of two
 };
@@ -293,31 +291,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_wait();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_p;
-  grid_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       const uint64_t policy = (int)blockIdx.y < keep ? l2_policy_evict_last() : l2_policy_evict_first();
-      auto load_b = [&](int it) {
-        const int s = it % Cfg::NSTAGE;
-        const uint32_t b_dst = base + s * Cfg::STAGE + Cfg::A_BYTES;
-        if (h == 0) mbar_arrive_expect_tx(full_bar(s), 2 * Cfg::STAGE);  // both CTAs' bytes land on this barrier
-        for (int nh = 0; nh < Cfg::NI; ++nh)
-          tma_load_2d_pair_hint(b_dst + nh * (Cfg::NMMA / 2) * 128, &tmB, full_bar(s), k_begin + it * Cfg::KC,
-                                n0 + nh * Cfg::NMMA + (int)h * (Cfg::NMMA / 2), policy);
-      };
-      const int early = iters < Cfg::NSTAGE ? iters : Cfg::NSTAGE;
-      for (int it = 0; it < early; ++it) load_b(it);
-      grid_wait();
       for (int it = 0; it < iters; ++it) {
         const int s = it % Cfg::NSTAGE;
-        if (it >= Cfg::NSTAGE) {
-          if (!mbar_wait(empty_bar(s), (it / Cfg::NSTAGE - 1) & 1u, wctx, 111)) break;
-          load_b(it);
-        }
-        tma_load_2d_pair(base + s * Cfg::STAGE, &tmA, full_bar(s), k_begin + it * Cfg::KC, m0);
+        if (it >= Cfg::NSTAGE && !mbar_wait(empty_bar(s), (it / Cfg::NSTAGE - 1) & 1u, wctx, 111)) break;
+        const uint32_t a_dst = base + s * Cfg::STAGE, b_dst = a_dst + Cfg::A_BYTES;
+        if (h == 0) mbar_arrive_expect_tx(full_bar(s), 2 * Cfg::STAGE);  // both CTAs' bytes land on this barrier
+        const int k = k_begin + it * Cfg::KC;
+        tma_load_2d_pair(a_dst, &tmA, full_bar(s), k, m0);
+        for (int nh = 0; nh < Cfg::NI; ++nh)
+          tma_load_2d_pair_hint(b_dst + nh * (Cfg::NMMA / 2) * 128, &tmB, full_bar(s), k,
+                                n0 + nh * Cfg::NMMA + (int)h * (Cfg::NMMA / 2), policy);
       }
     }
   } else if (warp == 1) {
@@ -344,7 +333,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     const int q = warp & 3;
-    grid_wait();
     const bool ok = mbar_wait(done_bar, 0, wctx, 113);
     tcgen05_fence_after();
     store_tile<NT>(&tmOut, base, tmem_base, q, lane, n0, (int)blockIdx.z * M_total + m0 + q * 32, iters == 0 || !ok);
@@ -358,7 +346,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 template <int NT>
 int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int N_total, long long K_total, int nsplit,
-                     bool overlap, int* status, cudaStream_t s) {
+                     int* status, cudaStream_t s) {
   using Cfg = PairCfg<NT>;
   CUtensorMap tmA, tmB, tmOut;
   if (!make_tmap_f32_out(&tmOut, out, (uint64_t)nsplit * M_total, (uint64_t)N_total) ||
@@ -372,18 +360,16 @@ int launch_gemm_pair(const void* A, const void* B, float* out, int M_total, int 
   cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 2 : 1;
+  cfg.numAttrs = 1;
   long long kps = (K_total + nsplit - 1) / nsplit;
   kps = (kps + Cfg::KC - 1) / Cfg::KC * Cfg::KC;
-  // A chain reads B again each step.  More of it than L2 holds (126 MB, of which the products take some) would push out all of
+  // Every step reads B again.  More of it than L2 holds (126 MB, of which the products take some) would push out all of
   // itself before it comes round again: 72 MB stay, the rest streams past.
   const double b_bytes = 2.0 * N_total * K_total, l2 = 72e6;
   const int tiles = N_total / NT, keep = b_bytes <= l2 ? tiles : (int)(tiles * (l2 / b_bytes));
@@ -405,7 +391,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int nspl
 
 template <bool MN_MAJOR, int NT>
 int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N_total, long long K_total, int nsplit,
-                int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr, bool overlap = false) {
+                int* status, cudaStream_t s, int slabs = 1, volatile int* host_status = nullptr) {
   using Cfg = GemmCfg<MN_MAJOR, NT>;
   CUtensorMap tmA, tmB, tmOut;
   bool ok;
@@ -430,19 +416,8 @@ int launch_gemm(const void* A, const void* B, float* partial, int M_total, int N
   dim3 grid((M_total + 127) / 128, (N_total + NT - 1) / NT, nsplit);
   {
     LaunchScope ls(K_DW, s);
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<MN_MAJOR, NT>, tmA, tmB, tmOut, M_total, N_total, K_total, kps,
-                                        chunks_per_slab, status, host_status));
+    gemm_tc_kernel<MN_MAJOR, NT><<<grid, GEMM_THREADS, Cfg::SMEM, s>>>(tmA, tmB, tmOut, M_total, N_total, K_total, kps,
+                                                                       chunks_per_slab, status, host_status);
   }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   return RINGRNN_OK;
@@ -491,24 +466,23 @@ int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, in
 // CTA-pair K-major GEMM: out[M,N] = A[M,K] * B[N,K]^T, M % 256 == 0, N a multiple of 256, 224 or 128 (the pair MMA wants N % 32 == 0) (N % NT == 0)
 int tc_gemm_pair(const void* A, const void* B, float* out, int M, int N, long long K, int* status, cudaStream_t s) {
   if (M % 256 != 0) return RINGRNN_ERR_SHAPE;
-  if (N % 256 == 0) return launch_gemm_pair<256>(A, B, out, M, N, K, 1, false, status, s);
-  if (N % 224 == 0) return launch_gemm_pair<224>(A, B, out, M, N, K, 1, false, status, s);
-  if (N % 128 == 0) return launch_gemm_pair<128>(A, B, out, M, N, K, 1, false, status, s);
+  if (N % 256 == 0) return launch_gemm_pair<256>(A, B, out, M, N, K, 1, status, s);
+  if (N % 224 == 0) return launch_gemm_pair<224>(A, B, out, M, N, K, 1, status, s);
+  if (N % 128 == 0) return launch_gemm_pair<128>(A, B, out, M, N, K, 1, status, s);
   return RINGRNN_ERR_SHAPE;
 }
 
-// One GEMM of a chain of kernels with programmatic dependent launch: partial[split][M][N] = A[M,K] * B[N,K]^T with tiles of nt
-// columns, by CTA pairs where M allows.  B must be older than the kernel before this one.
-int tc_gemm_chained(const void* A, const void* B, float* partial, int M, int N, long long K, int nsplit, int nt, int* status,
+// partial[split][M][N] = A[M,K] * B[N,K]^T with tiles of nt columns, by CTA pairs where M allows
+int tc_gemm_products(const void* A, const void* B, float* partial, int M, int N, long long K, int nsplit, int nt, int* status,
                     cudaStream_t s) {
   if (M % 256 == 0) {
-    if (nt == 512) return launch_gemm_pair<512>(A, B, partial, M, N, K, nsplit, true, status, s);
-    if (nt == 256) return launch_gemm_pair<256>(A, B, partial, M, N, K, nsplit, true, status, s);
-    if (nt == 128) return launch_gemm_pair<128>(A, B, partial, M, N, K, nsplit, true, status, s);
+    if (nt == 512) return launch_gemm_pair<512>(A, B, partial, M, N, K, nsplit, status, s);
+    if (nt == 256) return launch_gemm_pair<256>(A, B, partial, M, N, K, nsplit, status, s);
+    if (nt == 128) return launch_gemm_pair<128>(A, B, partial, M, N, K, nsplit, status, s);
   } else {
-    if (nt == 512) return launch_gemm<false, 512>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
-    if (nt == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
-    if (nt == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s, 1, nullptr, true);
+    if (nt == 512) return launch_gemm<false, 512>(A, B, partial, M, N, K, nsplit, status, s);
+    if (nt == 256) return launch_gemm<false, 256>(A, B, partial, M, N, K, nsplit, status, s);
+    if (nt == 128) return launch_gemm<false, 128>(A, B, partial, M, N, K, nsplit, status, s);
   }
   return RINGRNN_ERR_SHAPE;
 }

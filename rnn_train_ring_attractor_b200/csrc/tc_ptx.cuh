@@ -211,11 +211,6 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t bar, uint32_
                : "memory");
 }
 
-// ---- programmatic dependent launch: let the next kernel of the stream start its set-up / wait for the previous kernels
-// and their writes.  Both do nothing in a launch without the attribute.
-__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- TMA ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -92,6 +92,25 @@ def test_more_steps_than_a_grid_has_rows():
     assert orc.rel_err(got["bf16"][0][-3:], got["fp32"][0][-3:]) < TOL["bf16"]
 
 
+def test_several_waves_of_ctas_per_step_back_to_back():
+    """One GEMM per step of 544 CTAs and row kernels of 1024 blocks, forward and reverse, calls following one another without a
+    pause: the kernels' order is the stream's alone.  Sums in fixed order: every call gives the same bits."""
+    from rnn_train_ring_attractor_b200 import ring_rnn_cuda as op
+    N, B, T, a_dim = 2048, 1000, 20, 16
+    g = torch.Generator(device="cuda").manual_seed(0)
+    s = 0.5 / math.sqrt(N)
+    A, r0 = torch.rand(B, T, a_dim, generator=g, device="cuda"), torch.rand(B, N, generator=g, device="cuda") - 0.5
+    Wa = (torch.randn(a_dim, N, N, generator=g, device="cuda") * (s / 8)).requires_grad_(True)
+    Wo = (torch.randn(N, N, generator=g, device="cuda") * s).requires_grad_(True)
+    cot = torch.randn(T, B, N, generator=g, device="cuda")
+    first = None
+    for _ in range(6):
+        hist = op.ring_rnn_cuda_func(A, Wa, -0.003, 0.1, Wo, r0, 0.1, "silu")
+        out = [hist.detach()] + list(torch.autograd.grad(hist, [Wo, Wa], cot))
+        first = first or out
+    assert all(torch.isfinite(x).all() and torch.equal(x, y) for x, y in zip(first, out))
+
+
 @pytest.mark.parametrize("a_dim,cols", [(3, [0, 2]), (16, [0, 1]), (16, []), (64, [5, 63]), (7, list(range(7)))])
 def test_active_columns(a_dim, cols):
     from rnn_train_ring_attractor_b200.ring_rnn_cuda import active_columns
