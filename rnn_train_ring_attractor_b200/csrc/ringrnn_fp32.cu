@@ -662,16 +662,21 @@ __global__ void da_cluster_kernel(DevProblem p, const float* __restrict__ part, 
 
 // workspace layouts ----------------------------------------------------------------------------
 //   FWD : WT[n_mat][N][N]
-//   SAVED (only when the caller does not keep bump_history): hist[T][B][N], with cluster kernels also F'(re)[T][B][N]
+//   SAVED (only when the caller does not keep bump_history): hist[T][B][N], with cluster kernels and a history of up to 256 MB
+//         also F'(re)[T][B][N]
 //   BWD : WT[n_mat][N][N] | delta[T][B][N] | partial[ksplit][n_mat][N][N] | raw[N][N] |
-//         with cluster kernels F'(re)[T][B][N] (when the forward could not keep it) | dL/dA sums [C][n_mat-1][B][T]
+//         with cluster kernels dL/dA sums [C][n_mat-1][B][T]
 size_t fp32_fwd_workspace_bytes(const RingRnnProblem& p) {
   return align_up(sizeof(float) * (size_t)n_mat_of(p) * p.N * p.N, 256);
 }
+static size_t history_bytes(const RingRnnProblem& p) { return align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256); }
+// Whether a forward that keeps the history itself keeps F'(re) beside it.  The reverse pass can form it from the history, in
+// the place of delta; that costs a launch over all steps, so up to 256 MB the memory is spent.
+static bool keeps_dact(const RingRnnProblem& p) { return history_bytes(p) <= ((size_t)256 << 20); }
 size_t fp32_saved_bytes(const RingRnnProblem& p, int history_given) {
   if (history_given) return 0;
   fc::Shape h;
-  return (cluster_shape(p, n_mat_of(p), &h) ? 2 : 1) * align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256);
+  return (cluster_shape(p, n_mat_of(p), &h) && keeps_dact(p) ? 2 : 1) * history_bytes(p);
 }
 static size_t cluster_da_bytes(const RingRnnProblem& p, const fc::Shape& h) {
   return align_up(sizeof(float) * (size_t)h.C * (n_mat_of(p) - 1) * p.B * p.T, 256);
@@ -685,10 +690,9 @@ static size_t partial_bytes(const RingRnnProblem& p, int n_mat) {
 size_t fp32_bwd_workspace_bytes(const RingRnnProblem& p) {
   const int n_mat = n_mat_of(p);
   const size_t NN = (size_t)p.N * p.N;
-  size_t n = align_up(sizeof(float) * n_mat * NN, 256) + align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256) +
-             partial_bytes(p, n_mat) + align_up(sizeof(float) * NN, 256);
+  size_t n = align_up(sizeof(float) * n_mat * NN, 256) + history_bytes(p) + partial_bytes(p, n_mat) + align_up(sizeof(float) * NN, 256);
   fc::Shape h;
-  if (cluster_shape(p, n_mat, &h)) n += align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256) + cluster_da_bytes(p, h);
+  if (cluster_shape(p, n_mat, &h)) n += cluster_da_bytes(p, h);
   return n;
 }
 
@@ -705,8 +709,8 @@ int fp32_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s) 
   if (cluster_shape(p, dp.n_mat, &ca.sh)) {
     ca.p = dp;
     ca.hist = hist;
-    if (a.bump_history == nullptr && a.saved != nullptr)
-      ca.dact = reinterpret_cast<float*>(static_cast<char*>(a.saved) + align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256));
+    if (a.bump_history == nullptr && a.saved != nullptr && keeps_dact(p))
+      ca.dact = reinterpret_cast<float*>(static_cast<char*>(a.saved) + history_bytes(p));
     ca.dec_x = a.dec_x; ca.dec_y = a.dec_y; ca.dec_ta = a.dec_ta; ca.dec_u = a.dec_u; ca.dec_v = a.dec_v;
     ca.final_state = a.final_state;
     return launch_cluster_act<0>(p.activation, ca, 1, K_FWD, s);
@@ -750,17 +754,15 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
   if (cluster_shape(p, n_mat, &ca.sh)) {
     ca.p = dp;
     ca.hist = const_cast<float*>(hist);
-    const size_t tbn = align_up(sizeof(float) * (size_t)p.T * p.B * p.N, 256);
-    if (a.bump_history == nullptr) {  // the forward kept F'(re) beside the history
-      ca.dact = reinterpret_cast<float*>(static_cast<char*>(const_cast<void*>(a.saved)) + tbn);
-    } else {  // only the history: F'(re) of all steps at once first, off the sequential path
-      ca.dact = reinterpret_cast<float*>(w);
+    if (a.bump_history == nullptr && keeps_dact(p)) {  // the forward kept F'(re) beside the history
+      ca.dact = reinterpret_cast<float*>(static_cast<char*>(const_cast<void*>(a.saved)) + history_bytes(p));
+    } else {  // only the history: F'(re) of all steps at once first, off the sequential path, where delta goes later
+      ca.dact = delta;
       int splits = 148 / (ca.sh.tiles * ca.sh.C);
       if (splits > p.T) splits = p.T;
       rc = launch_cluster_act<1>(p.activation, ca, splits < 1 ? 1 : splits, K_BWD, s);
       if (rc != RINGRNN_OK) return rc;
     }
-    w += tbn;
     ca.grad_output = a.grad_output;
     ca.coef_x = a.coef_x; ca.coef_y = a.coef_y; ca.coef_s = a.coef_s; ca.dec_u = a.dec_u; ca.dec_v = a.dec_v;
     ca.delta = delta;

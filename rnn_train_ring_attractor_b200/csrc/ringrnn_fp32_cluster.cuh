@@ -39,7 +39,7 @@ struct Args {
   DevProblem p;
   Shape sh;
   float* hist;           // MODE 0: out or nullptr; 1, 2: in  [T,B,N]
-  float* dact;           // [T,B,N] F'(re): MODE 0 out or nullptr, 1 out, 2 in
+  float* dact;           // [T,B,N] F'(re): MODE 0 out or nullptr, 1 out, 2 in (may be delta: the same thread reads, then writes)
   // forward
   float* dec_x;          // [B,T] or nullptr
   float* dec_y;
@@ -309,6 +309,16 @@ __global__ void __launch_bounds__(THREADS, 1) cluster_kernel(const __grid_consta
       }
       return v;
     };
+    auto load2_own = [&](const float* base, int pair, int i) {  // of a tensor this thread may overwrite there: not a read-only load
+      float2 v = make_float2(0.f, 0.f);
+      const int b = b0 + 2 * pair;
+      if (i < N) {
+        const float* src = base + (size_t)b * N + i;
+        if (b < p.B) v.x = src[0];
+        if (b + 1 < p.B) v.y = src[N];
+      }
+      return v;
+    };
     auto save2 = [&](float* base, size_t row_stride, int pair, int i, float2 v) {
       const int b = b0 + 2 * pair;
       if (i < N) {
@@ -331,7 +341,7 @@ __global__ void __launch_bounds__(THREADS, 1) cluster_kernel(const __grid_consta
     struct Ahead { float2 d, go, r; };
     auto fetch = [&](int t, int pair, int n) {
       Ahead x;
-      x.d = load2(a.dact + t * slab, N, pair, i0 + n);
+      x.d = load2_own(a.dact + t * slab, pair, i0 + n);
       x.go = a.grad_output != nullptr ? load2(a.grad_output + t * slab, N, pair, i0 + n) : make_float2(0.f, 0.f);
       x.r = has_coef ? load2(a.hist + t * slab, N, pair, i0 + n) : make_float2(0.f, 0.f);
       return x;

@@ -92,6 +92,17 @@ def test_workspace_sizes(L):
     assert L.ringrnn_workspace_bytes(C.byref(pa), _lib.WS_FWD, 1) < L.ringrnn_workspace_bytes(C.byref(pf), _lib.WS_FWD, 1)
 
 
+def test_fp32_mode_holds_two_histories_beyond_what_it_can_spare(L):
+    """A long sequence in the fp32 mode: the history (the caller's or the library's) and delta, nothing else of that size.
+    B * T floats per CTA and column come on top for dL/dA, a fifth of a history at most."""
+    for N, B, T in ((250, 60000, 100), (128, 20000, 1000), (600, 3000, 500)):
+        p = _problem(B=B, T=T, N=N)
+        one = 4 * B * T * N
+        assert L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_SAVED, 0) < 1.001 * one
+        assert L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_SAVED, 1) == 0
+        assert L.ringrnn_workspace_bytes(C.byref(p), _lib.WS_BWD, 0) < 1.2 * one + (64 << 20)
+
+
 def test_bf16_mode_sizes_every_shape_and_checkpoints_shrink_the_saved_state(L):
     """bf16 mode takes any shape with up to 64 active action columns (persistent kernels or one GEMM per timestep);
     checkpoints replace the per-step saved tensors by T/K states."""

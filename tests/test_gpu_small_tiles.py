@@ -69,6 +69,21 @@ def test_small_tile_kernels_match_the_oracle(prec, shape):
         assert float(((f[k].cpu().double() - want.T).abs() / scale.clamp(min=1e-30)).max()) < (N + 8) * 2.0 ** -24, k
 
 
+@pytest.mark.parametrize("N,B,T", [(250, 600, 3), (32, 2100, 1000)])
+def test_fp32_backward_from_the_librarys_own_history(N, B, T):
+    """Without a history of the caller's the forward keeps one, and F'(re) of every step beside it up to 256 MB; otherwise the
+    reverse pass forms F' from the history.  The same arithmetic either way: the same bits."""
+    from gpu_helpers import canaries_intact, run_backward, run_forward
+    A, Wa, Wo, r0, cot = (t.cuda() for t in _case(N, B, T, 2, 7))
+    out = []
+    for history in (True, False):
+        f = run_forward(A, Wa * 0.3, Wo, r0, -0.03, 0.1, 0.1, "tanh", "fp32", history=history)
+        out.append(run_backward(A, Wa * 0.3, Wo, r0, -0.03, 0.1, 0.1, "tanh", f, grad_output=cot))
+        assert all(canaries_intact(x) for x in f["backs"] + out[-1]["backs"])
+    for k in ("dWo", "dWa", "dJ", "dr_init", "dA"):
+        assert torch.isfinite(out[0][k]).all() and torch.equal(out[0][k], out[1][k]), k
+
+
 def test_more_steps_than_a_grid_has_rows():
     """65535 is the largest extent of a grid's second dimension: sequences beyond it on the one-GEMM-per-step path, against
     the fp32 mode.  Bound: weights, state and delta are rounded to bf16 (2^-9 each), and what a step gets wrong the next ones
