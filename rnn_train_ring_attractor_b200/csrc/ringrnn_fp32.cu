@@ -429,6 +429,77 @@ __global__ void __launch_bounds__(DW_THREADS, 2) dw_fp32_kernel(DevProblem p, co
   }
 }
 
+// N <= 64: one tile of 64 x 64, 4 x 4 per thread, 16 rows at a time.  Most of the larger tile would be padding, and the FMAs on
+// it the bound: operator forward and backward, N = 16, B = 4000, 60 steps: 1648 us with tiles of 128, 1210 with these.
+constexpr int DW_SMALL_TILE = 64;
+constexpr int DW_SMALL_KC = 16;
+
+__global__ void __launch_bounds__(256) dw_fp32_small_kernel(DevProblem p, const float* __restrict__ delta,
+                                                            const float* __restrict__ hist, float* __restrict__ partial,
+                                                            int ksplit, long long k_per_split) {
+  __shared__ __align__(16) float dsm[DW_SMALL_KC][DW_SMALL_TILE];
+  __shared__ __align__(16) float rsm[DW_SMALL_KC][DW_SMALL_TILE];
+  const int N = p.N;
+  const int m = blockIdx.z / ksplit, s = blockIdx.z % ksplit;
+  const int i0 = blockIdx.y * DW_SMALL_TILE, j0 = blockIdx.x * DW_SMALL_TILE;
+  const long long K = (long long)p.T * p.B;
+  const long long k_begin = (long long)s * k_per_split;
+  const long long k_end = (k_begin + k_per_split < K) ? k_begin + k_per_split : K;
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const int lr = threadIdx.x / 16;        // k row this thread loads
+  const int lc = (threadIdx.x % 16) * 4;  // first of 4 columns it loads
+  float acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+
+  for (long long kk = k_begin; kk < k_end; kk += DW_SMALL_KC) {
+    const long long k = kk + lr;
+    float dv[4] = {0.f, 0.f, 0.f, 0.f}, rv[4] = {0.f, 0.f, 0.f, 0.f};
+    if (k < k_end) {
+      const int t = (int)(k / p.B), b = (int)(k % p.B);
+      const float sc = (m == 0) ? 1.f : __ldg(p.A + ((size_t)b * p.T + t) * p.a_dim + active_col(p, m - 1));
+      const float* drow = delta + (size_t)k * N;
+      const float* rrow = (t == 0) ? p.r_init + (size_t)b * N : hist + ((size_t)(t - 1) * p.B + b) * N;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if (i0 + lc + c < N) dv[c] = sc * __ldg(drow + i0 + lc + c);
+        if (j0 + lc + c < N) rv[c] = __ldg(rrow + j0 + lc + c);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      dsm[lr][lc + c] = dv[c];
+      rsm[lr][lc + c] = rv[c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < DW_SMALL_KC; ++q) {
+      const float4 a4 = *reinterpret_cast<const float4*>(&dsm[q][ty * 4]);
+      const float4 b4 = *reinterpret_cast<const float4*>(&rsm[q][tx * 4]);
+      const float av[4] = {a4.x, a4.y, a4.z, a4.w};
+      const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+    }
+  }
+  float* out = partial + ((size_t)s * p.n_mat + m) * N * N;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int i = i0 + ty * 4 + a;
+    if (i >= N) continue;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int j = j0 + tx * 4 + b;
+      if (j < N) out[(size_t)i * N + j] = acc[a][b];
+    }
+  }
+}
+
 // grad_Wo = J1 * sum_s partial[s][0], grad_Wa[cols[m-1]] = sum_s partial[s][m]; raw[] keeps the
 // unscaled m = 0 sum for the J0/J1 gradients.
 __global__ void dw_reduce_kernel(DevProblem p, const float* __restrict__ partial, int ksplit, float* grad_Wa,
@@ -513,7 +584,7 @@ namespace {
 int pick_ksplit(const RingRnnProblem& p, int n_mat) {
   const int tiles = ((p.N + DW_TILE - 1) / DW_TILE) * ((p.N + DW_TILE - 1) / DW_TILE) * n_mat;
   long long K = (long long)p.T * p.B;
-  int ks = 2 * 148 / tiles;  // two resident CTAs per SM
+  int ks = (p.N <= DW_SMALL_TILE ? 4 * 148 : 2 * 148) / tiles;  // small tiles: four CTAs per SM, larger ones: two
   if (ks < 1) ks = 1;
   if (ks > 64) ks = 64;
   while (ks > 1 && K / ks < 64) --ks;
@@ -585,11 +656,19 @@ int launch_transpose(const DevProblem& dp, float* WT, cudaStream_t s) {
 }
 
 // ---- cluster kernels (ringrnn_fp32_cluster.cuh): which requests, and in what shape -------------------------------
-// The shape with the least estimated time per step among those whose weights and buffers fit shared memory:
-// rounds of resident clusters x (FMA issue of one CTA's neurons for the tile + exchange and barrier).  Resident clusters on
-// a B200 (148 SMs, GPCs of unequal size): 15 of 8, 33 of 4.  No shape fits: the kernels above, weights through L2.
-bool cluster_shape(const RingRnnProblem& p, int n_mat, fc::Shape* out) {
-  const int resident[4] = {148, 74, 33, 15};
+// The shape with the least estimated cycles per step among those whose weights and buffers fit shared memory: rounds of
+// resident clusters x (FMA issue of one CTA's neurons for the tile + exchange and barrier).  Resident clusters on a B200 (148
+// SMs, GPCs of unequal size): 15 of 8, 33 of 4.
+//
+// A step really takes about twice the estimate (N = 250: 9.1-9.6 us per round of 480 samples against 4.6), and the kernels
+// above, two CTAs of 16 samples per SM at a time, about 226 cycles per neuron and matrix (0.345 us N with three).  They
+// win where no shape fits, and between the rounds of large batches; times of clusters against them, 60 steps with two
+// columns: forward N = 250 0.73 at 3000 samples, 0.94 at 4000, 0.70 at 8000, N = 200 0.96, 1.28, 1.13, N = 160 0.84 at 4000;
+// training N = 250 0.54, 0.66, 0.93.  From a history of the caller's the reverse pass needs F'(re) formed first, and with it
+// the operator's forward and backward (and dL/dA) N = 250 0.89 (0.97), 1.10 (1.20), 0.93 (1.00), N = 200 0.89 (0.98), 1.12
+// (1.23), 1.04 (1.13): clusters need more of an advantage there.
+constexpr int RESIDENT_CLUSTERS[4] = {148, 74, 33, 15};  // of 1, 2, 4, 8 CTAs
+bool cluster_shape(const RingRnnProblem& p, int n_mat, fc::Shape* out, bool from_history = false) {
   double best = 1e300;
   for (int lc = 0; lc < 4; ++lc) {
     const int C = 1 << lc;
@@ -601,7 +680,7 @@ bool cluster_shape(const RingRnnProblem& p, int n_mat, fc::Shape* out) {
     for (h.NO = 1; h.NO <= 4; ++h.NO) {
       h.tiles = (p.B + 8 * h.NO - 1) / (8 * h.NO);
       if (sizeof(float) * (size_t)fc::offsets(h, n_mat, 2).total > SMEM_MAX) continue;
-      const double rounds = (h.tiles + resident[lc] - 1) / resident[lc];
+      const double rounds = (h.tiles + RESIDENT_CLUSTERS[lc] - 1) / RESIDENT_CLUSTERS[lc];
       const double cost = rounds * (n_mat * (double)h.NC * h.NP * 8 * h.NO / 128 * 1.25 + 900 + (C > 1 ? 400 : 0));
       if (cost < best) {
         best = cost;
@@ -609,7 +688,14 @@ bool cluster_shape(const RingRnnProblem& p, int n_mat, fc::Shape* out) {
       }
     }
   }
-  return best < 1e300;
+  const double waves = ((p.B + 15) / 16 + 295) / 296;
+  return best * (from_history ? 2.6 : 2.0) < waves * 226.0 * p.N * n_mat;
+}
+
+// A cluster runs tile after tile, so that it loads its weights once.
+int clusters_of(const fc::Shape& h) {
+  const int resident = RESIDENT_CLUSTERS[h.C == 1 ? 0 : h.C == 2 ? 1 : h.C == 4 ? 2 : 3];
+  return h.tiles < resident ? h.tiles : resident;
 }
 
 template <int MODE, int ACT>
@@ -628,7 +714,7 @@ int launch_cluster(const fc::Args& a, int splits, int slot, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   RINGRNN_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
-  cfg.gridDim = dim3(a.sh.tiles * a.sh.C, splits, 1);
+  cfg.gridDim = dim3(clusters_of(a.sh) * a.sh.C, splits, 1);
   {
     LaunchScope ls(slot, s);
     RINGRNN_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a));
@@ -751,14 +837,14 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
   int rc;
   fc::Args ca;
   memset(&ca, 0, sizeof(ca));
-  if (cluster_shape(p, n_mat, &ca.sh)) {
+  if (cluster_shape(p, n_mat, &ca.sh, a.bump_history != nullptr)) {
     ca.p = dp;
     ca.hist = const_cast<float*>(hist);
     if (a.bump_history == nullptr && keeps_dact(p)) {  // the forward kept F'(re) beside the history
       ca.dact = reinterpret_cast<float*>(static_cast<char*>(const_cast<void*>(a.saved)) + history_bytes(p));
     } else {  // only the history: F'(re) of all steps at once first, off the sequential path, where delta goes later
       ca.dact = delta;
-      int splits = 148 / (ca.sh.tiles * ca.sh.C);
+      int splits = 148 / (clusters_of(ca.sh) * ca.sh.C);
       if (splits > p.T) splits = p.T;
       rc = launch_cluster_act<1>(p.activation, ca, splits < 1 ? 1 : splits, K_BWD, s);
       if (rc != RINGRNN_OK) return rc;
@@ -788,9 +874,15 @@ int fp32_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
 
   const long long K = (long long)p.T * p.B;
   long long kps = (K + ksplit - 1) / ksplit;
-  kps = (kps + DW_KC - 1) / DW_KC * DW_KC;
+  kps = (kps + DW_SMALL_KC - 1) / DW_SMALL_KC * DW_SMALL_KC;  // (a multiple of both kernels' rows at a time)
   dim3 grid((p.N + DW_TILE - 1) / DW_TILE, (p.N + DW_TILE - 1) / DW_TILE, n_mat * ksplit);
-  { LaunchScope ls(K_DW, s); dw_fp32_kernel<<<grid, DW_THREADS, 0, s>>>(dp, delta, hist, partial, ksplit, kps); }
+  {
+    LaunchScope ls(K_DW, s);
+    if (p.N <= DW_SMALL_TILE)
+      dw_fp32_small_kernel<<<grid, 256, 0, s>>>(dp, delta, hist, partial, ksplit, kps);
+    else
+      dw_fp32_kernel<<<grid, DW_THREADS, 0, s>>>(dp, delta, hist, partial, ksplit, kps);
+  }
   RINGRNN_CUDA_TRY(cudaGetLastError());
   RINGRNN_CUDA_TRY(cudaMemsetAsync(a.grad_Wa, 0, sizeof(float) * (size_t)p.a_dim * NN, s));
   { LaunchScope ls(K_REDUCE, s); dw_reduce_kernel<<<296, 256, 0, s>>>(dp, partial, ksplit, a.grad_Wa, a.grad_Wo, raw); }

@@ -33,7 +33,13 @@ LANE = [(1, 1, 1, 2, "tanh", -0.1, 0.1), (2, 17, 8, 1, "silu", -0.1, 0.1), (127,
         (512, 1056, 3, 2, "tanh", -0.02, 0.1), (300, 1057, 2, 2, "tanh", -0.02, 0.1)]
 # fp32 clusters: one CTA, two, four, eight; a last CTA with few neurons; several column counts; no shape that fits
 CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), (97, 9, 4, 2, "gelu", -0.1, 0.1),
-           (200, 300, 3, 2, "tanh", -0.1, 0.1), (257, 70, 3, 1, "silu", -0.05, 0.2), (320, 33, 2, 2, "tanh", -0.04, 0.1)]
+           (200, 300, 3, 2, "tanh", -0.1, 0.1), (257, 70, 3, 1, "silu", -0.05, 0.2), (320, 33, 2, 2, "tanh", -0.04, 0.1),
+           (250, 40, 3, 2, "gelu", -0.05, 0.1),
+           # more tiles than resident clusters (148 of one CTA, 74 of two, 33 of four, 15 of eight): a cluster runs several
+           (16, 5000, 2, 2, "tanh", -0.1, 0.1), (160, 1300, 2, 2, "silu", -0.05, 0.1), (200, 1000, 3, 2, "gelu", -0.05, 0.1),
+           (250, 600, 3, 2, "silu", -0.05, 0.1),
+           # a forward on clusters and a reverse pass on single CTAs, both on single CTAs
+           (200, 3000, 2, 2, "tanh", -0.05, 0.1), (200, 4000, 2, 2, "silu", -0.05, 0.1)]
 
 
 # one GEMM per step (more than two action columns): neurons off and on multiples of four (single and 16-byte accesses) and
