@@ -43,8 +43,9 @@ enum { RINGRNN_ACT_RELU = 0, RINGRNN_ACT_GELU = 1, RINGRNN_ACT_TANH = 2, RINGRNN
  * master state (the reference's WMMA path, cpp/kernels/fwd_1loop_tc_idx.cuh). */
 enum { RINGRNN_PREC_FP32 = 0, RINGRNN_PREC_BF16 = 1 };
 
-/* which buffer ringrnn_workspace_bytes() sizes */
-enum { RINGRNN_WS_FWD = 0, RINGRNN_WS_SAVED = 1, RINGRNN_WS_BWD = 2 };
+/* which buffer ringrnn_workspace_bytes() sizes; INFER: the scratch of a forward without `saved`, which may be less than FWD,
+ * the scratch that serves every forward */
+enum { RINGRNN_WS_FWD = 0, RINGRNN_WS_SAVED = 1, RINGRNN_WS_BWD = 2, RINGRNN_WS_INFER = 3 };
 
 #define RINGRNN_MAX_ACTIVE 64
 
@@ -54,10 +55,10 @@ enum { RINGRNN_WS_FWD = 0, RINGRNN_WS_SAVED = 1, RINGRNN_WS_BWD = 2 };
  * script pads the L/R signal to 16 columns with zeros, train_general_ring_no_gain.py:200-223);
  * n_active < 0 means "all a_dim columns" (the fp32 mode then takes any a_dim; the bf16 mode at most
  * RINGRNN_MAX_ACTIVE active columns).  Gradients of skipped columns are exactly zero.
- * ckpt_every = K > 0 (bf16 mode, persistent kernels): the forward keeps only the fp32 state every K steps and the
+ * ckpt_every = K > 0 (bf16 mode): the forward keeps only the fp32 state every K steps and the
  * backward recomputes each stretch of K steps from its checkpoint before it propagates through it -- the saved
  * storage shrinks from two bf16 tensors of T*B*N to T/K fp32 states of B*N, for one extra forward pass.  0 = keep every
- * step (the default; faster whenever the saved tensors fit).  The fp32 mode and the stepwise path ignore it. */
+ * step (the default; faster whenever the saved tensors fit).  The fp32 mode ignores it. */
 typedef struct RingRnnProblem {
   int B, T, N, a_dim;
   int activation; /* RINGRNN_ACT_*  */

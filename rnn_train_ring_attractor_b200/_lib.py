@@ -12,7 +12,7 @@ LIB_PATH = os.path.join(PKG, "libringrnn.so")
 MAX_ACTIVE = 64
 ACT = {"relu": 0, "gelu": 1, "tanh": 2, "silu": 3}  # cpp/ring_rnn_cuda.py:63
 PREC = {"fp32": 0, "bf16": 1}
-WS_FWD, WS_SAVED, WS_BWD = 0, 1, 2
+WS_FWD, WS_SAVED, WS_BWD, WS_INFER = 0, 1, 2, 3
 ERR_UNSUPPORTED = 5
 ERR_DEVICE = 6
 ERR_TOO_LARGE = 7

@@ -219,29 +219,36 @@ extern "C" const char* ringrnn_last_cuda_error_string(void) { return cudaGetErro
 
 extern "C" size_t ringrnn_workspace_bytes(const RingRnnProblem* p, int which, int history_given) {
   if (p == nullptr || check_problem(*p) != RINGRNN_OK) return (size_t)-1;
-  const bool bf16 = p->precision == RINGRNN_PREC_BF16;
-  if (bf16 && lane_supported(*p)) {
+  if (p->precision != RINGRNN_PREC_BF16) {
     switch (which) {
-      case RINGRNN_WS_FWD: return lane_fwd_workspace_bytes(*p);
-      case RINGRNN_WS_SAVED: return lane_saved_bytes(*p);
-      case RINGRNN_WS_BWD: return lane_bwd_workspace_bytes(*p);
+      case RINGRNN_WS_FWD:
+      case RINGRNN_WS_INFER: return fp32_fwd_workspace_bytes(*p);
+      case RINGRNN_WS_SAVED: return fp32_saved_bytes(*p, history_given);
+      case RINGRNN_WS_BWD: return fp32_bwd_workspace_bytes(*p);
       default: return (size_t)-1;
     }
   }
-  if (bf16 && !bf16_supported(*p)) {
-    // bf16 arithmetic, one GEMM per timestep: the shapes the persistent kernels do not take
-    if (!stepwise_supported(*p)) return (size_t)-1;
-    switch (which) {
-      case RINGRNN_WS_FWD: return stepwise_fwd_workspace_bytes(*p);
-      case RINGRNN_WS_SAVED: return stepwise_saved_bytes(*p);
-      case RINGRNN_WS_BWD: return stepwise_bwd_workspace_bytes(*p);
-      default: return (size_t)-1;
-    }
-  }
+  const Route train = training_route(*p);
+  if (train == Route::NONE) return (size_t)-1;
+  auto forward_bytes = [p](Route r) {
+    return r == Route::LANE    ? lane_fwd_workspace_bytes(*p)
+           : r == Route::TILES ? bf16_fwd_workspace_bytes(*p)
+                               : stepwise_fwd_workspace_bytes(*p);
+  };
   switch (which) {
-    case RINGRNN_WS_FWD: return bf16 ? bf16_fwd_workspace_bytes(*p) : fp32_fwd_workspace_bytes(*p);
-    case RINGRNN_WS_SAVED: return bf16 ? bf16_saved_bytes(*p) : fp32_saved_bytes(*p, history_given);
-    case RINGRNN_WS_BWD: return bf16 ? bf16_bwd_workspace_bytes(*p) : fp32_bwd_workspace_bytes(*p);
+    case RINGRNN_WS_FWD:
+    case RINGRNN_WS_INFER: {
+      // with and without a history: a caller may ask for one size and use it for both
+      const size_t a = forward_bytes(inference_route(*p, false)), b = forward_bytes(inference_route(*p, true));
+      const size_t c = which == RINGRNN_WS_FWD ? forward_bytes(train) : 0, ab = a > b ? a : b;
+      return ab > c ? ab : c;
+    }
+    case RINGRNN_WS_SAVED:
+      return train == Route::LANE ? lane_saved_bytes(*p) : train == Route::TILES ? bf16_saved_bytes(*p) : stepwise_saved_bytes(*p);
+    case RINGRNN_WS_BWD:
+      return train == Route::LANE    ? lane_bwd_workspace_bytes(*p)
+             : train == Route::TILES ? bf16_bwd_workspace_bytes(*p)
+                                     : stepwise_bwd_workspace_bytes(*p);
     default: return (size_t)-1;
   }
 }
@@ -262,12 +269,13 @@ extern "C" int ringrnn_fwd(const RingRnnFwdArgs* a, void* stream) {
   const DevProblem dp = to_dev(a->p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
-    if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    if (lane_supported(a->p)) {
+    const Route route = a->saved != nullptr ? training_route(a->p) : inference_route(a->p, a->bump_history != nullptr);
+    if (route == Route::NONE) return RINGRNN_ERR_UNSUPPORTED;
+    if (route == Route::LANE) {
       rc = lane_forward(*a, dp, s);
       return rc != RINGRNN_OK || a->status == nullptr ? rc : queue_status_report(a->status, s);
     }
-    rc = bf16_supported(a->p) ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
+    rc = route == Route::TILES ? bf16_forward(*a, dp, s) : stepwise_forward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }
@@ -290,12 +298,13 @@ extern "C" int ringrnn_bwd(const RingRnnBwdArgs* a, void* stream) {
   const DevProblem dp = to_dev(a->p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (a->p.precision == RINGRNN_PREC_BF16) {
-    if (!bf16_supported(a->p) && !stepwise_supported(a->p)) return RINGRNN_ERR_UNSUPPORTED;
-    if (lane_supported(a->p)) {
+    const Route route = training_route(a->p);
+    if (route == Route::NONE) return RINGRNN_ERR_UNSUPPORTED;
+    if (route == Route::LANE) {
       rc = lane_backward(*a, dp, s);
       return rc != RINGRNN_OK || a->status == nullptr ? rc : queue_status_report(a->status, s);
     }
-    rc = bf16_supported(a->p) ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
+    rc = route == Route::TILES ? bf16_backward(*a, dp, s) : stepwise_backward(*a, dp, s);
     if (rc != RINGRNN_OK) return rc;
     return queue_status_report(a->status != nullptr ? a->status : static_cast<const int*>(a->workspace), s);
   }

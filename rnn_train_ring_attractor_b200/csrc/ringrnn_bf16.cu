@@ -122,23 +122,69 @@ Layout layout_of(const RingRnnProblem& p) {
 
 }  // namespace
 
-// Which bf16 requests the persistent kernels take: N <= 1024 with up to two active action columns; N <= 512 with up to
-// RINGRNN_MAX_ACTIVE of them when the batch is large.  A persistent kernel keeps one cluster busy per 128 samples and
-// its step time grows with the number of weight groups, so with more than two columns the stepwise path (full-machine GEMMs,
-// ringrnn_stepwise.cu) is faster up to 2048 samples.  Operator forward and backward, T = 32, stepwise against persistent, ms:
-// B = 2048: N = 256 with 6 columns 1.11 / 1.43, N = 384 with 3 1.23 / 1.54, N = 512 with 8 1.99 / 2.10, N = 128 with 6 1.02 /
-// 1.02; B = 4096, N = 256 with 6: 1.85 / 1.49.
-// N > 512 with up to two columns: clusters of eight take 18 us per step of either direction at any batch, one GEMM per step
-// less than that up to 512 samples.  Training step, T = 64, stepwise against persistent, ms: N = 1024 B = 32 1.79 / 2.44, 256
-// 2.00 / 2.55, 512 2.29 / 2.62, 1024 3.22 / 2.75; N = 600 B = 100 1.53 / 2.42, 1000 2.71 / 2.69.
+// checkpoint interval in force (0 = every step is kept)
+int ckpt_interval(const RingRnnProblem& p) { return (p.ckpt_every > 0 && p.ckpt_every < p.T) ? p.ckpt_every : 0; }
+
+// ---- which kernels a bf16 request runs on --------------------------------------------------------------------------
+// Small tiles (ringrnn_lane.cu) take as many SMs as the batch has groups of 16-64 samples, tiles of 128 (this file) one cluster
+// per 128 samples at a step time that grows with the weight groups, the stepwise path (ringrnn_stepwise.cu) the whole machine
+// at two launches per step.  Each line lies where the measured times cross; all figures are times of the first against the
+// second kind of kernel, in us, T = 24, tanh, unless a ratio is given.  Training calls keep one route whether or not the
+// caller keeps a history: `saved` is laid out by it.
+//
+// Up to two columns, training:
+//   N <= 128, small tiles to 148 CTAs of 64 samples, against tiles of 128: step ratio 0.81 at 9472, 1.24 at 9600 (the reverse
+//     kernel's second round), 1.17 at 28000.
+//   N <= 256, to 74 clusters of 64: 0.87 at 4736, 1.38 at 4800, 1.40 at 20000 (T = 100, gelu: 0.92, 1.61).
+//   N <= 512, to two rounds of 33 clusters of 16: 0.95 at 1056 (T = 128: 1.02; operator forward and backward 0.90), 1.31 at 1100.
+//   N <= 1024, stepwise against tiles of 128: N = 1024 0.92 at 400 samples, 1.00 at 512 (operator 0.83), 1.13 at 640; N = 600
+//     0.86 at 512, 0.96 at 768.  Its scratch is a sixth more, so sequences whose saved state alone takes 16 GB stay with the tiles.
+// Up to two columns, inference: small tiles have no reverse kernel to wait for.
+//   N <= 128: 0.54 to 0.73 of the tiles' time from 9472 to 28000 samples without a history.  N <= 256: 0.65 to 0.99 with one;
+//   without, 1.04 to 1.48 beyond 4736.  N <= 1024 without a history: stepwise 0.83 to 0.97 at 384, 1.05 (T = 100: 1.09) at 512.
+// More columns, N <= 512 (beyond, stepwise): stepwise up to 1024 samples, tiles of 128 from 2049 on.  Between, stepwise
+//   against tiles, operator forward and backward / training step: N = 128 with 3 columns 1.26 / 1.54 at 2048, N = 256 with 3 1.04 /
+//   1.35, with 6 0.92 / 1.05, with 16 0.85 / 0.92; N = 512 with 3 to 16 0.78 to 0.91 / 0.81 to 1.01 at 1100, 0.83 to 1.03 /
+//   0.95 to 1.18 at 1280; N = 384 with 4 0.78 / 0.92 at 1100, 1.01 / 1.16 at 1280.  Forward only: N <= 256 1.05 to 1.94 from
+//   1100 on, N = 384 and 512 with a history 0.73 to 1.00 at 1100, 0.78 to 1.11 at 1280.  N <= 128 without a history: 1.07 to
+//   1.94 at 512 already.
 // RINGRNN_STEPWISE=1 sends every bf16 request to the stepwise path (for comparisons).
-bool bf16_supported(const RingRnnProblem& p) {
-  static const bool force_stepwise = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
-  if (force_stepwise) return false;
+constexpr int LANE_128_MAX_B = 148 * 64, LANE_256_MAX_B = 74 * 64, LANE_512_MAX_B = 33 * 16 * 2;
+
+static bool force_stepwise() {
+  static const bool on = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
+  return on;
+}
+
+Route training_route(const RingRnnProblem& p) {
+  if (!stepwise_supported(p)) return Route::NONE;
   const int NP = padded_n(p.N), n_act = n_active_of(p);
-  if (NP == 0 || p.B < 1 || p.T < 1) return false;
-  if (n_act <= 2) return NP <= 512 || p.B > 512;
-  return NP <= 512 && n_act <= RINGRNN_MAX_ACTIVE && p.B > 2048;
+  if (force_stepwise() || NP == 0) return Route::STEPWISE;
+  if (n_act <= 2) {
+    if (NP == 1024) {
+      const int steps = ckpt_interval(p) > 0 ? ckpt_interval(p) : p.T;
+      return p.B > 512 || (long long)steps * padded_b(p.B, p.N, n_act) * NP > (1ll << 32) ? Route::TILES : Route::STEPWISE;
+    }
+    return p.B <= (NP == 128 ? LANE_128_MAX_B : NP == 256 ? LANE_256_MAX_B : LANE_512_MAX_B) ? Route::LANE : Route::TILES;
+  }
+  if (NP == 1024 || p.B <= 1024) return Route::STEPWISE;
+  if (p.B > 2048) return Route::TILES;
+  return (NP == 256 && n_act >= 6) || (NP == 512 && p.B <= 1152) ? Route::STEPWISE : Route::TILES;
+}
+
+Route inference_route(const RingRnnProblem& p, bool history) {
+  const Route train = training_route(p);
+  if (train == Route::NONE || force_stepwise()) return train;
+  const int NP = padded_n(p.N), n_act = n_active_of(p);
+  if (NP == 0) return train;
+  if (n_act <= 2) {
+    if (NP == 128 || (NP == 256 && history)) return Route::LANE;
+    if (NP == 1024) return p.B > (history ? 512 : 384) ? Route::TILES : Route::STEPWISE;
+    return train;
+  }
+  if (NP == 128 && !history) return Route::TILES;
+  if (NP <= 512 && p.B > 1024 && (NP <= 256 || !history)) return Route::TILES;
+  return train;
 }
 
 // FWD workspace: status(1024) | Wf | R0 | dec partials
@@ -150,8 +196,6 @@ size_t bf16_fwd_workspace_bytes(const RingRnnProblem& p) {
 size_t sign_mask_bytes(const RingRnnProblem& p, const Layout& l) {
   return align_up((size_t)p.T * (l.NP / 32) * 2 * l.BP * 4, 1024);
 }
-// checkpoint interval in force (0 = every step is kept)
-int ckpt_interval(const RingRnnProblem& p) { return (p.ckpt_every > 0 && p.ckpt_every < p.T) ? p.ckpt_every : 0; }
 size_t ckpt_slot_bytes(const RingRnnProblem& p) { return (size_t)p.B * p.N * sizeof(float); }
 size_t saved_every_step_bytes(const RingRnnProblem& p) {
   const Layout l = layout_of(p);

@@ -123,7 +123,13 @@ int tc_gemm_slabs(const void* A, const void* B, float* partial, int M, int N, in
 int tc_gemm_pair(const void* A, const void* B, float* out, int M, int N, long long K, int* status, cudaStream_t s);
 
 // bf16 tensor-core path ----------------------------------------------------------------------
-bool bf16_supported(const RingRnnProblem& p);
+// The kernels a request of the bf16 mode runs on; ringrnn_bf16.cu has the rule and its figures.
+enum class Route { NONE, LANE, TILES, STEPWISE };
+// a forward that was given `saved`, and the backward; a forward without, which writes bump_history or does not
+Route training_route(const RingRnnProblem& p);
+Route inference_route(const RingRnnProblem& p, bool history);
+
+// persistent kernels, tiles of 128 samples (ringrnn_bf16.cu)
 size_t bf16_fwd_workspace_bytes(const RingRnnProblem& p);
 size_t bf16_saved_bytes(const RingRnnProblem& p);
 size_t bf16_bwd_workspace_bytes(const RingRnnProblem& p);
@@ -131,7 +137,6 @@ int bf16_forward(const RingRnnFwdArgs& a, const DevProblem& dp, cudaStream_t s);
 int bf16_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s);
 
 // bf16, N <= 256 (small batches: 512) and up to two active columns: neurons on the tensor-memory lanes (ringrnn_lane.cu)
-bool lane_supported(const RingRnnProblem& p);
 size_t lane_fwd_workspace_bytes(const RingRnnProblem& p);
 size_t lane_saved_bytes(const RingRnnProblem& p);
 size_t lane_bwd_workspace_bytes(const RingRnnProblem& p);
@@ -140,7 +145,7 @@ int lane_backward(const RingRnnBwdArgs& a, const DevProblem& dp, cudaStream_t s)
 
 // bf16 stepwise path: one tensor-core GEMM per timestep (ringrnn_stepwise.cu), for the shapes the persistent
 // kernels do not take
-bool stepwise_supported(const RingRnnProblem& p);
+bool stepwise_supported(const RingRnnProblem& p);  // what the bf16 mode takes at all: the other paths take part of it
 size_t stepwise_fwd_workspace_bytes(const RingRnnProblem& p);
 size_t stepwise_saved_bytes(const RingRnnProblem& p);
 size_t stepwise_bwd_workspace_bytes(const RingRnnProblem& p);

@@ -235,18 +235,6 @@ void set_common(P& q, const RingRnnProblem& p, const DevProblem& dp, const LaneL
 
 }  // namespace
 
-// N in (256, 512]: two rounds of 33 resident clusters of 16 samples.  Training step N=512, T=128, against the tiles of 128
-// samples (tc_fwd.cu, tc_bwd.cu), which take one round up to 4096 samples: B = 64 1.37 against 2.67 ms, 512 1.50 / 2.84, 1024
-// 2.82 / 2.89 (with dL/dA, N=400 B=1000 T=100: 2.38 / 2.75), a third round 4.16 / 2.97.
-constexpr int LANE_512_MAX_B = 33 * 16 * 2;
-
-bool lane_supported(const RingRnnProblem& p) {
-  static const bool force_stepwise = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
-  if (force_stepwise) return false;
-  const int n_act = p.n_active < 0 ? p.a_dim : p.n_active;
-  return p.N >= 1 && (p.N <= 256 || (p.N <= 512 && p.B <= LANE_512_MAX_B)) && n_act <= 2 && p.B >= 1 && p.T >= 1;
-}
-
 // FWD workspace: status(1024) | the other CTAs' decode sums [CL-1][3][B][T]
 size_t lane_fwd_workspace_bytes(const RingRnnProblem& p) {
   const LaneLayout l = lane_layout(p);

@@ -1,9 +1,8 @@
 // bf16 mode, stepwise variant: one tensor-core GEMM per timestep instead of a persistent kernel.
 //
-// Used for shapes the persistent tcgen05 kernels do not take, or would leave most of the machine idle on (bf16_supported in
-// ringrnn_bf16.cu has the lines): N > 1024, more than two active action columns at N > 512 or up to 2048 samples, N > 512 up to
-// 512 samples.  Replaces, for those shapes, the same reference
-// kernels as the persistent path (cpp/kernels/fwd_1loop_tc_idx.cuh:265-277 and the five per-step launches of
+// Used for shapes the persistent tcgen05 kernels do not take, or would leave most of the machine idle on (training_route in
+// ringrnn_bf16.cu has the lines).  Replaces, for those shapes, the same reference kernels as the persistent path
+// (cpp/kernels/fwd_1loop_tc_idx.cuh:265-277 and the five per-step launches of
 // cpp/kernels/bwd_mixed_precision_aggressive.cuh:564-671), without materialising W_eff[B,N,N].
 //
 // With m = 0 for Wo and m = 1..n for the active action matrices (coefficient c_0 = 1 -- J1 is folded into the

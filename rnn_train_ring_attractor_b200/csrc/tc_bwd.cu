@@ -634,7 +634,8 @@ int tc_backward_launch(int NP, bool pair, const CUtensorMap& tmW, const CUtensor
     if (NP == 512) return launch_bwd_tc<512, false, true>(tmW, tmDL, tmDL32, p, s);
     return RINGRNN_ERR_UNSUPPORTED;
   }
-  // (two active columns, N <= 256 and small batches of N <= 512: tc_lane_bwd.cu)
+  if (NP == 128) return pair ? launch_bwd_tc<128, true>(tmW, tmDL, tmDL32, p, s) : launch_bwd_tc<128, false>(tmW, tmDL, tmDL32, p, s);
+  if (NP == 256) return pair ? launch_bwd_tc<256, true>(tmW, tmDL, tmDL32, p, s) : launch_bwd_tc<256, false>(tmW, tmDL, tmDL32, p, s);
   if (NP == 512) return pair ? launch_bwd_tc<512, true>(tmW, tmDL, tmDL32, p, s) : launch_bwd_tc<512, false>(tmW, tmDL, tmDL32, p, s);
   if (NP == 1024 && !pair) return launch_bwd_tc<1024, false>(tmW, tmDL, tmDL32, p, s);  // two K rounds per step, clusters of 8
   return RINGRNN_ERR_UNSUPPORTED;

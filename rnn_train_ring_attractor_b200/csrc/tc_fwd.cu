@@ -411,14 +411,13 @@ int tc_forward_launch(int act, int NP, bool pair, const CUtensorMap& tmW, const 
 #undef RINGRNN_TCG
     return RINGRNN_ERR_UNSUPPORTED;
   }
-// (two active columns, N <= 256 and small batches of N <= 512: tc_lane_fwd.cu)
 #define RINGRNN_TCF(ACT, NPV)                                                              \
   if (act == ACT && NP == NPV)                                                             \
     return pair ? launch_fwd_tc<ACT, NPV, true>(tmW, tmR0, p, s) : launch_fwd_tc<ACT, NPV, false>(tmW, tmR0, p, s);
-  RINGRNN_TCF(RINGRNN_ACT_RELU, 512)
-  RINGRNN_TCF(RINGRNN_ACT_GELU, 512)
-  RINGRNN_TCF(RINGRNN_ACT_TANH, 512)
-  RINGRNN_TCF(RINGRNN_ACT_SILU, 512)
+  RINGRNN_TCF(RINGRNN_ACT_RELU, 128) RINGRNN_TCF(RINGRNN_ACT_RELU, 256) RINGRNN_TCF(RINGRNN_ACT_RELU, 512)
+  RINGRNN_TCF(RINGRNN_ACT_GELU, 128) RINGRNN_TCF(RINGRNN_ACT_GELU, 256) RINGRNN_TCF(RINGRNN_ACT_GELU, 512)
+  RINGRNN_TCF(RINGRNN_ACT_TANH, 128) RINGRNN_TCF(RINGRNN_ACT_TANH, 256) RINGRNN_TCF(RINGRNN_ACT_TANH, 512)
+  RINGRNN_TCF(RINGRNN_ACT_SILU, 128) RINGRNN_TCF(RINGRNN_ACT_SILU, 256) RINGRNN_TCF(RINGRNN_ACT_SILU, 512)
 #undef RINGRNN_TCF
   if (NP == 1024 && !pair) {  // two K rounds per step, clusters of 8
     if (act == RINGRNN_ACT_RELU) return launch_fwd_tc<RINGRNN_ACT_RELU, 1024, false>(tmW, tmR0, p, s);

@@ -52,7 +52,7 @@ class RingRnnFusedFunc(Function):
             raise RuntimeError("target_angle must be (batch, seq_len)")
         dev = action_signal.device
         active = list(range(a_dim)) if ctx.needs_input_grad[0] else active_columns(action_signal)
-        prec, n_fwd, n_saved, n_bwd = plan(B, T, N, a_dim, act, len(active), precision, 0, int(ckpt_every))
+        prec, n_fwd, n_saved, n_bwd, _ = plan(B, T, N, a_dim, act, len(active), precision, 0, int(ckpt_every))
         if inv_count is None:
             inv_count = 1.0 / (B * T)
         u, v = decode_vectors(N, dev)
@@ -177,7 +177,7 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
         _check_tensor(name, t)
     dev = action_signal.device
     active = active_columns(action_signal)
-    prec, n_fwd, _, _ = plan(B, T, N, a_dim, act, len(active), precision, 0)
+    prec, _, _, _, n_infer = plan(B, T, N, a_dim, act, len(active), precision, 0)
     u, v = decode_vectors(N, dev)
     L = _lib.lib()
     with on_device(dev), torch.no_grad(), nvtx_range("ringrnn_rollout"):
@@ -185,7 +185,7 @@ def ring_rnn_rollout(action_signal, Wa, J0, J1, Wo, r_init, alpha, activation, p
                               Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active)
         xy = torch.empty(2, B, T, device=dev, dtype=torch.float32)
         final_state = torch.empty(B, N, device=dev, dtype=torch.float32)
-        ws = _scratch(n_fwd, dev)
+        ws = _scratch(n_infer, dev)
         a = _lib.FwdArgs()
         a.p = p
         a.dec_x, a.dec_y = xy[0].data_ptr(), xy[1].data_ptr()

@@ -135,12 +135,12 @@ def active_columns(action_signal):
     return cols
 
 
-_plans = {}  # (shape, precision asked for, history) -> (precision, forward / saved / backward bytes); sizes only, bounded
+_plans = {}  # (shape, precision asked for, history) -> (precision, sizes in bytes); bounded
 
 
 def plan(B, T, N, a_dim, act_code, n_active, requested, history, ckpt_every=0):
-    """(precision code, forward scratch, saved state, backward scratch in bytes) of a request: the precision resolved as
-    choose_precision does, the sizes as ringrnn_workspace_bytes reports them.  They depend on the shape alone, so a
+    """(precision code, forward scratch, saved state, backward scratch, scratch of a forward that saves nothing, in bytes) of
+    a request: the precision resolved as choose_precision does, the sizes as ringrnn_workspace_bytes reports them.  They depend on the shape alone, so a
     training loop asks the library once."""
     key = (B, T, N, a_dim, act_code, n_active, requested or _precision, history, ckpt_every)
     hit = _plans.get(key)
@@ -153,7 +153,8 @@ def plan(B, T, N, a_dim, act_code, n_active, requested, history, ckpt_every=0):
         for k in range(max(p.n_active, 0)):
             p.active_cols[k] = k
         L = _lib.lib()
-        sizes = [L.ringrnn_workspace_bytes(C.byref(p), w, history) for w in (_lib.WS_FWD, _lib.WS_SAVED, _lib.WS_BWD)]
+        sizes = [L.ringrnn_workspace_bytes(C.byref(p), w, history)
+                 for w in (_lib.WS_FWD, _lib.WS_SAVED, _lib.WS_BWD, _lib.WS_INFER)]
         if len(_plans) >= 256:
             _plans.clear()
         hit = _plans[key] = (prec, *sizes)
@@ -220,18 +221,19 @@ class RingRnnCudaFunc(Function):
         dev = action_signal.device
         # zero columns may be skipped only if nobody asks for the gradient with respect to the action signal
         active = list(range(a_dim)) if ctx.needs_input_grad[0] else active_columns(action_signal)
-        prec, n_fwd, n_saved, n_bwd = plan(batch_size, seq_len, N, a_dim, act, len(active), None, 1)
+        prec, n_fwd, n_saved, n_bwd, n_infer = plan(batch_size, seq_len, N, a_dim, act, len(active), None, 1)
         L = _lib.lib()
         with on_device(dev), nvtx_range("ringrnn_fwd"):
             p = _lib.make_problem(batch_size, seq_len, N, a_dim, act, prec, _scalar(J0), _scalar(J1), alpha,
                                   action_signal.data_ptr(), Wa.data_ptr(), Wo.data_ptr(), r_init.data_ptr(), active)
             bump_history = torch.empty(seq_len, batch_size, N, device=dev, dtype=action_signal.dtype)
-            ws = _scratch(n_fwd, dev)
+            keep = any(ctx.needs_input_grad)  # (true under no_grad too when a weight requires a gradient)
+            ws = _scratch(n_fwd if keep else n_infer, dev)
             a = _lib.FwdArgs()
             a.p = p
             a.bump_history = bump_history.data_ptr()
             saved = None
-            if any(ctx.needs_input_grad):  # nothing is kept for a backward that cannot come
+            if keep:
                 saved = _scratch(n_saved, dev)
                 a.saved, a.saved_bytes = saved.data_ptr(), saved.numel()
             a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()

@@ -130,6 +130,20 @@ def test_bf16_mode_sizes_every_shape_and_checkpoints_shrink_the_saved_state(L):
     assert L.ringrnn_workspace_bytes(C.byref(same), _lib.WS_SAVED, 0) == L.ringrnn_workspace_bytes(C.byref(base), _lib.WS_SAVED, 0)
 
 
+def test_scratch_of_a_forward_that_saves_nothing(L):
+    """RINGRNN_WS_FWD serves every forward; RINGRNN_WS_INFER those without `saved`, and is never more."""
+    less = 0
+    for prec in (0, 1):
+        for N in (16, 128, 200, 256, 400, 512, 600, 1024, 1100):
+            for B in (1, 384, 512, 1056, 1100, 2048, 5000, 10000):
+                for a_dim in (1, 2, 3, 6, 16):
+                    p = _problem(B=B, T=7, N=N, a_dim=a_dim, prec=prec)
+                    fwd, infer = (L.ringrnn_workspace_bytes(C.byref(p), w, 1) for w in (_lib.WS_FWD, _lib.WS_INFER))
+                    assert 0 < infer <= fwd < C.c_size_t(-1).value
+                    less += infer < fwd
+    assert less > 0
+
+
 def test_clip_adam_validates_arguments(L):
     assert L.ringrnn_clip_adam(None, 1, 1, 1, 10, 1e-3, 0.9, 0.999, 1e-8, 1, 1.0, 1, None) == 1
     assert L.ringrnn_clip_adam(1, 1, 1, 1, 10, 1e-3, 0.9, 0.999, 1e-8, 0, 1.0, 1, None) == 1   # steps count from 1

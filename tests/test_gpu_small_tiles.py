@@ -23,11 +23,12 @@ def _case(N, B, T, a_dim, seed):
             torch.randn(N, N, generator=g) * s, torch.rand(B, N, generator=g) - 0.5, torch.randn(T, B, N, generator=g))
 
 
-# neurons around the 128-lane and two-CTA limits; batches around 16, 32, 64 samples per unit (148 or 74 units resident) and
-# beyond one round of units; steps around the eight whose scalars are staged at a time; J1 = 0 (no ratio to J1)
+# neurons around the 128-lane and two-CTA limits; batches around 16, 32, 64 samples per unit (148 or 74 units resident), the
+# largest that train on them, and beyond; steps around the eight whose scalars are staged at a time; J1 = 0 (no ratio to J1)
 LANE = [(1, 1, 1, 2, "tanh", -0.1, 0.1), (2, 17, 8, 1, "silu", -0.1, 0.1), (127, 16, 9, 2, "gelu", -0.1, 0.1),
         (128, 2369, 7, 2, "tanh", -0.07, 0.3), (129, 15, 16, 2, "silu", -0.1, 0.1), (255, 1185, 3, 2, "gelu", -0.031, 0.1),
         (256, 2400, 9, 2, "tanh", -0.05, 0.0), (120, 9500, 2, 2, "silu", 0.0, 0.1), (100, 20001, 3, 2, "tanh", -0.1, 0.1),
+        (90, 9472, 3, 2, "gelu", -0.1, 0.1), (192, 4736, 2, 2, "silu", -0.05, 0.1),
         # four CTAs: neurons around 256 and 512, one and several rounds of 33 clusters of 16 samples, the last batch taken
         (257, 1, 1, 2, "tanh", -0.1, 0.1), (384, 17, 9, 1, "silu", -0.05, 0.1), (510, 33, 8, 2, "gelu", -0.013, 0.1),
         (512, 1056, 3, 2, "tanh", -0.02, 0.1), (300, 1057, 2, 2, "tanh", -0.02, 0.1)]
@@ -45,10 +46,14 @@ CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), 
 # one GEMM per step (more than two action columns): neurons off and on multiples of four (single and 16-byte accesses) and
 # beyond one round of 512 threads x 4 neurons, one and several K splits, and a batch that takes the concatenated operand
 STEPWISE = [(65, 3, 2, 3, "tanh", -0.1, 0.1), (130, 129, 3, 4, "silu", -0.1, 0.1), (384, 200, 3, 8, "gelu", -0.05, 0.1),
-            (600, 1900, 2, 3, "tanh", -0.02, 0.1), (2180, 5, 2, 3, "tanh", -0.01, 0.1), (513, 512, 2, 2, "tanh", -0.02, 0.1)]
+            (600, 1900, 2, 3, "tanh", -0.02, 0.1), (2180, 5, 2, 3, "tanh", -0.01, 0.1), (513, 512, 2, 2, "tanh", -0.02, 0.1),
+            (250, 2048, 2, 6, "tanh", -0.05, 0.1), (500, 1152, 2, 4, "silu", -0.02, 0.1)]
 
-# persistent tiles of 128 samples with several weight groups, and with two K rounds: batches above the stepwise path's
-GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1), (1000, 513, 3, 2, "tanh", -0.02, 0.1)]
+# persistent tiles of 128 samples with several weight groups, with two K rounds, and beyond the batches of the small tiles: the
+# smallest batches that train on them
+GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1), (1000, 513, 3, 2, "tanh", -0.02, 0.1),
+           (100, 1025, 3, 9, "tanh", -0.1, 0.1), (200, 1025, 2, 5, "gelu", -0.05, 0.1), (500, 1153, 2, 3, "silu", -0.02, 0.1),
+           (128, 9473, 3, 2, "gelu", -0.07, 0.1), (256, 4737, 3, 2, "tanh", -0.05, 0.1), (512, 1057, 4, 2, "gelu", -0.02, 0.1)]
 
 
 @pytest.mark.parametrize("prec,shape", [("bf16", s) for s in LANE + STEPWISE + GENERIC] + [("fp32", s) for s in CLUSTER],
@@ -73,6 +78,36 @@ def test_small_tile_kernels_match_the_oracle(prec, shape):
     for k, want in (("x", h @ u), ("y", h @ v), ("ta", h.abs().sum(2))):
         scale = (h.abs() @ (u.abs() if k == "x" else v.abs() if k == "y" else torch.ones(N, dtype=torch.float64))).T
         assert float(((f[k].cpu().double() - want.T).abs() / scale.clamp(min=1e-30)).max()) < (N + 8) * 2.0 ** -24, k
+
+
+# forward calls that save nothing may run on other kernels than those that do: both sides of each line
+INFER = [(100, 20001, 3, 2, "tanh"), (64, 9473, 9, 2, "gelu"), (256, 4736, 3, 2, "silu"), (256, 4737, 4, 2, "gelu"),
+         (1000, 384, 3, 2, "tanh"), (1000, 385, 3, 2, "tanh"), (1000, 512, 3, 2, "silu"), (64, 33, 5, 3, "silu"), (128, 1, 3, 16, "gelu"),
+         (128, 1025, 3, 16, "gelu"), (256, 1024, 3, 6, "tanh"), (256, 2048, 3, 6, "tanh"), (500, 1152, 3, 4, "silu"),
+         (500, 1153, 3, 4, "silu"), (300, 1025, 2, 5, "tanh")]
+
+
+@pytest.mark.parametrize("shape", INFER, ids=lambda v: "N%d-B%d-T%d-a%d-%s" % v)
+def test_forward_that_saves_nothing(shape):
+    from gpu_helpers import canaries_intact, run_forward
+    N, B, T, a_dim, act = shape
+    J0, J1 = -0.1 * min(1.0, 64.0 / N), 0.1
+    A, Wa, Wo, r0, _ = _case(N, B, T, a_dim, N + B)
+    rows = sorted({0, 1, B // 2, B - 1} & set(range(B)))  # samples do not interact
+    f64 = [x.double() for x in (A[rows], Wa, Wo, r0[rows])]
+    want = orc.ring_forward_lean(f64[0], f64[1], J0, J1, f64[2], f64[3], 0.1, act)
+    dev = [x.cuda() for x in (A, Wa, Wo, r0)]
+    for history in (False, True):
+        f = run_forward(*dev, J0, J1, 0.1, act, "bf16", None, history=history, decode=True, save=False)
+        assert all(canaries_intact(x) for x in f["backs"])
+        if history:
+            assert orc.rel_err(f["hist"][:, rows], want) < TOL["bf16"]
+        assert orc.rel_err(f["final"][rows], want[-1]) < TOL["bf16"]
+        u, v = f["u"].cpu().double(), f["v"].cpu().double()
+        for k, w in (("x", u), ("y", v)):
+            scale = (want.abs() @ w.abs()).T
+            assert float(((f[k][rows].cpu().double() - (want @ w).T).abs() / scale).max()) < 3 * TOL["bf16"], k
+        assert orc.rel_err(f["ta"][rows], want.abs().sum(2).T) < TOL["bf16"]
 
 
 @pytest.mark.parametrize("N,B,T", [(250, 600, 3), (32, 2100, 1000)])
