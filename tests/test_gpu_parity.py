@@ -216,7 +216,9 @@ def test_autograd_surface_against_reference_training_gradients(name):
 # in dWo at T=32 and any two precisions decorrelate at T=512 -- so that shape is compared at T=8, where errors are
 # still those of the arithmetic; (256, 192, 32) and (512, 192, 32, tanh) cover the longer horizon.
 FUSED_CASES = [(120, 128, 120, "tanh"), (24, 5, 12, "gelu"), (256, 64, 40, "relu"), (512, 192, 8, "gelu"),
-               (256, 192, 32, "gelu"), (512, 192, 32, "tanh"), (1024, 192, 12, "tanh"), (1280, 40, 5, "tanh")]
+               (256, 192, 32, "gelu"), (512, 192, 32, "tanh"), (1024, 192, 12, "tanh"), (1280, 40, 5, "tanh"),
+               # batches of the persistent tiles (the shapes above run on small tiles or one GEMM per step)
+               (512, 1100, 8, "gelu"), (1024, 520, 6, "tanh")]
 
 
 @pytest.mark.parametrize("cfg", FUSED_CASES, ids=lambda c: "N%d-B%d-T%d-%s" % c)
@@ -286,9 +288,10 @@ def test_fused_python_surface_and_rollout():
     assert torch.allclose(final2, final)
 
 
-@pytest.mark.parametrize("N,B,T", [(1024, 130, 9), (640, 300, 6), (1024, 260, 2), (1024, 64, 1)])
+@pytest.mark.parametrize("N,B,T", [(1024, 130, 9), (640, 300, 6), (1024, 260, 2), (1024, 64, 1),
+                                   (1024, 520, 9), (640, 600, 6), (1024, 2100, 2), (768, 513, 1)])
 def test_two_round_rollout_matches_the_training_forward(N, B, T, achieved):
-    """N > 512 (two K rounds): the CTAs of a cluster exchange the state through global memory -- through the saved
+    """N > 512; more than 512 samples (up to that, one GEMM per step either way) run in two K rounds: the CTAs of a cluster exchange the state through global memory -- through the saved
     state in training, through a three-block ring when nothing is saved.  Both forwards must decode the same angles
     and end in the same state, and agree with the oracle within the bf16-mode tolerance."""
     from rnn_train_ring_attractor_b200.fused import ring_rnn_fused, ring_rnn_rollout
@@ -457,8 +460,11 @@ def test_linearity_in_batch_at_scale(prec):
     assert orc.rel_err(acc_o, full["dWo"]) < 1e-5 and orc.rel_err(acc_a, full["dWa"]) < 1e-5
 
 
+# small tiles, one GEMM per step (N = 1024 with 130 samples, N = 192 with 1100 and five columns), persistent tiles of 128
 @pytest.mark.parametrize("cfg", [(256, 300, 50, "tanh", 16), (120, 128, 120, "tanh", 64), (512, 192, 12, "gelu", 5),
-                                 (1024, 130, 9, "tanh", 4), (96, 20000, 7, "silu", 3), (192, 1100, 10, "tanh", 4)],
+                                 (1024, 130, 9, "tanh", 4), (96, 20000, 7, "silu", 3), (192, 1100, 10, "tanh", 4),
+                                 (512, 1100, 12, "gelu", 5), (1024, 520, 9, "tanh", 4), (192, 2100, 10, "tanh", 4),
+                                 (256, 4800, 7, "silu", 3)],
                          ids=lambda c: "N%d-B%d-T%d-%s-K%d" % c)
 def test_checkpoint_and_recompute_matches_keeping_every_step(cfg):
     """ckpt_every = K: the forward keeps only the fp32 state every K steps, the backward recomputes each stretch from
@@ -468,7 +474,7 @@ def test_checkpoint_and_recompute_matches_keeping_every_step(cfg):
     N, B, T, act, K = cfg
     case = orc.make_case(N, B, T, act, seed=3)
     if N == 192:
-        # five active action columns on the persistent kernels (weight groups): the same run with a wider signal
+        # five active action columns (persistent tiles: weight groups): the same run with a wider signal
         g = torch.Generator().manual_seed(11)
         case.A = torch.rand(B, T, 5, generator=g) * 0.5
         case.Wa = torch.randn(5, N, N, generator=g) * 0.01
