@@ -283,7 +283,11 @@ int ringrnn_generate_trials(int B, int T, int N, int a_dim, unsigned long long s
  * j-th smallest ordering draw is below the trial's keep count; the target lags by one step), the [L, R] signal divided by
  * max_av, and the unit-norm Gaussian bump of width N/bump_width at the first target angle.
  *   draws  device, for n_all >= n trials: theta [n_all] | keep [n_all] | value [n_all][T-n0] | order [n_all][T-n0], all float
- *   A [n,T,2], target [n,T], r_init [n,N] out.  T - n0 <= 8192. */
+ *   A [n,T,2], target [n,T], r_init [n,N] out.  T - n0 <= 8192.
+ * Equal ordering draws of a trial rank by index.  The host's argsort ranks them as it likes: ringrnn_tied_trials sets tied[b]
+ * (device int [n]) to 1 for the trials that have any, else to 0, for a caller that wants the host's order to replace their
+ * ordering draws by ranks. */
+int ringrnn_tied_trials(int n, int n_all, int T, int n0, const float* draws, int* tied, void* stream);
 int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, const float* draws, float max_av, float bump_width,
                             float* A, float* target, float* r_init, void* stream);
 

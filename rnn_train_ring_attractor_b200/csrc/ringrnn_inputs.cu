@@ -111,25 +111,10 @@ __global__ void __launch_bounds__(128) initial_bump_kernel(int B, int N, const f
   }
 }
 
-// One block per trial.  The ordering draws are sorted in shared memory (bitonic, ties by index: a stable sort), then every
-// step's velocity, the running angle (fp64 like the host's cumulative sum, each thread a stretch of steps) and the action
-// signal.  Arithmetic in the order of the host generator.
+// The ordering draws of a trial, sorted in shared memory by a block (bitonic, equal draws by index): (draw bits, index)
 constexpr int ASSEMBLE_THREADS = 256;
-__global__ void __launch_bounds__(ASSEMBLE_THREADS) assemble_trials_kernel(int n_all, int T, int n0, int N,
-                                                                           const float* __restrict__ draws, float max_av,
-                                                                           float bump_width, int sort_len, float* __restrict__ A,
-                                                                           float* __restrict__ target,
-                                                                           float* __restrict__ r_init) {
-  extern __shared__ unsigned long long sorted[];  // [sort_len] (draw bits, index), then the velocities [T]
-  __shared__ double warp_sum[ASSEMBLE_THREADS / 32];
-  __shared__ float red[ASSEMBLE_THREADS / 32];
-  float* av = reinterpret_cast<float*>(sorted + sort_len);
-  const int b = blockIdx.x, rest = T - n0, tid = threadIdx.x;
-  const float two_pi = 6.283185307179586f;
-  const float theta0 = draws[b] * two_pi;
-  const int keep = (int)draws[n_all + b];
-  const float* value = draws + 2 * (size_t)n_all + (size_t)b * rest;
-  const float* order = draws + (size_t)n_all * (2 + rest) + (size_t)b * rest;
+__device__ __forceinline__ void sort_draws(const float* __restrict__ order, int rest, int sort_len, unsigned long long* sorted) {
+  const int tid = threadIdx.x;
   for (int i = tid; i < sort_len; i += ASSEMBLE_THREADS)
     sorted[i] = i < rest ? ((unsigned long long)__float_as_uint(order[i]) << 32) | (unsigned)i : ~0ull;
   __syncthreads();
@@ -145,6 +130,38 @@ __global__ void __launch_bounds__(ASSEMBLE_THREADS) assemble_trials_kernel(int n
       }
       __syncthreads();
     }
+}
+
+// tied[b] = whether two ordering draws of trial b are equal.  One block per trial.
+__global__ void __launch_bounds__(ASSEMBLE_THREADS) tied_trials_kernel(int n_all, int rest, const float* __restrict__ draws,
+                                                                       int sort_len, int* __restrict__ tied) {
+  extern __shared__ unsigned long long sorted[];
+  const int b = blockIdx.x;
+  sort_draws(draws + (size_t)n_all * (2 + rest) + (size_t)b * rest, rest, sort_len, sorted);
+  int any = 0;
+  for (int i = threadIdx.x; i + 1 < rest; i += ASSEMBLE_THREADS) any |= (sorted[i] >> 32) == (sorted[i + 1] >> 32);
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) tied[b] = any ? 1 : 0;
+}
+
+// One block per trial.  The ordering draws are sorted, then every step's velocity, the running angle (fp64 like the host's
+// cumulative sum, each thread a stretch of steps) and the action signal.  Arithmetic in the order of the host generator.
+__global__ void __launch_bounds__(ASSEMBLE_THREADS) assemble_trials_kernel(int n_all, int T, int n0, int N,
+                                                                           const float* __restrict__ draws, float max_av,
+                                                                           float bump_width, int sort_len, float* __restrict__ A,
+                                                                           float* __restrict__ target,
+                                                                           float* __restrict__ r_init) {
+  extern __shared__ unsigned long long sorted[];  // [sort_len] (draw bits, index), then the velocities [T]
+  __shared__ double warp_sum[ASSEMBLE_THREADS / 32];
+  __shared__ float red[ASSEMBLE_THREADS / 32];
+  float* av = reinterpret_cast<float*>(sorted + sort_len);
+  const int b = blockIdx.x, rest = T - n0, tid = threadIdx.x;
+  const float two_pi = 6.283185307179586f;
+  const float theta0 = draws[b] * two_pi;
+  const int keep = (int)draws[n_all + b];
+  const float* value = draws + 2 * (size_t)n_all + (size_t)b * rest;
+  const float* order = draws + (size_t)n_all * (2 + rest) + (size_t)b * rest;
+  sort_draws(order, rest, sort_len, sorted);
   for (int t = tid; t < T; t += ASSEMBLE_THREADS) {
     float v = 0.f;
     if (t >= n0) {
@@ -196,6 +213,12 @@ __global__ void __launch_bounds__(ASSEMBLE_THREADS) assemble_trials_kernel(int n
   for (int i = tid; i < N; i += ASSEMBLE_THREADS) r_init[(size_t)b * N + i] /= norm;
 }
 
+int padded_draws(int rest) {
+  int n = 2;
+  while (n < rest) n <<= 1;
+  return n;
+}
+
 }  // namespace
 }  // namespace ringrnn
 
@@ -230,6 +253,22 @@ extern "C" int ringrnn_generate_trials(int B, int T, int N, int a_dim, unsigned 
   return RINGRNN_OK;
 }
 
+extern "C" int ringrnn_tied_trials(int n, int n_all, int T, int n0, const float* draws, int* tied, void* stream) {
+  using namespace ringrnn;
+  if (n <= 0 || n_all < n || T <= 0 || n0 < 0 || n0 >= T) return RINGRNN_ERR_SHAPE;
+  if (!draws || !tied) return RINGRNN_ERR_ARG;
+  if (T - n0 > 8192) return RINGRNN_ERR_TOO_LARGE;
+  const int sort_len = padded_draws(T - n0);
+  RINGRNN_CUDA_TRY(cudaFuncSetAttribute(tied_trials_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 8));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  {
+    LaunchScope ls(K_PREP, s);
+    tied_trials_kernel<<<n, ASSEMBLE_THREADS, sort_len * 8, s>>>(n_all, T - n0, draws, sort_len, tied);
+  }
+  RINGRNN_CUDA_TRY(cudaGetLastError());
+  return RINGRNN_OK;
+}
+
 extern "C" int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, const float* draws, float max_av,
                                        float bump_width, float* A, float* target, float* r_init, void* stream) {
   using namespace ringrnn;
@@ -237,9 +276,7 @@ extern "C" int ringrnn_assemble_trials(int n, int n_all, int T, int n0, int N, c
   if (!draws || !A || !target || !r_init || !(max_av > 0.f) || !(bump_width > 0.f)) return RINGRNN_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(A) & 7) != 0) return RINGRNN_ERR_ARG;  // written two floats at a time
   if (T - n0 > 8192) return RINGRNN_ERR_TOO_LARGE;
-  int sort_len = 2;
-  while (sort_len < T - n0) sort_len <<= 1;
-  const int smem = sort_len * 8 + T * 4;
+  const int sort_len = padded_draws(T - n0), smem = sort_len * 8 + T * 4;
   if (smem > 200 * 1024) return RINGRNN_ERR_TOO_LARGE;
   RINGRNN_CUDA_TRY(cudaFuncSetAttribute(assemble_trials_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -225,6 +225,15 @@ def test_device_status_surface_without_a_gpu(L):
     _lib.raise_if_device_error()
 
 
+def test_tied_trials_validates_arguments(L):
+    assert L.ringrnn_tied_trials(0, 4, 10, 1, 1, 1, None) == 2      # no trials
+    assert L.ringrnn_tied_trials(4, 3, 10, 1, 1, 1, None) == 2      # fewer draws than trials
+    assert L.ringrnn_tied_trials(4, 4, 10, 10, 1, 1, None) == 2     # nothing to order
+    assert L.ringrnn_tied_trials(4, 4, 10, 1, None, 1, None) == 1
+    assert L.ringrnn_tied_trials(4, 4, 10, 1, 1, None, None) == 1
+    assert L.ringrnn_tied_trials(4, 4, 10000, 1, 1, 1, None) == 7   # more than a block sorts
+
+
 def test_generate_trials_validates_arguments(L):
     ratios = (C.c_float * 3)(0.2, 0.5, 0.8)
     ok = [8, 10, 16, 2, 1, 0, 0.3, 0.3, 0.1, ratios, 3, 0, 4.0, 1, 1, 1, 1, None]

@@ -189,6 +189,19 @@ def test_trials_from_host_draws_are_the_host_generators(n, batch, T):
     assert orc.rel_err(x["r_init"], inputs.initial_bump_gaussian(angle[:, 0], 120)) < 1e-5
 
 
+def test_equal_ordering_draws_rank_as_on_the_host():
+    """24-bit draws: of 1800 per trial, one trial in ten has two that are equal, and which of them comes first decides whether
+    a step moves.  Bit for bit the host generator's signal."""
+    from rnn_train_ring_attractor_b200 import inputs
+    n, batch, T = 203, 7, 2000
+    x = inputs.trials_from_host_draws(n, T, 16, batch, 0.3, torch.Generator().manual_seed(1), "cuda")
+    g = torch.Generator().manual_seed(1)
+    av, angle = (torch.cat(p)[:n] for p in zip(*[inputs.generate_av(batch, T, max_av=0.3, generator=g) for _ in range(29)]))
+    assert torch.equal(x["A"].cpu(), inputs.av_to_action_signal(av, 0.3))
+    d = (x["target"].cpu() - angle).abs()
+    assert float(torch.minimum(d, 2 * math.pi - d).max()) < 2e-5  # a few ulp of sums up to 32
+
+
 @pytest.mark.parametrize("T,ratio,max_av", [(40, 0.1, -0.3), (60000, 0.9, 0.1), (12000, 0.1, 0.1)])
 def test_trials_the_device_does_not_rank_come_from_the_host(T, ratio, max_av):
     """A negative max_av, a trial whose velocities and ordering draws together exceed shared memory, more than 8192 draws."""
