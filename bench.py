@@ -528,7 +528,7 @@ def run_ours(args, wl):
                    "l2": "working set (saved states + delta, several GB) exceeds the 126 MB L2; no flush needed"},
         "e2e": {"value": B_global * T / (ms_e2e * 1e-3), "unit": UNIT, "ms_per_step": ms_e2e,
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": 4,
-                "how": "public API ring_rnn_fused via dp.train_step; inputs in pinned host memory, H2D double-buffered on a "
+                "how": "public API dp.train_step on dp.fused_step_fn; inputs in pinned host memory, H2D double-buffered on a "
                        "copy stream, loss read back every step"},
         "gpu_launches": launches, "clocks": clocks, "roofline": roof, "cpu_baseline": cpu, "loss": loss_value,
         "grad_checksum": checksum,
