@@ -136,12 +136,15 @@ int ckpt_interval(const RingRnnProblem& p) { return (p.ckpt_every > 0 && p.ckpt_
 //   N <= 128, small tiles to 148 CTAs of 64 samples, against tiles of 128: step ratio 0.81 at 9472, 1.24 at 9600 (the reverse
 //     kernel's second round), 1.17 at 28000.
 //   N <= 256, to 74 clusters of 64: 0.87 at 4736, 1.38 at 4800, 1.40 at 20000 (T = 100, gelu: 0.92, 1.61).
-//   N <= 512, to two rounds of 33 clusters of 16: 0.95 at 1056 (T = 128: 1.02; operator forward and backward 0.90), 1.31 at 1100.
-//   N <= 1024, stepwise against tiles of 128: N = 1024 0.92 at 400 samples, 1.00 at 512 (operator 0.83), 1.13 at 640; N = 600
-//     0.86 at 512, 0.96 at 768.  Its scratch is a sixth more, so sequences whose saved state alone takes 16 GB stay with the tiles.
+//   N <= 512, to a round of 33 clusters of 16, beyond N = 480 to two: N = 512 0.95 at 1056 (T = 300: 1.00; operator forward and
+//     backward 0.90), 1.31 at 1100; N = 300 and 400, T = 300, 1.04 to 1.09 (operator 0.88 to 0.95) from 530 to 1056.
+//   N <= 1024, stepwise against tiles of 128: N = 600 0.86 at 512 samples (T = 200: 0.91), 0.96 at 768; N = 768 0.96 at 512; N =
+//     1024 0.92 at 384, 1.00 at 512 (T = 200: 1.05; operator 0.87), so to 384 there.  Its scratch is a sixth more, so sequences
+//     whose saved state alone takes 16 GB stay with the tiles.
 // Up to two columns, inference: small tiles have no reverse kernel to wait for.
 //   N <= 128: 0.54 to 0.73 of the tiles' time from 9472 to 28000 samples without a history.  N <= 256: 0.65 to 0.99 with one;
-//   without, 1.04 to 1.48 beyond 4736.  N <= 1024 without a history: stepwise 0.83 to 0.97 at 384, 1.05 (T = 100: 1.09) at 512.
+//   without, 1.04 to 1.48 beyond 4736.  N <= 480 from 530 to 1056: 0.87 to 0.96 with one, 1.02 to 1.03 without.  N <= 1024
+//   without a history: stepwise 0.83 to 0.97 at 384, 1.05 (T = 100: 1.09) at 512; with one 0.85 to 0.94 at 512.
 // More columns, N <= 512 (beyond, stepwise): stepwise up to 1024 samples, tiles of 128 from 2049 on.  Between, stepwise
 //   against tiles, operator forward and backward / training step: N = 128 with 3 columns 1.26 / 1.54 at 2048, N = 256 with 3 1.04 /
 //   1.35, with 6 0.92 / 1.05, with 16 0.85 / 0.92; N = 512 with 3 to 16 0.78 to 0.91 / 0.81 to 1.01 at 1100, 0.83 to 1.03 /
@@ -149,7 +152,7 @@ int ckpt_interval(const RingRnnProblem& p) { return (p.ckpt_every > 0 && p.ckpt_
 //   1100 on, N = 384 and 512 with a history 0.73 to 1.00 at 1100, 0.78 to 1.11 at 1280.  N <= 128 without a history: 1.07 to
 //   1.94 at 512 already.
 // RINGRNN_STEPWISE=1 sends every bf16 request to the stepwise path (for comparisons).
-constexpr int LANE_128_MAX_B = 148 * 64, LANE_256_MAX_B = 74 * 64, LANE_512_MAX_B = 33 * 16 * 2;
+constexpr int LANE_128_MAX_B = 148 * 64, LANE_256_MAX_B = 74 * 64, LANE_512_ROUND = 33 * 16;
 
 static bool force_stepwise() {
   static const bool on = getenv("RINGRNN_STEPWISE") != nullptr && getenv("RINGRNN_STEPWISE")[0] == '1';
@@ -163,9 +166,10 @@ Route training_route(const RingRnnProblem& p) {
   if (n_act <= 2) {
     if (NP == 1024) {
       const int steps = ckpt_interval(p) > 0 ? ckpt_interval(p) : p.T;
-      return p.B > 512 || (long long)steps * padded_b(p.B, p.N, n_act) * NP > (1ll << 32) ? Route::TILES : Route::STEPWISE;
+      return p.B > (p.N > 768 ? 384 : 512) || (long long)steps * padded_b(p.B, p.N, n_act) * NP > (1ll << 32) ? Route::TILES : Route::STEPWISE;
     }
-    return p.B <= (NP == 128 ? LANE_128_MAX_B : NP == 256 ? LANE_256_MAX_B : LANE_512_MAX_B) ? Route::LANE : Route::TILES;
+    const int lane_max = NP == 128 ? LANE_128_MAX_B : NP == 256 ? LANE_256_MAX_B : p.N > 480 ? 2 * LANE_512_ROUND : LANE_512_ROUND;
+    return p.B <= lane_max ? Route::LANE : Route::TILES;
   }
   if (NP == 1024 || p.B <= 1024) return Route::STEPWISE;
   if (p.B > 2048) return Route::TILES;
@@ -178,7 +182,7 @@ Route inference_route(const RingRnnProblem& p, bool history) {
   const int NP = padded_n(p.N), n_act = n_active_of(p);
   if (NP == 0) return train;
   if (n_act <= 2) {
-    if (NP == 128 || (NP == 256 && history)) return Route::LANE;
+    if (NP == 128 || (NP == 256 && history) || (NP == 512 && history && p.B <= 2 * LANE_512_ROUND)) return Route::LANE;
     if (NP == 1024) return p.B > (history ? 512 : 384) ? Route::TILES : Route::STEPWISE;
     return train;
   }

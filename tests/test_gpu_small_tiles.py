@@ -31,7 +31,7 @@ LANE = [(1, 1, 1, 2, "tanh", -0.1, 0.1), (2, 17, 8, 1, "silu", -0.1, 0.1), (127,
         (90, 9472, 3, 2, "gelu", -0.1, 0.1), (192, 4736, 2, 2, "silu", -0.05, 0.1),
         # four CTAs: neurons around 256 and 512, one and several rounds of 33 clusters of 16 samples, the last batch taken
         (257, 1, 1, 2, "tanh", -0.1, 0.1), (384, 17, 9, 1, "silu", -0.05, 0.1), (510, 33, 8, 2, "gelu", -0.013, 0.1),
-        (512, 1056, 3, 2, "tanh", -0.02, 0.1), (300, 1057, 2, 2, "tanh", -0.02, 0.1)]
+        (512, 1056, 3, 2, "tanh", -0.02, 0.1), (300, 1057, 2, 2, "tanh", -0.02, 0.1), (480, 528, 2, 2, "silu", -0.02, 0.1)]
 # fp32 clusters: one CTA, two, four, eight; a last CTA with few neurons; several column counts; no shape that fits
 CLUSTER = [(16, 3, 2, 2, "tanh", -0.1, 0.1), (33, 40, 5, 3, "silu", -0.1, 0.1), (97, 9, 4, 2, "gelu", -0.1, 0.1),
            (200, 300, 3, 2, "tanh", -0.1, 0.1), (257, 70, 3, 1, "silu", -0.05, 0.2), (320, 33, 2, 2, "tanh", -0.04, 0.1),
@@ -53,7 +53,8 @@ STEPWISE = [(65, 3, 2, 3, "tanh", -0.1, 0.1), (130, 129, 3, 4, "silu", -0.1, 0.1
 # smallest batches that train on them
 GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1), (1000, 513, 3, 2, "tanh", -0.02, 0.1),
            (100, 1025, 3, 9, "tanh", -0.1, 0.1), (200, 1025, 2, 5, "gelu", -0.05, 0.1), (500, 1153, 2, 3, "silu", -0.02, 0.1),
-           (128, 9473, 3, 2, "gelu", -0.07, 0.1), (256, 4737, 3, 2, "tanh", -0.05, 0.1), (512, 1057, 4, 2, "gelu", -0.02, 0.1)]
+           (128, 9473, 3, 2, "gelu", -0.07, 0.1), (256, 4737, 3, 2, "tanh", -0.05, 0.1), (512, 1057, 4, 2, "gelu", -0.02, 0.1),
+           (480, 529, 3, 2, "tanh", -0.02, 0.1), (800, 385, 2, 2, "silu", -0.02, 0.1)]
 
 
 @pytest.mark.parametrize("prec,shape", [("bf16", s) for s in LANE + STEPWISE + GENERIC] + [("fp32", s) for s in CLUSTER],
@@ -82,7 +83,7 @@ def test_small_tile_kernels_match_the_oracle(prec, shape):
 
 # forward calls that save nothing may run on other kernels than those that do: both sides of each line
 INFER = [(100, 20001, 3, 2, "tanh"), (64, 9473, 9, 2, "gelu"), (256, 4736, 3, 2, "silu"), (256, 4737, 4, 2, "gelu"),
-         (1000, 384, 3, 2, "tanh"), (1000, 385, 3, 2, "tanh"), (1000, 512, 3, 2, "silu"), (64, 33, 5, 3, "silu"), (128, 1, 3, 16, "gelu"),
+         (400, 529, 3, 2, "tanh"), (400, 1056, 2, 2, "gelu"), (400, 1057, 2, 2, "gelu"), (1000, 384, 3, 2, "tanh"), (1000, 385, 3, 2, "tanh"), (1000, 512, 3, 2, "silu"), (64, 33, 5, 3, "silu"), (128, 1, 3, 16, "gelu"),
          (128, 1025, 3, 16, "gelu"), (256, 1024, 3, 6, "tanh"), (256, 2048, 3, 6, "tanh"), (500, 1152, 3, 4, "silu"),
          (500, 1153, 3, 4, "silu"), (300, 1025, 2, 5, "tanh")]
 
