@@ -2,7 +2,9 @@
 
 The sweep in test_gpu_parity.py covers shapes at short horizons; the cases here run the full number of steps of each
 named configuration on a sub-batch the oracle finishes in seconds (every sample's recurrence is independent and the
-weight gradients are sums over samples, so a sub-batch exercises exactly the per-sample arithmetic of the full batch):
+weight gradients are sums over samples).  In bf16 mode the sub-batches of C3 and C4 run on the kernels for batches of their size
+(small tiles; one GEMM per step); the persistent tiles that the full batches run on are held over many steps by
+test_gpu_tiles_over_time.py:
 
   C2  N=256,  T=256,  relu, randn*0.01 weights            (B=32)
   C3  N=512,  T=512,  gelu, randn*0.01 weights            (B=128)

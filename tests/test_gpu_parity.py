@@ -50,9 +50,9 @@ FWD_SHAPES = [
     (120, 130, 65, 2, "gelu", False),
     (128, 128, 65, 2, "silu", False),
     (256, 130, 20, 16, "gelu", True),    # zero-padded action columns, as the root training script
-    # more than two active action columns, large batch: persistent kernels with weight groups of three matrices
+    # more than two active action columns, large batch: persistent kernels with weight groups of three matrices (in bf16 mode)
     (256, 1100, 3, 5, "silu", False),    # six matrices = two full groups
-    (512, 1030, 3, 16, "gelu", False),   # a_dim 16 as in the reference's published latency table: six groups
+    (512, 1030, 3, 16, "gelu", False),   # a_dim 16 as in the reference's published latency table (one GEMM per timestep)
     (100, 19300, 3, 3, "tanh", False),   # weight groups with several tiles per cluster (weights not resident)
     # more than two active action columns, small batch: one tensor-core GEMM per timestep
     (40, 33, 17, 4, "silu", False),
@@ -63,13 +63,15 @@ FWD_SHAPES = [
     (1024, 130, 4, 5, "tanh", False),    # N = 1024 with more than two active columns
     (1152, 40, 3, 2, "gelu", False),     # N > 1024, not a multiple of 256
     (2048, 64, 3, 4, "silu", False),
+    # small tiles: weights resident on one, two or four CTAs
     (256, 7, 9, 2, "tanh", False),
     (512, 16, 5, 2, "gelu", False),
-    (512, 260, 6, 2, "gelu", False),     # CTA pairs, cluster of 8, two 256-sample tiles (one mostly padding)
-    (384, 700, 4, 2, "tanh", False),     # N padded to 512, three tiles
-    (100, 513, 7, 2, "silu", False),     # five tiles, the last with one valid sample; weights resident in shared memory
-    (1024, 130, 6, 2, "gelu", False),    # two K rounds per step (16 chunks through 8 slots), cluster of 8, two tiles
-    (640, 300, 5, 2, "tanh", False),     # N padded to 1024, three tiles
+    (512, 260, 6, 2, "gelu", False),
+    (384, 700, 4, 2, "tanh", False),     # (tiles of 128, N padded to 512, six of them)
+    (100, 513, 7, 2, "silu", False),
+    # small batches of N > 512: one GEMM per timestep
+    (1024, 130, 6, 2, "gelu", False),
+    (640, 300, 5, 2, "tanh", False),
     (1024, 16, 3, 2, "silu", False),
     (24, 9, 4, 80, "tanh", False),       # more action columns than the tensor-core modes take: fp32 mode only, all columns
     # more tiles than clusters can be resident (148 / 33 / 15 for clusters of 1 / 4 / 8): every cluster runs several

@@ -54,7 +54,7 @@ STEPWISE = [(65, 3, 2, 3, "tanh", -0.1, 0.1), (130, 129, 3, 4, "silu", -0.1, 0.1
 GENERIC = [(256, 2060, 3, 5, "silu", -0.05, 0.1), (500, 2049, 2, 7, "gelu", -0.02, 0.1), (1000, 513, 3, 2, "tanh", -0.02, 0.1),
            (100, 1025, 3, 9, "tanh", -0.1, 0.1), (200, 1025, 2, 5, "gelu", -0.05, 0.1), (500, 1153, 2, 3, "silu", -0.02, 0.1),
            (128, 9473, 3, 2, "gelu", -0.07, 0.1), (256, 4737, 3, 2, "tanh", -0.05, 0.1), (512, 1057, 4, 2, "gelu", -0.02, 0.1),
-           (480, 529, 3, 2, "tanh", -0.02, 0.1), (800, 385, 2, 2, "silu", -0.02, 0.1)]
+           (480, 529, 3, 2, "tanh", -0.02, 0.1), (800, 385, 2, 2, "silu", -0.02, 0.1), (512, 1200, 3, 16, "gelu", -0.02, 0.1)]
 
 
 @pytest.mark.parametrize("prec,shape", [("bf16", s) for s in LANE + STEPWISE + GENERIC] + [("fp32", s) for s in CLUSTER],
